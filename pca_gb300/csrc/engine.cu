@@ -67,7 +67,7 @@ constexpr int kMaxBatch = 8192;
 /* engine_init's budget for an engine whose arena each solve supplies */
 constexpr size_t kArenaExternal = ~size_t(0);
 /* slots of the pinned host buffer */
-constexpr int kPinStatus = 0, kPinSurvivors = 1, kPinTotal = 2, kPinCount = 3, kPinFirst = 4,
+constexpr int kPinStatus = 0, kPinSurvivors = 1, kPinTotal = 2, kPinCount = 3,
               kPinHist = 64;
 /* A level whose children's states fit in this many bytes, or in an eighth
    of the arena's free space, is written into space for all of them, so its
@@ -121,6 +121,30 @@ __global__ void k_gather_paths(PathGather G, int S, const ulonglong2 *rec, uint6
     }
 }
 
+/* A task's DFS-first solving record of a first-only stage and the candidate
+   indices of its prefix path. key is all ones where the task has none. */
+struct FirstOut {
+    unsigned long long key, found;   /* found: programs of its records */
+    uint16_t path[SEARCH_MAX_DEPTH];
+};
+
+__global__ void k_gather_firsts(PathGather G, int S, const ulonglong2 *firsts, int t0, int t1,
+                                FirstOut *out)
+{
+    for (int t = t0 + blockIdx.x * blockDim.x + threadIdx.x; t < t1; t += gridDim.x * blockDim.x) {
+        const ulonglong2 f = firsts[t];
+        FirstOut &o = out[t];
+        o.key = f.x;
+        o.found = f.y + 1;
+        if (f.x == ~0ull) continue;
+        uint64_t q = f.x >> 36;
+        for (int d = S; d >= 1; d--) {
+            o.path[d - 1] = G.cidx[d][q];
+            q = G.parent[d][q];
+        }
+    }
+}
+
 }  // namespace pcagb
 
 using namespace pcagb;
@@ -131,12 +155,14 @@ struct pcagb_engine {
     cudaStream_t stream = nullptr;
     char *arena = nullptr;
     size_t cap = 0, bottom = 0, top = 0;
-    unsigned long long *d_small = nullptr;   /* [0] sol count [1] first [2] count
+    unsigned long long *d_small = nullptr;   /* [0] sol count [1] unused [2] count
                                                 [3] value-class evaluations run
                                                 [4] the work counter of the insert and
                                                 lean materialise kernels */
     uint32_t *d_status = nullptr;
     ulonglong2 *d_sol = nullptr;
+    ulonglong2 *d_firsts = nullptr;          /* [kMaxBatch] SolBuf::firsts */
+    FirstOut *d_first_out = nullptr, *h_first_out = nullptr;   /* [kMaxBatch], h: pinned */
     uint64_t sol_cap = 1u << 20;
     /* batch task table */
     int32_t *d_task_T = nullptr;
@@ -151,7 +177,7 @@ struct pcagb_engine {
     cudaEvent_t ev0 = nullptr, ev1 = nullptr, ev2 = nullptr, ev3 = nullptr;
     cudaEvent_t evk0 = nullptr, evk1 = nullptr;   /* around a lane-per-prefix launch */
     int occ_insert = 4, occ_suffix = 8, occ_mat = 4, occ_lanes = 4,
-        occ_mid_lanes = 4;   /* resident blocks per SM */
+        occ_states = 4;   /* resident blocks per SM */
     uint64_t launches = 0;
     uint64_t h2d = 0, d2h = 0;
     uint64_t insert_launches = 0, suffix_launches = 0, insert_children = 0;
@@ -164,8 +190,8 @@ struct pcagb_engine {
     double t_child_ms = 1.8e-7;     /* device ms per child of a level build */
     double t_child_lean_ms = 1.2e-7; /* the same for a lean level (k_materialize_probe) */
     double t_build_fixed_ms = 0.08; /* device ms of a level build's fixed part */
-    double t_eval_ms[4] = {0, 1.8e-9, 1.4e-9, 1.3e-9};  /* device ms per value-class
-                                                           evaluation, per suffix depth */
+    double t_eval_ms[4] = {0, 8e-10, 8e-12, 6e-12};  /* device ms per value-class
+                                                        evaluation, per suffix depth */
     double dedup_ratio = 0.35;      /* survivors / children of the last build */
     /* launch choices of the suffix stages, with their measured costs (ms
        per value-class evaluation, running averages; n = stages measured) */
@@ -605,6 +631,7 @@ struct TaskRun {
     bool done = false;
     int optimal_depth = -1;
     uint64_t nrec = 0;
+    uint64_t found = 0;            /* first-only: programs the stage found */
     std::vector<RawSol> sols;
     double t_done = 0;
     pcagb_result_t res{};
@@ -622,54 +649,62 @@ struct StageOrder {
     float ms_to_first = 0;
 };
 
+/* A solution being rebuilt from candidate indices. */
+struct SolBuilder {
+    const GenTables &gt = gen_tables();
+    RawSol sol;
+    uint32_t mask;
+
+    explicit SolBuilder(const TaskRun &tr) : mask((tr.root.live >> 1) & 127u) {}
+    uint32_t take(uint32_t c)   /* returns the register written */
+    {
+        const uint32_t idx = gt.cand_off[mask] + c, rd = UOP_RD(gt.cand_uop[idx]);
+        sol.kernel.push_back(gt.cand[idx]);
+        sol.key.push_back(c);
+        mask |= 1u << (rd - 1);
+        return rd;
+    }
+};
+
+PathGather path_gather(const pcagb_engine *e, int S)
+{
+    PathGather G{};
+    for (int d = 1; d <= S; d++) {
+        G.parent[d] = e->levels[d].parent;
+        G.cidx[d] = e->levels[d].cidx;
+    }
+    G.task = e->levels[S].task;
+    return G;
+}
+
 /* Turn solving records r0..r1 of the stage at depth K from level S into
- * the tasks' raw solutions (kept sorted in DFS order). `first` is the
- * packed DFS-first key, used instead of the records for one task in
- * first-only mode. */
-int take_records(pcagb_engine *e, int S, int K, std::vector<TaskRun> &runs, bool first_only,
-                 uint64_t r0, uint64_t r1, unsigned long long first)
+ * the tasks' raw solutions (kept sorted in DFS order). */
+int take_records(pcagb_engine *e, int S, int K, std::vector<TaskRun> &runs, uint64_t r0, uint64_t r1)
 {
     const GenTables &gt = gen_tables();
-    const Level &L = e->levels[S];
     const int s = K - S;
-    std::vector<ulonglong2> rec;
-    if (first_only && e->ntasks == 1) {
-        const uint64_t m1 = (first >> 24) & 4095, m2 = (first >> 12) & 4095, fc = first & 4095;
-        /* low 16 bits with bit 15 set: a candidate index, not a class */
-        rec.push_back(make_ulonglong2(first >> 36, (m1 << 32) | (m2 << 16) | (0x8000u | fc)));
-    } else {
-        if (r1 > e->sol_cap) {
-            set_err("%llu solving records exceed the buffer of %llu", (unsigned long long)r1,
-                    (unsigned long long)e->sol_cap);
-            return PCAGB_ELIMIT;
-        }
-        rec.resize(r1 - r0);
-        CK(e_copy(e, rec.data(), e->d_sol + r0, rec.size() * sizeof(ulonglong2),
-                  cudaMemcpyDeviceToHost, e->stream));
-        CK(cudaStreamSynchronize(e->stream));
+    if (r1 > e->sol_cap) {
+        set_err("%llu solving records exceed the buffer of %llu", (unsigned long long)r1,
+                (unsigned long long)e->sol_cap);
+        return PCAGB_ELIMIT;
     }
+    std::vector<ulonglong2> rec(r1 - r0);
     std::vector<uint16_t> paths(rec.size() * SEARCH_MAX_DEPTH, 0);
     std::vector<uint16_t> rtask(rec.size(), 0);
     {
         const size_t top0 = e->top;
-        ulonglong2 *d_rec = (ulonglong2 *)e->alloc_top(rec.size() * sizeof(ulonglong2));
         uint16_t *d_paths = (uint16_t *)e->alloc_top(paths.size() * 2);
         uint16_t *d_task = (uint16_t *)e->alloc_top(rtask.size() * 2);
-        if (!d_rec || !d_paths || !d_task) {
+        if (!d_paths || !d_task) {
             set_err("arena exhausted gathering paths");
             return PCAGB_ENOMEM;
         }
-        CK(e_copy(e, d_rec, rec.data(), rec.size() * sizeof(ulonglong2), cudaMemcpyHostToDevice,
-                  e->stream));
-        PathGather G{};
-        for (int d = 1; d <= S; d++) {
-            G.parent[d] = e->levels[d].parent;
-            G.cidx[d] = e->levels[d].cidx;
-        }
-        G.task = L.task;
-        k_gather_paths<<<64, 256, 0, e->stream>>>(G, S, d_rec, rec.size(), d_paths, d_task);
+        k_gather_paths<<<64, 256, 0, e->stream>>>(path_gather(e, S), S, e->d_sol + r0, rec.size(),
+                                                  d_paths, d_task);
         int rc = check_launch(e);
         if (rc) return rc;
+        CK(e_copy(e, rec.data(), e->d_sol + r0, rec.size() * sizeof(ulonglong2),
+                  cudaMemcpyDeviceToHost, e->stream));
         CK(e_copy(e, paths.data(), d_paths, paths.size() * 2, cudaMemcpyDeviceToHost, e->stream));
         CK(e_copy(e, rtask.data(), d_task, rtask.size() * 2, cudaMemcpyDeviceToHost, e->stream));
         CK(cudaStreamSynchronize(e->stream));
@@ -680,43 +715,24 @@ int take_records(pcagb_engine *e, int S, int K, std::vector<TaskRun> &runs, bool
         TaskRun &tr = runs[rtask[i]];
         touched[rtask[i]] = 1;
         tr.nrec++;
-        RawSol base;
-        uint32_t mask = (tr.root.live >> 1) & 127u;
-        auto take = [&](uint32_t c) {
-            const uint32_t idx = gt.cand_off[mask] + c;
-            base.kernel.push_back(gt.cand[idx]);
-            base.key.push_back(c);
-            mask |= 1u << (UOP_RD(gt.cand_uop[idx]) - 1);
-        };
-        for (int d = 0; d < S; d++) take(paths[i * SEARCH_MAX_DEPTH + d]);
+        SolBuilder base(tr);
+        for (int d = 0; d < S; d++) base.take(paths[i * SEARCH_MAX_DEPTH + d]);
         const uint32_t m1 = (uint32_t)(rec[i].y >> 32), m2 = (uint32_t)((rec[i].y >> 16) & 0xFFFF);
         const uint32_t low = (uint32_t)(rec[i].y & 0xFFFF);
-        if (s >= 2) take(m1);
-        if (s >= 3) take(m2);
+        if (s >= 2) base.take(m1);
+        if (s >= 3) base.take(m2);
         if (s == 0) {
-            base.out_reg = low;
-            base.key.push_back(0);
-            tr.sols.push_back(base);
+            base.sol.out_reg = low;
+            base.sol.key.push_back(0);
+            tr.sols.push_back(std::move(base.sol));
             continue;
         }
-        if (low & 0x8000u) {
-            RawSol r = base;
-            const uint32_t c = low & 0x7FFF;
-            const uint32_t idx = gt.cand_off[mask] + c;
-            r.kernel.push_back(gt.cand[idx]);
-            r.key.push_back(c);
-            r.out_reg = UOP_RD(gt.cand_uop[idx]);
-            tr.sols.push_back(r);
-            continue;
-        }
-        for (uint32_t c = 0; c < (uint32_t)gt.nc(mask); c++) {
-            const uint32_t idx = gt.cand_off[mask] + c;
-            if (gt.cand_vc[idx] != low) continue;
-            RawSol r = base;
-            r.kernel.push_back(gt.cand[idx]);
-            r.key.push_back(c);
-            r.out_reg = UOP_RD(gt.cand_uop[idx]);
-            tr.sols.push_back(r);
+        const uint16_t *of = &gt.cand_of[(gt.vc_off[base.mask] + low) * 8];
+        for (uint32_t rd = 1; rd < 8; rd++) {
+            if (of[rd] == 0xFFFF) continue;
+            SolBuilder r = base;
+            r.sol.out_reg = r.take(of[rd]);
+            tr.sols.push_back(std::move(r.sol));
         }
     }
     for (size_t t = 0; t < runs.size(); t++)
@@ -726,15 +742,55 @@ int take_records(pcagb_engine *e, int S, int K, std::vector<TaskRun> &runs, bool
     return PCAGB_OK;
 }
 
+/* First-only stages keep, per task, the DFS-first record and a count of the
+   programs found: gathered on the device and read back for tasks t0..t1-1
+   in one copy. enqueue_firsts enqueues it; take_firsts reads it after the
+   stream has been synchronised. */
+int enqueue_firsts(pcagb_engine *e, int S, int t0, int t1)
+{
+    if (t1 <= t0) return PCAGB_OK;
+    k_gather_firsts<<<(t1 - t0 + 127) / 128, 128, 0, e->stream>>>(path_gather(e, S), S, e->d_firsts,
+                                                                  t0, t1, e->d_first_out);
+    int rc = check_launch(e);
+    if (rc) return rc;
+    CK(e_copy(e, e->h_first_out + t0, e->d_first_out + t0, (t1 - t0) * sizeof(FirstOut),
+              cudaMemcpyDeviceToHost, e->stream));
+    return PCAGB_OK;
+}
+
+void take_firsts(pcagb_engine *e, int S, int K, std::vector<TaskRun> &runs, int t0, int t1)
+{
+    const int s = K - S;
+    for (int t = t0; t < t1; t++) {
+        const FirstOut &f = e->h_first_out[t];
+        if (f.key == ~0ull) continue;
+        TaskRun &tr = runs[t];
+        SolBuilder b(tr);
+        for (int d = 0; d < S; d++) b.take(f.path[d]);
+        if (s >= 2) b.take((uint32_t)(f.key >> 24 & 4095));
+        if (s >= 3) b.take((uint32_t)(f.key >> 12 & 4095));
+        const uint32_t last = (uint32_t)(f.key & 4095);
+        if (s == 0) {   /* a leaf: the register that holds the target */
+            b.sol.out_reg = last;
+            b.sol.key.push_back(0);
+        } else {
+            b.sol.out_reg = b.take(last);
+        }
+        tr.nrec = 1;
+        tr.found = f.found;
+        tr.sols.push_back(std::move(b.sol));
+    }
+}
+
 /* Work-item shapes of the suffix kernels, by suffix depth (index 0 is
    unused): at depth 1 the prefixes a warp scans at once (1: a warp per
    prefix, k_suffix; 32: a lane per prefix, k_suffix_lanes); at depths 2
-   and 3 the middle-instruction chunk a warp-per-item work item takes, or
-   kLaneShape: a lane per innermost middle (k_suffix_mid_lanes). */
+   and 3 kLaneShape, a lane per state (k_suffix_states), or, when the caller
+   forces it, the middle-instruction chunk of a warp per item (k_suffix). */
 constexpr uint32_t kLaneShape = 1024;
 constexpr uint32_t kChunkChoices[4][4] = {
     {1, 1, 1, 1}, {1, 32, 1, 32}, {8, 16, 32, kLaneShape}, {1, 2, 4, kLaneShape}};
-constexpr int kChunkOptions[4] = {1, 2, 4, 4};
+constexpr int kChunkOptions = 2;   /* explored, at depth 1 only */
 /* below this many prefixes a level gives a lane-per-prefix launch fewer
    warps than the SMs hold: the depth-1 default is then a warp per prefix */
 constexpr uint64_t kLanesMinPrefixes = 32ull * 152 * 4;
@@ -773,13 +829,34 @@ void launch_suffix_lanes(int ft, int g, cudaStream_t st, const LevelDev &L, cons
     else k_suffix_lanes<TPC, 2><<<g, kThreads, 0, st>>>(L, td, sb, R, lean);
 }
 
+/* A long stage of a solve that shares the GPU (a server's) runs in a few
+   CTAs: a launch holds its SMs until it ends, and requests admitted meanwhile
+   would wait for them. Six CTAs leave 146 SMs to the others and take about
+   as long as the stage took before it was a lane per state (is_power2 at
+   depth 5: 0.4 s, 9 ms on the whole GPU), which is also what the serving test
+   builds on: it submits requests 0.2 s into such a solve and expects their
+   answers before its own. The stages of requests up to depth 4 (0.2 ms)
+   are below the line. */
+constexpr double kBackgroundMs = 2.0;
+constexpr int kBackgroundCtas = 6;
+
+/* A lane per state (k_suffix_states): per_prefix states to a prefix, and the
+   shares their work is cut into so that the warps fill the GPU about twice
+   (at most 32 shares: a state has 12 to 55 (operand, group) pairs). Above
+   that a share only repeats the state's set-up. */
 template <int TPC, int SD>
-void launch_mid_lanes(int ft, int g, cudaStream_t st, const LevelDev &L, const TaskDev &td,
-                      const SolBuf &sb, uint32_t cpp, const PrefixRange &R)
+void launch_states(pcagb_engine *e, const LevelDev &L, const SolBuf &sb, uint32_t per_prefix,
+                   const PrefixRange &R, bool background)
 {
-    if (ft == 1) k_suffix_mid_lanes<TPC, SD, 1><<<g, kThreads, 0, st>>>(L, td, sb, cpp, R);
-    else if (ft == 3) k_suffix_mid_lanes<TPC, SD, 3><<<g, kThreads, 0, st>>>(L, td, sb, cpp, R);
-    else k_suffix_mid_lanes<TPC, SD, 2><<<g, kThreads, 0, st>>>(L, td, sb, cpp, R);
+    const int g = background ? kBackgroundCtas : e->grid(e->occ_states);
+    const uint64_t batches = (R.count * per_prefix + 31) / 32;
+    const uint64_t warps = (uint64_t)g * kStatesWarps;
+    uint32_t sl = 0;
+    while (sl < 5 && (batches << sl) < 2 * warps) sl++;
+    const unsigned blocks = (unsigned)std::min<uint64_t>(
+        (uint64_t)g, ((batches << sl) + kStatesWarps - 1) / kStatesWarps);
+    k_suffix_states<TPC, SD><<<std::max(blocks, 1u), kStatesWarps * 32, 0, e->stream>>>(L, e->td, sb,
+                                                                              per_prefix, sl, R);
 }
 
 template <int TPC, int SD>
@@ -809,8 +886,12 @@ int run_stage(pcagb_engine *e, int S, int K, std::vector<TaskRun> &runs, bool fi
     Level &L = e->levels[S];
     const int s = K - S;
     CK(cudaMemsetAsync(e->d_small, 0, 8, e->stream));
-    CK(cudaMemsetAsync(e->d_small + 1, 0xFF, 8, e->stream));
-    SolBuf sb{e->d_small, e->d_sol, e->sol_cap, e->d_small + 1, e->d_small + 3};
+    /* a batch's leaf check counts its records (the reference's "tried") */
+    const bool firsts = first_only && (s >= 1 || e->ntasks == 1);
+    if (firsts)
+        CK(cudaMemsetAsync(e->d_firsts, 0xFF, e->ntasks * sizeof(ulonglong2), e->stream));
+    SolBuf sb{e->d_small, e->d_sol, e->sol_cap, firsts ? e->d_firsts : nullptr, L.task,
+              e->d_small + 3};
     int tuned_ft = 0, tuned_ck = -1;   /* the launch choices this stage used */
     int lane_launches = 0;             /* lane-per-prefix launches of this stage */
     /* launch choices are explored and timed on single-task stages only: a
@@ -824,6 +905,7 @@ int run_stage(pcagb_engine *e, int S, int K, std::vector<TaskRun> &runs, bool fi
     const int g = e->grid(e->occ_suffix);
     int rc = PCAGB_OK;
     uint64_t taken = 0;  /* records already turned into solutions */
+    bool grouped = false;
     if (s == 0) {
         if (t16) k_leaf<16><<<e->grid(4), 256, 0, e->stream>>>(view(L), e->td, sb);
         else k_leaf<32><<<e->grid(4), 256, 0, e->stream>>>(view(L), e->td, sb);
@@ -841,7 +923,7 @@ int run_stage(pcagb_engine *e, int S, int K, std::vector<TaskRun> &runs, bool fi
            (an unmeasured one is tried first on a stage large enough) */
         const bool explore = evals_pred >= kTuneMinEvals && !so && nact_stage == 1 && e->measure;
         int ft = e->force_ft;
-        if (ft < 1 || ft > 3) ft = 1 + pick_option(&e->ft_ms[s][1], &e->ft_n[s][1], 3, 1, explore);
+        if (ft < 1 || ft > 3) ft = 1 + pick_option(&e->ft_ms[s][1], &e->ft_n[s][1], 3, 1, explore && s == 1);
         int ck = -1;
         uint32_t chunk = 1;
         /* a lane per prefix needs every prefix's last write: not at the root */
@@ -851,7 +933,18 @@ int run_stage(pcagb_engine *e, int S, int K, std::vector<TaskRun> &runs, bool fi
             ck = 1;
             chunk = 32;
         } else if (s >= 2 || lanes_ok) {
-            if (e->force_chunk >= 1) {
+            if (s == 2 && S == 0 && (e->force_chunk < 1 || e->force_chunk == (int)kLaneShape)) {
+                /* the roots at depth 2: a middle of zero (which the value
+                   forms leave out) and an ADDI reach the constants -1..-3
+                   here and at no later depth; few prefixes, so a warp per
+                   few middles, as few as fill the GPU */
+                chunk = (uint32_t)std::min<uint64_t>(
+                    8, std::max<uint64_t>(1, L.n * (uint64_t)ncmax / ((uint64_t)g * kWarpsPerBlock)));
+            } else if (s >= 2 && e->force_chunk < 1) {
+                /* a lane per state: measured 30-100x faster than the fastest
+                   warp-per-item chunk on every stage, so nothing is explored */
+                chunk = kLaneShape;
+            } else if (e->force_chunk >= 1) {
                 chunk = s == 1 ? (e->force_chunk >= 32 ? 32u : 1u)
                         : e->force_chunk == (int)kLaneShape ? kLaneShape
                                                              : (uint32_t)std::min(e->force_chunk, 64);
@@ -859,25 +952,24 @@ int run_stage(pcagb_engine *e, int S, int K, std::vector<TaskRun> &runs, bool fi
                 /* shapes are explored once the tests-per-lane choice is */
                 const bool ft_done = e->ft_n[s][1] >= kTuneSamples &&
                                      e->ft_n[s][2] >= kTuneSamples && e->ft_n[s][3] >= kTuneSamples;
-                /* unmeasured, the lane shapes: a stage that is not timed
-                   (an ordered or chunked first-only stage, or one too small
-                   to explore on) keeps its default, and the lanes measured
-                   2.3-3x faster on every stage that was timed; at depth 1 a
-                   level too small to fill the GPU with 32 prefixes a warp
+                /* unmeasured (a stage that is not timed: ordered, chunked
+                   first-only or too small to explore on), a lane per prefix;
+                   a level too small to fill the GPU with 32 prefixes a warp
                    stays a warp per prefix */
-                const int def = s == 1 ? (L.n >= kLanesMinPrefixes ? 1 : 0) : 3;
-                ck = pick_option(e->ck_ms[s], e->ck_n[s], kChunkOptions[s], def,
-                                 explore && ft_done);
+                const int def = L.n >= kLanesMinPrefixes ? 1 : 0;
+                ck = pick_option(e->ck_ms[s], e->ck_n[s], kChunkOptions, def, explore && ft_done);
                 chunk = kChunkChoices[s][ck];
             }
         }
-        /* work items per prefix: one (depth 1); the middle chunks; with a
-           lane per middle, 32 first middles (depth 2) or one (depth 3) */
+        /* work items per prefix: one (depth 1); with a lane per state one
+           state (depth 2) or one per first middle (depth 3); the middle
+           chunks */
         const uint32_t cpp =
             s == 1                ? 1u
-            : chunk == kLaneShape ? std::max(1u, s == 2 ? (uint32_t)(ncmax + 31) / 32
-                                                        : (uint32_t)ncmax)
+            : chunk == kLaneShape ? (s == 2 ? 1u : std::max(1u, (uint32_t)ncmax))
                                   : std::max(1u, (uint32_t)((ncmax + chunk - 1) / chunk));
+        const bool background =
+            !e->measure && (double)evals_pred * e->t_eval_ms[s] > kBackgroundMs;
         auto launch = [&](const PrefixRange &R) {
             const LevelDev V = view(L);
             if (s == 1) {
@@ -908,13 +1000,12 @@ int run_stage(pcagb_engine *e, int S, int K, std::vector<TaskRun> &runs, bool fi
                     k_count_evals<<<std::max(cb, 1u), 256, 0, e->stream>>>(V, e->td, R, sb);
                 }
             } else if (chunk == kLaneShape) {
-                const int gl = e->grid(e->occ_mid_lanes);
-                if (s == 2) {
-                    if (t16) launch_mid_lanes<16, 2>(ft, gl, e->stream, V, e->td, sb, cpp, R);
-                    else launch_mid_lanes<32, 2>(ft, gl, e->stream, V, e->td, sb, cpp, R);
+                if (t16) {
+                    if (s == 2) launch_states<16, 2>(e, V, sb, cpp, R, background);
+                    else launch_states<16, 3>(e, V, sb, cpp, R, background);
                 } else {
-                    if (t16) launch_mid_lanes<16, 3>(ft, gl, e->stream, V, e->td, sb, cpp, R);
-                    else launch_mid_lanes<32, 3>(ft, gl, e->stream, V, e->td, sb, cpp, R);
+                    if (s == 2) launch_states<32, 2>(e, V, sb, cpp, R, background);
+                    else launch_states<32, 3>(e, V, sb, cpp, R, background);
                 }
             } else if (s == 2) {
                 if (t16) launch_suffix<16, 2>(ft, g, e->stream, V, e->td, sb, cpp, chunk, R);
@@ -925,7 +1016,7 @@ int run_stage(pcagb_engine *e, int S, int K, std::vector<TaskRun> &runs, bool fi
             }
             return check_launch(e);
         };
-        tuned_ft = ft;
+        tuned_ft = s == 1 ? ft : 0;   /* the deeper stages have no choices to time */
         tuned_ck = ck;
         /* task groups of the progressive mode: [first task, end task) with
            the level range they occupy */
@@ -959,20 +1050,27 @@ int run_stage(pcagb_engine *e, int S, int K, std::vector<TaskRun> &runs, bool fi
             }
         }
         if (groups.size() > 1) {
+            grouped = true;
             for (const Group &G : groups) {
                 if (G.b1 > G.b0) {
                     rc = launch(PrefixRange{nullptr, G.b0, G.b1 - G.b0});
+                    if (rc) return rc;
+                }
+                if (firsts) {
+                    rc = enqueue_firsts(e, S, G.t0, G.t1);
                     if (rc) return rc;
                 }
                 CK(e_copy(e, &e->h_pin[kPinCount], e->d_small, 8, cudaMemcpyDeviceToHost,
                           e->stream));
                 CK(cudaStreamSynchronize(e->stream));
                 const uint64_t cnt = e->h_pin[kPinCount];
-                if (cnt > taken) {
-                    rc = take_records(e, S, K, runs, first_only, taken, cnt, 0);
+                if (firsts) {
+                    take_firsts(e, S, K, runs, G.t0, G.t1);
+                } else if (cnt > taken) {
+                    rc = take_records(e, S, K, runs, taken, cnt);
                     if (rc) return rc;
-                    taken = cnt;
                 }
+                taken = cnt;
                 (*on_tasks)(G.t0, G.t1);
             }
         } else {
@@ -1009,10 +1107,14 @@ int run_stage(pcagb_engine *e, int S, int K, std::vector<TaskRun> &runs, bool fi
         return PCAGB_ENOMEM;
     }
     cudaEventRecord(e->ev1, e->stream);
-    /* count, first key, (survivors), evaluations run so far in this solve */
+    if (firsts && !grouped) {
+        rc = enqueue_firsts(e, S, 0, e->ntasks);
+        if (rc) return rc;
+    }
+    /* count, (unused), (survivors), evaluations run so far in this solve */
     CK(e_copy(e, &e->h_pin[kPinCount], e->d_small, 32, cudaMemcpyDeviceToHost, e->stream));
     CK(cudaStreamSynchronize(e->stream));
-    const unsigned long long nrec = e->h_pin[kPinCount], first = e->h_pin[kPinFirst];
+    const unsigned long long nrec = e->h_pin[kPinCount];
     e->evals_run = e->h_pin[kPinCount + 3];
     float ms = 0;
     cudaEventElapsedTime(&ms, e->ev0, e->ev1);
@@ -1030,7 +1132,10 @@ int run_stage(pcagb_engine *e, int S, int K, std::vector<TaskRun> &runs, bool fi
         uint64_t evals = 0;
         for (size_t i = 0; i < L.hist.size(); i++)
             if (e->h_active[i >> 7]) evals += L.hist[i] * g[i & 127];
-        if (evals > 10000000ull) {
+        /* a stage long enough for its time to be its evaluations' and not
+           the launch's (some 10 us): the lanes per state of depths 2 and 3
+           decide 1e7 classes in a tenth of a microsecond */
+        if (evals > (s == 1 ? 10000000ull : 5000000000ull)) {
             const double per = ms / (double)evals;
             e->t_eval_ms[s] = 0.7 * e->t_eval_ms[s] + 0.3 * per;
             if (evals >= kTuneMinEvals && s <= 3 && nact_stage == 1) {
@@ -1039,8 +1144,12 @@ int run_stage(pcagb_engine *e, int S, int K, std::vector<TaskRun> &runs, bool fi
             }
         }
     }
+    if (firsts) {
+        if (!grouped) take_firsts(e, S, K, runs, 0, e->ntasks);
+        return PCAGB_OK;
+    }
     if (nrec <= taken) return PCAGB_OK;
-    return take_records(e, S, K, runs, first_only, taken, nrec, first);
+    return take_records(e, S, K, runs, taken, nrec);
 }
 
 /* Host-side step for the reference-key dedup of the solving leaves
@@ -1587,7 +1696,8 @@ int run_batch(pcagb_engine *e, std::vector<TaskRun> &runs, const pcagb_opts_t &o
                 tr.res.prefixes_to_first = sop ? sop->prefixes_to_first : LS.n;
                 tr.res.ms_to_first = sop ? sop->ms_to_first : 0.0;
                 tr.res.total_solutions =
-                    s == 0 || (o.first_only && nt == 1) ? tr.nrec : tr.sols.size();
+                    s == 0 || (o.first_only && nt == 1) ? tr.nrec
+                    : o.first_only                      ? tr.found : tr.sols.size();
                 notify(i);
             } else if (K >= tr.max_depth) {
                 tr.done = true;
@@ -1643,15 +1753,18 @@ int ensure_device_tables(int device)
     if (g_tables_ready[device]) return PCAGB_OK;
     const GenTables &gt = gen_tables();
     std::vector<uint16_t> first(gt.vc_uop.size(), 0);
+    std::vector<uint8_t> members(gt.vc_uop.size(), 0);
     for (int m = 0; m < 128; m++) {
         std::vector<bool> seen(gt.nvc(m), false);
         for (uint32_t c = 0; c < (uint32_t)gt.nc(m); c++) {
             uint16_t v = gt.cand_vc[gt.cand_off[m] + c];
             if (!seen[v]) { seen[v] = true; first[gt.vc_off[m] + v] = (uint16_t)c; }
+            members[gt.vc_off[m] + v]++;
         }
     }
     uint32_t *cand_uop = nullptr, *vc_uop = nullptr, *chunks = nullptr, *vcr_uop_d = nullptr;
     uint16_t *vc_first = nullptr, *vcr = nullptr;
+    uint8_t *vc_n = nullptr;
     {
         std::vector<uint32_t> vcr_uop(gt.vcr.size());
         for (int m = 0; m < 128; m++)
@@ -1697,10 +1810,27 @@ int ensure_device_tables(int device)
         CK(cudaMemcpyToSymbol(c_pr_off_g, &prop, sizeof prop));
         CK(cudaMemcpyToSymbol(c_pr, &pp, sizeof pp));
         CK(cudaMemcpyToSymbol(c_pr_cls, &pc, sizeof pc));
+        uint16_t *pra_d = nullptr, *co_d = nullptr;
+        CK(cudaMalloc(&pra_d, gt.pr_at.size() * 2));
+        CK(cudaMalloc(&co_d, gt.cand_of.size() * 2));
+        CK(cudaMemcpy(pra_d, gt.pr_at.data(), gt.pr_at.size() * 2, cudaMemcpyHostToDevice));
+        CK(cudaMemcpy(co_d, gt.cand_of.data(), gt.cand_of.size() * 2, cudaMemcpyHostToDevice));
+        const uint16_t *prap = pra_d, *cop = co_d;
+        CK(cudaMemcpyToSymbol(c_pr_at, &prap, sizeof prap));
+        CK(cudaMemcpyToSymbol(c_cand_of, &cop, sizeof cop));
+        uint32_t *evm_d = nullptr;
+        CK(cudaMalloc(&evm_d, gt.ev_mid.size() * 4));
+        CK(cudaMemcpy(evm_d, gt.ev_mid.data(), gt.ev_mid.size() * 4, cudaMemcpyHostToDevice));
+        const uint32_t *evmp = evm_d;
+        CK(cudaMemcpyToSymbol(c_ev_mid, &evmp, sizeof evmp));
     }
     CK(cudaMalloc(&cand_uop, gt.cand_uop.size() * 4));
     CK(cudaMalloc(&vc_uop, gt.vc_uop.size() * 4));
     CK(cudaMalloc(&vc_first, first.size() * 2));
+    CK(cudaMalloc(&vc_n, members.size()));
+    CK(cudaMemcpy(vc_n, members.data(), members.size(), cudaMemcpyHostToDevice));
+    const uint8_t *vn = vc_n;
+    CK(cudaMemcpyToSymbol(c_vc_n, &vn, sizeof vn));
     CK(cudaMalloc(&chunks, gt.chunks.size() * 4));
     {
         /* bit 31 of a device micro-op marks a candidate whose child is an
@@ -1758,12 +1888,8 @@ int engine_init(pcagb_engine *e, int device, size_t budget)
         PCAGB_PRELOAD(k_suffix_lanes<16, 1>); PCAGB_PRELOAD(k_suffix_lanes<16, 2>);
         PCAGB_PRELOAD(k_suffix_lanes<16, 3>); PCAGB_PRELOAD(k_suffix_lanes<32, 1>);
         PCAGB_PRELOAD(k_suffix_lanes<32, 2>); PCAGB_PRELOAD(k_suffix_lanes<32, 3>);
-        PCAGB_PRELOAD(k_suffix_mid_lanes<16, 2, 1>); PCAGB_PRELOAD(k_suffix_mid_lanes<16, 2, 2>);
-        PCAGB_PRELOAD(k_suffix_mid_lanes<16, 2, 3>); PCAGB_PRELOAD(k_suffix_mid_lanes<16, 3, 1>);
-        PCAGB_PRELOAD(k_suffix_mid_lanes<16, 3, 2>); PCAGB_PRELOAD(k_suffix_mid_lanes<16, 3, 3>);
-        PCAGB_PRELOAD(k_suffix_mid_lanes<32, 2, 1>); PCAGB_PRELOAD(k_suffix_mid_lanes<32, 2, 2>);
-        PCAGB_PRELOAD(k_suffix_mid_lanes<32, 2, 3>); PCAGB_PRELOAD(k_suffix_mid_lanes<32, 3, 1>);
-        PCAGB_PRELOAD(k_suffix_mid_lanes<32, 3, 2>); PCAGB_PRELOAD(k_suffix_mid_lanes<32, 3, 3>);
+        PCAGB_PRELOAD(k_suffix_states<16, 2>); PCAGB_PRELOAD(k_suffix_states<32, 2>);
+        PCAGB_PRELOAD(k_suffix_states<16, 3>); PCAGB_PRELOAD(k_suffix_states<32, 3>);
         PCAGB_PRELOAD(k_expand_insert<16>); PCAGB_PRELOAD(k_expand_insert<32>);
         PCAGB_PRELOAD(k_materialize<16>); PCAGB_PRELOAD(k_materialize<32>);
         PCAGB_PRELOAD(k_twins<16>); PCAGB_PRELOAD(k_twins<32>);
@@ -1771,7 +1897,7 @@ int engine_init(pcagb_engine *e, int device, size_t budget)
         PCAGB_PRELOAD(k_count_evals); PCAGB_PRELOAD(k_mark); PCAGB_PRELOAD(k_mark_all);
         PCAGB_PRELOAD(k_popc); PCAGB_PRELOAD(k_child_counts); PCAGB_PRELOAD(k_task_hist);
         PCAGB_PRELOAD(k_task_hist_smem); PCAGB_PRELOAD(k_scan_local); PCAGB_PRELOAD(k_scan_add);
-        PCAGB_PRELOAD(k_gather_paths); PCAGB_PRELOAD(k_check_perm);
+        PCAGB_PRELOAD(k_gather_paths); PCAGB_PRELOAD(k_gather_firsts); PCAGB_PRELOAD(k_check_perm);
 #undef PCAGB_PRELOAD
         cudaGetLastError();
         /* the insert kernel keeps each warp's children in shared memory:
@@ -1793,9 +1919,9 @@ int engine_init(pcagb_engine *e, int device, size_t budget)
         if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, k_suffix_lanes<32, 2>, kThreads, 0) ==
                 cudaSuccess && nb > 0)
             e->occ_lanes = nb;
-        if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, k_suffix_mid_lanes<32, 2, 2>,
-                                                          kThreads, 0) == cudaSuccess && nb > 0)
-            e->occ_mid_lanes = nb;
+        if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, k_suffix_states<32, 2>,
+                                                          kStatesWarps * 32, 0) == cudaSuccess && nb > 0)
+            e->occ_states = nb;
         cudaGetLastError();
     }
     size_t free_b = 0, total_b = 0;
@@ -1817,6 +1943,9 @@ int engine_init(pcagb_engine *e, int device, size_t budget)
     CK(cudaMalloc(&e->d_small, 256 * sizeof(unsigned long long)));
     CK(cudaMalloc(&e->d_status, 16));
     CK(cudaMalloc(&e->d_sol, e->sol_cap * sizeof(ulonglong2)));
+    CK(cudaMalloc(&e->d_firsts, kMaxBatch * sizeof(ulonglong2)));
+    CK(cudaMalloc(&e->d_first_out, kMaxBatch * sizeof(FirstOut)));
+    CK(cudaMallocHost(&e->h_first_out, kMaxBatch * sizeof(FirstOut)));
     CK(cudaMalloc(&e->d_task_T, kMaxBatch * 4));
     CK(cudaMalloc(&e->d_task_target, (size_t)kMaxBatch * 32 * 4));
     CK(cudaMalloc(&e->d_task_active, kMaxBatch));
@@ -2116,6 +2245,9 @@ void pcagb_engine_destroy(pcagb_engine_t *e)
     cudaFree(e->d_small);
     cudaFree(e->d_status);
     cudaFree(e->d_sol);
+    cudaFree(e->d_firsts);
+    cudaFree(e->d_first_out);
+    if (e->h_first_out) cudaFreeHost(e->h_first_out);
     cudaFree(e->d_task_T);
     cudaFree(e->d_task_target);
     cudaFree(e->d_task_active);

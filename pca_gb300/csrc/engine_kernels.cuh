@@ -45,6 +45,7 @@
 
 #include "pca_isa.h"
 #include "scan.cuh"
+#include "value_forms.h"
 
 namespace pcagb {
 
@@ -63,6 +64,7 @@ __constant__ uint32_t c_vc_off[129];
 __constant__ const uint32_t *c_cand_uop;   /* bit 31: a same-state duplicate of an earlier candidate */
 __constant__ const uint32_t *c_vc_uop;
 __constant__ const uint16_t *c_vc_first;   /* first candidate index per class */
+__constant__ const uint8_t *c_vc_n;        /* candidates per class */
 __constant__ uint32_t c_chunk_off[129];    /* op-uniform runs of candidates */
 __constant__ const uint32_t *c_chunks;
 __constant__ uint32_t c_vcr_off[128 * 8 + 1]; /* [mask*8 + r]: classes reading r */
@@ -73,6 +75,11 @@ __constant__ const uint32_t *c_pr;         /* a | b << 3 | opmask << 6 | imm << 
 __constant__ const uint16_t *c_pr_cls;     /* [entry][10] class index per opmask bit */
 __constant__ uint32_t c_pr_ev[128 * 8];    /* [mask*8 + r]: class evaluations of its pair list */
 __constant__ const uint32_t *c_ev_sd1;     /* the same in global memory, [mask*8 + 0] = all classes */
+__constant__ const uint16_t *c_pr_at;      /* GenTables::pr_at, cand_of */
+__constant__ const uint16_t *c_cand_of;
+__constant__ const uint32_t *c_ev_mid;     /* [dedup_mid][mask][A][B]: evaluations of the last two
+                                              positions from a state of that mask whose registers
+                                              A and B (0: none) they must read */
 __constant__ const uint32_t *c_pr_off_g;   /* c_pr_off in global memory (lanes of different masks) */
 
 /* Per-task parameters of a batch: device arrays indexed by task id. A
@@ -927,7 +934,10 @@ struct SolBuf {
     unsigned long long *count;    /* solving (prefix, mids, class) records */
     ulonglong2 *rec;              /* x = prefix rank, y = m1<<32 | m2<<16 | class */
     uint64_t cap;
-    unsigned long long *first;    /* atomicMin of a packed DFS-order key */
+    ulonglong2 *firsts;           /* first-only stages, in place of the records: per task the
+                                     smallest packed DFS-order key (x) and the programs of its
+                                     records less one (y; both start as all ones) */
+    const uint16_t *task;         /* task of each prefix (with firsts) */
     unsigned long long *evals;    /* value-class evaluations the suffix kernels ran
                                      (each class of an operand pair counts one) */
 };
@@ -940,16 +950,29 @@ __device__ __forceinline__ void flush_evals(const SolBuf &S, unsigned long long 
     if (lane == 0 && nev) atomicAdd(S.evals, nev);
 }
 
-__device__ __forceinline__ void record_solution(const SolBuf &S, uint64_t q, uint32_t m1,
-                                                uint32_t m2, uint32_t vc, uint32_t first_c)
+/* A solving record: prefix q, middles m1, m2, value class vc, whose first
+   candidate in DFS order is first_c and which has n of them. */
+__device__ __forceinline__ void record(const SolBuf &S, uint64_t q, uint32_t m1, uint32_t m2,
+                                       uint32_t vc, uint32_t first_c, uint32_t n)
 {
-    unsigned long long slot = atomicAdd(S.count, 1ull);
-    if (slot < S.cap)
-        S.rec[slot] = make_ulonglong2(q, ((unsigned long long)m1 << 32) | (m2 << 16) | vc);
-    unsigned long long key = ((unsigned long long)(q & 0xFFFFFFFull) << 36) |
+    const unsigned long long slot = atomicAdd(S.count, 1ull);
+    if (S.firsts) {
+        ulonglong2 *f = S.firsts + S.task[q];
+        atomicMin(&f->x, ((unsigned long long)(q & 0xFFFFFFFull) << 36) |
                              ((unsigned long long)m1 << 24) | ((unsigned long long)m2 << 12) |
-                             first_c;
-    atomicMin(S.first, key);
+                             first_c);
+        atomicAdd(&f->y, (unsigned long long)n);
+    } else if (slot < S.cap) {
+        S.rec[slot] = make_ulonglong2(q, ((unsigned long long)m1 << 32) | (m2 << 16) | vc);
+    }
+}
+
+/* The same by a class of mask m (index vc in its list). */
+__device__ __forceinline__ void record_solution(const SolBuf &S, uint64_t q, uint32_t m1,
+                                                uint32_t m2, uint32_t vc, uint32_t m)
+{
+    const uint32_t i = c_vc_off[m] + vc;
+    record(S, q, m1, m2, vc, c_vc_first[i], c_vc_n[i]);
 }
 
 /* Leaf check of a materialized level (count mode): state q solves through
@@ -968,7 +991,7 @@ __global__ void k_leaf(LevelDev P, TaskDev task, SolBuf S)
         for (uint32_t r = 1; r < 8; r++) {
             if (!((live >> r) & 1u)) continue;
             bool ok = lane >= T || P.regs[q * 8 * TPC + r * TPC + lane] == tgt;
-            if (__all_sync(0xFFFFFFFFu, ok) && lane == 0) record_solution(S, q, 0, 0, r, r);
+            if (__all_sync(0xFFFFFFFFu, ok) && lane == 0) record(S, q, 0, 0, r, r, 1);
         }
     }
 }
@@ -993,22 +1016,6 @@ __device__ __forceinline__ uint32_t pair_hits(uint32_t x, uint32_t y, uint32_t e
     return h;
 }
 
-__device__ __forceinline__ uint32_t pair_op(uint32_t k)
-{
-    switch (k) {
-    case 0: return PCA_OP_ADD;
-    case 1: return PCA_OP_SUB;
-    case 2: return PCA_OP_MUL;
-    case 3: return PCA_OP_AND;
-    case 4: return PCA_OP_OR;
-    case 5: return PCA_OP_XOR;
-    case 6: return PCA_OP_SHL;
-    case 7: return PCA_OP_SHR;
-    case 8: return PCA_OP_ASR;
-    default: return PCA_OP_ADDI;
-    }
-}
-
 /* Scan the value classes of mask m against the warp's state, with operand
  * registers remapped: a register equal to rd2 reads spare column 9, else a
  * register equal to rd1 reads column 8 (rd = 8 means "none").
@@ -1028,7 +1035,6 @@ __device__ __forceinline__ void scan_last(const WarpState<TPC> &ws, int T,
                                           const SolBuf &S, uint64_t q, uint32_t m1, uint32_t m2,
                                           uint32_t need1, uint32_t need2, unsigned long long &nev)
 {
-    const uint32_t vbase = c_vc_off[m];
     if (need1) {
         /* the classes reading need1, one operand pair (or ADDI) per lane,
            every op of the pair evaluated on the first two tests at once */
@@ -1070,13 +1076,14 @@ __device__ __forceinline__ void scan_last(const WarpState<TPC> &ws, int T,
                     }
                     if (__all_sync(0xFFFFFFFFu, ok) && lane == 0) {
                         const uint32_t cj = c_pr_cls[(uint64_t)(p0 + b0 + j) * 10 + k];
-                        record_solution(S, q, m1, m2, cj, c_vc_first[vbase + cj]);
+                        record_solution(S, q, m1, m2, cj, m);
                     }
                 }
             }
         }
         return;
     }
+    const uint32_t vbase = c_vc_off[m];
     const uint32_t *uops = c_vc_uop + vbase;
     const uint16_t *list = nullptr;
     const uint32_t nvc = c_vc_off[m + 1] - vbase;
@@ -1109,7 +1116,7 @@ __device__ __forceinline__ void scan_last(const WarpState<TPC> &ws, int T,
             if (lane < T) ok = pca_alu(UOP_OP(uj), ws.R[ra][lane], ws.R[rb][lane], UOP_IMM(uj)) == tgt;
             if (__all_sync(0xFFFFFFFFu, ok) && lane == 0) {
                 const uint32_t cj = list ? (uint32_t)list[b0 + j] : b0 + j;
-                record_solution(S, q, m1, m2, cj, c_vc_first[vbase + cj]);
+                record_solution(S, q, m1, m2, cj, m);
             }
         }
     }
@@ -1434,7 +1441,6 @@ k_suffix_lanes(LevelDev P, TaskDev task, SolBuf S, PrefixRange R, LeanDev lean)
                         y = b == rdL ? w : up[b * TPC];
                     }
                 }
-                const uint32_t vbase = c_vc_off[(liveL >> 1) & 127u];
                 while (hj) {
                     const uint32_t k = (uint32_t)(__ffs(hj) - 1);
                     hj &= hj - 1;
@@ -1443,7 +1449,7 @@ k_suffix_lanes(LevelDev P, TaskDev task, SolBuf S, PrefixRange R, LeanDev lean)
                         ok = (k == 9 ? ((x + e) & 0xFFFFu) : pca_alu(pair_op(k), x, y, 0)) == tgt;
                     if (__all_sync(0xFFFFFFFFu, ok) && lane == 0) {
                         const uint32_t cj = c_pr_cls[(uint64_t)pj * 10 + k];
-                        record_solution(S, qL, 0, 0, cj, c_vc_first[vbase + cj]);
+                        record_solution(S, qL, 0, 0, cj, (liveL >> 1) & 127u);
                     }
                 }
             }
@@ -1453,201 +1459,11 @@ k_suffix_lanes(LevelDev P, TaskDev task, SolBuf S, PrefixRange R, LeanDev lean)
     flush_evals(S, nev, lane);
 }
 
-/* The value of register x on test t after the middles (first FT tests):
-   the innermost middle's own value, else the first middle's (suffix depth
-   3), else the prefix's. */
-template <int FT>
-__device__ __forceinline__ uint32_t mid_val(const uint32_t (&V)[FT][8], int t, uint32_t x,
-                                            uint32_t rdA, uint32_t vA, uint32_t rdB, uint32_t vB)
-{
-    return x == rdB ? vB : x == rdA ? vA : V[t][x];
-}
+}  // namespace pcagb
 
-/* Suffix depths 2 and 3 with a lane per instruction of the innermost
- * middle. SD = 2: a work item is a prefix and 32 of its middle candidates,
- * one per lane; SD = 3: a work item is a prefix and one first middle, whose
- * second middles the lanes take 32 at a time. A lane computes its middle's
- * value on the first FT tests from the prefix's probe (and the first
- * middle's, computed by every lane), applies k_suffix's rules (same-state
- * middles skipped under OEP; a write overwritten unread skips the branch;
- * the last instruction reads the innermost write and the one write still
- * owed a read, at most one), and walks the operand pairs of its mask that
- * read its middle's write, every op of a pair evaluated at once. A pair that
- * passes the first FT tests is checked on every test by the warp (lane =
- * test, the whole chain recomputed from the level's columns) and recorded
- * as k_suffix records it, so the records are the same. */
-template <int TPC, int SD, int FT>
-__global__ void __launch_bounds__(kThreads, 4)
-k_suffix_mid_lanes(LevelDev P, TaskDev task, SolBuf S, uint32_t chunks_per_prefix, PrefixRange R)
-{
-    static_assert(SD == 2 || SD == 3, "middle lanes serve suffix depths 2 and 3");
-    __shared__ uint32_t sV[kWarpsPerBlock][FT][8];
-    const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
-    uint32_t (&V)[FT][8] = sV[wib];
-    const uint64_t nw = (uint64_t)gridDim.x * kWarpsPerBlock;
-    const uint64_t items = R.count * chunks_per_prefix;
-    uint64_t loaded = ~0ull;
-    uint32_t cur_task = ~0u, T = 0, t0 = 0, t1 = 0, t2 = 0;
-    bool cur_active = false;
-    unsigned long long nev = 0;
-    for (uint64_t it = (uint64_t)blockIdx.x * kWarpsPerBlock + wib; it < items; it += nw) {
-        const uint64_t qi = it / chunks_per_prefix;
-        const uint32_t ck = (uint32_t)(it - qi * chunks_per_prefix);
-        const uint64_t q = R.order ? (uint64_t)R.order[R.begin + qi] : R.begin + qi;
-        if (q >= P.n) continue;  /* orders are checked on the host; never index outside */
-        const uint32_t tid = P.task[q];
-        if (tid != cur_task) {
-            cur_task = tid;
-            cur_active = task.active[tid] != 0;
-            T = (uint32_t)task.T[tid];
-            t0 = task.target[tid * 32];
-            if (FT >= 2) t1 = task.target[tid * 32 + 1];
-            if (FT >= 3) t2 = task.target[tid * 32 + 2];
-        }
-        if (!cur_active) continue;
-        const uint32_t live = P.live[q], w0 = P.rdl[q];
-        const uint32_t m0 = (live >> 1) & 127u;
-        const uint32_t cb0 = c_cand_off[m0], nc0 = c_cand_off[m0 + 1] - cb0;
-        if (q != loaded) {
-            __syncwarp();
-            if (lane < FT * 8) V[lane >> 3][lane & 7] = P.probe[q * 32 + (lane & 7) * 4 + (lane >> 3)];
-            __syncwarp();
-            loaded = q;
-        }
-        /* the first middle: each lane's own (SD 2) or the work item's (SD 3) */
-        const uint32_t i1 = SD == 2 ? ck * 32 + (uint32_t)lane : ck;
-        if (SD == 3 && i1 >= nc0) continue;
-        bool act1 = i1 < nc0;
-        const uint32_t u1 = act1 ? c_cand_uop[cb0 + i1] : 0u;
-        if (task.dedup_mid && (u1 >> 31)) act1 = false;
-        const uint32_t rd1 = UOP_RD(u1);
-        const uint32_t owe0 = w0 && !uop_reads(u1, w0) ? w0 : 0u;
-        if (owe0 && rd1 == owe0) act1 = false;
-        if (SD == 3 && !act1) continue;    /* uniform for the warp at SD 3 */
-        uint32_t v1[FT];
-#pragma unroll
-        for (int t = 0; t < FT; t++)
-            v1[t] = pca_alu(UOP_OP(u1), V[t][UOP_A(u1)], V[t][UOP_B(u1)], UOP_IMM(u1));
-        /* (an inactive lane's micro-op is 0: rd 0, no bit to set) */
-        const uint32_t m1 = rd1 ? (m0 | (1u << (rd1 - 1))) & 127u : m0;
-        const uint32_t nc1 = SD == 3 ? c_cand_off[m1 + 1] - c_cand_off[m1] : 32u;
-        for (uint32_t b2 = 0; b2 < nc1; b2 += 32) {
-            /* the innermost middle of this lane and the last position's
-               requirements */
-            bool act = act1;
-            uint32_t i2 = 0, u2 = 0, rdA = 8, rdB = rd1, need1 = rd1, need2 = owe0, m = m1;
-            uint32_t vA[FT], vB[FT];
-#pragma unroll
-            for (int t = 0; t < FT; t++) {
-                vA[t] = 0;
-                vB[t] = v1[t];
-            }
-            if (SD == 3) {
-                i2 = b2 + (uint32_t)lane;
-                act = i2 < nc1;
-                u2 = act ? c_cand_uop[c_cand_off[m1] + i2] : 0u;
-                if (task.dedup_mid && (u2 >> 31)) act = false;
-                const uint32_t rd2 = UOP_RD(u2);
-                const uint32_t owe1 = uop_reads(u2, rd1) ? 0u : rd1;
-                const uint32_t owe0b = owe0 && !uop_reads(u2, owe0) ? owe0 : 0u;
-                if ((owe1 && rd2 == owe1) || (owe0b && rd2 == owe0b)) act = false;
-                if (owe1 && owe0b) act = false;   /* three registers to read */
-                need2 = owe1 ? owe1 : owe0b;
-                need1 = rd2;
-                m = rd2 ? (m1 | (1u << (rd2 - 1))) & 127u : m1;
-                rdA = rd1;
-                rdB = rd2;
-#pragma unroll
-                for (int t = 0; t < FT; t++) {
-                    vA[t] = v1[t];
-                    vB[t] = pca_alu(UOP_OP(u2), mid_val<FT>(V, t, UOP_A(u2), 8, 0, rd1, v1[t]),
-                                    mid_val<FT>(V, t, UOP_B(u2), 8, 0, rd1, v1[t]), UOP_IMM(u2));
-                }
-            }
-            uint32_t p0 = 0, np = 0;
-            if (act) {
-                p0 = c_pr_off_g[m * 8 + need1];
-                np = c_pr_off_g[m * 8 + need1 + 1] - p0;
-                if (!need2) nev += c_ev_sd1[m * 8 + need1];
-            }
-            uint32_t jn = np;
-#pragma unroll
-            for (int o = 16; o; o >>= 1) jn = max(jn, __shfl_xor_sync(0xFFFFFFFFu, jn, o));
-            for (uint32_t j = 0; j < jn; j++) {
-                uint32_t hits = 0;
-                if (j < np) {
-                    const uint32_t d = c_pr[p0 + j];
-                    const uint32_t a = d & 7u, b = (d >> 3) & 7u;
-                    if (!need2 || a == need2 || b == need2) {
-                        if (need2) nev += __popc((d >> 6) & 0x3FFu);
-                        const uint32_t e = (uint32_t)(uint16_t)(int16_t)(int8_t)(uint8_t)(d >> 16);
-                        hits = pair_hits(mid_val<FT>(V, 0, a, rdA, vA[0], rdB, vB[0]),
-                                         mid_val<FT>(V, 0, b, rdA, vA[0], rdB, vB[0]), e, t0) &
-                               (d >> 6) & 0x3FFu;
-                        if (FT >= 2 && T >= 2 && hits)
-                            hits &= pair_hits(
-                                mid_val<FT>(V, FT >= 2 ? 1 : 0, a, rdA, vA[FT >= 2 ? 1 : 0], rdB,
-                                            vB[FT >= 2 ? 1 : 0]),
-                                mid_val<FT>(V, FT >= 2 ? 1 : 0, b, rdA, vA[FT >= 2 ? 1 : 0], rdB,
-                                            vB[FT >= 2 ? 1 : 0]), e, t1);
-                        if (FT >= 3 && T >= 3 && hits)
-                            hits &= pair_hits(
-                                mid_val<FT>(V, FT >= 3 ? 2 : 0, a, rdA, vA[FT >= 3 ? 2 : 0], rdB,
-                                            vB[FT >= 3 ? 2 : 0]),
-                                mid_val<FT>(V, FT >= 3 ? 2 : 0, b, rdA, vA[FT >= 3 ? 2 : 0], rdB,
-                                            vB[FT >= 3 ? 2 : 0]), e, t2);
-                    }
-                }
-                uint32_t bal = __ballot_sync(0xFFFFFFFFu, hits != 0);
-                while (bal) {
-                    const int L = __ffs(bal) - 1;
-                    bal &= bal - 1;
-                    uint32_t hj = __shfl_sync(0xFFFFFFFFu, hits, L);
-                    const uint32_t uL1 = __shfl_sync(0xFFFFFFFFu, u1, L);
-                    const uint32_t uL2 = __shfl_sync(0xFFFFFFFFu, u2, L);
-                    const uint32_t iL1 = __shfl_sync(0xFFFFFFFFu, i1, L);
-                    const uint32_t iL2 = __shfl_sync(0xFFFFFFFFu, i2, L);
-                    const uint32_t mL = __shfl_sync(0xFFFFFFFFu, m, L);
-                    const uint32_t pj = __shfl_sync(0xFFFFFFFFu, p0, L) + j;
-                    const uint32_t d = c_pr[pj];
-                    const uint32_t a = d & 7u, b = (d >> 3) & 7u;
-                    const uint32_t e = (uint32_t)(uint16_t)(int16_t)(int8_t)(uint8_t)(d >> 16);
-                    /* the chain on test `lane`, from the level's columns */
-                    uint32_t x = 0, y = 0, tg = 0;
-                    if (lane < (int)T) {
-                        const uint16_t *col = P.regs + q * 8 * TPC + lane;
-                        const uint32_t r1 = UOP_RD(uL1);
-                        const uint32_t m1v = pca_alu(UOP_OP(uL1), col[UOP_A(uL1) * TPC],
-                                                     col[UOP_B(uL1) * TPC], UOP_IMM(uL1));
-                        uint32_t r2 = 8, m2v = 0;
-                        if (SD == 3) {
-                            r2 = UOP_RD(uL2);
-                            const uint32_t xa = UOP_A(uL2) == r1 ? m1v : col[UOP_A(uL2) * TPC];
-                            const uint32_t xb = UOP_B(uL2) == r1 ? m1v : col[UOP_B(uL2) * TPC];
-                            m2v = pca_alu(UOP_OP(uL2), xa, xb, UOP_IMM(uL2));
-                        }
-                        x = a == r2 ? m2v : a == r1 ? m1v : col[a * TPC];
-                        y = b == r2 ? m2v : b == r1 ? m1v : col[b * TPC];
-                        tg = task.target[tid * 32 + lane];
-                    }
-                    const uint32_t vbase = c_vc_off[mL];
-                    while (hj) {
-                        const uint32_t k = (uint32_t)(__ffs(hj) - 1);
-                        hj &= hj - 1;
-                        bool ok = true;
-                        if (lane < (int)T)
-                            ok = (k == 9 ? ((x + e) & 0xFFFFu) : pca_alu(pair_op(k), x, y, 0)) == tg;
-                        if (__all_sync(0xFFFFFFFFu, ok) && lane == 0) {
-                            const uint32_t cj = c_pr_cls[(uint64_t)pj * 10 + k];
-                            record_solution(S, q, iL1, SD == 3 ? iL2 : 0u, cj, c_vc_first[vbase + cj]);
-                        }
-                    }
-                }
-            }
-        }
-    }
-    flush_evals(S, nev, lane);
-}
+#include "suffix_forms.cuh"
+
+namespace pcagb {
 
 /* Value-class evaluations k_suffix<TPC, 1> runs over range R: a prefix of
    mask m whose last write is w0 scans the pair list of (m, w0), a root

@@ -68,6 +68,20 @@ struct GenTables {
     /* pr_ev[m*8+r]: class evaluations one pass over the pair list of (m, r)
        runs (every admitted op of every entry) */
     std::vector<uint32_t> pr_ev;
+    /* pr_at[(m*8 + r)*64 + (a | b << 3)]: place of the entry on operands a, b
+       in the pair list of (m, r), ADDI entries apart (those are the list's
+       last six, in immediate order); 0xFFFF: none */
+    std::vector<uint16_t> pr_at;
+    /* cand_of[(vc_off[m] + c)*8 + rd]: candidate of mask m's value class c
+       that writes rd; 0xFFFF: none */
+    std::vector<uint16_t> cand_of;
+    /* ev_mid[((d*128 + m)*8 + A)*8 + B]: class evaluations of a middle
+       instruction and the last one from a state of mask m, when they must
+       read registers A and B (0: none) between them: the middle overwrites
+       neither unread and leaves at most one unread, the last reads the
+       middle's write and the one left; d = 1 skips same-state middles
+       (cand_dupe) */
+    std::vector<uint32_t> ev_mid;
     int max_nc = 0;
     int max_nvc = 0;
 

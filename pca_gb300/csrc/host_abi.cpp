@@ -193,6 +193,44 @@ static GenTables build_tables()
     for (int i = 0; i < 128 * 8; i++)
         for (uint32_t e = t.pr_off[i]; e < t.pr_off[i + 1]; e++)
             t.pr_ev[i] += (uint32_t)__builtin_popcount((t.pr[e] >> 6) & 0x3FFu);
+    t.pr_at.assign(128 * 8 * 64, 0xFFFF);
+    for (uint32_t i = 0; i < 128 * 8; i++)
+        for (uint32_t e = t.pr_off[i]; e < t.pr_off[i + 1]; e++)
+            if (!(t.pr[e] >> 15 & 1u)) t.pr_at[i * 64 + (t.pr[e] & 63u)] = (uint16_t)(e - t.pr_off[i]);
+    t.cand_of.assign(t.vc_uop.size() * 8, 0xFFFF);
+    for (int m = 0; m < 128; m++)
+        for (uint32_t i = t.cand_off[m]; i < t.cand_off[m + 1]; i++)
+            t.cand_of[(t.vc_off[m] + t.cand_vc[i]) * 8 + UOP_RD(t.cand_uop[i])] =
+                (uint16_t)(i - t.cand_off[m]);
+    {
+        /* evaluations of one last position by (mask, its two reads) */
+        std::vector<uint32_t> last(128 * 64, 0);
+        for (int m = 0; m < 128; m++)
+            for (uint32_t r = 1; r < 8; r++)
+                for (uint32_t e = t.pr_off[m * 8 + r]; e < t.pr_off[m * 8 + r + 1]; e++) {
+                    const uint32_t d = t.pr[e], a = d & 7u, b = (d >> 3) & 7u;
+                    const uint32_t n = (uint32_t)__builtin_popcount((d >> 6) & 0x3FFu);
+                    last[(m * 8 + r) * 8] += n;
+                    for (uint32_t x = 1; x < 8; x++)
+                        if (a == x || b == x) last[(m * 8 + r) * 8 + x] += n;
+                }
+        t.ev_mid.assign(2 * 128 * 64, 0);
+        for (int m = 0; m < 128; m++)
+            for (uint32_t i = t.cand_off[m]; i < t.cand_off[m + 1]; i++) {
+                const uint32_t u = t.cand_uop[i], rd = UOP_RD(u);
+                const uint32_t reads = 1u << UOP_A(u) | 1u << UOP_B(u);
+                const uint32_t *l = &last[(((m | 1u << (rd - 1)) & 127u) * 8 + rd) * 8];
+                for (uint32_t A = 0; A < 8; A++)
+                    for (uint32_t B = 0; B < 8; B++) {
+                        const uint32_t a = A && !(reads >> A & 1u) ? A : 0u;
+                        const uint32_t b = B && !(reads >> B & 1u) ? B : 0u;
+                        if ((a && b) || (a && a == rd) || (b && b == rd)) continue;
+                        const uint32_t n = l[a ? a : b];
+                        t.ev_mid[(m * 8 + A) * 8 + B] += n;
+                        if (!t.cand_dupe[i]) t.ev_mid[((128 + m) * 8 + A) * 8 + B] += n;
+                    }
+            }
+    }
     for (int s = 0; s < 5; s++) t.ev[s].assign(128, 0);
     for (int m = 0; m < 128; m++) t.ev[1][m] = t.vc_off[m + 1] - t.vc_off[m];
     for (int s = 2; s < 5; s++)
