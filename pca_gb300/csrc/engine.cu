@@ -161,18 +161,27 @@ struct pcagb_engine {
                                                 lean materialise kernels */
     uint32_t *d_status = nullptr;
     ulonglong2 *d_sol = nullptr;
-    ulonglong2 *d_firsts = nullptr;          /* [kMaxBatch] SolBuf::firsts */
-    FirstOut *d_first_out = nullptr, *h_first_out = nullptr;   /* [kMaxBatch], h: pinned */
+    ulonglong2 *d_firsts = nullptr;          /* [cap_tasks] SolBuf::firsts */
+    FirstOut *d_first_out = nullptr;         /* [cap_tasks] */
     uint64_t sol_cap = 1u << 20;
     /* batch task table */
     int32_t *d_task_T = nullptr;
     uint32_t *d_task_target = nullptr;
     uint8_t *d_task_active = nullptr;
-    uint16_t *d_task_io = nullptr;           /* [kMaxBatch][3][32] in0, in1, target */
-    unsigned long long *d_hist = nullptr;    /* [kMaxBatch][128] */
+    uint16_t *d_task_io = nullptr;           /* [cap_tasks][3][32] in0, in1, target */
+    uint8_t *d_order = nullptr;              /* [cap_tasks][32] the caller's test at each place */
+    RootIn *d_roots = nullptr;               /* [cap_tasks] */
+    int cap_tasks = 0;                       /* tasks the per-task arrays hold (ensure_tasks) */
+    char *d_tasks = nullptr;                 /* the allocation behind the device ones */
+    unsigned long long *d_hist = nullptr;    /* [cap_tasks][128] */
     /* pinned host mirror of the small results (kPin* slots) and of d_hist:
        device-to-host reads of these never wait on their own */
     unsigned long long *h_pin = nullptr;
+    /* pinned too: first-only results, roots and active flags on their way to
+       the device */
+    FirstOut *h_first_out = nullptr;
+    RootIn *h_roots = nullptr;
+    uint8_t *h_up_active = nullptr;
     std::vector<uint8_t> h_active;           /* host copy of d_task_active */
     cudaEvent_t ev0 = nullptr, ev1 = nullptr, ev2 = nullptr, ev3 = nullptr;
     cudaEvent_t evk0 = nullptr, evk1 = nullptr;   /* around a lane-per-prefix launch */
@@ -626,7 +635,6 @@ struct TaskRun {
     search_state_t root;           /* level-0 state */
     int T = 0;
     uint16_t target[MAX_TESTS] = {};
-    std::vector<int> order;        /* device test order */
     int max_depth = 0, min_depth = 0;
     bool done = false;
     int optimal_depth = -1;
@@ -831,14 +839,14 @@ void launch_suffix_lanes(int ft, int g, cudaStream_t st, const LevelDev &L, cons
 
 /* A long stage of a solve that shares the GPU (a server's) runs in a few
    CTAs: a launch holds its SMs until it ends, and requests admitted meanwhile
-   would wait for them. Six CTAs leave 146 SMs to the others and take about
+   would wait for them. Four CTAs leave 148 SMs to the others and take about
    as long as the stage took before it was a lane per state (is_power2 at
-   depth 5: 0.4 s, 9 ms on the whole GPU), which is also what the serving test
+   depth 5: 0.4 s, 5 ms on the whole GPU), which is also what the serving test
    builds on: it submits requests 0.2 s into such a solve and expects their
    answers before its own. The stages of requests up to depth 4 (0.2 ms)
    are below the line. */
 constexpr double kBackgroundMs = 2.0;
-constexpr int kBackgroundCtas = 6;
+constexpr int kBackgroundCtas = 4;
 
 /* A lane per state (k_suffix_states): per_prefix states to a prefix, and the
    shares their work is cut into so that the warps fill the GPU about twice
@@ -1172,66 +1180,6 @@ void leaf_key(const task_spec_t *task, const search_state_t &root, const std::ve
     }
 }
 
-/* Test order for the suffix kernel. Its lanes evaluate value classes on
-   the first one or two tests and send survivors to a check of all tests, so
-   the fewer classes pass the first tests the less work is done. The order is
-   chosen greedily on (state, class) pairs sampled from the root and its
-   children: each next test is the one the fewest remaining pairs pass. A
-   permutation of the tests changes no result of the search (pruning keys,
-   DFS order, programs and counts are all independent of it). */
-std::vector<int> choose_test_order(const TaskRun &tr)
-{
-    const GenTables &gt = gen_tables();
-    const int T = tr.T;
-    search_ctx_t ctx;
-    memset(&ctx, 0, sizeof ctx);
-    ctx.num_tests = (uint8_t)T;
-    /* the root and up to 24 of its children, spread over the op blocks */
-    std::vector<search_state_t> sample(1, tr.root);
-    uint16_t cands[4096];
-    int n = gen_candidates(tr.root.live, cands, 4096);
-    const int stride = std::max(1, n / 24);
-    for (int i = 0; i < n; i += stride) {
-        search_state_t c;
-        if (search_state_step(&ctx, &tr.root, cands[i], &c)) sample.push_back(c);
-    }
-    std::vector<uint32_t> masks;
-    for (const search_state_t &st : sample) {
-        const uint32_t m = (st.live >> 1) & 127u;
-        for (uint32_t i = gt.vc_off[m]; i < gt.vc_off[m + 1]; i++) {
-            const uint32_t u = gt.vc_uop[i];
-            uint32_t pass = 0;
-            for (int t = 0; t < T; t++) {
-                uint32_t v = pca_alu(UOP_OP(u), st.regs[t][UOP_A(u)], st.regs[t][UOP_B(u)],
-                                     UOP_IMM(u));
-                if (v == tr.target[t]) pass |= 1u << t;
-            }
-            masks.push_back(pass);
-        }
-    }
-    std::vector<int> order;
-    uint32_t used = 0;
-    while ((int)order.size() < T && !masks.empty()) {
-        int best = -1;
-        size_t best_n = SIZE_MAX;
-        for (int t = 0; t < T; t++) {
-            if (used >> t & 1u) continue;
-            size_t cnt = 0;
-            for (uint32_t m : masks) cnt += m >> t & 1u;
-            if (cnt < best_n) { best_n = cnt; best = t; }
-        }
-        order.push_back(best);
-        used |= 1u << best;
-        std::vector<uint32_t> keep;
-        for (uint32_t m : masks)
-            if (m >> best & 1u) keep.push_back(m);
-        masks.swap(keep);
-    }
-    for (int t = 0; t < T; t++)
-        if (!(used >> t & 1u)) order.push_back(t);
-    return order;
-}
-
 uint64_t hist_sum(const Level &L, int t, const std::vector<uint64_t> &weight)
 {
     uint64_t s = 0;
@@ -1401,6 +1349,8 @@ int validate_order(pcagb_engine *e, const uint32_t *order, uint64_t n)
     return PCAGB_OK;
 }
 
+int ensure_tasks(pcagb_engine *e, int nt);
+
 /* Core batched IDDFS shared by every solve entry point. */
 struct OrderSpec {
     pcagb_order_cb cb = nullptr;
@@ -1443,8 +1393,9 @@ int run_batch(pcagb_engine *e, std::vector<TaskRun> &runs, const pcagb_opts_t &o
         maxK = std::max(maxK, tr.max_depth);
         memset(&tr.res, 0, sizeof tr.res);
         tr.res.optimal_depth = -1;
-        tr.order = choose_test_order(tr);
     }
+    CK(cudaSetDevice(e->device));
+    if (int prc = ensure_tasks(e, nt)) return prc;
     e->TPC = maxT <= 16 ? 16 : 32;
     e->no_oep = o.oep_mode == PCAGB_OEP_NONE;
     /* the last depth's split level may be built lean when nothing but its
@@ -1455,64 +1406,36 @@ int run_batch(pcagb_engine *e, std::vector<TaskRun> &runs, const pcagb_opts_t &o
     e->lean_K = !o.count_levels && !ord && !warp_forced && !o.full_levels ? maxK : -1;
     e->td = TaskDev{e->d_task_T, e->d_task_target, e->d_task_active,
                     o.oep_mode == PCAGB_OEP_EXACT_LIVE, o.oep_mode != PCAGB_OEP_NONE};
-    CK(cudaSetDevice(e->device));
-    CK(cudaMemsetAsync(e->d_status, 0, 4, e->stream));
-    CK(cudaMemsetAsync(e->d_small + 3, 0, 8, e->stream));
-    {
-        std::vector<int32_t> T(nt);
-        std::vector<uint32_t> tgt((size_t)nt * 32, 0);
-        for (int i = 0; i < nt; i++) {
-            T[i] = runs[i].T;
-            for (int t = 0; t < runs[i].T; t++)
-                tgt[(size_t)i * 32 + t] = runs[i].target[runs[i].order[t]];
-        }
-        std::vector<uint16_t> io((size_t)nt * 3 * 32, 0);
-        for (int i = 0; i < nt; i++)
-            for (int t = 0; t < runs[i].T; t++) {
-                const int o = runs[i].order[t];
-                io[((size_t)i * 3 + 0) * 32 + t] = runs[i].root.regs[o][1];
-                io[((size_t)i * 3 + 1) * 32 + t] = runs[i].root.regs[o][2];
-                io[((size_t)i * 3 + 2) * 32 + t] = runs[i].target[o];
-            }
-        CK(e_copy(e, e->d_task_T, T.data(), nt * 4, cudaMemcpyHostToDevice, e->stream));
-        CK(e_copy(e, e->d_task_target, tgt.data(), tgt.size() * 4, cudaMemcpyHostToDevice,
-                  e->stream));
-        CK(e_copy(e, e->d_task_io, io.data(), io.size() * 2, cudaMemcpyHostToDevice, e->stream));
-    }
-
-    /* level 0: one root per task */
+    /* level 0: one root per task. The roots go over in one copy; the test
+       order is chosen and level 0 laid out on the device (k_setup) */
     Level L0;
     if (alloc_level(e, L0, nt) != PCAGB_OK) { set_err("arena too small"); return PCAGB_ENOMEM; }
+    L0.hist.assign((size_t)nt * 128, 0);
+    for (int i = 0; i < nt; i++) {
+        const TaskRun &tr = runs[i];
+        RootIn &r = e->h_roots[i];
+        memset(&r, 0, sizeof r);
+        memcpy(r.regs, tr.root.regs, (size_t)tr.T * sizeof r.regs[0]);
+        memcpy(r.flags, tr.root.flags, tr.T);
+        memcpy(r.target, tr.target, (size_t)tr.T * 2);
+        r.live = tr.root.live;
+        r.T = (uint8_t)tr.T;
+        L0.hist[(size_t)i * 128 + ((tr.root.live >> 1) & 127)] = 1;
+    }
+    CK(e_copy(e, e->d_roots, e->h_roots, (size_t)nt * sizeof(RootIn), cudaMemcpyHostToDevice,
+              e->stream));
     {
-        const int TPC = e->TPC;
-        std::vector<uint16_t> regs((size_t)nt * 8 * TPC, 0), probe((size_t)nt * 32, 0);
-        std::vector<uint8_t> flags((size_t)nt * TPC, 0), live(nt);
-        std::vector<uint16_t> task(nt), cidx(nt, 0);
-        std::vector<uint32_t> parent(nt, 0);
-        L0.hist.assign((size_t)nt * 128, 0);
-        for (int i = 0; i < nt; i++) {
-            const TaskRun &tr = runs[i];
-            for (int t = 0; t < tr.T; t++) {
-                for (int r = 1; r < 8; r++) {
-                    regs[((size_t)i * 8 + r) * TPC + t] = tr.root.regs[tr.order[t]][r];
-                    if (t < 4) probe[(size_t)i * 32 + r * 4 + t] = tr.root.regs[tr.order[t]][r];
-                }
-                flags[(size_t)i * TPC + t] = tr.root.flags[tr.order[t]];
-            }
-            live[i] = tr.root.live;
-            task[i] = (uint16_t)i;
-            L0.hist[(size_t)i * 128 + ((tr.root.live >> 1) & 127)] = 1;
-        }
-        CK(e_copy(e, L0.regs, regs.data(), regs.size() * 2, cudaMemcpyHostToDevice, e->stream));
-        CK(e_copy(e, L0.flags, flags.data(), flags.size(), cudaMemcpyHostToDevice, e->stream));
-        CK(e_copy(e, L0.live, live.data(), nt, cudaMemcpyHostToDevice, e->stream));
-        CK(e_copy(e, L0.task, task.data(), nt * 2, cudaMemcpyHostToDevice, e->stream));
-        CK(e_copy(e, L0.parent, parent.data(), nt * 4, cudaMemcpyHostToDevice, e->stream));
-        CK(e_copy(e, L0.cidx, cidx.data(), nt * 2, cudaMemcpyHostToDevice, e->stream));
-        CK(cudaMemsetAsync(L0.rdl, 0, nt, e->stream));
-        CK(cudaMemsetAsync(L0.own, 0, nt, e->stream));
-        CK(cudaMemsetAsync(L0.twin, 0, nt, e->stream));
-        CK(e_copy(e, L0.probe, probe.data(), probe.size() * 2, cudaMemcpyHostToDevice, e->stream));
+        const LevelOut out{L0.regs, L0.flags, L0.live, L0.task, L0.parent, L0.cidx, L0.rdl, L0.own,
+                           L0.probe};
+        const SetupOut so{e->d_task_T, e->d_task_target, e->d_task_io, e->d_order, e->d_status,
+                          e->d_small + 3};
+        const uint32_t rounds = maxK >= 5 ? 8 : 1;
+        if (e->TPC == 16)
+            k_setup<16><<<nt, kSetupWarps * 32, 0, e->stream>>>(e->d_roots, rounds, out, L0.twin, so);
+        else
+            k_setup<32><<<nt, kSetupWarps * 32, 0, e->stream>>>(e->d_roots, rounds, out, L0.twin, so);
+        const int rc = check_launch(e);
+        if (rc) return rc;
     }
     e->levels.push_back(std::move(L0));
 
@@ -1566,7 +1489,8 @@ int run_batch(pcagb_engine *e, std::vector<TaskRun> &runs, const pcagb_opts_t &o
             nact += active[i];
         }
         if (!nact) break;
-        CK(e_copy(e, e->d_task_active, active.data(), nt, cudaMemcpyHostToDevice, e->stream));
+        memcpy(e->h_up_active, active.data(), nt);
+        CK(e_copy(e, e->d_task_active, e->h_up_active, nt, cudaMemcpyHostToDevice, e->stream));
         e->h_active = active;
         int S_target = o.count_levels ? K : K - 1;
         /* an ordered solve with an automatic split orders only the stages
@@ -1857,6 +1781,51 @@ int ensure_device_tables(int device)
     return PCAGB_OK;
 }
 
+/* The per-task arrays, on the device and pinned on the host, for a batch of
+   nt tasks: 256 at first, grown by the first larger batch (8,192, the most,
+   take 25 MB of both, whose allocation would take longer than the rest of an
+   engine's creation). */
+int ensure_tasks(pcagb_engine *e, int nt)
+{
+    if (nt <= e->cap_tasks) return PCAGB_OK;
+    int cap = std::max(e->cap_tasks, 256);
+    while (cap < nt) cap *= 2;
+    const size_t n = (size_t)cap;
+    CK(cudaStreamSynchronize(e->stream));
+    e->cap_tasks = 0;
+    CK(cudaFree(e->d_tasks));
+    if (e->h_pin) CK(cudaFreeHost(e->h_pin));
+    e->d_tasks = nullptr;
+    e->h_pin = nullptr;
+    struct { void **p; size_t bytes; } dev[] = {
+        {(void **)&e->d_firsts, n * sizeof(ulonglong2)},
+        {(void **)&e->d_first_out, n * sizeof(FirstOut)},
+        {(void **)&e->d_task_T, n * 4},
+        {(void **)&e->d_task_target, n * 32 * 4},
+        {(void **)&e->d_task_active, n},
+        {(void **)&e->d_task_io, n * 3 * 32 * 2},
+        {(void **)&e->d_order, n * 32},
+        {(void **)&e->d_roots, n * sizeof(RootIn)},
+        {(void **)&e->d_hist, n * 128 * sizeof(unsigned long long)}};
+    size_t total = 0;
+    for (auto &x : dev) total += (x.bytes + 255) & ~size_t(255);
+    CK(cudaMalloc(&e->d_tasks, total));
+    char *at = e->d_tasks;
+    for (auto &x : dev) {
+        *x.p = at;
+        at += (x.bytes + 255) & ~size_t(255);
+    }
+    const size_t pins = (kPinHist + n * 128) * sizeof(unsigned long long);
+    char *p = nullptr;
+    CK(cudaMallocHost(&p, pins + n * (sizeof(RootIn) + sizeof(FirstOut) + 1)));
+    e->h_pin = (unsigned long long *)p;
+    e->h_roots = (RootIn *)(p + pins);
+    e->h_first_out = (FirstOut *)(e->h_roots + n);
+    e->h_up_active = (uint8_t *)(e->h_first_out + n);
+    e->cap_tasks = cap;
+    return PCAGB_OK;
+}
+
 int engine_init(pcagb_engine *e, int device, size_t budget)
 {
     CK(cudaSetDevice(device));
@@ -1890,6 +1859,7 @@ int engine_init(pcagb_engine *e, int device, size_t budget)
         PCAGB_PRELOAD(k_suffix_lanes<32, 2>); PCAGB_PRELOAD(k_suffix_lanes<32, 3>);
         PCAGB_PRELOAD(k_suffix_states<16, 2>); PCAGB_PRELOAD(k_suffix_states<32, 2>);
         PCAGB_PRELOAD(k_suffix_states<16, 3>); PCAGB_PRELOAD(k_suffix_states<32, 3>);
+        PCAGB_PRELOAD(k_setup<16>); PCAGB_PRELOAD(k_setup<32>);
         PCAGB_PRELOAD(k_expand_insert<16>); PCAGB_PRELOAD(k_expand_insert<32>);
         PCAGB_PRELOAD(k_materialize<16>); PCAGB_PRELOAD(k_materialize<32>);
         PCAGB_PRELOAD(k_twins<16>); PCAGB_PRELOAD(k_twins<32>);
@@ -1943,16 +1913,7 @@ int engine_init(pcagb_engine *e, int device, size_t budget)
     CK(cudaMalloc(&e->d_small, 256 * sizeof(unsigned long long)));
     CK(cudaMalloc(&e->d_status, 16));
     CK(cudaMalloc(&e->d_sol, e->sol_cap * sizeof(ulonglong2)));
-    CK(cudaMalloc(&e->d_firsts, kMaxBatch * sizeof(ulonglong2)));
-    CK(cudaMalloc(&e->d_first_out, kMaxBatch * sizeof(FirstOut)));
-    CK(cudaMallocHost(&e->h_first_out, kMaxBatch * sizeof(FirstOut)));
-    CK(cudaMalloc(&e->d_task_T, kMaxBatch * 4));
-    CK(cudaMalloc(&e->d_task_target, (size_t)kMaxBatch * 32 * 4));
-    CK(cudaMalloc(&e->d_task_active, kMaxBatch));
-    CK(cudaMalloc(&e->d_task_io, (size_t)kMaxBatch * 3 * 32 * 2));
-    CK(cudaMalloc(&e->d_hist, (size_t)kMaxBatch * 128 * sizeof(unsigned long long)));
-    CK(cudaMallocHost(&e->h_pin, (kPinHist + (size_t)kMaxBatch * 128) * sizeof(unsigned long long)));
-    return PCAGB_OK;
+    return ensure_tasks(e, 1);
 }
 
 bool make_run(const task_spec_t *task, const pcagb_opts_t &o, TaskRun *tr)
@@ -2056,7 +2017,10 @@ int record_levels(pcagb_engine *e, const task_spec_t *task, const TaskRun &tr,
     for (auto &o : opt) st->optimal_states += (int)o.size();
 
     TestPos tp{};
-    for (int j = 0; j < tr.T; j++) tp.pos[tr.order[j]] = (uint8_t)j;
+    uint8_t placed[MAX_TESTS];   /* test order of the solve's one task */
+    CK(e_copy(e, placed, e->d_order, sizeof placed, cudaMemcpyDeviceToHost, e->stream));
+    CK(cudaStreamSynchronize(e->stream));
+    for (int j = 0; j < tr.T; j++) tp.pos[placed[j]] = (uint8_t)j;
     const size_t top0 = e->top;
     auto done = [&](int rc) {
         e->top = top0;
@@ -2241,19 +2205,12 @@ void pcagb_engine_destroy(pcagb_engine_t *e)
     if (!e) return;
     cudaSetDevice(e->device);
     if (e->stream) cudaStreamSynchronize(e->stream);
-    cudaFree(e->arena);
     cudaFree(e->d_small);
     cudaFree(e->d_status);
     cudaFree(e->d_sol);
-    cudaFree(e->d_firsts);
-    cudaFree(e->d_first_out);
-    if (e->h_first_out) cudaFreeHost(e->h_first_out);
-    cudaFree(e->d_task_T);
-    cudaFree(e->d_task_target);
-    cudaFree(e->d_task_active);
-    cudaFree(e->d_task_io);
-    cudaFree(e->d_hist);
+    cudaFree(e->d_tasks);
     if (e->h_pin) cudaFreeHost(e->h_pin);
+    cudaFree(e->arena);   /* last: the next engine's arena is then allocated 0.7 ms faster */
     for (cudaEvent_t ev : {e->ev0, e->ev1, e->ev2, e->ev3, e->evk0, e->evk1})
         if (ev) cudaEventDestroy(ev);
     if (e->stream) cudaStreamDestroy(e->stream);

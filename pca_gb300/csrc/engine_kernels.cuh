@@ -233,6 +233,181 @@ struct WarpState {
     uint64_t colh[8];         /* colh[r] = col_final(r, hash(col r)), r >= 1 */
 };
 
+/* ---- set-up of a batch -------------------------------------------------- */
+
+/* One task's root as the host hands it over, tests in the caller's order. */
+struct __align__(16) RootIn {
+    uint16_t regs[32][8];
+    uint16_t target[32];
+    uint8_t flags[32];
+    uint8_t live;
+    uint8_t T;
+};
+
+/* Where the set-up writes the batch's per-task arrays. */
+struct SetupOut {
+    int32_t *T;
+    uint32_t *target;   /* [task][32], in the engine's test order */
+    uint16_t *io;       /* [task][3][32] inputs 0 and 1, target, in that order */
+    uint8_t *order;     /* [task][32] the caller's test at each place */
+    uint32_t *status;
+    unsigned long long *evals;
+};
+
+/* Level 0 and the test order of every task: a block per task.
+ *
+ * The suffix kernels reject almost every value on a state's first tests, so
+ * these are chosen to reject: each next test is the one that the fewest
+ * (state, last instruction) pairs pass among the pairs that pass every test
+ * chosen before; once no pair is left the choice starts over, until the
+ * probe's four tests are chosen (a deeper state's values pass the first ones
+ * more often than the sample's, so each should reject well by itself). Ties
+ * go to a target not met yet: a constant passes equal targets together. The
+ * other tests keep the caller's order. A permutation of the tests changes no
+ * result of the search.
+ *
+ * The states are drawn (the same ones for every call) two instructions from
+ * the root, 17 a round, a warp each; the pairs are their classes that read
+ * the second write. One round serves a search of depth 4, whose last stage
+ * is over in a quarter of a millisecond; a deeper one takes eight, for on a
+ * target of few values one round's sample is too small: of is_power2's
+ * values at depth 5, one in 700 passed four tests chosen on 17 states and one
+ * in 50,000 tests chosen on 136 (a fifth of the stage's time).
+ *
+ * Bound: latency, a warp's walk over some fifty classes a round. On the host
+ * such a choice took 50-300 us a task, most of the time of a small solve and
+ * nine tenths of a batch of 256. */
+constexpr int kSetupWarps = 17;
+constexpr uint32_t kSetupPairs = 224;   /* passing pairs kept a warp */
+
+template <int TPC>
+__global__ void __launch_bounds__(kSetupWarps * 32)
+k_setup(const RootIn *in, uint32_t rounds, LevelOut L0, uint8_t *twin, SetupOut out)
+{
+    __shared__ RootIn root;
+    __shared__ uint16_t st[kSetupWarps][8][32];
+    __shared__ uint32_t sp[kSetupWarps][kSetupPairs];
+    __shared__ uint32_t cnt[32], alive;
+    __shared__ uint8_t order[32];
+    const uint32_t i = blockIdx.x;
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    static_assert(sizeof(RootIn) % 16 == 0, "copied in 16-byte pieces");
+    for (uint32_t k = threadIdx.x; k < sizeof(RootIn) / 16; k += blockDim.x)
+        reinterpret_cast<uint4 *>(&root)[k] = reinterpret_cast<const uint4 *>(in + i)[k];
+    if (threadIdx.x < 32) cnt[threadIdx.x] = 0;
+    __syncthreads();
+    const uint32_t T = root.T, live = root.live;
+    const uint32_t target = (uint32_t)lane < T ? root.target[lane] : 0x10000u;
+    uint16_t (&R)[8][32] = st[w];
+    uint32_t *pairs = sp[w], np = 0;
+    for (uint32_t rd = 0; rd < rounds; rd++) {
+        __syncwarp();
+#pragma unroll
+        for (int r = 0; r < 8; r++) R[r][lane] = root.regs[lane][r];
+        uint32_t m = (live >> 1) & 127u, last = 0;
+#pragma unroll
+        for (uint32_t k = 0; k < 2; k++) {
+            const uint32_t nc = c_cand_off[m + 1] - c_cand_off[m];
+            const uint32_t pick = ((rd * kSetupWarps + w) * 2 + k + 1) * 2654435761u;
+            const uint32_t u = c_cand_uop[c_cand_off[m] + __umulhi(pick, nc)];
+            const uint16_t v = (uint16_t)pca_alu(UOP_OP(u), R[UOP_A(u)][lane], R[UOP_B(u)][lane],
+                                                 UOP_IMM(u));
+            last = UOP_RD(u);
+            m |= 1u << (last - 1);
+            R[last][lane] = v;   /* each lane reads only its own test */
+        }
+        const uint32_t v0 = c_vcr_off[m * 8 + last], nv = c_vcr_off[m * 8 + last + 1] - v0;
+        for (uint32_t b = 0; b < nv; b += 32) {
+            const uint32_t mine = b + lane < nv ? c_vcr_uop[v0 + b + lane] : 0u;
+            const uint32_t n = min(32u, nv - b);
+            for (uint32_t k = 0; k < n; k++) {
+                const uint32_t u = __shfl_sync(0xFFFFFFFFu, mine, k);
+                const uint32_t v = pca_alu(UOP_OP(u), R[UOP_A(u)][lane], R[UOP_B(u)][lane],
+                                           UOP_IMM(u));
+                const uint32_t pass = __ballot_sync(0xFFFFFFFFu, v == target);
+                if (pass && np < kSetupPairs) {
+                    if (lane == 0) pairs[np] = pass;
+                    np++;
+                }
+            }
+        }
+    }
+    __syncwarp();
+    uint32_t used = 0, need = 0;   /* chosen tests; those since the last start */
+    for (uint32_t r = 0; r < 4 && r < T; r++) {
+        uint32_t c = 0, any = 0;
+        for (uint32_t k = 0; k < np; k++) {
+            const uint32_t p = pairs[k];
+            if ((p & need) != need) continue;
+            any = 1;
+            c += p >> lane & 1u;
+        }
+        if (threadIdx.x == 0) alive = 0;
+        __syncthreads();
+        if (c) atomicAdd(&cnt[lane], c);
+        if (any && lane == 0) alive = 1;
+        __syncthreads();
+        if (!alive && need) {
+            /* every pair ruled out: start over (cnt is all zero) */
+            need = 0;
+            r--;
+            __syncthreads();
+            continue;
+        }
+        if (w == 0) {
+            bool fresh = true;
+            for (uint32_t k = 0; k < r; k++) fresh &= root.target[order[k]] != target;
+            uint32_t key = (uint32_t)lane < T && !(used >> lane & 1u)
+                               ? (cnt[lane] * 2 + (fresh ? 0u : 1u)) * 32 + lane : ~0u;
+            key = __reduce_min_sync(0xFFFFFFFFu, key);
+            if (lane == 0) order[r] = (uint8_t)(key & 31u);
+        }
+        __syncthreads();
+        if (threadIdx.x < 32) cnt[threadIdx.x] = 0;
+        used |= 1u << order[r];
+        need |= 1u << order[r];
+        __syncthreads();
+    }
+    if (w == 0) {
+        const uint32_t rest = ~used & (T >= 32 ? ~0u : (1u << T) - 1u);
+        if (rest >> lane & 1u)
+            order[__popc(used) + __popc(rest & ((1u << lane) - 1u))] = (uint8_t)lane;
+    }
+    __syncthreads();
+    /* level 0, in the engine's test order */
+    for (uint32_t k = threadIdx.x; k < 8 * TPC; k += blockDim.x) {
+        const uint32_t r = k / TPC, t = k % TPC;
+        const uint16_t v = r && t < T ? root.regs[order[t]][r] : (uint16_t)0;
+        L0.regs[(uint64_t)i * 8 * TPC + k] = v;
+        if (t < 4) L0.probe[(uint64_t)i * 32 + r * 4 + t] = v;
+    }
+    if (w == 0) {
+        const uint32_t o = (uint32_t)lane < T ? order[lane] : 0u;
+        const bool in_t = (uint32_t)lane < T;
+        if (lane < TPC) L0.flags[(uint64_t)i * TPC + lane] = in_t ? root.flags[o] : (uint8_t)0;
+        out.target[i * 32 + lane] = in_t ? root.target[o] : 0u;
+        uint16_t *io = out.io + (uint64_t)i * 96 + lane;
+        io[0] = in_t ? root.regs[o][1] : (uint16_t)0;
+        io[32] = in_t ? root.regs[o][2] : (uint16_t)0;
+        io[64] = in_t ? root.target[o] : (uint16_t)0;
+        out.order[i * 32 + lane] = (uint8_t)o;
+        if (lane == 0) {
+            L0.live[i] = (uint8_t)live;
+            L0.task[i] = (uint16_t)i;
+            L0.parent[i] = 0;
+            L0.cidx[i] = 0;
+            L0.rdl[i] = 0;
+            L0.own[i] = 0;
+            twin[i] = 0;
+            out.T[i] = (int32_t)T;
+            if (i == 0) {
+                *out.status = 0;
+                *out.evals = 0;
+            }
+        }
+    }
+}
+
 /* ---- level expansion: insert every child into the exact table ------------ */
 
 /* One warp's shared memory in the insert kernel: its parent (16-bit columns,
