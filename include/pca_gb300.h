@@ -192,11 +192,13 @@ typedef struct {
                            from the deepest level that fits                  */
     /* Launch choices of the suffix stages; 0 = chosen by the autotuner
        from costs it measures. None changes an answer.                       */
-    int first_tests;    /* 1..3: tests a lane checks a value class on before
-                           the warp checks its survivors on every test       */
+    int first_tests;    /* 1..3: tests a lane checks a value on at the last
+                           position before the warp checks its survivors on
+                           every test (with a lane per prefix: 1, 2, or all
+                           four of the probe; with a lane per state: fixed)  */
     int suffix_chunk;   /* 1..64: first suffix instructions per work item of
                            the depth-2 and depth-3 suffix kernels, 1024: a
-                           lane per innermost middle instruction there; at
+                           lane per state there (the last two positions); at
                            depth 1 (past the root) 1 = a warp per prefix,
                            >= 32 = a lane per prefix                         */
     int stage_launch;   /* first-only solves of one task: -1 = one launch per
@@ -412,7 +414,7 @@ void *pcagb_engine_stream(pcagb_engine_t *e);
  * level build, and for each suffix depth s the cost of each launch choice
  * (first_tests 1..3 at [s][1..3], work-item shape c at [s][c]: for s >= 2
  * chunk_choices[s][c] first instructions per work item, 1024 meaning a lane
- * per innermost middle, for s = 1 the prefixes a warp scans at once, 1 or
+ * per state, for s = 1 the prefixes a warp scans at once, 1 or
  * 32) with the number of stages it was measured on; the host round trip of
  * a chunked launch. */
 typedef struct {

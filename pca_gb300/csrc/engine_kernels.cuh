@@ -1496,144 +1496,6 @@ k_suffix(LevelDev P, TaskDev task, SolBuf S, uint32_t chunks_per_prefix, uint32_
     flush_evals(S, nev, lane);
 }
 
-/* The last position (suffix depth 1) with a lane per prefix: a warp takes
- * 32 prefixes of range R at once, each lane the operand pairs of its own
- * prefix that read the prefix's last write (the read rule, as scan_last),
- * every op of a pair evaluated on the first FT tests at once. A lane holds
- * nothing but its prefix's first FT test values of r0..r7 (in shared
- * memory, [test][register][lane], so lanes reading different registers hit
- * different banks) instead of the whole state: per prefix 7 sectors of the
- * level instead of seven 64-byte columns, and the warp's instructions are
- * not repeated for every prefix. A pair that passes the first FT tests is
- * checked on every test by the whole warp (lane = test) straight from the
- * level and recorded as the warp-per-prefix kernel records it, so the
- * records are the same. Every prefix of a level past the root has a last
- * write (no candidate of the branchless set writes r0); root prefixes
- * (w0 = 0) are left to k_suffix. */
-template <int TPC, int FT>
-__global__ void __launch_bounds__(kThreads, 5)
-k_suffix_lanes(LevelDev P, TaskDev task, SolBuf S, PrefixRange R, LeanDev lean)
-{
-    __shared__ uint32_t sV[kWarpsPerBlock][FT][8][32];
-    const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
-    uint32_t (&V)[FT][8][32] = sV[wib];
-#pragma unroll
-    for (int t = 0; t < FT; t++) V[t][0][lane] = 0;
-    const uint64_t nw = (uint64_t)gridDim.x * kWarpsPerBlock;
-    uint32_t nev = 0;   /* this lane's prefixes' readable classes (the evaluation count) */
-    for (uint64_t base = ((uint64_t)blockIdx.x * kWarpsPerBlock + wib) * 32; base < R.count;
-         base += nw * 32) {
-        const uint64_t i = base + lane;
-        uint64_t q = ~0ull;
-        if (i < R.count) {
-            q = R.order ? (uint64_t)R.order[R.begin + i] : R.begin + i;
-            if (q >= P.n) q = ~0ull;   /* orders are checked on the host; never index outside */
-        }
-        uint32_t tid = 0, live = 0, w0 = 0, p0 = 0, np = 0, T = 0;
-        uint32_t t0 = 0, t1 = 0, t2 = 0;
-        if (q != ~0ull) {
-            tid = P.task[q];
-            live = P.live[q];
-            w0 = P.rdl[q];
-            if (task.active[tid] && w0) {
-                const uint32_t m = (live >> 1) & 127u;
-                p0 = c_pr_off_g[m * 8 + w0];
-                np = c_pr_off_g[m * 8 + w0 + 1] - p0;
-                nev += __ldg(c_ev_sd1 + m * 8 + w0);
-                T = (uint32_t)task.T[tid];
-                t0 = task.target[tid * 32];
-                if (FT >= 2) t1 = task.target[tid * 32 + 1];
-                if (FT >= 3) t2 = task.target[tid * 32 + 2];
-            }
-        }
-        __syncwarp();
-        if (np) {
-            /* the prefix's probe: registers 2h and 2h+1 on tests 0..3 in
-               16-byte piece h */
-            const uint4 *pp = reinterpret_cast<const uint4 *>(P.probe + q * 32);
-#pragma unroll
-            for (int h = 0; h < 4; h++) {
-                const uint4 w = pp[h];
-                const uint32_t lo[2] = {w.x, w.z}, hi[2] = {w.y, w.w};
-#pragma unroll
-                for (int k = 0; k < 2; k++) {
-                    const int r = 2 * h + k;
-                    if (r == 0) continue;
-                    V[0][r][lane] = lo[k] & 0xFFFFu;
-                    if (FT >= 2) V[FT >= 2 ? 1 : 0][r][lane] = lo[k] >> 16;
-                    if (FT >= 3) V[FT >= 3 ? 2 : 0][r][lane] = hi[k] & 0xFFFFu;
-                }
-            }
-        }
-        __syncwarp();
-        uint32_t jn = np;
-#pragma unroll
-        for (int o = 16; o; o >>= 1) jn = max(jn, __shfl_xor_sync(0xFFFFFFFFu, jn, o));
-        for (uint32_t j = 0; j < jn; j++) {
-            uint32_t hits = 0;
-            if (j < np) {
-                const uint32_t d = c_pr[p0 + j];
-                const uint32_t a = d & 7u, b = (d >> 3) & 7u;
-                const uint32_t e = (uint32_t)(uint16_t)(int16_t)(int8_t)(uint8_t)(d >> 16);
-                hits = pair_hits(V[0][a][lane], V[0][b][lane], e, t0) & (d >> 6) & 0x3FFu;
-                if (FT >= 2 && T >= 2 && hits)
-                    hits &= pair_hits(V[FT >= 2 ? 1 : 0][a][lane], V[FT >= 2 ? 1 : 0][b][lane], e, t1);
-                if (FT >= 3 && T >= 3 && hits)
-                    hits &= pair_hits(V[FT >= 3 ? 2 : 0][a][lane], V[FT >= 3 ? 2 : 0][b][lane], e, t2);
-            }
-            uint32_t bal = __ballot_sync(0xFFFFFFFFu, hits != 0);
-            while (bal) {
-                const int L = __ffs(bal) - 1;
-                bal &= bal - 1;
-                uint32_t hj = __shfl_sync(0xFFFFFFFFu, hits, L);
-                const unsigned long long qL = __shfl_sync(0xFFFFFFFFu, (unsigned long long)q, L);
-                const uint32_t tidL = __shfl_sync(0xFFFFFFFFu, tid, L);
-                const uint32_t liveL = __shfl_sync(0xFFFFFFFFu, live, L);
-                const uint32_t pj = __shfl_sync(0xFFFFFFFFu, p0, L) + j;
-                const uint32_t d = c_pr[pj];
-                const uint32_t a = d & 7u, b = (d >> 3) & 7u;
-                const uint32_t e = (uint32_t)(uint16_t)(int16_t)(int8_t)(uint8_t)(d >> 16);
-                const int TL = task.T[tidL];
-                const uint32_t tgt = lane < TL ? task.target[tidL * 32 + lane] : 0u;
-                uint32_t x = 0, y = 0;
-                if (!lean.up_regs) {
-                    if (lane < TL) {
-                        x = P.regs[(qL * 8 + a) * TPC + lane];
-                        y = P.regs[(qL * 8 + b) * TPC + lane];
-                    }
-                } else {
-                    /* a lean level: the prefix's registers are its parent's
-                       but for the one its last instruction wrote */
-                    const uint64_t pL = P.parent[qL];
-                    const uint32_t uL = c_cand_uop[c_cand_off[(lean.up_live[pL] >> 1) & 127u] +
-                                                   lean.cidx[qL]];
-                    const uint32_t rdL = UOP_RD(uL);
-                    if (lane < TL) {
-                        const uint16_t *up = lean.up_regs + pL * 8 * TPC + lane;
-                        const uint32_t w = pca_alu(UOP_OP(uL), up[UOP_A(uL) * TPC],
-                                                   up[UOP_B(uL) * TPC], UOP_IMM(uL)) & 0xFFFFu;
-                        x = a == rdL ? w : up[a * TPC];
-                        y = b == rdL ? w : up[b * TPC];
-                    }
-                }
-                while (hj) {
-                    const uint32_t k = (uint32_t)(__ffs(hj) - 1);
-                    hj &= hj - 1;
-                    bool ok = true;
-                    if (lane < TL)
-                        ok = (k == 9 ? ((x + e) & 0xFFFFu) : pca_alu(pair_op(k), x, y, 0)) == tgt;
-                    if (__all_sync(0xFFFFFFFFu, ok) && lane == 0) {
-                        const uint32_t cj = c_pr_cls[(uint64_t)pj * 10 + k];
-                        record_solution(S, qL, 0, 0, cj, (liveL >> 1) & 127u);
-                    }
-                }
-            }
-        }
-    }
-    /* the stage's evaluation count (k_count_evals' sum for these prefixes) */
-    flush_evals(S, nev, lane);
-}
-
 }  // namespace pcagb
 
 #include "suffix_forms.cuh"

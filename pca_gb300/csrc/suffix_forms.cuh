@@ -1,6 +1,7 @@
 /*
  * suffix_forms.cuh -- the suffix kernels over value forms (included by
- * engine_kernels.cuh): the last two positions, a lane per state.
+ * engine_kernels.cuh): the last position, a lane per prefix, and the last two, a
+ * lane per state.
  */
 #pragma once
 
@@ -46,6 +47,117 @@ __device__ __forceinline__ void record_last(const SolBuf &S, uint32_t m, uint32_
         const uint32_t c = c_pr_cls[(uint64_t)pair_index(m, v, ab, k, f - kFAddi) * 10 + k];
         record_solution(S, q, m1, m2, c, m);
     }
+}
+
+/* ---- suffix depth 1 --------------------------------------------------------- */
+
+/* The last position, a lane per prefix. The last instruction reads the
+ * prefix's last write v; the other operand is one of the prefix's other
+ * live registers or v itself. A lane holds its prefix's 64-byte probe
+ * (r0..r7 on the first four tests) in registers and evaluates the thirteen
+ * forms of (v, x) for each live x, and the twelve of v, two tests to a word:
+ * on the first test (FT = 1), on the first two (2), or on all four (3).
+ * What is left is checked on every test by the warp (lane = test), from the
+ * level's columns or, on a lean level, from the parent's columns and the
+ * prefix's last instruction.
+ *
+ * Bound: integer issue (59% active), about 700 warp instructions for 32
+ * prefixes, and 75 bytes of HBM a prefix. 5.3M prefixes of is_power2: 0.52 ms
+ * walking the generator's operand pairs from memory (2,000 instructions, the
+ * operands looked up in shared memory), 0.21-0.28 ms by forms, 0.15 ms where
+ * the targets are less alike (popcount); reading the prefixes takes 0.06. */
+template <int TPC, int FT>
+__global__ void __launch_bounds__(kThreads, 4)
+k_suffix_lanes(LevelDev P, TaskDev task, SolBuf S, PrefixRange R, LeanDev lean)
+{
+    const int lane = threadIdx.x & 31;
+    const uint64_t nt = (uint64_t)gridDim.x * kThreads;
+    const uint64_t n_round = (R.count + 31) & ~31ull;
+    uint32_t nev = 0;   /* this lane's prefixes' readable classes (the evaluation count) */
+    for (uint64_t i = (uint64_t)blockIdx.x * kThreads + threadIdx.x; i < n_round; i += nt) {
+        uint64_t q = ~0ull;
+        if (i < R.count) {
+            q = R.order ? (uint64_t)R.order[R.begin + i] : R.begin + i;
+            if (q >= P.n) q = ~0ull;   /* orders are checked on the host; never index outside */
+        }
+        uint32_t tid = 0, live = 0, w0 = 0, T = 0, t01 = 0, t23 = 0;
+        uint4 pr[4] = {};
+        if (q != ~0ull) {
+            tid = P.task[q];
+            live = P.live[q];
+            w0 = P.rdl[q];
+            const uint4 *pp = reinterpret_cast<const uint4 *>(P.probe + q * 32);
+#pragma unroll
+            for (int h = 0; h < 4; h++) pr[h] = pp[h];
+            if (task.active[tid] && w0) {
+                T = (uint32_t)task.T[tid];
+                nev += __ldg(c_ev_sd1 + ((live >> 1) & 127u) * 8 + w0);
+                const uint4 tt = *reinterpret_cast<const uint4 *>(task.target + tid * 32);
+                t01 = FT >= 2 && T >= 2 ? tt.x | tt.y << 16 : tt.x * 0x10001u;
+                t23 = tt.z | (T >= 4 ? tt.w : tt.z) << 16;
+            } else {
+                w0 = 0;
+            }
+        }
+        /* register r's words (two tests each); a lone test fills both halves */
+        auto word = [&](uint32_t r, int p) -> uint32_t {
+            const uint4 w = r < 2 ? pr[0] : r < 4 ? pr[1] : r < 6 ? pr[2] : pr[3];
+            const uint32_t u = p ? (r & 1 ? w.w : w.y) : (r & 1 ? w.z : w.x);
+            const bool lone = p ? T < 4 : FT == 1 || T < 2;
+            return lone ? __byte_perm(u, 0, 0x1010) : u;
+        };
+        const uint32_t v01 = word(w0, 0), v23 = FT >= 3 ? word(w0, 1) : 0u;
+        /* x = 1..7: another live register; 8: v alone */
+#pragma unroll 1
+        for (uint32_t x = 1; x <= 8; x++) {
+            const bool self = x == 8;
+            const bool on = w0 && (self || (((live >> x) & 1u) && x != w0));
+            if (!__any_sync(0xFFFFFFFFu, on)) continue;
+            uint32_t hits = 0;
+            if (on) {
+                hits = self ? self_mask2(v01, t01) : pair_mask2(v01, word(x, 0), t01);
+                if (FT >= 3 && T >= 3 && hits)
+                    hits &= self ? self_mask2(v23, t23) : pair_mask2(v23, word(x, 1), t23);
+            }
+            uint32_t bal = __ballot_sync(0xFFFFFFFFu, hits != 0);
+            while (bal) {
+                const int L = __ffs(bal) - 1;
+                bal &= bal - 1;
+                const unsigned long long qL = __shfl_sync(0xFFFFFFFFu, (unsigned long long)q, L);
+                const uint32_t tidL = __shfl_sync(0xFFFFFFFFu, tid, L);
+                const uint32_t liveL = __shfl_sync(0xFFFFFFFFu, live, L);
+                const uint32_t wL = __shfl_sync(0xFFFFFFFFu, w0, L);
+                const uint32_t hL = __shfl_sync(0xFFFFFFFFu, hits, L);
+                const int TL = task.T[tidL];
+                uint32_t ok = ~0u;
+                if (lane < TL) {
+                    uint32_t a, b;
+                    const uint32_t xr = self ? wL : (uint32_t)x;
+                    if (!lean.up_regs) {
+                        a = P.regs[(qL * 8 + wL) * TPC + lane];
+                        b = P.regs[(qL * 8 + xr) * TPC + lane];
+                    } else {
+                        /* a lean level: the prefix's registers are its
+                           parent's but for the one its last instruction wrote */
+                        const uint64_t pL = P.parent[qL];
+                        const uint32_t uL = c_cand_uop[c_cand_off[(lean.up_live[pL] >> 1) & 127u] +
+                                                       lean.cidx[qL]];
+                        const uint16_t *up = lean.up_regs + pL * 8 * TPC + lane;
+                        a = pca_alu(UOP_OP(uL), up[UOP_A(uL) * TPC], up[UOP_B(uL) * TPC],
+                                    UOP_IMM(uL)) & 0xFFFFu;
+                        b = up[xr * TPC];
+                    }
+                    const uint32_t tg = task.target[tidL * 32 + lane];
+                    ok = self ? self_mask(a, tg) : pair_mask(a, b, tg);
+                }
+                const uint32_t forms = __reduce_and_sync(0xFFFFFFFFu, ok) & hL;
+                if (forms >> lane & 1u)   /* a form a lane */
+                    record_last(S, (liveL >> 1) & 127u, wL, (uint32_t)x, self, 1u << lane, qL, 0, 0);
+            }
+        }
+    }
+    /* the stage's evaluation count (k_count_evals' sum for these prefixes) */
+    flush_evals(S, nev, lane);
 }
 
 /* One warp's shared memory in k_suffix_states, a column per lane: the
@@ -100,7 +212,11 @@ __device__ __forceinline__ LastKeys load_keys(const uint32_t (&K)[14][32], int l
  * Work items are 32 states and one of 2^slices_log2 shares of their
  * (x, group) pairs, so small levels fill the GPU too.
  *
- * Bound: integer issue. */
+ * Bound: integer issue, the ALU pipe first (72% of it at 59% issue). 5.3M
+ * prefixes, suffix depth 2, every middle and last instruction: 376 ms with a
+ * lane per middle that evaluates the operand pairs, 3.4 ms here (popcount;
+ * is_power2, whose values pass more tests, 425 and 5.3); depth 3 from 100K
+ * two-input states' parents 3.3 -> 0.2 ms. */
 template <int TPC, int SD>
 __global__ void __launch_bounds__(kStatesWarps * 32, 8)
 k_suffix_states(LevelDev P, TaskDev task, SolBuf S, uint32_t per_prefix, uint32_t slices_log2,

@@ -268,6 +268,23 @@ PCA_HD uint32_t form_value2(uint32_t kind, uint32_t f, uint32_t x, uint32_t y)
                                : ldi_imm(f) * 0x10001u;
 }
 
+/* which forms give t on both tests */
+PCA_HD uint32_t pair_mask2(uint32_t v, uint32_t x, uint32_t t)
+{
+    uint32_t h = 0;
+    PCA_UNROLL
+    for (uint32_t f = 0; f < kPairForms; f++) h |= (uint32_t)(pair_value2(f, v, x) == t) << f;
+    return h;
+}
+
+PCA_HD uint32_t self_mask2(uint32_t v, uint32_t t)
+{
+    uint32_t h = 0;
+    PCA_UNROLL
+    for (uint32_t f = 0; f < kSelfForms; f++) h |= (uint32_t)(self_value2(f, v) == t) << f;
+    return h;
+}
+
 /* The v for which some form of (v, x) gives t, on two tests at once: v equals
    add, sub, rsub or xr; v & x == t; v | x == t; (v & mulm) == mulc;
    (v & shlm) == shlc (v << x); (v & shrm) == shrc (v >> x of either kind, so

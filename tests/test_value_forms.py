@@ -35,6 +35,9 @@ static int keys(uint32_t v, uint32_t x, uint32_t t, uint32_t w, uint32_t y, uint
     for (uint32_t f = 0; f < kSelfForms; f++)
         if (self_value2(f, V) != (self_value(f, v) | self_value(f, w) << 16))
             return fail("self_value2", f, V, 0, 0);
+    if (pair_mask2(V, X, G) != (pair_mask(v, x, t) & pair_mask(w, y, s)) ||
+        self_mask2(V, G) != (self_mask(v, t) & self_mask(w, s)))
+        return fail("mask2", V, X, G, 0);
     /* every form that solves both tests is matched */
     if ((pair_mask(v, x, t) & pair_mask(w, y, s)) && !last_any(V, last_keys(X, G)))
         return fail("pair", V, X, G, 0);
