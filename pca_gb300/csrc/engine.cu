@@ -915,8 +915,15 @@ int run_stage(pcagb_engine *e, int S, int K, std::vector<TaskRun> &runs, bool fi
     uint64_t taken = 0;  /* records already turned into solutions */
     bool grouped = false;
     if (s == 0) {
-        if (t16) k_leaf<16><<<e->grid(4), 256, 0, e->stream>>>(view(L), e->td, sb);
-        else k_leaf<32><<<e->grid(4), 256, 0, e->stream>>>(view(L), e->td, sb);
+        /* at depth 1 every live register: the root's may hold the target
+           when its own check was skipped (min_depth) */
+        if (K == 1) {
+            if (t16) k_leaf<16><<<e->grid(4), 256, 0, e->stream>>>(view(L), e->td, sb);
+            else k_leaf<32><<<e->grid(4), 256, 0, e->stream>>>(view(L), e->td, sb);
+        } else {
+            if (t16) k_leaf_last<16><<<e->grid(8), kThreads, 0, e->stream>>>(view(L), e->td, sb);
+            else k_leaf_last<32><<<e->grid(8), kThreads, 0, e->stream>>>(view(L), e->td, sb);
+        }
         rc = check_launch(e);
         if (rc) return rc;
     } else if (s <= 3) {
@@ -1864,6 +1871,7 @@ int engine_init(pcagb_engine *e, int device, size_t budget)
         PCAGB_PRELOAD(k_materialize<16>); PCAGB_PRELOAD(k_materialize<32>);
         PCAGB_PRELOAD(k_twins<16>); PCAGB_PRELOAD(k_twins<32>);
         PCAGB_PRELOAD(k_leaf<16>); PCAGB_PRELOAD(k_leaf<32>);
+        PCAGB_PRELOAD(k_leaf_last<16>); PCAGB_PRELOAD(k_leaf_last<32>);
         PCAGB_PRELOAD(k_count_evals); PCAGB_PRELOAD(k_mark); PCAGB_PRELOAD(k_mark_all);
         PCAGB_PRELOAD(k_popc); PCAGB_PRELOAD(k_child_counts); PCAGB_PRELOAD(k_task_hist);
         PCAGB_PRELOAD(k_task_hist_smem); PCAGB_PRELOAD(k_scan_local); PCAGB_PRELOAD(k_scan_add);
@@ -2166,6 +2174,11 @@ thread_local uint64_t t_last_explored = 0;
    and device but keeps its own levels. */
 cudaStream_t pcagb_internal_stream(pcagb_engine_t *e) { return e->stream; }
 int pcagb_internal_device(pcagb_engine_t *e) { return e->device; }
+void pcagb_internal_arena(pcagb_engine_t *e, char **base, size_t *bytes)
+{
+    *base = e->arena;
+    *bytes = e->arena ? e->cap : 0;
+}
 
 extern "C" {
 

@@ -863,13 +863,15 @@ __global__ void k_child_counts(const uint8_t *live, const uint16_t *task, const 
 template <int TPC>
 struct MatState {
     __align__(16) uint16_t PR[8 * TPC];
-    __align__(16) uint16_t CB[TPC];
-    __align__(16) uint8_t FB[TPC];
+    __align__(16) uint16_t CB[32];   /* 32 / TPC children at a time */
+    __align__(16) uint8_t FB[32];
 };
 
-/* Write the marked children of each parent, in rank (DFS) order. A child's
-   register block (8 x TPC halves) is written as TPC 16-byte pieces, one per
-   lane, and its flags as TPC/16 pieces: lane t first computes the new value
+/* Write the marked children of each parent, in rank (DFS) order, by TPC lanes
+   each (with 16 tests two children at a time: level 3 of an 11-test search,
+   5.3M states, 0.62 -> 0.48 ms). A child's register block (8 x TPC halves) is
+   written as TPC 16-byte pieces, one per lane, and its flags as TPC/16
+   pieces: lane t first computes the new value
    and flags of test t into shared memory, then lane L copies piece L from
    the parent's block, or from the new column when the piece lies in the
    written register's column. Level blocks start on 256-byte boundaries (the
@@ -881,15 +883,16 @@ k_materialize(LevelDev P, TaskDev task, const uint32_t *bitmap, const uint64_t *
               LevelOut C, uint32_t split_log2, uint32_t *fcr, const uint32_t *fcr_up)
 {
     static_assert(TPC == 16 || TPC == 32, "a state holds 16 or 32 tests");
-    constexpr int kPieces = 8 * TPC * 2 / 16;   /* = TPC: lanes 0..TPC-1 */
+    constexpr int kPieces = 8 * TPC * 2 / 16;   /* = TPC: a piece a lane of the group */
     constexpr int kFlagPieces = TPC / 16;
     constexpr int kPiecesPerCol = TPC / 8;
     __shared__ MatState<TPC> sms[kWarpsPerBlock];
     const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
+    const int t = lane % TPC, grp = lane / TPC;   /* test (and piece), child of the pair */
     MatState<TPC> &ms = sms[wib];
-    const uint32_t my_col = (uint32_t)lane / kPiecesPerCol;   /* column of piece `lane` */
-    const uint4 *my_new = reinterpret_cast<const uint4 *>(ms.CB) + lane % kPiecesPerCol;
-    const uint4 *my_old = reinterpret_cast<const uint4 *>(ms.PR) + lane;
+    const uint32_t my_col = (uint32_t)t / kPiecesPerCol;   /* column of piece t */
+    const uint4 *my_new = reinterpret_cast<const uint4 *>(ms.CB + grp * TPC) + t % kPiecesPerCol;
+    const uint4 *my_old = reinterpret_cast<const uint4 *>(ms.PR) + t;
     const uint64_t nw = (uint64_t)gridDim.x * kWarpsPerBlock;
     const uint32_t split = 1u << split_log2;
     /* work items as in k_expand_insert: a parent, or a slice of its
@@ -905,7 +908,7 @@ k_materialize(LevelDev P, TaskDev task, const uint32_t *bitmap, const uint64_t *
         if (lane < kPieces)
             reinterpret_cast<uint4 *>(ms.PR)[lane] =
                 reinterpret_cast<const uint4 *>(P.regs + q * 8 * TPC)[lane];
-        const uint32_t pf = lane < TPC ? P.flags[q * TPC + lane] : 0u;
+        const uint32_t pf = P.flags[q * TPC + t];
         const uint32_t live = P.live[q];
         __syncwarp();
         const uint32_t m = (live >> 1) & 127u;
@@ -945,32 +948,38 @@ k_materialize(LevelDev P, TaskDev task, const uint32_t *bitmap, const uint64_t *
             }
             uint32_t bal = __ballot_sync(0xFFFFFFFFu, keep);
             while (bal) {
-                const int j = __ffs(bal) - 1;
+                /* this lane group's child: the first set bit, or the second */
+                uint32_t mine = bal;
                 bal &= bal - 1;
-                const uint64_t rk = __shfl_sync(0xFFFFFFFFu, rank, j);
-                const uint32_t uj = __shfl_sync(0xFFFFFFFFu, u, j);
+                if (TPC == 16) {
+                    mine = grp ? bal : mine;
+                    bal &= bal - 1;
+                }
+                const int j = __ffs((int)mine) - 1;
+                const uint64_t rk = __shfl_sync(0xFFFFFFFFu, rank, j < 0 ? 0 : j);
+                const uint32_t uj = __shfl_sync(0xFFFFFFFFu, u, j < 0 ? 0 : j);
                 const uint32_t op = UOP_OP(uj), rd = UOP_RD(uj);
-                if (lane < TPC) {
-                    const uint32_t a = ms.PR[UOP_A(uj) * TPC + lane];
-                    const uint32_t b = ms.PR[UOP_B(uj) * TPC + lane];
+                {
+                    const uint32_t a = ms.PR[UOP_A(uj) * TPC + t];
+                    const uint32_t b = ms.PR[UOP_B(uj) * TPC + t];
                     uint32_t res = pca_alu(op, a, b, UOP_IMM(uj));
                     uint32_t f = pca_alu_flags(op, a, b, UOP_IMM(uj), res, pf);
-                    if (lane >= T) { res = 0; f = 0; }
+                    if (t >= T) { res = 0; f = 0; }
                     ms.CB[lane] = (uint16_t)res;
                     ms.FB[lane] = (uint8_t)f;
                 }
                 __syncwarp();
-                if (lane < kPieces) {
+                if (j >= 0) {
                     const uint4 pv = *(my_col == rd ? my_new : my_old);
-                    reinterpret_cast<uint4 *>(C.regs + rk * 8 * TPC)[lane] = pv;
+                    reinterpret_cast<uint4 *>(C.regs + rk * 8 * TPC)[t] = pv;
                     /* the lane holding tests 0..7 of a column also writes
                        tests 0..3 of it into the probe (8 lanes, 64 bytes) */
-                    if (lane % kPiecesPerCol == 0)
+                    if (t % kPiecesPerCol == 0)
                         reinterpret_cast<uint2 *>(C.probe + rk * 32)[my_col] = make_uint2(pv.x, pv.y);
+                    if (t < kFlagPieces)
+                        reinterpret_cast<uint4 *>(C.flags + rk * TPC)[t] =
+                            reinterpret_cast<const uint4 *>(ms.FB + grp * TPC)[t];
                 }
-                if (lane < kFlagPieces)
-                    reinterpret_cast<uint4 *>(C.flags + rk * TPC)[lane] =
-                        reinterpret_cast<const uint4 *>(ms.FB)[lane];
                 __syncwarp();
             }
         }
@@ -1167,6 +1176,47 @@ __global__ void k_leaf(LevelDev P, TaskDev task, SolBuf S)
             if (!((live >> r) & 1u)) continue;
             bool ok = lane >= T || P.regs[q * 8 * TPC + r * TPC + lane] == tgt;
             if (__all_sync(0xFFFFFFFFu, ok) && lane == 0) record(S, q, 0, 0, r, r, 1);
+        }
+    }
+}
+
+/* The leaf check past depth 1. At depth K - 1 no state held the target in a
+ * live register (its leaf check found nothing), so a state of level K can
+ * hold it only in the register its last instruction wrote. A lane per state
+ * compares that register's four probe tests (8 of the probe's 64 bytes); a
+ * state that passes is checked on every test by the warp.
+ *
+ * Bound: HBM latency and bandwidth, 45 bytes a state (a 32-byte sector of the
+ * probe, task, rdl). A warp per state reading all live columns took 1.97 ms
+ * for 5.3M states of 11 tests; this 0.06 ms. */
+template <int TPC>
+__global__ void __launch_bounds__(kThreads)
+k_leaf_last(LevelDev P, TaskDev task, SolBuf S)
+{
+    const int lane = threadIdx.x & 31;
+    const uint64_t n_round = (P.n + 31) & ~31ull;
+    for (uint64_t q = (uint64_t)blockIdx.x * kThreads + threadIdx.x; q < n_round;
+         q += (uint64_t)gridDim.x * kThreads) {
+        uint32_t tid = 0, r = 0;
+        bool pass = false;
+        if (q < P.n) {
+            tid = P.task[q];
+            r = P.rdl[q];
+            const uint2 v = *reinterpret_cast<const uint2 *>(P.probe + q * 32 + r * 4);
+            const uint4 t = *reinterpret_cast<const uint4 *>(task.target + tid * 32);
+            /* tests past the task's are zero in both */
+            pass = task.active[tid] && r && v.x == (t.x | t.y << 16) && v.y == (t.z | t.w << 16);
+        }
+        uint32_t bal = __ballot_sync(0xFFFFFFFFu, pass);
+        while (bal) {
+            const int j = __ffs((int)bal) - 1;
+            bal &= bal - 1;
+            const unsigned long long qj = __shfl_sync(0xFFFFFFFFu, (unsigned long long)q, j);
+            const uint32_t tj = __shfl_sync(0xFFFFFFFFu, tid, j);
+            const uint32_t rj = __shfl_sync(0xFFFFFFFFu, r, j);
+            const bool ok = lane >= task.T[tj] ||
+                            P.regs[(qj * 8 + rj) * TPC + lane] == task.target[tj * 32 + lane];
+            if (__all_sync(0xFFFFFFFFu, ok) && lane == 0) record(S, qj, 0, 0, rj, rj, 1);
         }
     }
 }
