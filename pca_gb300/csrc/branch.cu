@@ -170,6 +170,66 @@ __host__ __device__ __forceinline__ uint16_t bcand(const BTab &b, uint32_t m, ui
     return b.post[b.post_off[m] + (c - nbr)];
 }
 
+/* The candidate tables on a device, uploaded once and kept until the process
+   exits (400 KB). */
+struct DevTables {
+    uint32_t *pre_off = nullptr, *post_off = nullptr;
+    uint16_t *pre = nullptr, *post = nullptr;
+};
+
+int device_tables(int device, const DevTables **out)
+{
+    static std::mutex mu;
+    static DevTables tabs[64];
+    std::lock_guard<std::mutex> lk(mu);
+    if (device < 0 || device >= 64) { set_berr("device %d out of range", device); return PCAGB_EINVAL; }
+    DevTables &d = tabs[device];
+    if (!d.post) {
+        const BranchTables &bt = branch_tables();
+        DevTables n;
+        BCK(cudaMalloc(&n.pre_off, 129 * 4));
+        BCK(cudaMalloc(&n.post_off, 129 * 4));
+        BCK(cudaMalloc(&n.pre, bt.pre.size() * 2));
+        BCK(cudaMalloc(&n.post, bt.post.size() * 2));
+        BCK(cudaMemcpy(n.pre_off, bt.pre_off.data(), 129 * 4, cudaMemcpyHostToDevice));
+        BCK(cudaMemcpy(n.post_off, bt.post_off.data(), 129 * 4, cudaMemcpyHostToDevice));
+        /* bit 0 of a device word (padding in these formats) marks a candidate
+           that writes the same value and flags as an earlier one of its mask
+           on every state: the copies of x with its Z/N flags (ADD and OR and
+           XOR rd,r0,x; AND and OR rd,x,x), zero with Z (AND and the shifts
+           rd,r0,x; XOR rd,x,x), zero with Z and C (SUB rd,x,x). Its child is
+           that sibling's state by a larger index, so never kept */
+        std::vector<uint16_t> pre(bt.pre);
+        for (int m = 0; m < 128; m++) {
+            std::vector<uint32_t> seen;
+            for (uint32_t i = bt.pre_off[m]; i < bt.pre_off[m + 1]; i++) {
+                const uint32_t w = pre[i], op = w >> 11, rd = (w >> 8) & 7u;
+                const uint32_t a = (w >> 5) & 7u, b = (w >> 2) & 7u;
+                uint32_t key = 0;
+                if ((op == PCA_OP_ADD || op == PCA_OP_OR || op == PCA_OP_XOR) && a == 0 && b)
+                    key = 1u << 8 | rd << 4 | b;
+                else if ((op == PCA_OP_AND || op == PCA_OP_OR) && a == b && a)
+                    key = 1u << 8 | rd << 4 | a;
+                else if ((op == PCA_OP_AND || op == PCA_OP_SHL || op == PCA_OP_SHR ||
+                          op == PCA_OP_ASR) && a == 0 && b)
+                    key = 2u << 8 | rd << 4;
+                else if (op == PCA_OP_XOR && a == b && a)
+                    key = 2u << 8 | rd << 4;
+                else if (op == PCA_OP_SUB && a == b && a)
+                    key = 3u << 8 | rd << 4;
+                if (!key) continue;
+                if (std::find(seen.begin(), seen.end(), key) != seen.end()) pre[i] |= 1u;
+                else seen.push_back(key);
+            }
+        }
+        BCK(cudaMemcpy(n.pre, pre.data(), pre.size() * 2, cudaMemcpyHostToDevice));
+        BCK(cudaMemcpy(n.post, bt.post.data(), bt.post.size() * 2, cudaMemcpyHostToDevice));
+        d = n;
+    }
+    *out = &d;
+    return PCAGB_OK;
+}
+
 /* ---- one instruction on one test (src/vm.c:59-203) ----------------------- */
 
 __device__ __forceinline__ uint32_t zn(uint32_t v)
@@ -269,6 +329,9 @@ struct BLevel {
     uint8_t *live = nullptr;    /* [n] */
     uint32_t *parent = nullptr;
     uint16_t *cidx = nullptr;
+    uint8_t *rdl = nullptr;        /* [n] register the last instruction wrote (0: none,
+                                      or by a DIV or MOD) */
+    uint32_t *fcr = nullptr;       /* [n][8] first kept child whose rdl is r (once expanded) */
     uint64_t *child_off = nullptr; /* [n+1] */
     uint64_t children = 0;
 };
@@ -278,7 +341,24 @@ struct BDev {
     const uint8_t *flags, *skip, *live;
     const uint64_t *child_off;
     uint64_t n;
+    const uint32_t *parent;
+    const uint8_t *rdl;
+    const uint32_t *fcr_up;        /* fcr of the level above (null: the root level) */
 };
+
+/* The register a child of state q must not overwrite unread, or 0. When q's
+   last instruction z wrote w and is not the first kept sibling z1 writing it,
+   a child y that overwrites w without reading it (and sets the flags) is in
+   registers, flags and resume positions the child y of z1, which has a
+   smaller index: neither z nor z1 is a BR or can fault, so both run y on the
+   same tests, a test that runs z runs y, and one that runs neither keeps the
+   registers it had before. So it is never the kept one, and need not be
+   looked at. */
+__device__ __forceinline__ uint32_t dead_write(const BDev &P, uint64_t q)
+{
+    const uint32_t w = P.fcr_up ? P.rdl[q] : 0u;
+    return w && P.fcr_up[(uint64_t)P.parent[q] * 8 + w] < (uint32_t)q ? w : 0u;
+}
 
 __device__ __forceinline__ uint64_t bmix(uint64_t x)
 {
@@ -309,6 +389,100 @@ __device__ uint64_t child_key(const BDev &P, uint64_t q, uint32_t insn, uint32_t
         h = bmix(h ^ x) + 0x2545F4914F6CDD1Dull;
     }
     return h;
+}
+
+/* One instruction as the expansion kernels take it: operands a = R[ra],
+   b = R[rb] and the register it writes (0: none: CMP, BR, a write to r0). */
+struct BUop {
+    uint32_t op, ra, rb, wr, imm;
+};
+
+__device__ __forceinline__ BUop buop(uint32_t insn)
+{
+    BUop u;
+    u.op = insn >> 11;
+    const uint32_t rd = (insn >> 8) & 7u, rs = (insn >> 5) & 7u, rt = (insn >> 2) & 7u;
+    const bool cmp = u.op == (uint32_t)kOpCmp, addi = u.op == PCA_OP_ADDI;
+    u.ra = cmp || addi ? rd : rs;
+    u.rb = cmp ? rs : u.op == (uint32_t)kOpBr ? rd : rt;   /* a BR's condition */
+    u.wr = cmp || u.op == (uint32_t)kOpBr ? 0u : rd;
+    u.imm = insn & 0xFFu;
+    return u;
+}
+
+/* Is candidate u (word insn) of a state whose dead write is w known to give
+   an earlier child's state? */
+__device__ __forceinline__ bool never_kept(uint32_t insn, const BUop &u, uint32_t w)
+{
+    if (u.op < PCA_OP_LDI && (insn & 1u)) return true;   /* a same-state sibling */
+    return w && u.wr == w && u.op != PCA_OP_LDI && u.op != (uint32_t)kOpDiv &&
+           u.op != (uint32_t)kOpMod && u.ra != w && u.rb != w;
+}
+
+/* bexec on one test with the operands at hand: the written register's value
+   (old when the test does not run the instruction), the flags and the resume
+   position afterwards. */
+__device__ __forceinline__ uint32_t bvalue(const BUop &u, uint32_t p, uint32_t a, uint32_t b,
+                                           uint32_t old, uint32_t f0, uint32_t skip0, uint32_t *f,
+                                           uint32_t *skip)
+{
+    *f = f0;
+    *skip = skip0;
+    if (skip0 > p) return old;  /* jumped over, or stopped by a fault */
+    uint32_t v;
+    switch (u.op) {
+    case PCA_OP_ADD: v = (a + b) & 0xFFFFu; *f = f_add(a, b); break;
+    case PCA_OP_SUB: v = (a - b) & 0xFFFFu; *f = f_sub(a, b); break;
+    case PCA_OP_MUL: {
+        const uint32_t prod = a * b;
+        v = prod & 0xFFFFu;
+        *f = zn(v) | (prod > 0xFFFFu ? PCA_FC : 0u);
+        break;
+    }
+    case kOpDiv:
+    case kOpMod: {
+        if (b == 0) {
+            *skip = kFault;
+            return old;
+        }
+        const int sa = (int)(int16_t)(uint16_t)a, sb = (int)(int16_t)(uint16_t)b;
+        v = (uint32_t)(uint16_t)(u.op == (uint32_t)kOpDiv ? sa / sb : sa % sb);
+        *f = zn(v);
+        break;
+    }
+    case PCA_OP_AND: v = a & b; *f = zn(v); break;
+    case PCA_OP_OR:  v = a | b; *f = zn(v); break;
+    case PCA_OP_XOR: v = a ^ b; *f = zn(v); break;
+    case PCA_OP_SHL: v = (a << (b & 15u)) & 0xFFFFu; *f = zn(v); break;
+    case PCA_OP_SHR: v = a >> (b & 15u); *f = zn(v); break;
+    case PCA_OP_ASR: v = (uint32_t)(uint16_t)((int16_t)(uint16_t)a >> (b & 15u)); *f = zn(v); break;
+    case kOpCmp: *f = f_sub(a, b); return old;
+    case kOpBr: {
+        const uint32_t Z = f0 & PCA_FZ, N = (f0 & PCA_FN) != 0, C = f0 & PCA_FC,
+                       V = (f0 & PCA_FV) != 0;
+        bool take = false;
+        switch (u.rb) {
+        case 0: take = true; break;
+        case 1: take = Z != 0; break;
+        case 2: take = Z == 0; break;
+        case 3: take = N != V; break;
+        case 4: take = N == V; break;
+        case 5: take = C == 0; break;
+        case 6: take = C != 0; break;
+        }
+        if (take) *skip = p + 1 + (uint32_t)(int32_t)(int8_t)(uint8_t)u.imm;
+        return old;
+    }
+    case PCA_OP_LDI: v = u.imm; break;
+    case PCA_OP_ADDI: {
+        const uint32_t s = (uint32_t)(int32_t)(int8_t)(uint8_t)u.imm & 0xFFFFu;
+        *f = f_add(a, s);
+        v = (a + s) & 0xFFFFu;
+        break;
+    }
+    default: return old;
+    }
+    return v;
 }
 
 /* Two children equal in registers and flags on every test (warp-wide: lane = test). */
@@ -346,34 +520,161 @@ __global__ void k_bchild_counts(BDev P, BTab tab, uint64_t *cnt)
 constexpr uint64_t kBRefMask = (1ull << 40) - 1;
 constexpr uint32_t kBMaxProbes = 1u << 16;
 
-/* One warp per parent, one lane per candidate (32 at a time): BR children
-   are kept (their bit set at once), the others go through the exact table. */
+/* ---- hashing: a chain over four tests a word, mixed per column ------------- */
+
+__device__ __forceinline__ uint64_t bchain(uint64_t h, uint64_t w)
+{
+    h = (h ^ w) * 0x9E3779B97F4A7C15ull;
+    return (h << 27) | (h >> 37);
+}
+
+__device__ __forceinline__ uint64_t bcol(uint32_t r, uint64_t h)
+{
+    return bmix(h + (uint64_t)r * 0xD6E8FEB86659FD93ull);
+}
+
+/* One warp's shared memory in k_bexpand: its parent (a row stride of TP + 2
+   halves, so that lanes reading different columns of one test hit different
+   banks), its columns' hashes, and each lane's child: the written column and
+   the flags, which the compares read. */
+template <int TP>
+struct BWarp {
+    uint64_t colh[8];
+    uint64_t flagsA[TP / 16][32];   /* 4 bits a test */
+    uint16_t R[8][TP + 2];
+    uint16_t colA[TP][33];
+    uint8_t F[TP], S[TP];
+};
+
+/* Children A (lane j's, of the warp's parent qa) and B (parent qb, candidate
+   ub) equal in registers and flags on every test: lane = test. */
+template <int TP>
+__device__ bool bchild_same(const BDev &P, const BWarp<TP> &A, uint32_t wa, int j, uint64_t qa,
+                            uint64_t qb, const BUop &ub, uint32_t p, int T, int lane)
+{
+    bool ok = true;
+    if (lane < T) {
+        const uint32_t va = A.colA[lane][j];
+        const uint32_t fa = (uint32_t)(A.flagsA[lane >> 4][j] >> (4 * (lane & 15))) & 15u;
+        uint32_t B[8], f0, s0;
+        if (qb == qa) {
+#pragma unroll
+            for (int r = 0; r < 8; r++) B[r] = A.R[r][lane];
+            f0 = A.F[lane];
+            s0 = A.S[lane];
+        } else {
+            const uint16_t *col = P.regs + qb * 8 * TP + lane;
+#pragma unroll
+            for (int r = 0; r < 8; r++) B[r] = col[r * TP];
+            f0 = P.flags[qb * TP + lane];
+            s0 = P.skip[qb * TP + lane];
+        }
+        uint32_t a = 0, b = 0, old = 0, f, sk;
+#pragma unroll
+        for (uint32_t r = 0; r < 8; r++) {
+            a = r == ub.ra ? B[r] : a;
+            b = r == ub.rb ? B[r] : b;
+            old = r == ub.wr ? B[r] : old;
+        }
+        const uint32_t vb = bvalue(ub, p, a, b, old, f0, s0, &f, &sk);
+        ok = fa == f;
+#pragma unroll
+        for (uint32_t r = 1; r < 8; r++)
+            ok &= (r == wa ? va : (uint32_t)A.R[r][lane]) == (r == ub.wr ? vb : B[r]);
+    }
+    return __all_sync(0xFFFFFFFFu, ok);
+}
+
+/* One warp per parent (or one of 2^split_log2 slices of its candidates, so
+   that a level of few parents fills the GPU), one lane per candidate: BR
+   children are kept (their bit set at once), the others go through the exact
+   table. The parent sits in shared memory; a lane hashes its child from the
+   parent's column hashes, the one column it writes and its flags, and leaves
+   both in shared memory for the compares.
+
+   Bound: integer issue. Hashing every register of every test of every child
+   from global memory took 6.9 ms for relu's depth-3 last level (11 tests,
+   22.5M children, 8.2M kept); this 4.1 ms (5.9 without never_kept). */
 template <int TP>
 __global__ void __launch_bounds__(kBThreads)
 k_bexpand(BDev P, BTab tab, int T, uint32_t p, unsigned long long *table, uint64_t tmask,
-          uint32_t *bitmap, uint32_t *status)
+          uint32_t *bitmap, uint32_t *status, uint32_t split_log2)
 {
+    __shared__ BWarp<TP> sw[kWarps];
     const int lane = threadIdx.x & 31;
+    BWarp<TP> &W = sw[threadIdx.x >> 5];
     const uint64_t nw = (uint64_t)gridDim.x * kWarps;
-    for (uint64_t q = ((uint64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5; q < P.n; q += nw) {
+    const uint32_t split = 1u << split_log2;
+    for (uint64_t it = ((uint64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+         it < P.n << split_log2; it += nw) {
+        const uint64_t q = it >> split_log2;
         const uint32_t m = (P.live[q] >> 1) & 127u;
         const uint32_t nc = bcount(tab, m);
-        for (uint32_t c0 = 0; c0 < nc; c0 += 32) {
+        const uint64_t off = P.child_off[q];
+        __syncwarp();
+        if (lane < TP) {
+#pragma unroll
+            for (int r = 0; r < 8; r++) W.R[r][lane] = P.regs[(q * 8 + r) * TP + lane];
+            W.F[lane] = P.flags[q * TP + lane];
+            W.S[lane] = P.skip[q * TP + lane];
+        }
+        __syncwarp();
+        if (lane >= 1 && lane < 8) {
+            uint64_t h = 0x243F6A8885A308D3ull;
+            for (int t = 0; t < T; t += 4)
+                h = bchain(h, (uint64_t)W.R[lane][t] | (uint64_t)W.R[lane][t + 1] << 16 |
+                                  (uint64_t)W.R[lane][t + 2] << 32 |
+                                  (uint64_t)W.R[lane][t + 3] << 48);
+            W.colh[lane] = bcol(lane, h);
+        }
+        if (lane == 0) W.colh[0] = 0;
+        __syncwarp();
+        uint64_t regsum = 0;
+#pragma unroll
+        for (int r = 1; r < 8; r++) regsum += W.colh[r];
+        const uint32_t dead = dead_write(P, q);
+        for (uint32_t c0 = ((uint32_t)it & (split - 1)) * 32; c0 < nc; c0 += 32 << split_log2) {
             const uint32_t c = c0 + lane;
             const bool valid = c < nc;
             const uint32_t insn = valid ? bcand(tab, m, c) : 0u;
-            const bool br = valid && (insn >> 11) == (uint32_t)kOpBr;
+            const BUop u = buop(insn);
+            const bool br = valid && u.op == (uint32_t)kOpBr;
             if (br) {
-                const uint64_t L = P.child_off[q] + c;
+                const uint64_t L = off + c;
                 atomicOr(&bitmap[L >> 5], 1u << (L & 31));
             }
-            uint64_t H = 0;
-            if (valid && !br) H = child_key<TP>(P, q, insn, p, T);
+            bool done = !valid || br || never_kept(insn, u, dead);
+            if (__all_sync(0xFFFFFFFFu, done)) continue;
+            uint64_t h = 0x243F6A8885A308D3ull, hf = 0x13198A2E03707344ull, wf = 0;
+            __syncwarp();   /* the previous compares are done with colA */
+#pragma unroll 1
+            for (int t0 = 0; t0 < T; t0 += 4) {
+                uint64_t w = 0;
+#pragma unroll
+                for (int k = 0; k < 4; k++) {
+                    const int t = t0 + k;   /* columns are zero past T */
+                    uint32_t f = 0, sk, v = 0;
+                    if (t < T)
+                        v = bvalue(u, p, W.R[u.ra][t], W.R[u.rb][t], W.R[u.wr][t], W.F[t], W.S[t],
+                                   &f, &sk);
+                    W.colA[t][lane] = (uint16_t)v;
+                    w |= (uint64_t)v << (16 * k);
+                    wf |= (uint64_t)f << (4 * (t & 15));
+                }
+                h = bchain(h, w);
+                if ((t0 & 15) == 12 || t0 + 4 >= T) {
+                    hf = bchain(hf, wf);
+                    W.flagsA[t0 >> 4][lane] = wf;
+                    wf = 0;
+                }
+            }
+            __syncwarp();
+            uint64_t H = regsum + bmix(hf);
+            if (u.wr) H += bcol(u.wr, h) - W.colh[u.wr];
             const uint64_t ref = (q << 12) | c;
             const unsigned long long mine = ((H >> 40) << 40) | (ref + 1);
             uint64_t idx = H & tmask;
             uint32_t probes = 0;
-            bool done = !valid || br;
             while (__any_sync(0xFFFFFFFFu, !done)) {
                 bool needcmp = false;
                 unsigned long long s = 0;
@@ -386,17 +687,21 @@ k_bexpand(BDev P, BTab tab, int T, uint32_t p, unsigned long long *table, uint64
                     }
                     if (!done) needcmp = (s >> 40) == (mine >> 40);
                 }
+                uint32_t insn_b = 0;
+                if (needcmp) {
+                    const uint64_t oref = (s & kBRefMask) - 1;
+                    insn_b = bcand(tab, (P.live[oref >> 12] >> 1) & 127u, (uint32_t)(oref & 4095));
+                }
                 uint32_t req = __ballot_sync(0xFFFFFFFFu, needcmp);
                 bool eq = false;
                 while (req) {
                     const int j = __ffs(req) - 1;
                     req &= req - 1;
-                    const uint32_t ij = __shfl_sync(0xFFFFFFFFu, insn, j);
+                    const uint32_t wj = __shfl_sync(0xFFFFFFFFu, u.wr, j);
+                    const uint32_t ij = __shfl_sync(0xFFFFFFFFu, insn_b, j);
                     const unsigned long long sj = __shfl_sync(0xFFFFFFFFu, s, j);
-                    const uint64_t oref = (sj & kBRefMask) - 1;
-                    const uint64_t qb = oref >> 12;
-                    const uint32_t ib = bcand(tab, (P.live[qb] >> 1) & 127u, (uint32_t)(oref & 4095));
-                    const bool e = bchild_equal<TP>(P, q, ij, qb, ib, p, T, lane);
+                    const uint64_t qb = ((sj & kBRefMask) - 1) >> 12;
+                    const bool e = bchild_same<TP>(P, W, wj, j, q, qb, buop(ij), p, T, lane);
                     if (lane == j) eq = e;
                 }
                 if (!done) {
@@ -442,46 +747,102 @@ __global__ void k_bpopc(const uint32_t *bitmap, uint64_t words, uint64_t *off)
         off[i] = __popc(bitmap[i]);
 }
 
-/* One warp per parent: its kept children, lane = test. */
+/* One warp per parent (or a slice of its candidates): the lanes settle 32
+   candidates at a time (kept?, rank, links); the kept children are then
+   written by TP lanes each (two at a time with 16 tests): lane t computes
+   test t into shared memory, and the child's registers (TP 16-byte pieces),
+   flags and resume positions go out a piece a lane, from the parent's block
+   staged in the level's layout or from the new column.
+
+   Bound: HBM writes (18 TP + 8 bytes a child) and their issue. A warp that
+   looked at the candidates one by one and wrote two bytes a lane took 2.5 ms
+   for relu's depth-3 last level (11 tests, 22.5M children, 8.2M kept); one
+   child at a time 1.46; this 0.81 ms. */
+template <int TP>
+struct BMat {
+    __align__(16) uint16_t PR[8 * TP];
+    __align__(16) uint16_t CB[32];
+    __align__(16) uint8_t FB[32], SB[32];
+};
+
 template <int TP>
 __global__ void __launch_bounds__(kBThreads)
 k_bmaterialize(BDev P, BTab tab, int T, uint32_t p, const uint32_t *bitmap,
-               const uint64_t *word_rank, BLevel C)
+               const uint64_t *word_rank, BLevel C, uint32_t *fcr, uint32_t split_log2)
 {
-    const int lane = threadIdx.x & 31;
+    constexpr int kPerCol = TP / 8;   /* 16-byte pieces of a column */
+    __shared__ BMat<TP> sm[kWarps];
+    const int lane = threadIdx.x & 31, t = lane % TP, g = lane / TP;
+    BMat<TP> &W = sm[threadIdx.x >> 5];
+    const uint32_t my_col = (uint32_t)(t / kPerCol);
+    const uint4 *my_new = reinterpret_cast<const uint4 *>(W.CB + g * TP) + t % kPerCol;
+    const uint4 *my_old = reinterpret_cast<const uint4 *>(W.PR) + t;
     const uint64_t nw = (uint64_t)gridDim.x * kWarps;
-    for (uint64_t q = ((uint64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5; q < P.n; q += nw) {
-        const uint32_t m = (P.live[q] >> 1) & 127u;
+    const uint32_t split = 1u << split_log2;
+    for (uint64_t it = ((uint64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+         it < P.n << split_log2; it += nw) {
+        const uint64_t q = it >> split_log2;
+        const uint32_t live = P.live[q], m = (live >> 1) & 127u;
         const uint32_t nc = bcount(tab, m);
         const uint64_t base = P.child_off[q];
-        uint32_t R[8] = {0, 0, 0, 0, 0, 0, 0, 0}, f0 = 0, s0 = 0;
-        if (lane < TP) {
-#pragma unroll
-            for (int r = 0; r < 8; r++) R[r] = P.regs[(q * 8 + r) * TP + lane];
-            f0 = P.flags[q * TP + lane];
-            s0 = P.skip[q * TP + lane];
-        }
-        for (uint32_t c = 0; c < nc; c++) {
-            const uint64_t L = base + c;
-            if (!(bitmap[L >> 5] >> (L & 31) & 1u)) continue;
-            const uint64_t k = word_rank[L >> 5] + __popc(bitmap[L >> 5] & ((1u << (L & 31)) - 1u));
-            const uint32_t insn = bcand(tab, m, c);
-            uint32_t v = 0, f = f0, sk = s0, rd = 0;
-            if (lane < T) rd = bexec(insn, p, R, f0, s0, &v, &f, &sk);
-            if (lane < TP) {
-#pragma unroll
-                for (int r = 0; r < 8; r++)
-                    C.regs[(k * 8 + r) * TP + lane] = (uint16_t)(lane < T ? (rd == (uint32_t)r ? v : R[r]) : 0u);
-                C.flags[k * TP + lane] = (uint8_t)(lane < T ? f : 0u);
-                C.skip[k * TP + lane] = (uint8_t)(lane < T ? sk : 0u);
+        __syncwarp();
+        if (lane < TP)
+            reinterpret_cast<uint4 *>(W.PR)[lane] =
+                reinterpret_cast<const uint4 *>(P.regs + q * 8 * TP)[lane];
+        const uint32_t f0 = P.flags[q * TP + t], s0 = P.skip[q * TP + t];
+        __syncwarp();
+        for (uint32_t c0 = ((uint32_t)it & (split - 1)) * 32; c0 < nc; c0 += 32 << split_log2) {
+            const uint32_t c = c0 + lane;
+            uint32_t insn = 0;
+            uint64_t k = 0;
+            bool keep = false;
+            if (c < nc) {
+                const uint64_t L = base + c;
+                const uint32_t wv = bitmap[L >> 5];
+                keep = wv >> (L & 31) & 1u;
+                if (keep) {
+                    k = word_rank[L >> 5] + __popc(wv & ((1u << (L & 31)) - 1u));
+                    insn = bcand(tab, m, c);
+                    const BUop u = buop(insn);
+                    const uint32_t w = u.op == (uint32_t)kOpDiv || u.op == (uint32_t)kOpMod ? 0u : u.wr;
+                    C.live[k] = (uint8_t)(live | (1u << u.wr & 0xFEu));
+                    C.parent[k] = (uint32_t)q;
+                    C.cidx[k] = (uint16_t)c;
+                    C.rdl[k] = (uint8_t)w;
+                    if (w) atomicMin(&fcr[q * 8 + w], (uint32_t)k);
+                }
             }
-            if (lane == 0) {
-                const uint32_t op = insn >> 11, rdi = (insn >> 8) & 7u;
-                uint32_t nl = P.live[q];
-                if (op != (uint32_t)kOpCmp && op != (uint32_t)kOpBr && rdi != 0) nl |= 1u << rdi;
-                C.live[k] = (uint8_t)nl;
-                C.parent[k] = (uint32_t)q;
-                C.cidx[k] = (uint16_t)c;
+            uint32_t bal = __ballot_sync(0xFFFFFFFFu, keep);
+            while (bal) {
+                /* this lane group's child: the first set bit, or the second */
+                uint32_t mine = bal;
+                bal &= bal - 1;
+                if (TP == 16) {
+                    mine = g ? bal : mine;
+                    bal &= bal - 1;
+                }
+                const int j = __ffs((int)mine) - 1;
+                const uint64_t kj = __shfl_sync(0xFFFFFFFFu, k, j < 0 ? 0 : j);
+                const BUop u = buop(__shfl_sync(0xFFFFFFFFu, insn, j < 0 ? 0 : j));
+                uint32_t f = 0, sk = 0, v = 0;
+                if (t < T)
+                    v = bvalue(u, p, W.PR[u.ra * TP + t], W.PR[u.rb * TP + t], W.PR[u.wr * TP + t],
+                               f0, s0, &f, &sk);
+                W.CB[lane] = (uint16_t)v;
+                W.FB[lane] = (uint8_t)f;
+                W.SB[lane] = (uint8_t)sk;
+                __syncwarp();
+                if (j >= 0) {
+                    reinterpret_cast<uint4 *>(C.regs + kj * 8 * TP)[t] =
+                        u.wr && my_col == u.wr ? *my_new : *my_old;
+                    if (t < TP / 16) {
+                        reinterpret_cast<uint4 *>(C.flags + kj * TP)[t] =
+                            reinterpret_cast<const uint4 *>(W.FB + g * TP)[t];
+                        reinterpret_cast<uint4 *>(C.skip + kj * TP)[t] =
+                            reinterpret_cast<const uint4 *>(W.SB + g * TP)[t];
+                    }
+                }
+                __syncwarp();
             }
         }
     }
@@ -489,23 +850,54 @@ k_bmaterialize(BDev P, BTab tab, int T, uint32_t p, const uint32_t *bitmap,
 
 /* Output check of a complete kernel (tools/enumerate.c:262-286 with
    tasks/spec.c:187-212): OUT r passes on a test that did not fault and
-   holds the target in r. Bit r of mask[i] is set when it passes on all. */
+   holds the target in r. Bit r of mask[i] is set when it passes on all.
+   Per block of kLeafBlock states, sums[2 b] and [2 b + 1] receive the passing
+   (state, register) pairs and the live registers. Eight lanes a state, a
+   register each: 16 bytes (eight tests) of its column against the packed
+   target, the others only where those match.
+
+   Bound: HBM, the register block read once. A warp per state and register
+   took 3.3 ms for relu's depth-3 last level (8.2M states), this 0.3 ms. */
+constexpr uint64_t kLeafBlock = 4096;
 template <int TP>
-__global__ void k_bleaf(BDev P, int T, const uint32_t *target, uint8_t *mask)
+__global__ void __launch_bounds__(256)
+k_bleaf(BDev P, int T, const uint32_t *target, uint8_t *mask, uint32_t *sums)
 {
-    const int lane = threadIdx.x & 31;
-    const uint64_t nw = (uint64_t)gridDim.x * (blockDim.x >> 5);
-    for (uint64_t q = ((uint64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5; q < P.n; q += nw) {
-        const uint32_t live = P.live[q];
-        uint32_t ok = 0;
-        for (int r = 1; r < 8; r++) {
-            if (!(live >> r & 1u)) continue;
-            bool good = true;
-            if (lane < T)
-                good = P.skip[q * TP + lane] != kFault && P.regs[(q * 8 + r) * TP + lane] == target[lane];
-            if (__all_sync(0xFFFFFFFFu, good)) ok |= 1u << r;
+    __shared__ __align__(16) uint16_t tgt[TP];
+    __shared__ uint32_t total[2];
+    const int lane = threadIdx.x & 31, r = lane & 7;
+    if (threadIdx.x < TP) tgt[threadIdx.x] = (uint16_t)(threadIdx.x < T ? target[threadIdx.x] : 0u);
+    for (uint64_t b = blockIdx.x; b * kLeafBlock < P.n; b += gridDim.x) {
+        if (threadIdx.x < 2) total[threadIdx.x] = 0;
+        __syncthreads();
+        uint32_t pairs = 0, outs = 0;
+        for (uint64_t k = threadIdx.x >> 3; k < kLeafBlock; k += blockDim.x >> 3) {
+            const uint64_t q = b * kLeafBlock + k;
+            bool ok = q < P.n;
+            uint32_t live = 0;
+            if (ok) {
+                live = P.live[q];
+                ok = r && (live >> r & 1u);
+                const uint4 *col = reinterpret_cast<const uint4 *>(P.regs + (q * 8 + r) * TP);
+                /* unused tests are zero in both */
+                for (int i = 0; ok && i < (T + 7) / 8; i++) {
+                    const uint4 v = col[i], w = reinterpret_cast<const uint4 *>(tgt)[i];
+                    ok = v.x == w.x && v.y == w.y && v.z == w.z && v.w == w.w;
+                }
+                for (int t = 0; ok && t < T; t++) ok = P.skip[q * TP + t] != kFault;
+            }
+            const uint32_t bal = __ballot_sync(0xFFFFFFFFu, ok) >> (lane & 24) & 0xFFu;
+            if (r == 0 && q < P.n) {
+                mask[q] = (uint8_t)bal;
+                pairs += __popc(bal);
+                outs += __popc(live >> 1);
+            }
         }
-        if (lane == 0) mask[q] = (uint8_t)ok;
+        if (r == 0 && pairs) atomicAdd(&total[0], pairs);
+        if (r == 0) atomicAdd(&total[1], outs);
+        __syncthreads();
+        if (threadIdx.x < 2) sums[2 * b + threadIdx.x] = total[threadIdx.x];
+        __syncthreads();
     }
 }
 
@@ -569,10 +961,12 @@ k_bsuffix(BDev P, BTab tab, int T, uint32_t p, const uint32_t *target, BSol *out
         const uint32_t live = P.live[q];
         const uint32_t m = (live >> 1) & 127u;
         const uint32_t nc = bcount(tab, m);
+        const uint32_t dead = dead_write(P, q);
         for (uint32_t c0 = 0; c0 < nc; c0 += 32) {
             const uint32_t c = c0 + lane;
             if (c >= nc) continue;
             const uint32_t insn = bcand(tab, m, c);
+            if (never_kept(insn, buop(insn), dead)) continue;
             const uint32_t op = insn >> 11, rdi = (insn >> 8) & 7u;
             const uint32_t wr = (op != (uint32_t)kOpCmp && op != (uint32_t)kOpBr && rdi != 0) ? rdi : 0u;
             /* a register the child leaves as the parent's can hold the
@@ -654,6 +1048,42 @@ __global__ void k_bpath(BPath L, int K, const uint32_t *qs, const uint16_t *cs, 
     }
 }
 
+/* A state on a solution's path: its rank in its level, its liveness, the
+   candidate that its child on the path took and its child offset. */
+struct BStep {
+    uint64_t child_off;
+    uint32_t rank;
+    uint16_t cidx;
+    uint8_t live, pad;
+};
+
+struct BPathAll {
+    const uint32_t *parent[17];
+    const uint16_t *cidx[17];
+    const uint8_t *live[17];
+    const uint64_t *child_off[17];
+};
+
+/* out[i][d], d = 0..K: the path of state leaf[i] of level K. */
+__global__ void k_bpath_all(BPathAll L, int K, const uint32_t *leaf, int ns, BStep *out)
+{
+    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < ns; i += gridDim.x * blockDim.x) {
+        uint32_t st = leaf[i];
+        uint16_t c = 0;
+        for (int d = K; d >= 0; d--) {
+            BStep s;
+            s.child_off = d < K ? L.child_off[d][st] : 0;
+            s.rank = st;
+            s.cidx = c;
+            s.live = L.live[d][st];
+            s.pad = 0;
+            out[(size_t)i * (K + 1) + d] = s;
+            c = L.cidx[d][st];
+            st = L.parent[d][st];
+        }
+    }
+}
+
 /* ---- host driver ----------------------------------------------------------- */
 
 struct BranchRun {
@@ -666,7 +1096,15 @@ struct BranchRun {
     uint32_t *d_pre_off = nullptr, *d_post_off = nullptr;
     uint16_t *d_pre = nullptr, *d_post = nullptr;
     uint32_t *d_status = nullptr;
-    std::vector<void *> allocs;
+    /* the engine's arena, idle during a branch-mode solve, from its bottom;
+       what does not fit in it comes from the device's pool */
+    char *arena = nullptr;
+    size_t arena_cap = 0, arena_used = 0;
+    struct Alloc {
+        void *p;
+        size_t before;   /* arena_used before it; ~0: a pool allocation */
+    };
+    std::vector<Alloc> allocs;
     uint64_t h2d = 0, d2h = 0;
     int launches = 0;
 
@@ -679,26 +1117,38 @@ struct BranchRun {
     void release(size_t keep)
     {
         while (allocs.size() > keep) {
-            cudaFreeAsync(allocs.back(), st);
+            const Alloc &a = allocs.back();
+            if (a.before == ~size_t(0)) cudaFreeAsync(a.p, st);
+            else arena_used = a.before;
             allocs.pop_back();
         }
     }
     template <class X>
     X *alloc(size_t count)
     {
+        const size_t bytes = (std::max<size_t>(count * sizeof(X), 16) + 255) & ~size_t(255);
+        if (bytes <= arena_cap - arena_used) {
+            allocs.push_back({arena + arena_used, arena_used});
+            arena_used += bytes;
+            return (X *)allocs.back().p;
+        }
         void *p = nullptr;
-        if (cudaMallocAsync(&p, std::max<size_t>(count * sizeof(X), 16), st) != cudaSuccess) {
+        if (cudaMallocAsync(&p, bytes, st) != cudaSuccess) {
             cudaGetLastError();
             return nullptr;
         }
-        allocs.push_back(p);
+        allocs.push_back({p, ~size_t(0)});
         return (X *)p;
     }
     BTab tab(int mf) const { return BTab{d_pre_off, d_post_off, d_pre, d_post, mf}; }
     int grid(int per_sm) const { return sms * per_sm; }
 };
 
-BDev bdev(const BLevel &L) { return BDev{L.regs, L.flags, L.skip, L.live, L.child_off, L.n}; }
+BDev bdev(const BLevel &L, const BLevel *up = nullptr)
+{
+    return BDev{L.regs, L.flags, L.skip, L.live, L.child_off, L.n, L.parent, L.rdl,
+                up ? up->fcr : nullptr};
+}
 
 int alloc_blevel(BranchRun &b, BLevel &L, uint64_t n)
 {
@@ -709,7 +1159,8 @@ int alloc_blevel(BranchRun &b, BLevel &L, uint64_t n)
     L.live = b.alloc<uint8_t>(n);
     L.parent = b.alloc<uint32_t>(n);
     L.cidx = b.alloc<uint16_t>(n);
-    if (!L.regs || !L.flags || !L.skip || !L.live || !L.parent || !L.cidx) {
+    L.rdl = b.alloc<uint8_t>(n);
+    if (!L.regs || !L.flags || !L.skip || !L.live || !L.parent || !L.cidx || !L.rdl) {
         set_berr("device memory exhausted for a level of %llu states", (unsigned long long)n);
         return PCAGB_ENOMEM;
     }
@@ -746,6 +1197,15 @@ int bscan(BranchRun &b, uint64_t *a, uint64_t n)
     return rc;
 }
 
+/* log2 of the slices a level's parents are cut into so that its warps fill
+   the grid (at most 32). */
+uint32_t slices(uint64_t parents, int grid)
+{
+    uint32_t l = 0;
+    while (l < 5 && (parents << (l + 1)) <= (uint64_t)grid * kWarps) l++;
+    return l;
+}
+
 /* Expand level P (position p of a depth-K pass) into C. Fills the number of
    generated children. */
 /* Children of every state of P at a position with mf forward offsets:
@@ -775,7 +1235,8 @@ int count_bchildren(BranchRun &b, BLevel &P, int mf)
     return PCAGB_OK;
 }
 
-int build_blevel(BranchRun &b, BLevel &P, uint32_t p, int mf, BLevel &C)
+/* `up`: the level above P (null at the root). */
+int build_blevel(BranchRun &b, BLevel &P, const BLevel *up, uint32_t p, int mf, BLevel &C)
 {
     const BTab tab = b.tab(mf);
     int rc = P.child_off ? PCAGB_OK : count_bchildren(b, P, mf);
@@ -787,14 +1248,18 @@ int build_blevel(BranchRun &b, BLevel &P, uint32_t p, int mf, BLevel &C)
     uint32_t *bitmap = b.alloc<uint32_t>(words + 1);
     unsigned long long *table = b.alloc<unsigned long long>(slots);
     uint64_t *rank = b.alloc<uint64_t>(words + 1);
-    if (!bitmap || !table || !rank) { set_berr("device memory exhausted expanding a level"); return PCAGB_ENOMEM; }
+    P.fcr = b.alloc<uint32_t>(P.n * 8);
+    if (!bitmap || !table || !rank || !P.fcr) { set_berr("device memory exhausted expanding a level"); return PCAGB_ENOMEM; }
     BCK(cudaMemsetAsync(bitmap, 0, (words + 1) * 4, b.st));
     BCK(cudaMemsetAsync(table, 0, slots * 8, b.st));
     BCK(cudaMemsetAsync(b.d_status, 0, 4, b.st));
+    BCK(cudaMemsetAsync(P.fcr, 0xFF, P.n * 8 * sizeof(uint32_t), b.st));
     if (b.TP == 16)
-        k_bexpand<16><<<b.grid(4), kBThreads, 0, b.st>>>(bdev(P), tab, b.T, p, table, slots - 1, bitmap, b.d_status);
+        k_bexpand<16><<<b.grid(6), kBThreads, 0, b.st>>>(bdev(P, up), tab, b.T, p, table, slots - 1,
+                                                        bitmap, b.d_status, slices(P.n, b.grid(6)));
     else
-        k_bexpand<32><<<b.grid(4), kBThreads, 0, b.st>>>(bdev(P), tab, b.T, p, table, slots - 1, bitmap, b.d_status);
+        k_bexpand<32><<<b.grid(6), kBThreads, 0, b.st>>>(bdev(P, up), tab, b.T, p, table, slots - 1,
+                                                        bitmap, b.d_status, slices(P.n, b.grid(6)));
     rc = blaunch(b);
     if (rc) return rc;
     k_bmark<<<b.grid(4), 256, 0, b.st>>>(table, slots, P.child_off, bitmap);
@@ -819,36 +1284,14 @@ int build_blevel(BranchRun &b, BLevel &P, uint32_t p, int mf, BLevel &C)
     if (rc) return rc;
     if (kept) {
         if (b.TP == 16)
-            k_bmaterialize<16><<<b.grid(4), kBThreads, 0, b.st>>>(bdev(P), tab, b.T, p, bitmap, rank, C);
+            k_bmaterialize<16><<<b.grid(8), kBThreads, 0, b.st>>>(bdev(P), tab, b.T, p, bitmap, rank, C,
+                                                                 P.fcr, slices(P.n, b.grid(8)));
         else
-            k_bmaterialize<32><<<b.grid(4), kBThreads, 0, b.st>>>(bdev(P), tab, b.T, p, bitmap, rank, C);
+            k_bmaterialize<32><<<b.grid(8), kBThreads, 0, b.st>>>(bdev(P), tab, b.T, p, bitmap, rank, C,
+                                                                 P.fcr, slices(P.n, b.grid(8)));
         rc = blaunch(b);
         if (rc) return rc;
     }
-    return PCAGB_OK;
-}
-
-/* Host copies of a level's tree links. */
-struct HostLevel {
-    std::vector<uint32_t> parent;
-    std::vector<uint16_t> cidx;
-    std::vector<uint8_t> live;
-    uint64_t children = 0;
-};
-
-int fetch_links(BranchRun &b, const BLevel &L, HostLevel &H, bool links)
-{
-    H.live.resize(L.n);
-    BCK(cudaMemcpyAsync(H.live.data(), L.live, L.n, cudaMemcpyDeviceToHost, b.st));
-    b.d2h += L.n;
-    if (links) {
-        H.parent.resize(L.n);
-        H.cidx.resize(L.n);
-        BCK(cudaMemcpyAsync(H.parent.data(), L.parent, L.n * 4, cudaMemcpyDeviceToHost, b.st));
-        BCK(cudaMemcpyAsync(H.cidx.data(), L.cidx, L.n * 2, cudaMemcpyDeviceToHost, b.st));
-        b.d2h += L.n * 6;
-    }
-    BCK(cudaStreamSynchronize(b.st));
     return PCAGB_OK;
 }
 
@@ -900,6 +1343,37 @@ int solution_kernels(BranchRun &b, const BranchTables &bt, std::vector<BLevel> &
     return PCAGB_OK;
 }
 
+/* The paths (K + 1 steps each) of ns states of level K, gathered on the
+   device so that no level's links cross the bus. */
+template <class F>
+int solution_paths(BranchRun &b, std::vector<BLevel> &lv, int K, size_t ns, F &&leaf,
+                   std::vector<BStep> *steps)
+{
+    BPathAll L{};
+    for (int d = 0; d <= K; d++) {
+        L.parent[d] = lv[d].parent;
+        L.cidx[d] = lv[d].cidx;
+        L.live[d] = lv[d].live;
+        L.child_off[d] = lv[d].child_off;
+    }
+    std::vector<uint32_t> q(ns);
+    for (size_t i = 0; i < ns; i++) q[i] = (uint32_t)leaf(i);
+    steps->resize(ns * (K + 1));
+    uint32_t *d_q = b.alloc<uint32_t>(ns);
+    BStep *d_out = b.alloc<BStep>(steps->size());
+    if (!d_q || !d_out) { set_berr("device memory exhausted"); return PCAGB_ENOMEM; }
+    BCK(cudaMemcpyAsync(d_q, q.data(), ns * 4, cudaMemcpyHostToDevice, b.st));
+    k_bpath_all<<<(unsigned)((ns + 127) / 128), 128, 0, b.st>>>(L, K, d_q, (int)ns, d_out);
+    int rc = blaunch(b);
+    if (rc) return rc;
+    BCK(cudaMemcpyAsync(steps->data(), d_out, steps->size() * sizeof(BStep), cudaMemcpyDeviceToHost,
+                        b.st));
+    BCK(cudaStreamSynchronize(b.st));
+    b.h2d += ns * 4;
+    b.d2h += steps->size() * sizeof(BStep);
+    return PCAGB_OK;
+}
+
 /* The last position of a depth-K pass without building level K: solving
  * children from k_bsuffix; a child counts only if it is the depth-first
  * first of its key (the pruner would have dropped it otherwise), the
@@ -916,6 +1390,7 @@ int64_t branch_suffix(BranchRun &b, const BranchTables &bt, std::vector<BLevel> 
                       int *sol_lens, int cap, bool first_only, uint64_t *searched)
 {
     BLevel &P = lv[K - 1];
+    const BLevel *up = K >= 2 ? &lv[K - 2] : nullptr;
     const BTab tab = b.tab(0);
     const uint32_t p = (uint32_t)(K - 1);
     const uint64_t kCap = 1ull << 22;
@@ -930,10 +1405,10 @@ int64_t branch_suffix(BranchRun &b, const BranchTables &bt, std::vector<BLevel> 
         const uint64_t q1 = std::min(P.n, q0 + step);
         BCK(cudaMemsetAsync(d_cnt, 0, 8, b.st));
         if (b.TP == 16)
-            k_bsuffix<16><<<b.grid(4), kBThreads, 0, b.st>>>(bdev(P), tab, b.T, p, b.d_target,
+            k_bsuffix<16><<<b.grid(4), kBThreads, 0, b.st>>>(bdev(P, up), tab, b.T, p, b.d_target,
                                                              d_sol, d_cnt, kCap, q0, q1);
         else
-            k_bsuffix<32><<<b.grid(4), kBThreads, 0, b.st>>>(bdev(P), tab, b.T, p, b.d_target,
+            k_bsuffix<32><<<b.grid(4), kBThreads, 0, b.st>>>(bdev(P, up), tab, b.T, p, b.d_target,
                                                              d_sol, d_cnt, kCap, q0, q1);
         int rc = blaunch(b);
         if (rc) return rc;
@@ -1065,6 +1540,7 @@ int64_t branch_suffix(BranchRun &b, const BranchTables &bt, std::vector<BLevel> 
 /* Internal accessors of engine.cu. */
 cudaStream_t pcagb_internal_stream(pcagb_engine_t *e);
 int pcagb_internal_device(pcagb_engine_t *e);
+void pcagb_internal_arena(pcagb_engine_t *e, char **base, size_t *bytes);
 
 extern "C" {
 
@@ -1110,26 +1586,28 @@ int solve_branch(pcagb_engine_t *e, const task_spec_t *task, int max_depth,
     b.st = pcagb_internal_stream(e);
     BCK(cudaSetDevice(pcagb_internal_device(e)));
     BCK(cudaDeviceGetAttribute(&b.sms, cudaDevAttrMultiProcessorCount, pcagb_internal_device(e)));
+    pcagb_internal_arena(e, &b.arena, &b.arena_cap);
+    {
+        const DevTables *dt = nullptr;
+        const int rc = device_tables(pcagb_internal_device(e), &dt);
+        if (rc) return rc;
+        b.d_pre_off = dt->pre_off;
+        b.d_post_off = dt->post_off;
+        b.d_pre = dt->pre;
+        b.d_post = dt->post;
+    }
     b.task = task;
     b.T = task->num_tests;
     b.TP = b.T <= 16 ? 16 : 32;
     b.d_target = b.alloc<uint32_t>(32);
-    b.d_pre_off = b.alloc<uint32_t>(129);
-    b.d_post_off = b.alloc<uint32_t>(129);
-    b.d_pre = b.alloc<uint16_t>(bt.pre.size());
-    b.d_post = b.alloc<uint16_t>(bt.post.size());
     b.d_status = b.alloc<uint32_t>(1);
-    if (!b.d_target || !b.d_pre_off || !b.d_post_off || !b.d_pre || !b.d_post || !b.d_status) {
+    if (!b.d_target || !b.d_status) {
         set_berr("device memory exhausted");
         return PCAGB_ENOMEM;
     }
     uint32_t tgt[32] = {0};
     for (int t = 0; t < b.T; t++) tgt[t] = task->tests[t].out[0];
     BCK(cudaMemcpyAsync(b.d_target, tgt, sizeof tgt, cudaMemcpyHostToDevice, b.st));
-    BCK(cudaMemcpyAsync(b.d_pre_off, bt.pre_off.data(), 129 * 4, cudaMemcpyHostToDevice, b.st));
-    BCK(cudaMemcpyAsync(b.d_post_off, bt.post_off.data(), 129 * 4, cudaMemcpyHostToDevice, b.st));
-    BCK(cudaMemcpyAsync(b.d_pre, bt.pre.data(), bt.pre.size() * 2, cudaMemcpyHostToDevice, b.st));
-    BCK(cudaMemcpyAsync(b.d_post, bt.post.data(), bt.post.size() * 2, cudaMemcpyHostToDevice, b.st));
 
     /* level 0: the IN scaffold's state */
     search_ctx_t ctx;
@@ -1155,6 +1633,7 @@ int solve_branch(pcagb_engine_t *e, const task_spec_t *task, int max_depth,
         BCK(cudaMemcpyAsync(lv[0].live, &live0, 1, cudaMemcpyHostToDevice, b.st));
         BCK(cudaMemcpyAsync(lv[0].parent, &zero, 4, cudaMemcpyHostToDevice, b.st));
         BCK(cudaMemcpyAsync(lv[0].cidx, &zero, 2, cudaMemcpyHostToDevice, b.st));
+        BCK(cudaMemsetAsync(lv[0].rdl, 0, 1, b.st));
         uint64_t tried = 0, pruned = 0;
         bool unbuilt_last = false;
         for (int d = 0; d < K; d++) {
@@ -1167,7 +1646,7 @@ int solve_branch(pcagb_engine_t *e, const task_spec_t *task, int max_depth,
                     break;
                 }
             }
-            int rc = build_blevel(b, lv[d], (uint32_t)d, mf, lv[d + 1]);
+            int rc = build_blevel(b, lv[d], d ? &lv[d - 1] : nullptr, (uint32_t)d, mf, lv[d + 1]);
             if (rc) return rc;
             tried += lv[d + 1].n;
             pruned += lv[d].children - lv[d + 1].n;
@@ -1198,32 +1677,29 @@ int solve_branch(pcagb_engine_t *e, const task_spec_t *task, int max_depth,
         }
         res->level_children[K] = K ? lv[K - 1].children : 1;
         res->level_survivors[K] = lv[K].n;
-        /* the output check of every complete kernel */
+        /* the output check of every complete kernel, its sums per block */
         const BLevel &LK = lv[K];
+        const uint64_t blocks = (LK.n + kLeafBlock - 1) / kLeafBlock;
         uint8_t *d_mask = b.alloc<uint8_t>(LK.n);
-        if (!d_mask) { set_berr("device memory exhausted"); return PCAGB_ENOMEM; }
+        uint32_t *d_sums = b.alloc<uint32_t>(blocks * 2);
+        if (!d_mask || !d_sums) { set_berr("device memory exhausted"); return PCAGB_ENOMEM; }
+        std::vector<uint32_t> sums(blocks * 2);
         if (LK.n) {
+            const unsigned g = (unsigned)std::min<uint64_t>(blocks, (uint64_t)b.grid(8));
             if (b.TP == 16)
-                k_bleaf<16><<<b.grid(4), 256, 0, b.st>>>(bdev(LK), b.T, b.d_target, d_mask);
+                k_bleaf<16><<<g, 256, 0, b.st>>>(bdev(LK), b.T, b.d_target, d_mask, d_sums);
             else
-                k_bleaf<32><<<b.grid(4), 256, 0, b.st>>>(bdev(LK), b.T, b.d_target, d_mask);
+                k_bleaf<32><<<g, 256, 0, b.st>>>(bdev(LK), b.T, b.d_target, d_mask, d_sums);
             int rc = blaunch(b);
             if (rc) return rc;
+            BCK(cudaMemcpyAsync(sums.data(), d_sums, sums.size() * 4, cudaMemcpyDeviceToHost, b.st));
+            BCK(cudaStreamSynchronize(b.st));
+            b.d2h += sums.size() * 4;
         }
-        std::vector<HostLevel> H(K + 1);
-        for (int d = 0; d <= K; d++) {
-            int rc = fetch_links(b, lv[d], H[d], d > 0);
-            if (rc) return rc;
-            H[d].children = lv[d].children;
-        }
-        std::vector<uint8_t> mask(LK.n);
-        BCK(cudaMemcpyAsync(mask.data(), d_mask, LK.n, cudaMemcpyDeviceToHost, b.st));
-        BCK(cudaStreamSynchronize(b.st));
-        b.d2h += LK.n;
         uint64_t outputs = 0, nsol = 0;
-        for (uint64_t i = 0; i < LK.n; i++) {
-            outputs += __builtin_popcount(H[K].live[i] >> 1);
-            nsol += __builtin_popcount(mask[i]);
+        for (uint64_t i = 0; i < blocks; i++) {
+            nsol += sums[2 * i];
+            outputs += sums[2 * i + 1];
         }
         if (nsol == 0) {
             res->tried[K] = tried + outputs;
@@ -1232,46 +1708,54 @@ int solve_branch(pcagb_engine_t *e, const task_spec_t *task, int max_depth,
             res->candidates[K] = res->tried[K];
             continue;
         }
-        /* solutions: the first 100 (state, register) pairs in depth-first
-           order; the reference's pass stops there, so its counters are
-           those of the depth-first walk up to that leaf */
+        /* solutions: the (state, register) pairs of the leaves in depth-first
+           order (the level's) up to the one that brings their number to 100.
+           The reference's pass stops there, so its counters are those of the
+           depth-first walk up to that leaf */
         const uint64_t kMax = 100;
-        std::vector<std::vector<uint64_t>> first(K);
-        for (int d = 0; d < K; d++) {
-            first[d].assign(lv[d].n + 1, 0);
-            for (uint32_t p : H[d + 1].parent) first[d][p + 1]++;
-            for (uint64_t i = 0; i < lv[d].n; i++) first[d][i + 1] += first[d][i];
-        }
         struct Sol { uint64_t state; int reg; };
         std::vector<Sol> sols;
-        uint64_t w_tried = 0, w_pruned = 0;
-        bool stop = false;
-        auto walk = [&](auto &&self, int d, uint64_t i) -> void {
-            if (d == K) {
-                const uint32_t live = H[K].live[i];
-                w_tried += __builtin_popcount(live >> 1);
+        uint64_t w_out = 0, last = LK.n;   /* outputs tried; the leaf it stops at (n: none) */
+        std::vector<uint8_t> mask(kLeafBlock), live(kLeafBlock);
+        for (uint64_t blk = 0; blk < blocks && last == LK.n; blk++) {
+            if (!sums[2 * blk]) {
+                w_out += sums[2 * blk + 1];
+                continue;
+            }
+            const uint64_t i0 = blk * kLeafBlock, n = std::min(kLeafBlock, LK.n - i0);
+            BCK(cudaMemcpyAsync(mask.data(), d_mask + i0, n, cudaMemcpyDeviceToHost, b.st));
+            BCK(cudaMemcpyAsync(live.data(), LK.live + i0, n, cudaMemcpyDeviceToHost, b.st));
+            BCK(cudaStreamSynchronize(b.st));
+            b.d2h += 2 * n;
+            for (uint64_t i = 0; i < n && last == LK.n; i++) {
+                w_out += __builtin_popcount(live[i] >> 1);
                 for (int r = 1; r < 8; r++)
-                    if (mask[i] >> r & 1u) sols.push_back(Sol{i, r});
-                if (sols.size() >= kMax) stop = true;
-                return;
+                    if (mask[i] >> r & 1u) sols.push_back(Sol{i0 + i, r});
+                if (sols.size() >= kMax) last = i0 + i;
             }
-            const uint64_t nchild = (d + 1 <= K) ? first[d][i + 1] - first[d][i] : 0;
-            const uint32_t m = (H[d].live[i] >> 1) & 127u;
-            BTab ht{bt.pre_off.data(), bt.post_off.data(), bt.pre.data(), bt.post.data(), K - d - 1};
-            const uint64_t ncand = bcount(ht, m);
-            uint64_t seen = 0;
-            for (uint64_t j = first[d][i]; j < first[d][i + 1]; j++) {
-                /* candidates before this child that it did not visit were pruned */
-                w_pruned += H[d + 1].cidx[j] - seen;
-                seen = (uint64_t)H[d + 1].cidx[j] + 1;
-                w_tried++;
-                self(self, d + 1, j);
-                if (stop) return;
+        }
+        /* the paths of the solutions (and so of the last leaf): for each, its
+           ancestor's rank, liveness, candidate index on the path and child
+           offset at every level */
+        std::vector<BStep> steps;
+        int rc = solution_paths(b, lv, K, sols.size(), [&](size_t i) { return sols[i].state; }, &steps);
+        if (rc) return rc;
+        uint64_t w_tried = w_out, w_pruned = 0;
+        if (last == LK.n) {
+            /* the whole walk */
+            w_tried += tried;
+            w_pruned = pruned;
+        } else {
+            /* states of a level come in depth-first order, so the walk has
+               visited those up to the last leaf's ancestor at each; the
+               candidates before the path's, less the children kept of them,
+               were pruned */
+            const BStep *s = &steps[(sols.size() - 1) * (size_t)(K + 1)];
+            for (int d = 1; d <= K; d++) {
+                w_tried += (uint64_t)s[d].rank + 1;
+                w_pruned += s[d - 1].child_off + s[d - 1].cidx - s[d].rank;
             }
-            (void)nchild;
-            w_pruned += ncand - seen;
-        };
-        walk(walk, 0, 0);
+        }
         res->tried[K] = w_tried;
         pruned_cum += w_pruned;
         res->pruned_cum[K] = pruned_cum;
@@ -1279,22 +1763,18 @@ int solve_branch(pcagb_engine_t *e, const task_spec_t *task, int max_depth,
         res->optimal_depth = K;
         res->total_solutions = sols.size();
         int stored = 0;
-        for (const Sol &s : sols) {
+        for (size_t i = 0; i < sols.size(); i++) {
             if (stored >= cap || !sol_progs) break;
-            std::vector<uint16_t> kern(K);
-            uint64_t i = s.state;
-            for (int d = K; d >= 1; d--) {
-                const uint32_t p = H[d].parent[i];
-                BTab ht{bt.pre_off.data(), bt.post_off.data(), bt.pre.data(), bt.post.data(), K - d};
-                kern[d - 1] = bcand(ht, (H[d - 1].live[p] >> 1) & 127u, H[d].cidx[i]);
-                i = p;
-            }
             uint16_t prog[16] = {0};
             int n = 0;
             for (int q = 0; q < task->num_inputs; q++)
                 prog[n++] = (uint16_t)PCA_ENC_I(PCA_OP_IN, q + 1, task->input_ports[q]);
-            for (uint16_t w : kern) prog[n++] = w;
-            prog[n++] = (uint16_t)PCA_ENC_I(PCA_OP_OUT, s.reg, task->output_ports[0]);
+            for (int d = 0; d < K; d++) {
+                const BStep &s = steps[i * (size_t)(K + 1) + d];
+                BTab ht{bt.pre_off.data(), bt.post_off.data(), bt.pre.data(), bt.post.data(), K - d - 1};
+                prog[n++] = bcand(ht, (s.live >> 1) & 127u, s.cidx);
+            }
+            prog[n++] = (uint16_t)PCA_ENC_I(PCA_OP_OUT, sols[i].reg, task->output_ports[0]);
             prog[n++] = (uint16_t)PCA_ENC_R(PCA_OP_HLT, 0, 0, 0);
             if (task_evaluate(task, prog, n) != task->num_tests) {
                 set_berr("internal: a branch-mode solution failed the VM re-check");
