@@ -158,7 +158,8 @@ struct pcagb_engine {
     unsigned long long *d_small = nullptr;   /* [0] sol count [1] unused [2] count
                                                 [3] value-class evaluations run
                                                 [4] the work counter of the insert and
-                                                lean materialise kernels */
+                                                lean materialise kernels
+                                                [5] column ids given out */
     uint32_t *d_status = nullptr;
     ulonglong2 *d_sol = nullptr;
     ulonglong2 *d_firsts = nullptr;          /* [cap_tasks] SolBuf::firsts */
@@ -409,16 +410,65 @@ uint32_t split_log2(uint64_t parents, int grid)
 
 template <int TPC>
 int launch_expand(pcagb_engine *e, const Level &P, const uint32_t *fcr_up,
-                  unsigned long long *table, uint64_t tmask)
+                  unsigned long long *table, uint64_t tmask, const IdDev &ids)
 {
     const int g = e->grid(e->occ_insert);
     /* the work-item counter the kernel's warps draw from */
     uint32_t *next = reinterpret_cast<uint32_t *>(e->d_small + 4);
     CK(cudaMemsetAsync(next, 0, 4, e->stream));
-    k_expand_insert<TPC><<<g, kThreads, 0, e->stream>>>(view(P), e->td, table, tmask,
-                                                        e->d_status, split_log2(P.n, g), fcr_up,
-                                                        next);
+    if (ids.tab) {
+        k_state_ids<TPC><<<e->grid(4), kThreads, 0, e->stream>>>(view(P), ids, e->d_status);
+        const int rc = check_launch(e);
+        if (rc) return rc;
+        k_expand_insert<TPC, true><<<g, kThreads, 0, e->stream>>>(
+            view(P), e->td, table, tmask, e->d_status, split_log2(P.n, g), fcr_up, next, ids);
+    } else {
+        k_expand_insert<TPC, false><<<g, kThreads, 0, e->stream>>>(
+            view(P), e->td, table, tmask, e->d_status, split_log2(P.n, g), fcr_up, next, ids);
+    }
     return check_launch(e);
+}
+
+/* Scratch for the column ids of an expansion of level P, from the arena's
+   top (given back by the caller); no ids (tab null) where it does not fit a
+   quarter of the free arena, so that no level that fits without it stops
+   fitting, or where the level is too small to gain: at 159 to 311 parents the
+   insert takes 0.06-0.08 ms with ids and 0.08-0.11 without, at one parent the
+   extra pass and the clearing cost more than there is to compare. */
+constexpr uint64_t kIdParents = 64;
+int alloc_ids(pcagb_engine *e, const Level &P, IdDev *out)
+{
+    IdDev D{};
+    *out = D;
+    if (P.n < kIdParents) return PCAGB_OK;
+    const GenTables &gt = gen_tables();
+    uint64_t classes = 0;
+    for (size_t i = 0; i < P.hist.size(); i++)
+        if (P.hist[i] && e->h_active[i >> 7]) {
+            D.stride = std::max(D.stride, (uint32_t)gt.nvc((int)(i & 127)));
+            classes += P.hist[i] * (uint64_t)gt.nvc((int)(i & 127));
+        }
+    /* distinct columns: at most the registers and classes together, measured
+       a tenth of that; warps drop parts of their batches */
+    const uint64_t warps = (uint64_t)e->grid(e->occ_insert) * kWarpsPerBlock;
+    const uint64_t cap = std::min<uint64_t>((classes + 7 * P.n) / 4 + warps * kIdBatch, 1u << 30);
+    uint64_t slots = 1024;
+    while (slots < 2 * cap) slots <<= 1;
+    const uint64_t bytes = slots * 8 + cap * e->TPC * 2 + P.n * 32 + P.n * D.stride * 20;
+    if (bytes > (e->top - e->bottom) / 4) return PCAGB_OK;
+    D.tab = (unsigned long long *)e->alloc_top(slots * 8);
+    D.cols = (uint64_t *)e->alloc_top(cap * e->TPC * 2);
+    D.ids = (uint32_t *)e->alloc_top(P.n * 32);
+    D.cls_id = (uint32_t *)e->alloc_top(P.n * D.stride * 4);
+    D.cls_flags = (uint4 *)e->alloc_top(P.n * D.stride * 16);
+    if (!D.tab || !D.cols || !D.ids || !D.cls_id || !D.cls_flags) return PCAGB_OK;
+    D.mask = slots - 1;
+    D.cap = (uint32_t)cap;
+    D.next = reinterpret_cast<uint32_t *>(e->d_small + 5);
+    CK(cudaMemsetAsync(D.next, 0, 4, e->stream));
+    CK(cudaMemsetAsync(D.tab, 0, slots * 8, e->stream));
+    *out = D;
+    return PCAGB_OK;
 }
 
 template <int TPC>
@@ -448,11 +498,21 @@ int launch_materialize(pcagb_engine *e, const Level &P, const uint32_t *fcr_up,
  * free arena is materialised into space for every child and its survivor
  * count, status, scan total and histogram come back in one round trip; a
  * larger level reads the survivor count first and allocates exactly. */
-int build_level(pcagb_engine *e, int d, bool lean = false)
+int build_level(pcagb_engine *e, int d, bool lean = false, bool use_ids = true)
 {
     const GenTables &gt = gen_tables();
     Level &P = e->levels[d];
     const size_t bottom0 = e->bottom, top0 = e->top;
+    bool with_ids = false;
+    /* the ids ran out: once more without them */
+    auto retry = [&]() -> int {
+        e->bottom = bottom0;
+        e->top = top0;
+        P.child_off = nullptr;
+        P.fcr = nullptr;
+        CK(cudaMemsetAsync(e->d_status, 0, 4, e->stream));
+        return build_level(e, d, lean, false);
+    };
     auto fail = [&](int rc) {
         e->bottom = bottom0;
         e->top = top0;
@@ -531,9 +591,17 @@ int build_level(pcagb_engine *e, int d, bool lean = false)
         CK(cudaMemsetAsync(bitmap, 0, words * 4 + 4, e->stream));
         CK(cudaMemsetAsync(e->d_small + 2, 0, 8, e->stream));
         cudaEventRecord(e->ev2, e->stream);
-        int rc = e->TPC == 16 ? launch_expand<16>(e, P, fcr_up, table, slots - 1)
-                              : launch_expand<32>(e, P, fcr_up, table, slots - 1);
+        /* the column ids' scratch lives on the top only while the insert
+           runs, as the twins' table above */
+        const size_t top_ids = e->top;
+        IdDev ids{};
+        int rc = use_ids ? alloc_ids(e, P, &ids) : PCAGB_OK;
         if (rc) return rc;
+        rc = e->TPC == 16 ? launch_expand<16>(e, P, fcr_up, table, slots - 1, ids)
+                          : launch_expand<32>(e, P, fcr_up, table, slots - 1, ids);
+        if (rc) return rc;
+        e->top = top_ids;
+        with_ids = ids.tab != nullptr;
         cudaEventRecord(e->ev3, e->stream);
         k_mark<<<e->grid(4), 256, 0, e->stream>>>(table, slots, P.child_off, bitmap,
                                                   e->d_small + 2);
@@ -544,6 +612,7 @@ int build_level(pcagb_engine *e, int d, bool lean = false)
                   e->stream));
         if (!one_sync) {
             CK(cudaStreamSynchronize(e->stream));
+            if (with_ids && (uint32_t)e->h_pin[kPinStatus] == kStatusColumns) return retry();
             if ((uint32_t)e->h_pin[kPinStatus]) {
                 set_err("expansion of level %d hit a device limit (status %u)", d + 1,
                         (uint32_t)e->h_pin[kPinStatus]);
@@ -587,6 +656,11 @@ int build_level(pcagb_engine *e, int d, bool lean = false)
     if (rc) return rc;
     CK(cudaStreamSynchronize(e->stream));
     if (one_sync && !e->no_oep) {
+        if (with_ids && (uint32_t)e->h_pin[kPinStatus] == kStatusColumns) {
+            e->insert_launches--;
+            e->insert_children -= children;
+            return retry();
+        }
         if ((uint32_t)e->h_pin[kPinStatus]) {
             set_err("expansion of level %d hit a device limit (status %u)", d + 1,
                     (uint32_t)e->h_pin[kPinStatus]);
@@ -1749,6 +1823,27 @@ int ensure_device_tables(int device)
         const uint16_t *prap = pra_d, *cop = co_d;
         CK(cudaMemcpyToSymbol(c_pr_at, &prap, sizeof prap));
         CK(cudaMemcpyToSymbol(c_cand_of, &cop, sizeof cop));
+        std::vector<uint16_t> kid(gt.cand_of);
+        for (int m = 0; m < 128; m++)
+            for (uint32_t i = gt.vc_off[m] * 8; i < gt.vc_off[m + 1] * 8; i++)
+                if (kid[i] != 0xFFFF && gt.cand_dupe[gt.cand_off[m] + kid[i]]) kid[i] = 0xFFFF;
+        std::vector<uint2> ck2(gt.cand_uop.size());
+        for (size_t i = 0; i < ck2.size(); i++) ck2[i] = make_uint2(gt.cand_uop[i], gt.cand_vc[i]);
+        uint2 *ck2_d = nullptr;
+        uint32_t *coff_d = nullptr;
+        CK(cudaMalloc(&ck2_d, ck2.size() * sizeof(uint2)));
+        CK(cudaMalloc(&coff_d, 129 * 4));
+        CK(cudaMemcpy(ck2_d, ck2.data(), ck2.size() * sizeof(uint2), cudaMemcpyHostToDevice));
+        CK(cudaMemcpy(coff_d, gt.cand_off.data(), 129 * 4, cudaMemcpyHostToDevice));
+        const uint2 *ck2p = ck2_d;
+        const uint32_t *coffp = coff_d;
+        CK(cudaMemcpyToSymbol(c_cand_k, &ck2p, sizeof ck2p));
+        CK(cudaMemcpyToSymbol(c_cand_off_g, &coffp, sizeof coffp));
+        uint16_t *kid_d = nullptr;
+        CK(cudaMalloc(&kid_d, kid.size() * 2));
+        CK(cudaMemcpy(kid_d, kid.data(), kid.size() * 2, cudaMemcpyHostToDevice));
+        const uint16_t *kidp = kid_d;
+        CK(cudaMemcpyToSymbol(c_kid, &kidp, sizeof kidp));
         uint32_t *evm_d = nullptr;
         CK(cudaMalloc(&evm_d, gt.ev_mid.size() * 4));
         CK(cudaMemcpy(evm_d, gt.ev_mid.data(), gt.ev_mid.size() * 4, cudaMemcpyHostToDevice));
@@ -1776,13 +1871,13 @@ int ensure_device_tables(int device)
     CK(cudaMemcpy(chunks, gt.chunks.data(), gt.chunks.size() * 4, cudaMemcpyHostToDevice));
     CK(cudaMemcpyToSymbol(c_cand_off, gt.cand_off.data(), 129 * 4));
     CK(cudaMemcpyToSymbol(c_vc_off, gt.vc_off.data(), 129 * 4));
-    CK(cudaMemcpyToSymbol(c_chunk_off, gt.chunk_off.data(), 129 * 4));
+    CK(cudaMemcpyToSymbol(c_vchunk_off, gt.chunk_off.data(), 129 * 4));
     const uint32_t *cu = cand_uop, *vu = vc_uop, *ck = chunks;
     const uint16_t *vf = vc_first;
     CK(cudaMemcpyToSymbol(c_cand_uop, &cu, sizeof cu));
     CK(cudaMemcpyToSymbol(c_vc_uop, &vu, sizeof vu));
     CK(cudaMemcpyToSymbol(c_vc_first, &vf, sizeof vf));
-    CK(cudaMemcpyToSymbol(c_chunks, &ck, sizeof ck));
+    CK(cudaMemcpyToSymbol(c_vchunks, &ck, sizeof ck));
     CK(cudaDeviceSynchronize());
     g_tables_ready[device] = true;
     return PCAGB_OK;
@@ -1867,7 +1962,9 @@ int engine_init(pcagb_engine *e, int device, size_t budget)
         PCAGB_PRELOAD(k_suffix_states<16, 2>); PCAGB_PRELOAD(k_suffix_states<32, 2>);
         PCAGB_PRELOAD(k_suffix_states<16, 3>); PCAGB_PRELOAD(k_suffix_states<32, 3>);
         PCAGB_PRELOAD(k_setup<16>); PCAGB_PRELOAD(k_setup<32>);
-        PCAGB_PRELOAD(k_expand_insert<16>); PCAGB_PRELOAD(k_expand_insert<32>);
+        PCAGB_PRELOAD(k_expand_insert<16, true>); PCAGB_PRELOAD(k_expand_insert<32, true>);
+        PCAGB_PRELOAD(k_expand_insert<16, false>); PCAGB_PRELOAD(k_expand_insert<32, false>);
+        PCAGB_PRELOAD(k_state_ids<16>); PCAGB_PRELOAD(k_state_ids<32>);
         PCAGB_PRELOAD(k_materialize<16>); PCAGB_PRELOAD(k_materialize<32>);
         PCAGB_PRELOAD(k_twins<16>); PCAGB_PRELOAD(k_twins<32>);
         PCAGB_PRELOAD(k_leaf<16>); PCAGB_PRELOAD(k_leaf<32>);
@@ -1880,12 +1977,16 @@ int engine_init(pcagb_engine *e, int device, size_t budget)
         cudaGetLastError();
         /* the insert kernel keeps each warp's children in shared memory:
            its occupancy needs the largest shared-memory carveout */
-        cudaFuncSetAttribute(k_expand_insert<32>, cudaFuncAttributePreferredSharedMemoryCarveout,
-                             cudaSharedmemCarveoutMaxShared);
-        cudaFuncSetAttribute(k_expand_insert<16>, cudaFuncAttributePreferredSharedMemoryCarveout,
-                             cudaSharedmemCarveoutMaxShared);
+        const auto carve = [](auto *kernel) {
+            cudaFuncSetAttribute(kernel, cudaFuncAttributePreferredSharedMemoryCarveout,
+                                 cudaSharedmemCarveoutMaxShared);
+        };
+        carve(k_expand_insert<16, true>);
+        carve(k_expand_insert<32, true>);
+        carve(k_expand_insert<16, false>);
+        carve(k_expand_insert<32, false>);
         int nb = 0;
-        if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, k_expand_insert<32>, kThreads, 0) ==
+        if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, k_expand_insert<32, true>, kThreads, 0) ==
                 cudaSuccess && nb > 0)
             e->occ_insert = nb;
         if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, k_suffix<32, 1, 2>, kThreads, 0) ==

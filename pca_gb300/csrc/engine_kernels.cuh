@@ -65,8 +65,12 @@ __constant__ const uint32_t *c_cand_uop;   /* bit 31: a same-state duplicate of 
 __constant__ const uint32_t *c_vc_uop;
 __constant__ const uint16_t *c_vc_first;   /* first candidate index per class */
 __constant__ const uint8_t *c_vc_n;        /* candidates per class */
-__constant__ uint32_t c_chunk_off[129];    /* op-uniform runs of candidates */
-__constant__ const uint32_t *c_chunks;
+__constant__ uint32_t c_vchunk_off[129];   /* op-uniform runs of value classes */
+__constant__ const uint32_t *c_vchunks;    /* first class << 8 | classes (at most 32) */
+__constant__ const uint2 *c_cand_k;        /* micro-op and value class of each candidate */
+__constant__ const uint32_t *c_cand_off_g; /* c_cand_off in global memory (lanes of different masks) */
+__constant__ const uint16_t *c_kid;        /* [class][8] candidate of the class by destination;
+                                              0xFFFF: none, or a same-state duplicate */
 __constant__ uint32_t c_vcr_off[128 * 8 + 1]; /* [mask*8 + r]: classes reading r */
 __constant__ const uint32_t *c_vcr_uop;    /* their micro-ops */
 __constant__ const uint16_t *c_vcr;        /* their indices in the mask's class list */
@@ -166,16 +170,13 @@ __device__ __forceinline__ uint64_t task_final(uint32_t task)
     return fmix64(0x9E3779B97F4A7C15ull * (task + 1));
 }
 
-template <int TPC, typename E>
-__device__ __forceinline__ uint64_t hash_column(const E *col)
+/* a column's hash, two tests to a word */
+template <int TPC>
+__device__ __forceinline__ uint64_t hash_column(const uint32_t *col)
 {
     uint64_t h = 0x243F6A8885A308D3ull;
 #pragma unroll
-    for (int t = 0; t < TPC; t += 4) {
-        uint64_t w = (uint64_t)col[t] | ((uint64_t)col[t + 1] << 16) |
-                     ((uint64_t)col[t + 2] << 32) | ((uint64_t)col[t + 3] << 48);
-        h = chain(h, w);
-    }
+    for (int t = 0; t < TPC / 2; t += 2) h = chain(h, (uint64_t)col[t + 1] << 32 | col[t]);
     return h;
 }
 
@@ -410,172 +411,326 @@ k_setup(const RootIn *in, uint32_t rounds, LevelOut L0, uint8_t *twin, SetupOut 
 
 /* ---- level expansion: insert every child into the exact table ------------ */
 
-/* One warp's shared memory in the insert kernel: its parent (16-bit columns,
-   a row stride of TPC + 2 halves so that lanes reading different operand
-   columns of one test hit different banks) and the new column and flags of
-   each lane's child in the current chunk, which the warp-wide compares read
-   instead of recomputing them. */
+/* ---- flags of a state as four planes -----------------------------------------
+   A plane (Z, N, C, V) holds one flag on every test, a bit a test: test t at
+   bit TPC/2 - 1 - t/2, the odd tests sixteen higher (two tests of a word
+   enter a plane by one shift and add). */
+template <int TPC>
+__device__ __forceinline__ uint32_t plane_bit(int t)
+{
+    return (uint32_t)(TPC / 2 - 1 - (t >> 1) + 16 * (t & 1));
+}
+
+/* the bits of the tests below T */
+template <int TPC>
+__device__ __forceinline__ uint32_t plane_mask(int T)
+{
+    const uint32_t even = (uint32_t)(T + 1) / 2, odd = (uint32_t)T / 2;
+    return ((1u << even) - 1u) << (TPC / 2 - even) | ((1u << odd) - 1u) << (TPC / 2 - odd) << 16;
+}
+
+/* One warp's shared memory in the insert kernel: its parent (two tests to a
+   word, a row stride of TPC / 2 + 1 words so that lanes reading different
+   operand columns of one test hit different banks), the column, flags and
+   hashes of each value class of the current chunk (a class a lane), and the
+   chunk's children. */
 template <int TPC>
 struct InsertState {
-    uint64_t colh[8];           /* colh[r] = col_final(r, hash(col r)), r >= 1 */
-    uint64_t flagsA[TPC / 16][32]; /* [word][lane]: the lane's child flags, 4 bits a test */
-    uint16_t R[8][TPC + 2];
-    uint16_t colA[TPC][33];     /* [test][lane]: odd stride, a test row per lane is conflict free */
+    uint4 flagsA[33];                      /* [class] Z, N, C, V planes; [32]: the parent's */
+    uint64_t colA[32][TPC / 4 + 1];        /* [class][four tests] */
+    uint64_t colh[8];                      /* colh[r] = col_final(r, hash(col r)), r >= 1 */
+    uint64_t hA[32], hfA[32];              /* [class] the column's and the flags' hash */
+    uint32_t idA[32], ids[8];              /* column ids: the classes', the parent's registers' */
+    uint32_t R[8][TPC / 2 + 1];
     uint8_t F[TPC];
+    uint8_t kids[256];                     /* class << 3 | destination */
 };
 
-template <int TPC>
-__device__ __forceinline__ void load_insert_state(InsertState<TPC> &ws, const uint16_t *regs,
-                                                  const uint8_t *flags, uint64_t q, int lane)
-{
-    if (lane < TPC) {
-        const uint16_t *src = regs + q * 8 * TPC + lane;
-#pragma unroll
-        for (int r = 0; r < 8; r++) ws.R[r][lane] = src[r * TPC];
-        ws.F[lane] = flags[q * TPC + lane];
-    }
-}
-
-/* The op is a template parameter here: a warp expands a run of candidates
-   that share one op, so the switch is resolved at compile time and the
-   lanes never diverge on it. */
-template <int OP>
-__device__ __forceinline__ uint32_t alu_t(uint32_t a, uint32_t b, uint32_t imm)
-{
-    if constexpr (OP == PCA_OP_ADD) return (a + b) & 0xFFFFu;
-    else if constexpr (OP == PCA_OP_SUB) return (a - b) & 0xFFFFu;
-    else if constexpr (OP == PCA_OP_MUL) return (a * b) & 0xFFFFu;
-    else if constexpr (OP == PCA_OP_AND) return a & b;
-    else if constexpr (OP == PCA_OP_OR) return a | b;
-    else if constexpr (OP == PCA_OP_XOR) return a ^ b;
-    else if constexpr (OP == PCA_OP_SHL) return (a << (b & 15u)) & 0xFFFFu;
-    else if constexpr (OP == PCA_OP_SHR) return a >> (b & 15u);
-    else if constexpr (OP == PCA_OP_ASR) return (uint32_t)(uint16_t)((int16_t)(uint16_t)a >> (b & 15u));
-    else if constexpr (OP == PCA_OP_LDI) return imm;
-    else return (a + (uint32_t)(int32_t)(int8_t)(uint8_t)imm) & 0xFFFFu; /* ADDI */
-}
-
-template <int OP>
-__device__ __forceinline__ uint32_t flags_t(uint32_t a, uint32_t b, uint32_t imm, uint32_t res,
-                                            uint32_t old)
-{
-    if constexpr (OP == PCA_OP_LDI) return old;
-    else if constexpr (OP == PCA_OP_ADD || OP == PCA_OP_SUB || OP == PCA_OP_MUL ||
-                       OP == PCA_OP_ADDI)
-        return pca_alu_flags(OP, a, b, imm, res, old);
-    else return pca_zn(res);
-}
-
-/* Hash of the child's new column (chain over 4 tests per word) and of its
-   flags (16 tests per word), tests >= T contributing zeros; the column and
-   the flags are also left in the warp's shared memory for the compares. The
-   loop over word groups is kept rolled: eleven op variants of a fully
-   unrolled loop overflow the instruction cache. */
+/* A class's new column and flags, two tests to a word; the op is a template
+   parameter: a warp takes a run of classes that share one, so the switch is
+   resolved at compile time and the lanes never diverge on it. Leaves the
+   column and the planes in shared memory and returns their hashes (tests >= T
+   are zero in both). */
 template <int TPC, int OP>
-__device__ __forceinline__ void child_hashes(InsertState<TPC> &ws, uint32_t ra, uint32_t rb,
+__device__ __forceinline__ void class_values(InsertState<TPC> &ws, uint32_t ra, uint32_t rb,
                                              uint32_t imm, int T, int lane, uint64_t &h,
                                              uint64_t &hf)
 {
+    const uint32_t imm2 = OP == PCA_OP_LDI ? imm * 0x10001u
+                                           : (uint32_t)(uint16_t)(int16_t)(int8_t)(uint8_t)imm * 0x10001u;
+    constexpr bool kCarry = OP == PCA_OP_ADD || OP == PCA_OP_SUB || OP == PCA_OP_MUL ||
+                            OP == PCA_OP_ADDI;
+    constexpr bool kOver = kCarry && OP != PCA_OP_MUL;
+    uint32_t Z = 0, N = 0, C = 0, V = 0;
     h = 0x243F6A8885A308D3ull;
-    hf = 0x13198A2E03707344ull;
-    uint64_t wf = 0;
 #pragma unroll 1
-    for (int t0 = 0; t0 < TPC; t0 += 4) {
-        uint64_t w = 0;
+    for (int i = 0; i < TPC / 4; i++) {
+        uint32_t v[2];
 #pragma unroll
-        for (int j = 0; j < 4; j++) {
-            const int t = t0 + j;
-            const uint32_t a = ws.R[ra][t], b = ws.R[rb][t];
-            uint32_t res = alu_t<OP>(a, b, imm);
-            uint32_t f = flags_t<OP>(a, b, imm, res, ws.F[t]);
-            if (t >= T) { res = 0; f = 0; }
-            ws.colA[t][lane] = (uint16_t)res;
-            w |= (uint64_t)res << (16 * j);
-            wf |= (uint64_t)f << (4 * (t & 15));
+        for (int k = 0; k < 2; k++) {
+            const uint32_t a = ws.R[ra][2 * i + k];
+            const uint32_t b = OP == PCA_OP_ADDI ? imm2 : ws.R[rb][2 * i + k];
+            uint32_t r, c = 0, o = 0;
+            if constexpr (OP == PCA_OP_ADD || OP == PCA_OP_ADDI) {
+                r = add2(a, b);
+                c = (a & b) | ((a | b) & ~r);
+                o = ~(a ^ b) & (a ^ r);
+            } else if constexpr (OP == PCA_OP_SUB) {
+                r = sub2(a, b);
+                c = ~((~a & b) | ((~a | b) & r));   /* no borrow */
+                o = (a ^ b) & (a ^ r);
+            } else if constexpr (OP == PCA_OP_MUL) {
+                const uint32_t p0 = (a & 0xFFFFu) * (b & 0xFFFFu), p1 = (a >> 16) * (b >> 16);
+                r = halves(p0, p1 << 16);
+                c = (p0 > 0xFFFFu ? 0x8000u : 0u) | (p1 > 0xFFFFu ? 0x80000000u : 0u);
+            } else if constexpr (OP == PCA_OP_AND) r = a & b;
+            else if constexpr (OP == PCA_OP_OR) r = a | b;
+            else if constexpr (OP == PCA_OP_XOR) r = a ^ b;
+            else if constexpr (OP == PCA_OP_SHL) r = shl2(a, b);
+            else if constexpr (OP == PCA_OP_SHR) r = shr2(a, b);
+            else if constexpr (OP == PCA_OP_ASR) r = asr2(a, b);
+            else r = imm2;
+            if constexpr (OP != PCA_OP_LDI) {
+                const uint32_t nz = ((r & 0x7FFF7FFFu) + 0x7FFF7FFFu) | r;
+                Z = Z * 2 + (~nz >> 15 & 0x10001u);
+                N = N * 2 + (r >> 15 & 0x10001u);
+                if constexpr (kCarry) C = C * 2 + (c >> 15 & 0x10001u);
+                if constexpr (kOver) V = V * 2 + (o >> 15 & 0x10001u);
+            }
+            v[k] = r;
         }
+        const int left = T - 4 * i;   /* tests of this word */
+        if (left < 4) {
+            v[0] = left >= 2 ? v[0] : left == 1 ? v[0] & 0xFFFFu : 0u;
+            v[1] = left == 3 ? v[1] & 0xFFFFu : 0u;
+        }
+        const uint64_t w = (uint64_t)v[1] << 32 | v[0];
+        ws.colA[lane][i] = w;
         h = chain(h, w);
-        if ((t0 & 15) == 12) {
-            hf = chain(hf, wf);
-            ws.flagsA[t0 >> 4][lane] = wf;
-            wf = 0;
-        }
     }
+    uint4 f;
+    if constexpr (OP == PCA_OP_LDI) {
+        f = ws.flagsA[32];
+    } else {
+        const uint32_t m = plane_mask<TPC>(T);
+        f = make_uint4(Z & m, N & m, C & m, V & m);
+    }
+    ws.flagsA[lane] = f;
+    hf = chain(chain(0x13198A2E03707344ull, (uint64_t)f.y << 32 | f.x), (uint64_t)f.w << 32 | f.z);
 }
 
 template <int TPC>
-__device__ __forceinline__ void child_hashes_any(uint32_t op, InsertState<TPC> &ws, uint32_t ra,
+__device__ __forceinline__ void class_values_any(uint32_t op, InsertState<TPC> &ws, uint32_t ra,
                                                  uint32_t rb, uint32_t imm, int T, int lane,
                                                  uint64_t &h, uint64_t &hf)
 {
     switch (op) {
-    case PCA_OP_ADD: child_hashes<TPC, PCA_OP_ADD>(ws, ra, rb, imm, T, lane, h, hf); break;
-    case PCA_OP_SUB: child_hashes<TPC, PCA_OP_SUB>(ws, ra, rb, imm, T, lane, h, hf); break;
-    case PCA_OP_MUL: child_hashes<TPC, PCA_OP_MUL>(ws, ra, rb, imm, T, lane, h, hf); break;
-    case PCA_OP_AND: child_hashes<TPC, PCA_OP_AND>(ws, ra, rb, imm, T, lane, h, hf); break;
-    case PCA_OP_OR: child_hashes<TPC, PCA_OP_OR>(ws, ra, rb, imm, T, lane, h, hf); break;
-    case PCA_OP_XOR: child_hashes<TPC, PCA_OP_XOR>(ws, ra, rb, imm, T, lane, h, hf); break;
-    case PCA_OP_SHL: child_hashes<TPC, PCA_OP_SHL>(ws, ra, rb, imm, T, lane, h, hf); break;
-    case PCA_OP_SHR: child_hashes<TPC, PCA_OP_SHR>(ws, ra, rb, imm, T, lane, h, hf); break;
-    case PCA_OP_ASR: child_hashes<TPC, PCA_OP_ASR>(ws, ra, rb, imm, T, lane, h, hf); break;
-    case PCA_OP_LDI: child_hashes<TPC, PCA_OP_LDI>(ws, ra, rb, imm, T, lane, h, hf); break;
-    default: child_hashes<TPC, PCA_OP_ADDI>(ws, ra, rb, imm, T, lane, h, hf); break;
+    case PCA_OP_ADD: class_values<TPC, PCA_OP_ADD>(ws, ra, rb, imm, T, lane, h, hf); break;
+    case PCA_OP_SUB: class_values<TPC, PCA_OP_SUB>(ws, ra, rb, imm, T, lane, h, hf); break;
+    case PCA_OP_MUL: class_values<TPC, PCA_OP_MUL>(ws, ra, rb, imm, T, lane, h, hf); break;
+    case PCA_OP_AND: class_values<TPC, PCA_OP_AND>(ws, ra, rb, imm, T, lane, h, hf); break;
+    case PCA_OP_OR: class_values<TPC, PCA_OP_OR>(ws, ra, rb, imm, T, lane, h, hf); break;
+    case PCA_OP_XOR: class_values<TPC, PCA_OP_XOR>(ws, ra, rb, imm, T, lane, h, hf); break;
+    case PCA_OP_SHL: class_values<TPC, PCA_OP_SHL>(ws, ra, rb, imm, T, lane, h, hf); break;
+    case PCA_OP_SHR: class_values<TPC, PCA_OP_SHR>(ws, ra, rb, imm, T, lane, h, hf); break;
+    case PCA_OP_ASR: class_values<TPC, PCA_OP_ASR>(ws, ra, rb, imm, T, lane, h, hf); break;
+    case PCA_OP_LDI: class_values<TPC, PCA_OP_LDI>(ws, ra, rb, imm, T, lane, h, hf); break;
+    default: class_values<TPC, PCA_OP_ADDI>(ws, ra, rb, imm, T, lane, h, hf); break;
     }
 }
 
-/* Exact compare of child A (lane jA's child of the warp's parent, its new
-   column and flags in shared memory, micro-op uA) with child B (parent qB of
-   the level in HBM + micro-op uB), the whole warp cooperating: lane t
-   rebuilds test t of child B (every register, the flags) and __all_sync
-   decides. The requesting lane has already checked the task and (when it is
-   part of the key) the live mask. All lanes must call it. */
-template <int TPC>
-__device__ bool warp_child_equal(const LevelDev &P, const InsertState<TPC> &A, uint64_t qA, int T,
-                                 int jA, uint32_t uA, uint64_t qB, uint32_t uB, int lane)
+/* ---- exact column ids --------------------------------------------------------
+   Every distinct register column met while a level is expanded (its states'
+   registers, its classes' values) gets an id from an exact table: a column is
+   written to `cols` under a fresh id, then published in a slot [tag 24][id + 1:
+   40]; a tag match is settled by comparing the whole column. Equal ids are
+   equal columns and equal columns have equal ids, so two children are the
+   same state when their register ids and flag planes are: a lane compares its
+   own, where comparing the columns takes the warp and a hundred instructions
+   a pair. The table and the arrays live only while the level is expanded. */
+struct IdDev {
+    unsigned long long *tab;   /* [mask + 1] slots; null: no ids (compare columns) */
+    uint64_t mask;
+    uint64_t *cols;            /* [cap][TPC / 4] */
+    uint32_t cap;
+    uint32_t *next;            /* ids given out, kIdBatch at a time to a warp */
+    uint32_t *ids;             /* [n][8] of the level's registers; r0's place: task << 8 | live */
+    uint32_t *cls_id;          /* [n][stride] of its classes' columns */
+    uint4 *cls_flags;          /* [n][stride] planes of its classes */
+    uint32_t stride;
+};
+constexpr uint32_t kIdBatch = 64;
+constexpr uint32_t kStatusColumns = 4u;    /* out of ids or slots: expand without them */
+
+__device__ __forceinline__ unsigned long long load_acquire(const unsigned long long *p)
 {
-    const uint32_t rdA = UOP_RD(uA), rdB = UOP_RD(uB);
+    unsigned long long v;
+    asm volatile("ld.acquire.gpu.global.u64 %0, [%1];" : "=l"(v) : "l"(p) : "memory");
+    return v;
+}
+
+/* A warp's ids not yet used: [at, end). */
+struct IdPool {
+    uint32_t at = 0, end = 0;
+};
+
+/* The id of this lane's column (col, hash h) where `want`; all lanes call it. */
+template <int TPC>
+__device__ __forceinline__ uint32_t intern(const IdDev &D, const uint64_t *col, uint64_t h,
+                                           bool want, IdPool &pool, uint32_t *status, int lane)
+{
+    const uint64_t H = fmix64(h);
+    const unsigned long long tag = H >> 40;
+    uint64_t idx = H & D.mask;
+    uint32_t mine = ~0u, id = 0, probes = 0;
+    bool done = !want;
+    while (__any_sync(0xFFFFFFFFu, !done)) {
+        unsigned long long s = done ? 1ull : load_acquire(&D.tab[idx]);
+        const bool need = !done && s == 0 && mine == ~0u;
+        const uint32_t bal = __ballot_sync(0xFFFFFFFFu, need);
+        if (bal) {
+            const uint32_t n = __popc(bal);
+            if (pool.end - pool.at < n) {   /* the rest of the old batch is dropped */
+                uint32_t b = 0;
+                if (lane == 0) b = atomicAdd(D.next, kIdBatch);
+                pool.at = __shfl_sync(0xFFFFFFFFu, b, 0);
+                pool.end = pool.at + kIdBatch;
+            }
+            if (need) {
+                mine = pool.at + __popc(bal & ((1u << lane) - 1u));
+                if (mine >= D.cap) {
+                    atomicOr(status, kStatusColumns);
+                    done = true;
+                } else {
+                    uint4 *dst = reinterpret_cast<uint4 *>(D.cols + (uint64_t)mine * (TPC / 4));
+#pragma unroll
+                    for (int i = 0; i < TPC / 8; i++)
+                        dst[i] = make_uint4((uint32_t)col[2 * i], (uint32_t)(col[2 * i] >> 32),
+                                            (uint32_t)col[2 * i + 1], (uint32_t)(col[2 * i + 1] >> 32));
+                    __threadfence();
+                }
+            }
+            pool.at += n;
+        }
+        if (!done && s == 0) {
+            s = atomicCAS(&D.tab[idx], 0ull, tag << 40 | (mine + 1ull));
+            if (s == 0) {
+                id = mine;
+                done = true;
+            } else {
+                __threadfence();   /* its column, published before the slot */
+            }
+        }
+        if (!done) {
+            bool eq = (s >> 40) == tag;
+            if (eq) {
+                const uint32_t o = (uint32_t)(s & kRefMask) - 1u;
+                const uint4 *src = reinterpret_cast<const uint4 *>(D.cols + (uint64_t)o * (TPC / 4));
+#pragma unroll
+                for (int i = 0; i < TPC / 8; i++) {
+                    const uint4 w = __ldcg(src + i);
+                    eq &= col[2 * i] == ((uint64_t)w.y << 32 | w.x) &&
+                          col[2 * i + 1] == ((uint64_t)w.w << 32 | w.z);
+                }
+                if (eq) {
+                    id = o;
+                    done = true;
+                }
+            }
+            if (!eq) {
+                idx = (idx + 1) & D.mask;
+                if (++probes >= kMaxProbes) {
+                    atomicOr(status, kStatusColumns);
+                    done = true;
+                }
+            }
+        }
+    }
+    return id;
+}
+
+/* Ids of a level's registers: eight lanes a state, a register each. */
+template <int TPC>
+__global__ void __launch_bounds__(kThreads)
+k_state_ids(LevelDev P, IdDev D, uint32_t *status)
+{
+    __shared__ uint64_t sc[kWarpsPerBlock][32][TPC / 4 + 1];
+    const int lane = threadIdx.x & 31, r = lane & 7;
+    uint64_t *col = sc[threadIdx.x >> 5][lane];
+    IdPool pool;
+    const uint64_t nw = (uint64_t)gridDim.x * kWarpsPerBlock;
+    for (uint64_t w = ((uint64_t)blockIdx.x * kThreads + threadIdx.x) >> 5; w * 4 < P.n; w += nw) {
+        const uint64_t q = w * 4 + (lane >> 3);
+        const bool want = q < P.n && r;
+        uint64_t h = 0x243F6A8885A308D3ull;
+        if (want) {
+            const uint4 *src = reinterpret_cast<const uint4 *>(P.regs + (q * 8 + r) * TPC);
+#pragma unroll
+            for (int i = 0; i < TPC / 8; i++) {
+                const uint4 v = src[i];
+                col[2 * i] = (uint64_t)v.y << 32 | v.x;
+                col[2 * i + 1] = (uint64_t)v.w << 32 | v.z;
+                h = chain(chain(h, col[2 * i]), col[2 * i + 1]);
+            }
+        }
+        const uint32_t id = intern<TPC>(D, col, h, want, pool, status, lane);
+        if (q < P.n) D.ids[q * 8 + r] = r ? id : (uint32_t)P.task[q] << 8 | P.live[q];
+    }
+}
+
+/* Exact compare of child A (class jA of the warp's parent written to rdA; its
+   column and flags in shared memory) with child B (parent qB of the level in
+   HBM + micro-op uB), the whole warp cooperating: lane t rebuilds test t of
+   child B (every register, the flags) and __all_sync decides. The requesting
+   lane has already checked the task and (when it is part of the key) the live
+   mask. All lanes must call it. Used where a level's column ids do not fit. */
+template <int TPC>
+__device__ bool warp_child_equal(const LevelDev &P, const InsertState<TPC> &A, int T, int jA,
+                                 uint32_t rdA, uint64_t qB, uint32_t uB, int lane)
+{
     bool ok = true;
     if (lane < T) {
-        const uint32_t resA = A.colA[lane][jA];
-        const uint32_t fA = (uint32_t)(A.flagsA[lane >> 4][jA] >> (4 * (lane & 15))) & 15u;
-        if (qB == qA) {
-            /* same parent (about a fifth of the duplicates): only the written
-               columns and the flags can differ, and the parent is in shared
-               memory */
-            const uint32_t a2 = A.R[UOP_A(uB)][lane], b2 = A.R[UOP_B(uB)][lane];
-            const uint32_t resB = pca_alu(UOP_OP(uB), a2, b2, UOP_IMM(uB));
-            const uint32_t fB = pca_alu_flags(UOP_OP(uB), a2, b2, UOP_IMM(uB), resB, A.F[lane]);
-            ok = fA == fB;
-            if (rdA == rdB) {
-                ok &= resA == resB;
-            } else {
-                ok &= resA == A.R[rdA][lane];   /* B keeps the parent's rdA column */
-                ok &= resB == A.R[rdB][lane];   /* A keeps the parent's rdB column */
-            }
-        } else {
-            const uint16_t *RB = P.regs + qB * 8 * TPC + lane;
-            const uint32_t a2 = RB[UOP_A(uB) * TPC], b2 = RB[UOP_B(uB) * TPC];
-            const uint32_t resB = pca_alu(UOP_OP(uB), a2, b2, UOP_IMM(uB));
-            const uint32_t fB = pca_alu_flags(UOP_OP(uB), a2, b2, UOP_IMM(uB), resB,
-                                              P.flags[qB * TPC + lane]);
-            ok = fA == fB;
+        const uint32_t rdB = UOP_RD(uB);
+        const uint32_t resA = reinterpret_cast<const uint16_t *>(A.colA[jA])[lane];
+        const uint4 f = A.flagsA[jA];
+        const uint32_t b = plane_bit<TPC>(lane);
+        const uint32_t fA = (f.x >> b & 1u) | (f.y >> b & 1u) << 1 | (f.z >> b & 1u) << 2 |
+                            (f.w >> b & 1u) << 3;
+        const uint16_t *RB = P.regs + qB * 8 * TPC + lane;
+        const uint32_t a2 = RB[UOP_A(uB) * TPC], b2 = RB[UOP_B(uB) * TPC];
+        const uint32_t resB = pca_alu(UOP_OP(uB), a2, b2, UOP_IMM(uB));
+        const uint32_t fB = pca_alu_flags(UOP_OP(uB), a2, b2, UOP_IMM(uB), resB,
+                                          P.flags[qB * TPC + lane]);
+        ok = fA == fB;
 #pragma unroll
-            for (uint32_t r = 1; r < 8; r++) {
-                const uint32_t vA = r == rdA ? resA : (uint32_t)A.R[r][lane];
-                const uint32_t vB = r == rdB ? resB : (uint32_t)RB[r * TPC];
-                ok &= vA == vB;
-            }
+        for (uint32_t r = 1; r < 8; r++) {
+            const uint32_t vA = r == rdA ? resA
+                                         : (uint32_t)reinterpret_cast<const uint16_t *>(A.R[r])[lane];
+            const uint32_t vB = r == rdB ? resB : (uint32_t)RB[r * TPC];
+            ok &= vA == vB;
         }
     }
     return __all_sync(0xFFFFFFFFu, ok);
 }
 
-/* Six CTAs per SM (40 registers a thread, 26 KB of shared memory a CTA at
-   32 tests): measured 3% faster than eight CTAs at 32 registers, whose
-   spills cost more than the extra warps hide. */
-template <int TPC>
-__global__ void __launch_bounds__(kThreads, 6)
+/* A child's new column and flags depend on its value class alone, not on the
+   destination, so a warp forms the values of its parent's classes, a class a
+   lane, in runs of one op, gives their columns exact ids, and then takes the
+   run's children (class, destination) that may be a representative, 32 at a
+   time. IDS: two children are compared by ids; else, on a level whose ids do
+   not fit, column by column (warp_child_equal).
+
+   Bound: memory latency (45% issue; a tag match is four dependent loads) with
+   32 warps an SM, 64 registers a thread: five CTAs of 48 registers spill and
+   measured 4% slower. Level 3 of a 32-test search (24,547 parents, 15.5M
+   children, 7.9M of them looked up, 5.3M kept): hashing each child's column
+   and comparing columns by the warp took 943M warp instructions, 1.40 ms;
+   hashing by class 695M, 1.16 ms; with ids 311M, 0.61 ms (0.75 with the
+   ids of the level's registers and the clearing of their table). */
+template <int TPC, bool IDS>
+__global__ void __launch_bounds__(kThreads, 4)
 k_expand_insert(LevelDev P, TaskDev task, unsigned long long *table, uint64_t tmask,
-                uint32_t *status, uint32_t split_log2, const uint32_t *fcr_up, uint32_t *next)
+                uint32_t *status, uint32_t split_log2, const uint32_t *fcr_up, uint32_t *next, IdDev D)
 {
     __shared__ InsertState<TPC> sws[kWarpsPerBlock];
     const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
@@ -591,6 +746,7 @@ k_expand_insert(LevelDev P, TaskDev task, unsigned long long *table, uint64_t tm
        measured 1.59 -> 1.48 ms per solve). Items < 2^33 (levels below 2^28
        states, slices only for levels below 2^12). */
     const uint64_t items = P.n << split_log2;
+    IdPool pool;
     uint32_t nx = 0;
     if (lane == 0) nx = atomicAdd(next, 1u);
     for (uint64_t it = __shfl_sync(0xFFFFFFFFu, nx, 0); it < items;
@@ -602,38 +758,79 @@ k_expand_insert(LevelDev P, TaskDev task, unsigned long long *table, uint64_t tm
         if (!task.active[tid]) continue;
         const int T = task.T[tid];
         __syncwarp();
-        load_insert_state<TPC>(ws, P.regs, P.flags, q, lane);
+        if (lane < TPC) {
+            const uint4 w = reinterpret_cast<const uint4 *>(P.regs + q * 8 * TPC)[lane];
+            uint32_t *row = &ws.R[lane / (TPC / 8)][lane % (TPC / 8) * 4];
+            row[0] = w.x; row[1] = w.y; row[2] = w.z; row[3] = w.w;
+            ws.F[lane] = P.flags[q * TPC + lane];
+        }
+        if (IDS && lane < 8) ws.ids[lane] = D.ids[q * 8 + lane];
         const uint32_t live = P.live[q];
         __syncwarp();
         if (lane >= 1 && lane < 8) ws.colh[lane] = col_final(lane, hash_column<TPC>(ws.R[lane]));
+        if (lane >= 8 && lane < 12) {   /* the parent's flags, a plane a lane */
+            uint32_t x = 0;
+            for (int t = 0; t < TPC; t += 2)
+                x = x * 2 + (ws.F[t] >> (lane - 8) & 1u) + ((ws.F[t + 1] >> (lane - 8) & 1u) << 16);
+            reinterpret_cast<uint32_t *>(&ws.flagsA[32])[lane - 8] = x;
+        }
         __syncwarp();
         uint64_t regsum = task_final(tid);
 #pragma unroll
         for (int r = 1; r < 8; r++) regsum += ws.colh[r];
         const uint32_t m = (live >> 1) & 127u;
-        const uint32_t base = c_cand_off[m];
-        const uint32_t k0 = c_chunk_off[m], k1 = c_chunk_off[m + 1];
+        const uint32_t v0 = c_vc_off[m];
+        const uint32_t k0 = c_vchunk_off[m], k1 = c_vchunk_off[m + 1];
         const uint32_t per = (k1 - k0 + split - 1) >> split_log2;
         const uint32_t ka = min(k1, k0 + g * per), kb = min(k1, ka + per);
         const uint32_t wdead = deadable_writes(P, fcr_up, q);
         const uint32_t wldi = fcr_up && (P.own[q] & 1u) ? P.rdl[q] : 0u;
         const bool twin_later = P.twin[q] != 0;
         for (uint32_t k = ka; k < kb; k++) {
-            const uint32_t ch = c_chunks[k], start = ch >> 8, cnt = ch & 255u;
-            bool valid = (uint32_t)lane < cnt;
-            const uint32_t c = start + (valid ? lane : 0);
-            const uint32_t u = c_cand_uop[base + c];
-            const uint32_t op = UOP_OP(u), rd = UOP_RD(u);
-            if ((wdead >> rd & 1u) && op != PCA_OP_LDI && !uop_reads(u, rd)) valid = false;
-            if (ldi_swap(u, wldi)) valid = false;
-            if (u >> 31) valid = false;   /* an earlier sibling's state (same value and flags) */
-            if (twin_later && op != PCA_OP_LDI) valid = false;   /* k_twins */
-            if (!__any_sync(0xFFFFFFFFu, valid)) continue;
-            uint64_t h, hf;
-            __syncwarp();   /* the previous chunk's compares are done with colA */
-            child_hashes_any<TPC>(op, ws, UOP_A(u), UOP_B(u), UOP_IMM(u), T, lane, h, hf);
+            const uint32_t ch = c_vchunks[k], start = ch >> 8, cnt = ch & 255u;
+            const uint32_t uv = c_vc_uop[v0 + start + min((uint32_t)lane, cnt - 1)];
+            const uint32_t op = UOP_OP(uv);
+            if (twin_later && op != PCA_OP_LDI) continue;   /* k_twins */
+            /* the children that may be a representative (c_kid leaves out
+               the same-state duplicates of an earlier sibling) */
+            uint32_t nk = 0;
+            __syncwarp();   /* the previous chunk's children are done */
+            for (uint32_t i0 = 0; i0 < cnt * 8; i0 += 32) {
+                const uint32_t i = i0 + lane, rd = i & 7u;
+                const uint32_t u = __shfl_sync(0xFFFFFFFFu, uv, (int)(i >> 3) & 31);
+                bool valid = i < cnt * 8 && c_kid[(v0 + start) * 8 + i] != 0xFFFFu;
+                const bool reads_rd = uop_reads(u, rd);
+                if ((wdead >> rd & 1u) && op != PCA_OP_LDI && !reads_rd) valid = false;
+                if (ldi_swap((u & ~(7u << 5)) | rd << 5, wldi)) valid = false;
+                const uint32_t bal = __ballot_sync(0xFFFFFFFFu, valid);
+                if (valid) ws.kids[nk + __popc(bal & ((1u << lane) - 1u))] = (uint8_t)i;
+                nk += __popc(bal);
+            }
+            if (!nk) continue;
+            {
+                uint64_t h, hf;
+                class_values_any<TPC>(op, ws, UOP_A(uv), UOP_B(uv), UOP_IMM(uv), T, lane, h, hf);
+                ws.hA[lane] = h;
+                ws.hfA[lane] = hf;
+                if (IDS) {
+                    const bool mine = (uint32_t)lane < cnt;
+                    const uint32_t id = intern<TPC>(D, ws.colA[lane], h, mine, pool, status, lane);
+                    ws.idA[lane] = id;
+                    if (mine) {
+                        const uint64_t at = q * D.stride + start + lane;
+                        D.cls_id[at] = id;
+                        D.cls_flags[at] = ws.flagsA[lane];
+                    }
+                    __threadfence();   /* before any slot names these classes */
+                }
+            }
             __syncwarp();
-            uint64_t H = regsum - ws.colh[rd] + col_final(rd, h) + hf;
+            for (uint32_t i0 = 0; i0 < nk; i0 += 32) {
+            const bool valid = i0 + lane < nk;
+            const uint32_t kid = ws.kids[valid ? i0 + lane : 0];
+            const uint32_t cls = kid >> 3, rd = kid & 7u;
+            const uint32_t c = c_kid[(v0 + start) * 8 + kid];
+            uint64_t H = regsum - ws.colh[rd] + col_final(rd, ws.hA[cls]) + ws.hfA[cls];
             if (task.key_live) H += live_final(live | (1u << rd));
             const uint64_t ref = (q << 12) | c;
             const unsigned long long mine = ((H >> 40) << 40) | (ref + 1);
@@ -646,42 +843,70 @@ k_expand_insert(LevelDev P, TaskDev task, unsigned long long *table, uint64_t tm
                 bool needcmp = false;
                 unsigned long long s = 0;
                 if (!done) {
-                    s = *((volatile unsigned long long *)&table[idx]);
+                    s = IDS ? load_acquire(&table[idx])
+                            : *((volatile unsigned long long *)&table[idx]);
                     if (s == 0) {
                         const unsigned long long old = atomicCAS(&table[idx], 0ull, mine);
-                        if (old == 0) done = true;
-                        else s = old;
+                        if (old == 0) {
+                            done = true;
+                        } else {
+                            s = old;
+                            if (IDS) __threadfence();   /* as after an acquiring load */
+                        }
                     }
                     if (!done) needcmp = (s >> 40) == (mine >> 40);
                 }
                 /* a tag match first settles the stored child's task, live
-                   mask and micro-op in its own lane (all lanes at once);
-                   only a match on those takes a warp-wide compare */
+                   mask and micro-op in its own lane (all lanes at once) */
                 uint64_t qB = 0;
-                uint32_t uB = 0;
+                uint32_t uB = 0, cB = 0;
+                uint4 b0 = make_uint4(0, 0, 0, 0), b1 = b0;   /* the parent's ids */
                 if (needcmp) {
                     const uint64_t oref = (s & kRefMask) - 1;
                     qB = oref >> 12;
-                    uint32_t liveB = live;
-                    if (qB != q) {
-                        const uint32_t tB = P.task[qB];
+                    uint32_t liveB = live, tB = tid;
+                    if (IDS) {
+                        const uint4 *src = reinterpret_cast<const uint4 *>(D.ids + qB * 8);
+                        b0 = src[0];
+                        b1 = src[1];
+                        liveB = b0.x & 0xFFu;
+                        tB = b0.x >> 8;
+                    } else if (qB != q) {
+                        tB = P.task[qB];
                         liveB = P.live[qB];
-                        needcmp = tB == tid;
                     }
-                    uB = c_cand_uop[c_cand_off[(liveB >> 1) & 127u] + (uint32_t)(oref & 4095)];
+                    needcmp = tB == tid;
+                    const uint2 k = c_cand_k[c_cand_off_g[(liveB >> 1) & 127u] + (uint32_t)(oref & 4095)];
+                    uB = k.x;
+                    cB = k.y;
                     if (task.key_live && (live | (1u << rd)) != (liveB | (1u << UOP_RD(uB))))
                         needcmp = false;
                 }
-                uint32_t req = __ballot_sync(0xFFFFFFFFu, needcmp);
                 bool eq = false;
-                while (req) {
-                    const int j = __ffs(req) - 1;
-                    req &= req - 1;
-                    const uint32_t uj = __shfl_sync(0xFFFFFFFFu, u, j);
-                    const uint32_t ubj = __shfl_sync(0xFFFFFFFFu, uB, j);
-                    const uint64_t qbj = __shfl_sync(0xFFFFFFFFu, qB, j);
-                    const bool e = warp_child_equal<TPC>(P, ws, q, T, j, uj, qbj, ubj, lane);
-                    if (lane == j) eq = e;
+                if (IDS) {
+                    if (needcmp) {
+                        const uint64_t at = qB * D.stride + cB;
+                        const uint32_t idB = __ldcg(D.cls_id + at);
+                        const uint4 fB = __ldcg(D.cls_flags + at), fA = ws.flagsA[cls];
+                        const uint32_t B[8] = {b0.x, b0.y, b0.z, b0.w, b1.x, b1.y, b1.z, b1.w};
+                        const uint32_t idA = ws.idA[cls], rdB = UOP_RD(uB);
+                        eq = fA.x == fB.x && fA.y == fB.y && fA.z == fB.z && fA.w == fB.w;
+#pragma unroll
+                        for (uint32_t r = 1; r < 8; r++)
+                            eq &= (r == rd ? idA : ws.ids[r]) == (r == rdB ? idB : B[r]);
+                    }
+                } else {
+                    uint32_t req = __ballot_sync(0xFFFFFFFFu, needcmp);
+                    while (req) {
+                        const int j = __ffs(req) - 1;
+                        req &= req - 1;
+                        const uint32_t kj = __shfl_sync(0xFFFFFFFFu, kid, j);
+                        const uint32_t ubj = __shfl_sync(0xFFFFFFFFu, uB, j);
+                        const uint64_t qbj = __shfl_sync(0xFFFFFFFFu, qB, j);
+                        const bool e = warp_child_equal<TPC>(P, ws, T, (int)(kj >> 3), kj & 7u, qbj,
+                                                             ubj, lane);
+                        if (lane == j) eq = e;
+                    }
                 }
                 if (!done) {
                     if (needcmp && eq) {
@@ -702,6 +927,7 @@ k_expand_insert(LevelDev P, TaskDev task, unsigned long long *table, uint64_t tm
                         }
                     }
                 }
+            }
             }
         }
     }

@@ -36,9 +36,9 @@ struct GenTables {
     std::vector<uint16_t> cand_vc;     /* value class index within mask    */
     std::vector<uint32_t> vc_off;      /* size 129                         */
     std::vector<uint32_t> vc_uop;      /* one micro-op per value class     */
-    /* per mask: runs of <= 32 consecutive candidates with one op, so a warp
-       expanding a state works on a single op at a time; entry =
-       start << 8 | count, start relative to the mask's candidate list */
+    /* per mask: runs of <= 32 consecutive value classes with one op, so a
+       warp expanding a state works on a single op at a time; entry =
+       start << 8 | count, start relative to the mask's class list */
     std::vector<uint32_t> chunk_off;   /* size 129 */
     std::vector<uint32_t> chunks;
     /* f[s][m]: programs decided by s more instructions from mask m:

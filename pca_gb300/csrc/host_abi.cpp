@@ -97,11 +97,11 @@ static GenTables build_tables()
     t.chunk_off.assign(129, 0);
     for (int m = 0; m < 128; m++) {
         t.chunk_off[m] = (uint32_t)t.chunks.size();
-        const uint32_t base = t.cand_off[m], n = t.cand_off[m + 1] - base;
+        const uint32_t base = t.vc_off[m], n = t.vc_off[m + 1] - base;
         uint32_t s = 0;
         while (s < n) {
             uint32_t e = s;
-            while (e < n && e - s < 32 && UOP_OP(t.cand_uop[base + e]) == UOP_OP(t.cand_uop[base + s])) e++;
+            while (e < n && e - s < 32 && UOP_OP(t.vc_uop[base + e]) == UOP_OP(t.vc_uop[base + s])) e++;
             t.chunks.push_back(s << 8 | (e - s));
             s = e;
         }
