@@ -698,10 +698,22 @@ int build_level(pcagb_engine *e, int d, bool lean = false, bool use_ids = true)
     return PCAGB_OK;
 }
 
+/* A solution: the candidate index taken at each position (its DFS-order key)
+   and the register that holds the output. */
 struct RawSol {
-    std::vector<uint16_t> kernel;  /* kernel instructions */
-    uint32_t out_reg = 0;
-    std::vector<uint32_t> key;     /* DFS-order key: candidate indices */
+    uint16_t cand[SEARCH_MAX_DEPTH];
+    uint8_t len = 0, out_reg = 0;
+};
+
+/* A solving record of a stage: prefix q of the split level, middles and value
+   class (y, as SolBuf::rec), its path at TaskRun::paths[at * SEARCH_MAX_DEPTH].
+   By (q, middles) records come in DFS order; those equal there are one
+   prefix's, whose solutions interleave by the last candidate. */
+struct Record {
+    uint64_t q, y;
+    uint32_t at;
+    uint64_t prefix() const { return y >> 16; }
+    bool operator<(const Record &o) const { return q != o.q ? q < o.q : y < o.y; }
 };
 
 /* One task of a batch, host side. */
@@ -715,6 +727,12 @@ struct TaskRun {
     uint64_t nrec = 0;
     uint64_t found = 0;            /* first-only: programs the stage found */
     std::vector<RawSol> sols;
+    /* the optimal depth's records (all solutions wanted): expanded to the
+       programs the caller takes by expand_records */
+    std::vector<Record> recs;
+    std::vector<uint16_t> paths;
+    int rec_S = 0, rec_s = 0;      /* split level and suffix depth of the records */
+    uint64_t nsols = 0;            /* programs of the records */
     double t_done = 0;
     pcagb_result_t res{};
 };
@@ -740,13 +758,87 @@ struct SolBuilder {
     explicit SolBuilder(const TaskRun &tr) : mask((tr.root.live >> 1) & 127u) {}
     uint32_t take(uint32_t c)   /* returns the register written */
     {
-        const uint32_t idx = gt.cand_off[mask] + c, rd = UOP_RD(gt.cand_uop[idx]);
-        sol.kernel.push_back(gt.cand[idx]);
-        sol.key.push_back(c);
+        const uint32_t rd = UOP_RD(gt.cand_uop[gt.cand_off[mask] + c]);
+        sol.cand[sol.len++] = (uint16_t)c;
         mask |= 1u << (rd - 1);
         return rd;
     }
 };
+
+/* the kernel's instruction words */
+std::vector<uint16_t> sol_kernel(const TaskRun &tr, const RawSol &s)
+{
+    const GenTables &gt = gen_tables();
+    uint32_t mask = (tr.root.live >> 1) & 127u;
+    std::vector<uint16_t> k(s.len);
+    for (int i = 0; i < s.len; i++) {
+        const uint32_t at = gt.cand_off[mask] + s.cand[i];
+        k[i] = gt.cand[at];
+        mask |= 1u << (UOP_RD(gt.cand_uop[at]) - 1);
+    }
+    return k;
+}
+
+/* A record's prefix and middles. */
+SolBuilder record_prefix(const TaskRun &tr, const Record &r)
+{
+    SolBuilder b(tr);
+    for (int d = 0; d < tr.rec_S; d++) b.take(tr.paths[(size_t)r.at * SEARCH_MAX_DEPTH + d]);
+    if (tr.rec_s >= 2) b.take((uint32_t)(r.y >> 32));
+    if (tr.rec_s >= 3) b.take((uint32_t)((r.y >> 16) & 0xFFFF));
+    return b;
+}
+
+/* The first `most` solutions of the task's records in DFS order (every one
+   with most = ~0), appended to tr.sols. */
+void expand_records(TaskRun &tr, size_t most)
+{
+    std::vector<Record> &recs = tr.recs;
+    if (!most || recs.empty()) return;
+    /* each record has a solution at least, so the first `most` records, with
+       the rest of the last one's prefix, hold them */
+    size_t n = recs.size();
+    if (most < n) {
+        std::partial_sort(recs.begin(), recs.begin() + most, recs.end());
+        n = most;
+        const Record last = recs[n - 1];
+        for (size_t i = n; i < recs.size(); i++)
+            if (recs[i].q == last.q && recs[i].prefix() == last.prefix())
+                std::swap(recs[n++], recs[i]);
+    } else {
+        std::sort(recs.begin(), recs.end());
+    }
+    const GenTables &gt = gen_tables();
+    std::vector<RawSol> group;
+    for (size_t i = 0; i < n && tr.sols.size() < most;) {
+        SolBuilder base = record_prefix(tr, recs[i]);
+        size_t j = i;
+        group.clear();
+        for (; j < n && recs[j].q == recs[i].q && recs[j].prefix() == recs[i].prefix(); j++) {
+            const uint32_t low = (uint32_t)(recs[j].y & 0xFFFF);
+            if (tr.rec_s == 0) {   /* a leaf and the register that holds the target */
+                group.push_back(base.sol);
+                group.back().out_reg = (uint8_t)low;
+                continue;
+            }
+            const uint16_t *of = &gt.cand_of[(gt.vc_off[base.mask] + low) * 8];
+            for (uint32_t rd = 1; rd < 8; rd++) {
+                if (of[rd] == 0xFFFF) continue;
+                SolBuilder r = base;
+                r.sol.out_reg = (uint8_t)r.take(of[rd]);
+                group.push_back(r.sol);
+            }
+        }
+        std::sort(group.begin(), group.end(), [](const RawSol &a, const RawSol &b) {
+            const uint16_t x = a.len ? a.cand[a.len - 1] : 0, y = b.len ? b.cand[b.len - 1] : 0;
+            return x != y ? x < y : a.out_reg < b.out_reg;
+        });
+        for (const RawSol &r : group)
+            if (tr.sols.size() < most) tr.sols.push_back(r);
+        i = j;
+    }
+    recs.clear();
+}
 
 PathGather path_gather(const pcagb_engine *e, int S)
 {
@@ -759,8 +851,8 @@ PathGather path_gather(const pcagb_engine *e, int S)
     return G;
 }
 
-/* Turn solving records r0..r1 of the stage at depth K from level S into
- * the tasks' raw solutions (kept sorted in DFS order). */
+/* Hand solving records r0..r1 of the stage at depth K from level S to their
+ * tasks, with their paths. */
 int take_records(pcagb_engine *e, int S, int K, std::vector<TaskRun> &runs, uint64_t r0, uint64_t r1)
 {
     const GenTables &gt = gen_tables();
@@ -792,35 +884,22 @@ int take_records(pcagb_engine *e, int S, int K, std::vector<TaskRun> &runs, uint
         CK(cudaStreamSynchronize(e->stream));
         e->top = top0;
     }
-    std::vector<uint8_t> touched(runs.size(), 0);
     for (size_t i = 0; i < rec.size(); i++) {
         TaskRun &tr = runs[rtask[i]];
-        touched[rtask[i]] = 1;
         tr.nrec++;
-        SolBuilder base(tr);
-        for (int d = 0; d < S; d++) base.take(paths[i * SEARCH_MAX_DEPTH + d]);
-        const uint32_t m1 = (uint32_t)(rec[i].y >> 32), m2 = (uint32_t)((rec[i].y >> 16) & 0xFFFF);
-        const uint32_t low = (uint32_t)(rec[i].y & 0xFFFF);
-        if (s >= 2) base.take(m1);
-        if (s >= 3) base.take(m2);
+        tr.rec_S = S;
+        tr.rec_s = s;
+        const Record r{rec[i].x, rec[i].y, (uint32_t)(tr.paths.size() / SEARCH_MAX_DEPTH)};
+        tr.recs.push_back(r);
+        tr.paths.insert(tr.paths.end(), &paths[i * SEARCH_MAX_DEPTH],
+                        &paths[i * SEARCH_MAX_DEPTH] + SEARCH_MAX_DEPTH);
         if (s == 0) {
-            base.sol.out_reg = low;
-            base.sol.key.push_back(0);
-            tr.sols.push_back(std::move(base.sol));
+            tr.nsols++;
             continue;
         }
-        const uint16_t *of = &gt.cand_of[(gt.vc_off[base.mask] + low) * 8];
-        for (uint32_t rd = 1; rd < 8; rd++) {
-            if (of[rd] == 0xFFFF) continue;
-            SolBuilder r = base;
-            r.sol.out_reg = r.take(of[rd]);
-            tr.sols.push_back(std::move(r.sol));
-        }
+        const uint16_t *of = &gt.cand_of[(gt.vc_off[record_prefix(tr, r).mask] + (rec[i].y & 0xFFFF)) * 8];
+        for (uint32_t rd = 1; rd < 8; rd++) tr.nsols += of[rd] != 0xFFFF;
     }
-    for (size_t t = 0; t < runs.size(); t++)
-        if (touched[t])
-            std::sort(runs[t].sols.begin(), runs[t].sols.end(),
-                      [](const RawSol &a, const RawSol &b) { return a.key < b.key; });
     return PCAGB_OK;
 }
 
@@ -853,14 +932,13 @@ void take_firsts(pcagb_engine *e, int S, int K, std::vector<TaskRun> &runs, int 
         if (s >= 3) b.take((uint32_t)(f.key >> 12 & 4095));
         const uint32_t last = (uint32_t)(f.key & 4095);
         if (s == 0) {   /* a leaf: the register that holds the target */
-            b.sol.out_reg = last;
-            b.sol.key.push_back(0);
+            b.sol.out_reg = (uint8_t)last;
         } else {
-            b.sol.out_reg = b.take(last);
+            b.sol.out_reg = (uint8_t)b.take(last);
         }
         tr.nrec = 1;
         tr.found = f.found;
-        tr.sols.push_back(std::move(b.sol));
+        tr.sols.push_back(b.sol);
     }
 }
 
@@ -1244,7 +1322,7 @@ int run_stage(pcagb_engine *e, int S, int K, std::vector<TaskRun> &runs, bool fi
 /* Host-side step for the reference-key dedup of the solving leaves
    (tools/enumerate.c:380-384 applies OEP to leaves too). */
 void leaf_key(const task_spec_t *task, const search_state_t &root, const std::vector<uint16_t> &k,
-              std::vector<uint8_t> *key)
+              std::string *key)
 {
     search_ctx_t ctx;
     search_ctx_init(&ctx, task);
@@ -1255,9 +1333,8 @@ void leaf_key(const task_spec_t *task, const search_state_t &root, const std::ve
     }
     key->clear();
     for (int t = 0; t < task->num_tests; t++) {
-        const uint8_t *p = (const uint8_t *)s.regs[t];
-        key->insert(key->end(), p, p + 16);
-        key->push_back(s.flags[t]);
+        key->append((const char *)s.regs[t], 16);
+        key->push_back((char)s.flags[t]);
     }
 }
 
@@ -1530,8 +1607,7 @@ int run_batch(pcagb_engine *e, std::vector<TaskRun> &runs, const pcagb_opts_t &o
             for (int t = 0; t < tr.T && ok; t++) ok = tr.root.regs[t][r] == tr.target[t];
             if (ok) {
                 RawSol s0;
-                s0.out_reg = r;
-                s0.key.push_back(r);
+                s0.out_reg = (uint8_t)r;
                 tr.sols.push_back(s0);
             }
         }
@@ -1702,7 +1778,8 @@ int run_batch(pcagb_engine *e, std::vector<TaskRun> &runs, const pcagb_opts_t &o
                 tr.res.ms_to_first = sop ? sop->ms_to_first : 0.0;
                 tr.res.total_solutions =
                     s == 0 || (o.first_only && nt == 1) ? tr.nrec
-                    : o.first_only                      ? tr.found : tr.sols.size();
+                    : o.first_only                      ? tr.found
+                    : ord && !ordered_stage             ? tr.nrec : tr.nsols;
                 notify(i);
             } else if (K >= tr.max_depth) {
                 tr.done = true;
@@ -2055,19 +2132,19 @@ bool make_run(const task_spec_t *task, const pcagb_opts_t &o, TaskRun *tr)
 int emit_solutions(const task_spec_t *task, const pcagb_opts_t &o, TaskRun &tr,
                    uint16_t *sol_progs, int *sol_lens, int sol_cap)
 {
-    std::vector<RawSol> &sols = tr.sols;
     /* The reference applies its pruner to the last level too: among solving
        programs with equal final regs+flags only the DFS-first is printed. */
-    if (o.oep_mode == PCAGB_OEP_EXACT && !o.count_levels && tr.optimal_depth > 0 &&
-        !o.first_only) {
+    const bool distinct = o.oep_mode == PCAGB_OEP_EXACT && !o.count_levels &&
+                          tr.optimal_depth > 0 && !o.first_only;
+    expand_records(tr, distinct ? ~size_t(0) : sol_progs ? (size_t)std::max(sol_cap, 0) : 0);
+    std::vector<RawSol> &sols = tr.sols;
+    if (distinct) {
         std::vector<RawSol> kept;
-        std::vector<std::vector<uint8_t>> seen;
-        std::vector<uint8_t> key;
+        std::unordered_set<std::string> seen;
+        std::string key;
         for (RawSol &s : sols) {
-            leaf_key(task, tr.root, s.kernel, &key);
-            if (std::find(seen.begin(), seen.end(), key) != seen.end()) continue;
-            seen.push_back(key);
-            kept.push_back(s);
+            leaf_key(task, tr.root, sol_kernel(tr, s), &key);
+            if (seen.insert(key).second) kept.push_back(s);
         }
         sols.swap(kept);
         tr.res.total_solutions = sols.size();
@@ -2079,7 +2156,7 @@ int emit_solutions(const task_spec_t *task, const pcagb_opts_t &o, TaskRun &tr,
         int n = 0;
         for (int i = 0; i < task->num_inputs; i++)
             prog[n++] = PCA_ENC_I(PCA_OP_IN, i + 1, task->input_ports[i]);
-        for (uint16_t insn : s.kernel) prog[n++] = insn;
+        for (uint16_t insn : sol_kernel(tr, s)) prog[n++] = insn;
         prog[n++] = PCA_ENC_I(PCA_OP_OUT, s.out_reg, task->output_ports[0]);
         prog[n++] = PCA_ENC_R(PCA_OP_HLT, 0, 0, 0);
         if (task_evaluate(task, prog, n) != task->num_tests) {
@@ -2583,8 +2660,9 @@ int pcagb_complete(pcagb_engine_t *e, const search_ctx_t *ctx, const search_stat
     if (states_explored) *states_explored = explored;
     if (tr.optimal_depth < 0 || tr.sols.empty()) return 0;
     const RawSol &s = tr.sols.front();
-    for (size_t i = 0; i < s.kernel.size(); i++) solution_insns[i] = s.kernel[i];
-    *solution_len = (int)s.kernel.size();
+    const std::vector<uint16_t> kernel = sol_kernel(tr, s);
+    for (size_t i = 0; i < kernel.size(); i++) solution_insns[i] = kernel[i];
+    *solution_len = (int)kernel.size();
     return 1;
 }
 

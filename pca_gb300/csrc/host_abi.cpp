@@ -512,10 +512,26 @@ int task_load(const char *path, task_spec_t *spec)
 int task_evaluate(const task_spec_t *spec, const uint16_t *prog, int prog_len)
 {
     int passed = 0;
+    pca_vm_t vm;
+    pca_init(&vm);
+    pca_load(&vm, prog, (size_t)prog_len);
+    /* A program without ST leaves the memory zero, and the stack is only read
+       below what the test itself pushed: such a test needs no new machine
+       (clearing and loading one is most of the time of a short program). */
+    bool stores = false;
+    for (int i = 0; i < prog_len && i < PCA_PROG_SIZE; i++)
+        stores |= PCA_INSN_OP(prog[i]) == PCA_OP_ST;
     for (int t = 0; t < spec->num_tests; t++) {
-        pca_vm_t vm;
-        pca_init(&vm);
-        pca_load(&vm, prog, (size_t)prog_len);
+        if (t && stores) {
+            pca_init(&vm);
+            pca_load(&vm, prog, (size_t)prog_len);
+        } else if (t) {
+            memset(vm.r, 0, sizeof vm.r);
+            memset(vm.ports, 0, sizeof vm.ports);
+            vm.pc = vm.sp = vm.flags = 0;
+            vm.status = PCA_RUNNING;
+            vm.cycles = 0;
+        }
         for (int i = 0; i < spec->num_inputs; i++)
             vm.ports[spec->input_ports[i]] = spec->tests[t].in[i];
         pca_run(&vm, spec->max_cycles);

@@ -404,14 +404,20 @@ RESULT_ARRAYS = ("candidates", "evaluations", "tried", "pruned_cum", "level_chil
                  "level_survivors", "gpu_ms_lanes")
 
 
+def _programs(progs, lens, base: int, stored: int) -> list:
+    """Programs base .. base + stored of a result's arrays (one slice each:
+    element by element a few thousand take milliseconds)."""
+    flat = progs[base * 16:(base + stored) * 16]
+    return [flat[k * 16:k * 16 + n] for k, n in enumerate(lens[base:base + stored])]
+
+
 def solution_from_result(r: "SolveResult", progs, lens, base: int, max_depth: int) -> "Solution":
     """A Solution from a pcagb_result_t and its programs (progs[(base + k) *
     16 ...], lens[base + k] for k < r.stored)."""
     sol = Solution(optimal_depth=r.optimal_depth, total_solutions=r.total_solutions)
     for name in RESULT_SCALARS:
         setattr(sol, name, getattr(r, name))
-    for k in range(r.stored):
-        sol.programs.append([progs[(base + k) * 16 + j] for j in range(lens[base + k])])
+    sol.programs = _programs(progs, lens, base, r.stored)
     last = r.optimal_depth if r.optimal_depth >= 0 else max_depth
     for name in RESULT_ARRAYS:
         arr = getattr(r, name)
@@ -469,8 +475,7 @@ class Engine:
         sol = Solution(optimal_depth=r.optimal_depth, total_solutions=r.total_solutions)
         for name in RESULT_SCALARS:
             setattr(sol, name, getattr(r, name))
-        for i in range(r.stored):
-            sol.programs.append([progs[i * 16 + j] for j in range(lens[i])])
+        sol.programs = _programs(progs, lens, 0, r.stored)
         last = max(r.optimal_depth, max_depth if r.optimal_depth < 0 else r.optimal_depth)
         for name in RESULT_ARRAYS:
             arr = getattr(r, name)
@@ -517,8 +522,7 @@ class Engine:
             for name in RESULT_SCALARS:
                 setattr(sol, name, getattr(r, name))
             base = i * cap
-            for k in range(r.stored):
-                sol.programs.append([progs[(base + k) * 16 + j] for j in range(lens[base + k])])
+            sol.programs = _programs(progs, lens, base, r.stored)
             last = r.optimal_depth if r.optimal_depth >= 0 else max_depth
             for name in RESULT_ARRAYS:
                 arr2 = getattr(r, name)
@@ -599,8 +603,7 @@ class Engine:
         sol = Solution(optimal_depth=r.optimal_depth, total_solutions=r.total_solutions)
         for name in RESULT_SCALARS:
             setattr(sol, name, getattr(r, name))
-        for i in range(r.stored):
-            sol.programs.append([progs[i * 16 + j] for j in range(lens[i])])
+        sol.programs = _programs(progs, lens, 0, r.stored)
         sol.candidates = [r.candidates[k] for k in range(MAXD)]
         return sol
 
@@ -637,8 +640,7 @@ class Engine:
                               f"{self.lib.pcagb_branch_last_error().decode()}")
         sol = Solution(optimal_depth=r.optimal_depth, total_solutions=r.total_solutions)
         sol.seconds = r.seconds
-        for i in range(r.stored):
-            sol.programs.append([progs[i * 16 + j] for j in range(lens[i])])
+        sol.programs = _programs(progs, lens, 0, r.stored)
         last = r.optimal_depth if r.optimal_depth >= 0 else max_depth
         sol.tried = [r.tried[k] for k in range(last + 1)]
         sol.pruned_cum = [r.pruned_cum[k] for k in range(last + 1)]
