@@ -3,35 +3,55 @@
  * generation tensor cores (tcgen05 + TMEM + TMA), fused from the level's
  * states to the pooled state vector.
  *
- * One persistent CTA per SM walks tiles of 128 feature rows (4 states x 32
- * test rows). Roles: warp 0 streams the weights by TMA (256 x 64 bf16 slabs
- * of W1 then W2, 128-byte swizzle) through a 3-stage ring; warp 1 owns TMEM
- * and one of its threads issues tcgen05.mma (M=128, N=256, K=16, BF16 in,
- * FP32 accumulate); warps 2..17 are the epilogue, four per TMEM lane quarter
- * (one state), each owning 64 of the 256 units. Per tile:
- *   features  the 176 bit features of each (state, test) row (the columns
- *             of k_features in valuenet.cu), expanded to BF16 in registers
- *             straight into the swizzled K-major operand A1;
- *   layer E1  A1 x W1^T into TMEM columns 0..255;
+ * One persistent pair of CTAs (a cluster of two on neighbouring SMs) walks
+ * tiles of 256 feature rows: 8 states x 32 test rows, 4 states a CTA. Both
+ * layers are tcgen05.mma.cta_group::2 products (M = 256, N = 256, K = 16,
+ * BF16 in, FP32 accumulate), so each SM keeps half of the weights: its 128
+ * units of W1 and of W2 (112 KB) are loaded once by TMA and stay in shared
+ * memory for every tile. Per tile, in each CTA:
+ *   features  the 176 bit features of each of its (state, test) rows (the
+ *             columns of k_features in valuenet.cu), expanded to BF16 in
+ *             registers straight into the swizzled K-major operand A1;
+ *   layer E1  A1 x W1^T: TMEM lanes = the CTA's 128 rows, columns 0..255 =
+ *             the units;
  *   epi 1     tcgen05.ld, + bias, ReLU and BF16 rounding in one packed
- *             convert, into the operand A2 (swizzled, K-major);
- *   layer E2  A2 x W2^T into TMEM columns 256..511;
- *   epi 2     the same on E2's accumulators, written back over the warp's
- *             own part of A2, then pooled: each lane sums (fp32, tests in
- *             order) and maxes (packed bf16) 2 units over the task's T test
- *             rows and writes P[528] = mean(256) | max(256) | live bits(8) |
- *             depth | zeros -- the same values as k_pool on the same H2.
- * A1 and A2 are separate buffers, so the next tile's features and E1 run on
- * the tensor core while the epilogue finishes the current tile's E2.
+ *             convert, held in registers until the previous tile's E2 has
+ *             read A2, then stored there (swizzled, K-major);
+ *   layer E2  W2 x A2^T, the operands exchanged: TMEM lanes = the CTA's 128
+ *             units, columns 256..511 = the pair's 256 rows;
+ *   epi 2     each lane owns a unit: + bias, ReLU, BF16, the sum (fp32,
+ *             tests in order) and the maximum over a state's T columns, all
+ *             in registers, and writes P[528] = mean(256) | max(256) | live
+ *             bits(8) | depth | zeros -- the values of k_pool on the same
+ *             H2. H2 is written nowhere.
  * The activations X, H1 and H2 never reach HBM: per state the kernel reads
- * the level record (17 x T bytes) and writes 1,056 bytes; the weights (224
- * KB) are re-read from L2 once per tile.
+ * the level record (17 x T bytes) and writes 1,056 bytes.
  *
- * Synchronisation is by mbarriers only; every wait is bounded by the global
- * timer (kWaitNs). A wait that runs out sets the CTA's abort flag and the
- * status word, every role leaves its loop, the producer waits for its own
- * TMA copies, the MMA thread waits for its own MMAs, and TMEM is freed
- * before the CTA returns.
+ * Roles: warp 0's first thread loads the weights; warp 1 owns TMEM and, in
+ * the first CTA, one of its threads issues every MMA; eight front warps
+ * write the features and E1's epilogue, eight back warps E2's (two warps
+ * each per TMEM lane quarter). E1 is issued as two halves of 128 units, so
+ * that the front starts on the first while the second runs. The MMAs run in
+ * the order E1(i + 1), E2(i): the front's work on tile i + 1 and the
+ * features of tile i + 2 run while E2(i) does, the back's on tile i while
+ * E1(i + 2) does.
+ *
+ * What bounds it: 27 MMAs of 128 cycles a tile, 3,456, and the hand-overs
+ * between the roles: 5,600 cycles a tile, tensor pipe 60% busy. In the
+ * one-CTA form (weights streamed, H2 pooled through shared memory by the
+ * same 16 warps) the operands, 224 KB of weight slabs a tile and H2's way
+ * were 800 KB of shared-memory traffic a tile of 128 rows and each warp
+ * waited for its own record loads, 10,900 cycles. Measured on the way
+ * (131,072 states of 16 to 32 tests): the pair alone 1.21 -> 0.85 ms; front
+ * and back apart, accumulators fetched ahead and nothing computed from a
+ * record when it is loaded 0.67; the quotient below and E1 in halves 0.63.
+ * 4,096 states: 47 -> 31 us.
+ *
+ * Synchronisation is by mbarriers (and one cluster barrier at each end);
+ * every wait is bounded by the global timer (kWaitNs). A wait that runs out
+ * sets the CTA's abort flag and the status word, every role of the CTA
+ * leaves its loop, and the other CTA's waits run out in turn; the MMA thread
+ * waits for its own MMAs, and TMEM is freed once both CTAs are done.
  */
 #include <cuda.h>
 #include <cuda_bf16.h>
@@ -44,42 +64,45 @@
 
 namespace {
 
-constexpr int kRows = 128;            /* feature rows per tile */
-constexpr int kStatesPerTile = 4;
-constexpr int kUnits = 256;           /* N of both encoder layers */
+constexpr int kRows = 128;            /* feature rows per CTA and tile */
+constexpr int kStatesPerTile = 8;     /* of a pair */
+constexpr int kUnits = 256;           /* units of both encoder layers */
+constexpr int kHalfUnits = kUnits / 2; /* of one CTA's weights */
 constexpr int kFeat = 176;            /* feature columns (164 used) */
-constexpr int kKB1 = 3, kKB2 = 4;     /* 64-column K blocks of E1 (176 -> 192) and E2 */
-constexpr int kSlabs = kKB1 + kKB2;   /* weight slabs per tile */
-constexpr int kStages = 3;
-constexpr int kEpiWarps = 16;
-constexpr int kEpiThreads = 32 * kEpiWarps;
-constexpr int kThreads = 64 + kEpiThreads; /* warp 0 TMA, warp 1 MMA + TMEM, 2..17 epilogue */
-constexpr int kABlock = kRows * 128;  /* 16 KB: 128 rows x 64 bf16 */
-constexpr int kWBlock = kUnits * 128; /* 32 KB: 256 rows x 64 bf16 */
+constexpr int kKB1 = 3, kKB2 = 4;     /* 64-column K blocks of E1 (176 of 192) and E2 */
+constexpr int kFrontWarps = 8, kBackWarps = 8;
+constexpr int kThreads = 64 + 32 * (kFrontWarps + kBackWarps); /* warp 0 TMA, 1 MMA + TMEM */
+constexpr int kBlock = kRows * 128;   /* 16 KB: 128 rows x 64 bf16 of any operand */
 constexpr int kOffA1 = 0;                             /* 48 KB */
-constexpr int kOffA2 = kOffA1 + kKB1 * kABlock;       /* 64 KB */
-constexpr int kOffW = kOffA2 + kKB2 * kABlock;        /* 96 KB */
-constexpr int kOffBias = kOffW + kStages * kWBlock;   /* 2 x 256 fp32 */
-constexpr int kOffBar = kOffBias + 2 * kUnits * 4;
+constexpr int kOffA2 = kOffA1 + kKB1 * kBlock;        /* 64 KB */
+constexpr int kOffW1 = kOffA2 + kKB2 * kBlock;        /* 48 KB */
+constexpr int kOffW2 = kOffW1 + kKB1 * kBlock;        /* 64 KB */
+constexpr int kOffBias = kOffW2 + kKB2 * kBlock;      /* b1: 256 fp32 */
+constexpr int kOffBar = kOffBias + kUnits * 4;
 constexpr int kSmemBytes = kOffBar + 256 + 1024;      /* + alignment slack */
 constexpr int kPoolCols = 528;
 constexpr unsigned long long kWaitNs = 1000000000ull; /* 1 s per wait */
-static_assert(kOffA2 % 1024 == 0 && kOffW % 1024 == 0, "swizzle atoms need 1024-byte alignment");
+static_assert(kRows == kHalfUnits, "A and B blocks are the same size");
 static_assert(kSmemBytes <= 227 * 1024, "shared memory");
 
-/* barrier slots (8 bytes each) */
-constexpr int kBarWFull = 0, kBarWEmpty = kStages, kBarA1 = 2 * kStages, kBarA2 = kBarA1 + 1,
-              kBarD1 = kBarA1 + 2, kBarD2 = kBarA1 + 3, kBarDrain = kBarA1 + 4,
-              kBarCount = kBarA1 + 5;
+/* barrier slots (8 bytes each). Counted in the pair's first CTA (an arrival
+   per front or back warp of both): A1 and A2 written, the halves of D1 and
+   D2 drained. In each CTA: weights landed, E1's halves done (the second: A1
+   read), E2's four K blocks done (that block of A2 read; the last one: D2
+   complete), all MMAs done. */
+constexpr int kBarA1 = 0, kBarA2 = 1, kBarFree1 = 2, kBarFree2 = 4, kBarW = 5, kBarD1 = 6,
+              kBarE2 = 8, kBarDrain = kBarE2 + kKB2, kBarCount = kBarDrain + 1;
 constexpr int kOffTmemSlot = kBarCount * 8;
 constexpr int kOffAbort = kOffTmemSlot + 4;
 static_assert(kOffAbort + 4 <= 256, "barrier area");
 
 /* Instruction descriptor of tcgen05.mma kind::f16: D f32 (bits 4-5 = 1),
    A and B bf16 (bits 7-9, 10-12 = 1), both K-major, N >> 3 at bits 17-22,
-   M >> 4 at bits 24-28. */
-constexpr uint32_t kIdesc = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(kUnits >> 3) << 17) |
-                            ((uint32_t)(kRows >> 4) << 24);
+   M >> 4 at bits 24-28. Of the pair: M = 256, N = 128 (E1, a half of the
+   units) or 256 (E2). */
+constexpr uint32_t kIdescM256 = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(256 >> 4) << 24);
+constexpr uint32_t kIdescE1 = kIdescM256 | ((uint32_t)(kHalfUnits >> 3) << 17);
+constexpr uint32_t kIdescE2 = kIdescM256 | ((uint32_t)(2 * kRows >> 3) << 17);
 
 __device__ __forceinline__ uint32_t smem_u32(const void *p)
 {
@@ -98,9 +121,20 @@ __device__ __forceinline__ void mbar_init(uint32_t bar, uint32_t count)
     asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(bar), "r"(count) : "memory");
 }
 
-__device__ __forceinline__ void mbar_arrive(uint32_t bar)
+/* arrive on the barrier at this offset of the cluster's first CTA */
+__device__ __forceinline__ void mbar_arrive_first(uint32_t bar)
 {
-    asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(bar) : "memory");
+    asm volatile(
+        "{\n\t.reg .b32 ra;\n\t"
+        "mapa.shared::cluster.u32 ra, %0, 0;\n\t"
+        "mbarrier.arrive.shared::cluster.b64 _, [ra];\n\t}" ::"r"(bar)
+        : "memory");
+}
+
+__device__ __forceinline__ void cluster_sync()
+{
+    asm volatile("barrier.cluster.arrive.release.aligned;\n\t"
+                 "barrier.cluster.wait.acquire.aligned;" ::: "memory");
 }
 
 __device__ __forceinline__ void mbar_expect_tx(uint32_t bar, uint32_t bytes)
@@ -127,6 +161,7 @@ __device__ __forceinline__ bool mbar_test(uint32_t bar, uint32_t parity)
 __device__ bool mbar_wait(uint32_t bar, uint32_t parity, volatile int *abort_flag, int *status,
                           int code)
 {
+    if (mbar_test(bar, parity)) return true;
     const unsigned long long t0 = global_ns();
     for (uint32_t i = 0;; i++) {
         if (mbar_test(bar, parity)) return true;
@@ -185,13 +220,25 @@ __device__ __forceinline__ uint64_t sw128_mn_desc(uint32_t saddr)
     return d;
 }
 
-__device__ __forceinline__ void mma_f16(uint32_t dtmem, uint64_t a, uint64_t b, uint32_t acc)
+/* one product of the pair: A and B at these offsets of both CTAs */
+__device__ __forceinline__ void mma_pair(uint32_t dtmem, uint64_t a, uint64_t b, uint32_t idesc,
+                                         uint32_t acc)
 {
     asm volatile(
         "{\n\t.reg .pred p;\n\t"
         "setp.ne.b32 p, %4, 0;\n\t"
-        "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}" ::"r"(dtmem),
-        "l"(a), "l"(b), "r"(kIdesc), "r"(acc)
+        "tcgen05.mma.cta_group::2.kind::f16 [%0], %1, %2, %3, p;\n\t}" ::"r"(dtmem),
+        "l"(a), "l"(b), "r"(idesc), "r"(acc)
+        : "memory");
+}
+
+/* arrive on the barrier at this offset of both CTAs of the pair once the
+   thread's products so far are done */
+__device__ __forceinline__ void mma_commit_pair(uint32_t bar)
+{
+    asm volatile(
+        "tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 "
+        "[%0], %1;" ::"r"(bar), "h"((uint16_t)3)
         : "memory");
 }
 
@@ -202,7 +249,9 @@ __device__ __forceinline__ void mma_commit(uint32_t bar)
         : "memory");
 }
 
-__device__ __forceinline__ void tmem_ld32(uint32_t taddr, uint32_t (&r)[32])
+/* 32 columns of this warp's lanes into registers; r is not to be read before
+   tmem_wait(r) */
+__device__ __forceinline__ void tmem_ld32_async(uint32_t taddr, uint32_t (&r)[32])
 {
     asm volatile(
         "tcgen05.ld.sync.aligned.32x32b.x32.b32 "
@@ -215,7 +264,25 @@ __device__ __forceinline__ void tmem_ld32(uint32_t taddr, uint32_t (&r)[32])
           "=r"(r[25]), "=r"(r[26]), "=r"(r[27]), "=r"(r[28]), "=r"(r[29]), "=r"(r[30]),
           "=r"(r[31])
         : "r"(taddr));
-    asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+}
+
+__device__ __forceinline__ void tmem_wait(uint32_t (&r)[32])
+{
+    asm volatile("tcgen05.wait::ld.sync.aligned;"
+                 : "+r"(r[0]), "+r"(r[1]), "+r"(r[2]), "+r"(r[3]), "+r"(r[4]), "+r"(r[5]),
+                   "+r"(r[6]), "+r"(r[7]), "+r"(r[8]), "+r"(r[9]), "+r"(r[10]), "+r"(r[11]),
+                   "+r"(r[12]), "+r"(r[13]), "+r"(r[14]), "+r"(r[15]), "+r"(r[16]), "+r"(r[17]),
+                   "+r"(r[18]), "+r"(r[19]), "+r"(r[20]), "+r"(r[21]), "+r"(r[22]), "+r"(r[23]),
+                   "+r"(r[24]), "+r"(r[25]), "+r"(r[26]), "+r"(r[27]), "+r"(r[28]), "+r"(r[29]),
+                   "+r"(r[30]), "+r"(r[31])
+                 :
+                 : "memory");
+}
+
+__device__ __forceinline__ void tmem_ld32(uint32_t taddr, uint32_t (&r)[32])
+{
+    tmem_ld32_async(taddr, r);
+    tmem_wait(r);
 }
 
 /* Byte offset of 16-byte chunk c (0..7) of row r in a 128-byte-swizzled
@@ -225,17 +292,50 @@ __device__ __forceinline__ uint32_t sw128_off(int r, int c)
     return (uint32_t)(r * 128 + ((c ^ (r & 7)) << 4));
 }
 
-/* 8 bits of b as 8 bf16 values 0.0 / 1.0 (bit 0 first): bit 2j selects
-   0x3F80 in the low half of word j, bit 2j+1 0x3F80 in the high half. */
-__device__ __forceinline__ uint4 bits_to_bf16x8(uint32_t b)
+/* 8 bits of a 16-bit word w (the low or the high byte) as 8 bf16 values 0.0 /
+   1.0, the byte's bit 0 first. y has the byte's bit 2j at 2j and bit 2j + 1
+   at 16 + 2j; the two, times 0x3F80 >> 2j, are the halves of output word j. */
+__device__ __forceinline__ uint4 byte_to_bf16x8(uint32_t w, int high)
 {
-    uint32_t w[4];
-#pragma unroll
-    for (int j = 0; j < 4; j++) {
-        const uint32_t t = b >> (2 * j);
-        w[j] = (t & 1u) * 0x3F80u + (t & 2u) * 0x1FC00000u;
-    }
-    return make_uint4(w[0], w[1], w[2], w[3]);
+    const uint32_t y = high ? (w >> 8) | (w << 7) : w | (w << 15);
+    return make_uint4((y & 0x00010001u) * 0x3F80u, (y & 0x00040004u) * (0x3F80u >> 2),
+                      (y & 0x00100010u) * (0x3F80u >> 4), (y & 0x00400040u) * (0x3F80u >> 6));
+}
+
+/* v / T rounded to nearest, v >= 0 and 1 <= T <= 32 (T = 0: v is 0), with
+   r = 1 / T rounded to nearest: Markstein's correction of a quotient
+   (Computation of elementary functions on the IBM RISC System/6000
+   processor, 1990). Away from the ends of the range its steps scale with v,
+   and over all 2^23 significands and each T it gives the division's value;
+   at the ends it is the division. A division for each of the four sums of a
+   lane takes 1,400 cycles of a tile beside the other warps, this a tenth. */
+__device__ __forceinline__ float quotient(float v, int T, float r)
+{
+    if (v > 0.f && !(v > 1e-30f && v < 1e38f)) return v / (float)T;
+    const float q = v * r;
+    return __fmaf_rn(__fmaf_rn(-(float)T, q, v), r, q);
+}
+
+/* s + the low half + the high half of x, in this order */
+__device__ __forceinline__ float add_bf16x2(float s, uint32_t x)
+{
+    asm("{\n\t.reg .b16 l, h;\n\tmov.b32 {l, h}, %1;\n\t"
+        "add.rn.f32.bf16 %0, l, %0;\n\tadd.rn.f32.bf16 %0, h, %0;\n\t}"
+        : "+f"(s)
+        : "r"(x));
+    return s;
+}
+
+/* (a.x + b.x, a.y + b.y), each rounded as a single addition */
+__device__ __forceinline__ float2 add_f32x2(uint32_t ax, uint32_t ay, float bx, float by)
+{
+    float2 d;
+    asm("{\n\t.reg .b64 a, b, c;\n\t"
+        "mov.b64 a, {%2, %3};\n\tmov.b64 b, {%4, %5};\n\t"
+        "add.rn.f32x2 c, a, b;\n\tmov.b64 {%0, %1}, c;\n\t}"
+        : "=f"(d.x), "=f"(d.y)
+        : "r"(ax), "r"(ay), "f"(bx), "f"(by));
+    return d;
 }
 
 /* relu(lo), relu(hi) rounded to bf16, lo in the low half. */
@@ -253,7 +353,7 @@ __device__ __forceinline__ uint32_t max_bf16x2(uint32_t a, uint32_t b)
     return d;
 }
 
-__global__ void __launch_bounds__(kThreads, 1)
+__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads, 1)
 k_encode_pool_tc(const __grid_constant__ CUtensorMap map_w1, const __grid_constant__ CUtensorMap map_w2,
                  const float *__restrict__ b1, const float *__restrict__ b2,
                  const uint16_t *__restrict__ regs, const uint8_t *__restrict__ flags,
@@ -265,261 +365,303 @@ k_encode_pool_tc(const __grid_constant__ CUtensorMap map_w1, const __grid_consta
     extern __shared__ uint8_t smem_raw[];
     uint8_t *smem = (uint8_t *)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
     const uint32_t sA1 = smem_u32(smem + kOffA1), sA2 = smem_u32(smem + kOffA2);
-    const uint32_t sW = smem_u32(smem + kOffW);
+    const uint32_t sW1 = smem_u32(smem + kOffW1), sW2 = smem_u32(smem + kOffW2);
     const uint32_t sBar = smem_u32(smem + kOffBar);
     uint32_t *tmem_slot = (uint32_t *)(smem + kOffBar + kOffTmemSlot);
     volatile int *abort_flag = (volatile int *)(smem + kOffBar + kOffAbort);
     float *sb1 = (float *)(smem + kOffBias);
-    float *sb2 = sb1 + kUnits;
     auto bar = [&](int i) { return sBar + 8u * (uint32_t)i; };
 
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int rank = blockIdx.x & 1;                     /* in the pair */
+    const int pair = blockIdx.x >> 1, pairs = gridDim.x >> 1;
     const int ntiles = (n + kStatesPerTile - 1) / kStatesPerTile;
+    const int mine = pair < ntiles ? (ntiles - 1 - pair) / pairs + 1 : 0;
 
     if (threadIdx.x == 0) {
-        for (int s = 0; s < kStages; s++) {
-            mbar_init(bar(kBarWFull + s), 1);
-            mbar_init(bar(kBarWEmpty + s), 1);
-        }
-        mbar_init(bar(kBarA1), kEpiThreads);
-        mbar_init(bar(kBarA2), kEpiThreads);
-        mbar_init(bar(kBarD1), 1);
-        mbar_init(bar(kBarD2), 1);
-        mbar_init(bar(kBarDrain), 1);
+        for (int i = 0; i < kBarCount; i++)
+            mbar_init(bar(i), i < kBarFree2 ? 2 * kFrontWarps : i == kBarFree2 ? 2 * kBackWarps : 1);
         *abort_flag = 0;
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
         fence_async_smem();
+        mbar_expect_tx(bar(kBarW), (kKB1 + kKB2) * kBlock);
+        for (int k = 0; k < kKB1; k++)
+            for (int u = 0; u < 2; u++)      /* its quarter of each half of the units */
+                tma_load_2d(sW1 + k * kBlock + u * (kBlock / 2), &map_w1, bar(kBarW), 64 * k,
+                            kHalfUnits * u + kHalfUnits / 2 * rank);
+        for (int k = 0; k < kKB2; k++)
+            tma_load_2d(sW2 + k * kBlock, &map_w2, bar(kBarW), 64 * k, kHalfUnits * rank);
     }
-    for (int i = threadIdx.x; i < kUnits; i += kThreads) {
-        sb1[i] = b1[i];
-        sb2[i] = b2[i];
-    }
+    for (int i = threadIdx.x; i < kUnits; i += kThreads) sb1[i] = b1[i];
     if (warp == 1) {
-        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], 512;" ::"r"(
+        asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], 512;" ::"r"(
                          smem_u32(tmem_slot))
                      : "memory");
-        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::2.sync.aligned;" ::: "memory");
     }
     tc_before();
     __syncthreads();
     tc_after();
     const uint32_t tmem = *tmem_slot;
+    /* both CTAs' barriers are set up, their TMEM is theirs, their weights
+       have landed */
+    mbar_wait(bar(kBarW), 0, abort_flag, status, 1);
+    __syncwarp();
+    cluster_sync();
 
-    if (warp == 0) {
-        /* ---- TMA producer: weight slabs through the ring ---- */
-        if (lane == 0) {
-            uint32_t j = 0;
-            bool ok = true;
-            for (int tile = blockIdx.x; tile < ntiles && ok; tile += gridDim.x) {
-                for (int s = 0; s < kSlabs && ok; s++, j++) {
-                    const uint32_t st = j % kStages, ph = (j / kStages) & 1u;
-                    ok = mbar_wait(bar(kBarWEmpty + st), ph ^ 1u, abort_flag, status, 1);
-                    if (!ok) break;
-                    mbar_expect_tx(bar(kBarWFull + st), kWBlock);
-                    if (s < kKB1)
-                        tma_load_2d(sW + st * kWBlock, &map_w1, bar(kBarWFull + st), s * 64, 0);
-                    else
-                        tma_load_2d(sW + st * kWBlock, &map_w2, bar(kBarWFull + st),
-                                    (s - kKB1) * 64, 0);
-                }
-            }
-            /* wait for the copies this thread issued (the last one per stage) */
-            const uint32_t issued = j;
-            for (uint32_t st = 0; st < kStages && st < issued; st++) {
-                const uint32_t last = issued - 1 - ((issued - 1 - st) % kStages);
-                const unsigned long long t0 = global_ns();
-                while (!mbar_test(bar(kBarWFull + st), (last / kStages) & 1u) &&
-                       global_ns() - t0 < kWaitNs) {
-                }
-            }
-        }
-    } else if (warp == 1) {
-        /* ---- MMA issuer ---- */
-        if (lane == 0) {
-            uint32_t j = 0;
-            bool ok = true;
-            int it = 0;
-            for (int tile = blockIdx.x; tile < ntiles && ok; tile += gridDim.x, it++) {
-                for (int layer = 0; layer < 2 && ok; layer++) {
-                    ok = mbar_wait(bar(layer ? kBarA2 : kBarA1), it & 1, abort_flag, status, 2);
-                    if (!ok) break;
-                    tc_after();
-                    const int nkb = layer ? kKB2 : kKB1;
-                    const uint32_t d = tmem + (layer ? (uint32_t)kUnits : 0u);
-                    const uint32_t a = layer ? sA2 : sA1;
-                    for (int kb = 0; kb < nkb; kb++, j++) {
-                        const uint32_t st = j % kStages, ph = (j / kStages) & 1u;
-                        ok = mbar_wait(bar(kBarWFull + st), ph, abort_flag, status, 3);
-                        if (!ok) break;
-                        tc_after();
-                        const uint32_t a0 = a + kb * kABlock, b0 = sW + st * kWBlock;
+    if (warp == 1) {
+        /* ---- MMA issuer (first CTA) ---- */
+        if (lane == 0 && rank == 0) {
+            auto wait = [&](int which, int tile, int code) {
+                return mbar_wait(bar(which), tile & 1, abort_flag, status, code);
+            };
+            /* unrolled: a product takes this thread 100 to 120 cycles to
+               issue, in a loop 190, longer than the tensor core needs */
+            auto e1 = [&](int i) {
+                if (!wait(kBarA1, i, 2)) return false;
 #pragma unroll
-                        for (int k = 0; k < 4; k++)
-                            mma_f16(d, sw128_desc(a0 + 32 * k), sw128_desc(b0 + 32 * k),
-                                    (kb | k) != 0);
-                        mma_commit(bar(kBarWEmpty + st));
-                    }
-                    if (!ok) break;
-                    mma_commit(bar(layer ? kBarD2 : kBarD1));
+                for (int u = 0; u < 2; u++) {
+                    if (i && !wait(kBarFree1 + u, i - 1, 3)) return false;
+                    tc_after();
+#pragma unroll
+                    for (int k = 0; k < kFeat / 16; k++)
+                        mma_pair(tmem + kHalfUnits * u,
+                                 sw128_desc(sA1 + (k >> 2) * kBlock + 32 * (k & 3)),
+                                 sw128_desc(sW1 + (k >> 2) * kBlock + u * (kBlock / 2) + 32 * (k & 3)),
+                                 kIdescE1, k != 0);
+                    mma_commit_pair(bar(kBarD1 + u));
                 }
+                return true;
+            };
+            auto e2 = [&](int i) {
+                if (!wait(kBarA2, i, 4)) return false;
+                if (i && !wait(kBarFree2, i - 1, 5)) return false;
+                tc_after();
+#pragma unroll
+                for (int k = 0; k < 4 * kKB2; k++) {
+                    mma_pair(tmem + kUnits, sw128_desc(sW2 + (k >> 2) * kBlock + 32 * (k & 3)),
+                             sw128_desc(sA2 + (k >> 2) * kBlock + 32 * (k & 3)), kIdescE2, k != 0);
+                    if ((k & 3) == 3) mma_commit_pair(bar(kBarE2 + (k >> 2)));
+                }
+                return true;
+            };
+            bool ok = mine > 0 && e1(0);
+            for (int i = 0; i < mine && ok; i++) {
+                if (i + 1 < mine) ok = e1(i + 1);
+                ok = ok && e2(i);
             }
             /* every MMA this thread issued has finished before TMEM is freed */
-            mma_commit(bar(kBarDrain));
+            mma_commit_pair(bar(kBarDrain));
             const unsigned long long t0 = global_ns();
             while (!mbar_test(bar(kBarDrain), 0) && global_ns() - t0 < kWaitNs) {
             }
         }
-    } else {
-        /* ---- epilogue warps ---- */
-        const int q = warp & 3;              /* TMEM lane quarter = the tile's state */
-        const int h = (warp - 2) >> 2;       /* units [64h, 64h + 64) */
-        const int r = q * 32 + lane;         /* tile row = TMEM lane */
+    } else if (warp >= 2 && warp < 2 + kFrontWarps) {
+        /* ---- front warps: features, and E1's epilogue into A2 ---- */
+        const int q = warp & 3;              /* TMEM lane quarter = the CTA's state */
+        const int h = (warp - 2) >> 2;       /* its K blocks of A2: h and h + 2 */
+        const int r = q * 32 + lane;         /* row of A1 and A2 = TMEM lane */
         const uint32_t lane_base = (uint32_t)(q * 32) << 16;
 
         /* A state's level record, loaded one tile ahead of its features:
-           the three 16-bit words of this warp's quarter of the feature row
-           (h = 0: in0 in1 target; 1: r1 r2 r3; 2: r4 r5 r6; 3: r7 flags 0)
-           for test `lane`, the task's T and (h = 0, lanes 0..15) the pooled
-           row's tail. The task id is loaded a tile earlier still, so no
-           load waits on another in the loop. */
+           the 16-bit words of this warp's half of the feature row (h = 0:
+           in0 in1 target r1 r2 r3; 1: r4 r5 r6 r7 flags) for test `lane`,
+           the task's tests and (h = 0, lanes 0..15) the pooled row's tail.
+           The task id is loaded a tile earlier still and nothing is computed
+           from what was loaded until its tile, so nothing in the loop waits
+           for a load. */
         struct Rec {
             int s, T;
-            uint32_t w[3];
-            float g;  /* P column 512 + lane: live bit / depth / 0 */
+            uint32_t w[6];
+            uint32_t g;  /* lane < 8: live mask, 8: depth, else 0 */
         };
-        auto task_of = [&](int tile) -> int {
-            const int st = tile * kStatesPerTile + q;
-            return (tile < ntiles && st < n) ? (int)task[st] : -1;
+        auto own = [&](int i) {
+            return i < mine ? (pair + i * pairs) * kStatesPerTile + 4 * rank + q : n;
         };
-        auto load_rec = [&](int tile, int tid, Rec &rc) {
-            rc.s = tile * kStatesPerTile + q;
+        auto task_of = [&](int s) -> int { return s < n ? (int)task[s] : -1; };
+        auto load_rec = [&](int i, int tid, Rec &rc) {
+            rc.s = own(i);
             rc.T = 0;
-            rc.g = 0.f;
-            rc.w[0] = rc.w[1] = rc.w[2] = 0;
+            rc.g = 0;
+#pragma unroll
+            for (int k = 0; k < 6; k++) rc.w[k] = 0;
             if (tid < 0) return;
-            rc.T = min(task_T[tid], TP);
-            if (h == 0 && lane < 8) rc.g = (float)((live[rc.s] >> lane) & 1u);
-            else if (h == 0 && lane == 8) rc.g = (float)depth[rc.s];
+            rc.T = task_T[tid];
+            if (h == 0 && lane < 9) rc.g = (lane < 8 ? live : depth)[rc.s];
             if (lane >= TP) return;
-            const size_t s8 = (size_t)rc.s * 8;
+            const uint16_t *rg = regs + (size_t)rc.s * 8 * TP + lane;
             if (h == 0) {
 #pragma unroll
-                for (int k = 0; k < 3; k++) rc.w[k] = task_io[((size_t)tid * 3 + k) * 32 + lane];
-            } else if (h < 3) {
-#pragma unroll
-                for (int k = 0; k < 3; k++) rc.w[k] = regs[(s8 + 3 * h - 2 + k) * TP + lane];
+                for (int k = 0; k < 3; k++) {
+                    rc.w[k] = task_io[((size_t)tid * 3 + k) * 32 + lane];
+                    rc.w[3 + k] = rg[(1 + k) * TP];
+                }
             } else {
-                rc.w[0] = regs[(s8 + 7) * TP + lane];
-                rc.w[1] = flags[(size_t)rc.s * TP + lane] & 0xFu;
+#pragma unroll
+                for (int k = 0; k < 4; k++) rc.w[k] = rg[(4 + k) * TP];
+                rc.w[4] = flags[(size_t)rc.s * TP + lane];
             }
         };
-        /* bit features of (state, test lane), chunks [6h, 6h + 6) of the
-           row's 24 16-byte chunks, into A1 (rows of tests >= T are zero) */
+        /* bit features of (state, test lane), this half's chunks of the
+           row's 22 16-byte chunks, into A1 (rows past the task's tests are
+           zero), and the pooled row's tail */
         auto features = [&](const Rec &rc) {
             const bool valid = lane < rc.T;
 #pragma unroll
-            for (int k = 0; k < 6; k++) {
-                const int c = 6 * h + k;
-                const uint32_t byte = valid ? (rc.w[k >> 1] >> ((k & 1) * 8)) & 0xFFu : 0u;
-                *(uint4 *)(smem + kOffA1 + (c >> 3) * kABlock + sw128_off(r, c & 7)) =
-                    bits_to_bf16x8(byte);
+            for (int k = 0; k < 12; k++) {
+                const int c = 12 * h + k;
+                if (c >= kFeat / 8) break;
+                *(uint4 *)(smem + kOffA1 + (c >> 3) * kBlock + sw128_off(r, c & 7)) =
+                    byte_to_bf16x8(!valid ? 0u : c >= 20 ? rc.w[k >> 1] & 0xFu : rc.w[k >> 1],
+                                   k & 1);
             }
             fence_async_smem();
-            mbar_arrive(bar(kBarA1));
+            __syncwarp();
+            if (lane == 0) mbar_arrive_first(bar(kBarA1));
+            if (h == 0 && lane < 16 && rc.s < n)
+                P[(size_t)rc.s * kPoolCols + 2 * kUnits + lane] =
+                    __float2bfloat16((float)(lane < 8 ? (rc.g >> lane) & 1u : rc.g));
         };
 
-        /* accumulators of units [64h, 64h + 64) of one layer: + bias, ReLU,
-           bf16, into this warp's part of A2 */
-        auto drain = [&](uint32_t col_base, const float *bias) {
-#pragma unroll 1
+        /* a K block (64 units) of E1: + bias, ReLU, bf16, into registers */
+        auto drain = [&](int kb, uint32_t (&w)[32]) {
+#pragma unroll
             for (int g = 0; g < 2; g++) {
-            const int col0 = 64 * h + 32 * g;
-            uint32_t acc[32];
-            tmem_ld32(tmem + col_base + lane_base + col0, acc);
+                uint32_t acc[32];
+                tmem_ld32(tmem + lane_base + (uint32_t)(64 * kb + 32 * g), acc);
 #pragma unroll
-            for (int c = 0; c < 4; c++) {
-                const float4 bl = *(const float4 *)(bias + col0 + 8 * c);
-                const float4 bh = *(const float4 *)(bias + col0 + 8 * c + 4);
-                const uint32_t *a = acc + 8 * c;
-                const uint32_t w0 = relu_bf16x2(__uint_as_float(a[0]) + bl.x, __uint_as_float(a[1]) + bl.y);
-                const uint32_t w1 = relu_bf16x2(__uint_as_float(a[2]) + bl.z, __uint_as_float(a[3]) + bl.w);
-                const uint32_t w2 = relu_bf16x2(__uint_as_float(a[4]) + bh.x, __uint_as_float(a[5]) + bh.y);
-                const uint32_t w3 = relu_bf16x2(__uint_as_float(a[6]) + bh.z, __uint_as_float(a[7]) + bh.w);
-                const int chunk = (col0 >> 3) + c;
-                *(uint4 *)(smem + kOffA2 + (chunk >> 3) * kABlock + sw128_off(r, chunk & 7)) =
-                    make_uint4(w0, w1, w2, w3);
-            }
-            }
-        };
-
-        /* mean (fp32 over tests in order, as k_pool) and max of units
-           64h + 2 lane, + 1 over the state's T rows of H2 in A2 */
-        auto pool = [&](const Rec &rc) {
-            const int chunk = 8 * h + (lane >> 2);
-            const uint8_t *base = smem + kOffA2 + (chunk >> 3) * kABlock + ((lane & 3) << 2);
-            float s0 = 0.f, s1 = 0.f;
-            uint32_t m01 = 0u;                /* ReLU outputs are >= 0 */
-            for (int t0 = 0; t0 < rc.T; t0 += 8) {
-                uint32_t v[8];
-#pragma unroll
-                for (int k = 0; k < 8; k++)
-                    v[k] = *(const uint32_t *)(base + sw128_off(32 * q + t0 + k, chunk & 7));
-                const bool full = t0 + 8 <= rc.T;
-#pragma unroll
-                for (int k = 0; k < 8; k++) {
-                    const uint32_t x = (full || t0 + k < rc.T) ? v[k] : 0u;
-                    s0 += __uint_as_float(x << 16);
-                    s1 += __uint_as_float(x & 0xFFFF0000u);
-                    m01 = max_bf16x2(m01, x);
+                for (int c = 0; c < 8; c++) {
+                    const float4 b = *(const float4 *)(sb1 + 64 * kb + 32 * g + 4 * c);
+                    const float2 u = add_f32x2(acc[4 * c], acc[4 * c + 1], b.x, b.y);
+                    const float2 v = add_f32x2(acc[4 * c + 2], acc[4 * c + 3], b.z, b.w);
+                    w[16 * g + 2 * c] = relu_bf16x2(u.x, u.y);
+                    w[16 * g + 2 * c + 1] = relu_bf16x2(v.x, v.y);
                 }
             }
-            const float fT = (float)(rc.T > 0 ? rc.T : 1);
-            __nv_bfloat162 mean = __floats2bfloat162_rn(s0 / fT, s1 / fT);
-            __nv_bfloat16 *row = P + (size_t)rc.s * kPoolCols;
-            *(uint32_t *)(row + 64 * h + 2 * lane) = *reinterpret_cast<uint32_t *>(&mean);
-            *(uint32_t *)(row + kUnits + 64 * h + 2 * lane) = m01;
-            if (h == 0 && lane < 16) row[2 * kUnits + lane] = __float2bfloat16(rc.g);
         };
 
-        const int G = (int)gridDim.x;
-        int it = 0;
-        int tile = blockIdx.x;
-        Rec cur, nxt;
-        load_rec(tile, task_of(tile), cur);
-        int tid_next = task_of(tile + G);
-        if (tile < ntiles) features(cur);
-        for (; tile < ntiles; tile += G, it++) {
-            /* the next tile's record, in flight while E1 drains */
-            load_rec(tile + G, tid_next, nxt);
-            tid_next = task_of(tile + 2 * G);
-            /* E1 -> A2 */
-            bool ok = mbar_wait(bar(kBarD1), it & 1, abort_flag, status, 4);
+        Rec rec;
+        load_rec(0, task_of(own(0)), rec);
+        int tid_next = task_of(own(1));
+        if (mine) features(rec);
+        load_rec(1, tid_next, rec);
+        tid_next = task_of(own(2));
+        for (int i = 0; i < mine; i++) {
+            bool ok = true;
+#pragma unroll 1
+            for (int u = 0; u < 2; u++) {
+                const int kb = 2 * u + h;
+                uint32_t w[32];
+                ok = mbar_wait(bar(kBarD1 + u), i & 1, abort_flag, status, 6);
+                if (!__all_sync(0xffffffffu, ok)) break;
+                tc_after();
+                drain(kb, w);
+                tc_before();
+                __syncwarp();
+                if (lane == 0) mbar_arrive_first(bar(kBarFree1 + u));
+                if (u == 0) {
+                    /* E1 has read A1 once its second half is done: the next
+                       tile's features */
+                    ok = mbar_wait(bar(kBarD1 + 1), i & 1, abort_flag, status, 6);
+                    if (!__all_sync(0xffffffffu, ok)) break;
+                    if (i + 1 < mine) features(rec);
+                }
+                /* into A2 once the previous tile's E2 has read the block */
+                if (i) {
+                    ok = mbar_wait(bar(kBarE2 + kb), (i - 1) & 1, abort_flag, status, 7);
+                    if (!__all_sync(0xffffffffu, ok)) break;
+                }
+#pragma unroll
+                for (int c = 0; c < 8; c++)
+                    *(uint4 *)(smem + kOffA2 + kb * kBlock + sw128_off(r, c)) =
+                        make_uint4(w[4 * c], w[4 * c + 1], w[4 * c + 2], w[4 * c + 3]);
+            }
             if (!__all_sync(0xffffffffu, ok)) break;
-            tc_after();
-            drain(0u, sb1);
-            tc_before();
             fence_async_smem();
-            mbar_arrive(bar(kBarA2));
-            /* next tile's features while E2 runs */
-            if (tile + G < ntiles) features(nxt);
-            /* E2 -> H2 (over this warp's part of A2) -> pooling */
-            ok = mbar_wait(bar(kBarD2), it & 1, abort_flag, status, 5);
+            __syncwarp();
+            if (lane == 0) mbar_arrive_first(bar(kBarA2));
+            load_rec(i + 2, tid_next, rec);
+            tid_next = task_of(own(i + 3));
+        }
+    } else if (warp >= 2) {
+        /* ---- back warps: E2's epilogue and pooling ---- */
+        const int q = warp & 3;
+        const int h = (warp - 2 - kFrontWarps) >> 2;      /* states 4h .. 4h + 3 of the tile */
+        const int unit = kHalfUnits * rank + q * 32 + lane;
+        const uint32_t lane_base = (uint32_t)(q * 32) << 16;
+        const float bias2 = b2[unit];
+        /* lane k < 4 holds the tests of state k of tile i, loaded ahead as
+           the front's records are */
+        auto state_of = [&](int i) {
+            return i < mine && lane < 4 ? (pair + i * pairs) * kStatesPerTile + 4 * h + lane : n;
+        };
+        auto task_of = [&](int s) -> int { return s < n ? (int)task[s] : -1; };
+        auto tests_of = [&](int tid) { return tid < 0 ? 0 : min(task_T[tid], TP); };
+        int T_cur = tests_of(task_of(state_of(0))), tid_next = task_of(state_of(1));
+        for (int i = 0; i < mine; i++) {
+            const int T_next = tests_of(tid_next);
+            tid_next = task_of(state_of(i + 2));
+            const bool ok = mbar_wait(bar(kBarE2 + kKB2 - 1), i & 1, abort_flag, status, 8);
             if (!__all_sync(0xffffffffu, ok)) break;
             tc_after();
-            drain((uint32_t)kUnits, sb2);
-            tc_before();
-            __syncwarp();
-            if (cur.s < n) pool(cur);
-            __syncwarp();
-            cur = nxt;
+            const int s0 = (pair + i * pairs) * kStatesPerTile + 4 * h;
+            /* the four states' accumulators + bias, ReLU, bf16: D2 is drained
+               before anything is summed */
+            const uint32_t d2 = tmem + kUnits + lane_base + (uint32_t)(128 * h);
+            uint32_t x[4][16];
+#pragma unroll
+            for (int k = 0; k < 4; k++) {
+                uint32_t acc[32];
+                tmem_ld32(d2 + 32 * k, acc);
+                if (k == 3) {
+                    tc_before();
+                    __syncwarp();
+                    if (lane == 0) mbar_arrive_first(bar(kBarFree2));
+                }
+#pragma unroll
+                for (int j = 0; j < 16; j++) {
+                    const float2 u = add_f32x2(acc[2 * j], acc[2 * j + 1], bias2, bias2);
+                    x[k][j] = relu_bf16x2(u.x, u.y);
+                }
+            }
+            const float r_cur = 1.f / (float)(T_cur > 0 ? T_cur : 1);
+#pragma unroll
+            for (int k = 0; k < 4; k++) {
+                /* sum (fp32, tests in order, as k_pool) and max of this
+                   lane's unit over the state's T columns, 8 tests at a time:
+                   T is the warp's, so whole groups past it are skipped and
+                   only the last one looks at each test */
+                const int T = __shfl_sync(0xffffffffu, T_cur, k);
+                const float r = __shfl_sync(0xffffffffu, r_cur, k);
+                float v = 0.f;
+                uint32_t m = 0u;              /* ReLU outputs are >= 0 */
+#pragma unroll
+                for (int g = 0; g < 4; g++) {
+                    if (8 * g >= T) break;
+#pragma unroll
+                    for (int j = 4 * g; j < 4 * g + 4; j++) {
+                        if (8 * g + 8 > T)
+                            x[k][j] &= (2 * j < T ? 0xFFFFu : 0u) | (2 * j + 1 < T ? 0xFFFF0000u : 0u);
+                        v = add_bf16x2(v, x[k][j]);
+                        m = max_bf16x2(m, x[k][j]);
+                    }
+                }
+                if (s0 + k >= n) continue;
+                m = max_bf16x2(m, m >> 16);
+                __nv_bfloat16 *row = P + (size_t)(s0 + k) * kPoolCols + unit;
+                row[0] = __float2bfloat16(quotient(v, T, r));
+                reinterpret_cast<uint16_t *>(row)[kUnits] = (uint16_t)m;
+            }
+            T_cur = T_next;
         }
     }
     __syncwarp();
     tc_before();
     __syncthreads();
+    cluster_sync();
     tc_after();
     if (warp == 1)
-        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, 512;" ::"r"(tmem)
+        asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, 512;" ::"r"(tmem)
                      : "memory");
 }
 
@@ -876,14 +1018,15 @@ EncodeTiledFn encode_fn()
     return fn;
 }
 
-/* Tensor map of a row-major [256][K] bf16 weight, 64 x 256 boxes, 128B swizzle. */
-bool weight_map(CUtensorMap *m, const void *W, int K)
+/* Tensor map of a row-major [256][K] bf16 weight, boxes of 64 columns x `units`
+   rows, 128B swizzle. */
+bool weight_map(CUtensorMap *m, const void *W, int K, int units)
 {
     EncodeTiledFn fn = encode_fn();
     if (!fn) return false;
     cuuint64_t dims[2] = {(cuuint64_t)K, (cuuint64_t)kUnits};
     cuuint64_t strides[1] = {(cuuint64_t)K * 2};
-    cuuint32_t box[2] = {64, (cuuint32_t)kUnits};
+    cuuint32_t box[2] = {64, (cuuint32_t)units};
     cuuint32_t estr[2] = {1, 1};
     return fn(m, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, const_cast<void *>(W), dims, strides, box,
               estr, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B,
@@ -1068,7 +1211,7 @@ extern "C" int pcagb_vnet_encode_pool_tc(const void *W1, const float *b1, const 
         ((uintptr_t)W1 & 15) || ((uintptr_t)W2 & 15))
         return PCAGB_EINVAL;
     CUtensorMap m1, m2;
-    if (!weight_map(&m1, W1, kFeat) || !weight_map(&m2, W2, kUnits)) return PCAGB_ECUDA;
+    if (!weight_map(&m1, W1, kFeat, kHalfUnits / 2) || !weight_map(&m2, W2, kUnits, kHalfUnits)) return PCAGB_ECUDA;
     int dev = 0, sms = 0;
     if (cudaGetDevice(&dev) != cudaSuccess ||
         cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess)
@@ -1081,8 +1224,8 @@ extern "C" int pcagb_vnet_encode_pool_tc(const void *W1, const float *b1, const 
     });
     if (attr_err != cudaSuccess) return PCAGB_ECUDA;
     const int ntiles = (n + kStatesPerTile - 1) / kStatesPerTile;
-    const int grid = ntiles < sms ? ntiles : sms;
-    k_encode_pool_tc<<<grid, kThreads, kSmemBytes, (cudaStream_t)stream>>>(
+    const int pairs = ntiles < sms / 2 ? ntiles : sms / 2;
+    k_encode_pool_tc<<<2 * pairs, kThreads, kSmemBytes, (cudaStream_t)stream>>>(
         m1, m2, b1, b2, regs, flags, live, task, depth, TP, n, task_io, task_T,
         (__nv_bfloat16 *)P, status);
     return cudaGetLastError() == cudaSuccess ? PCAGB_OK : PCAGB_ECUDA;

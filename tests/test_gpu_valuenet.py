@@ -281,3 +281,33 @@ def test_adam_applies_each_layers_gradient():
         cols = 521 if k == "T1" else want.shape[1]   # T1's padding columns stay zero
         assert rel(net.W[k][:, :cols], want[:, :cols]) < 1e-5, k
         assert rel(net.b[k], b0[k] - 1e-3 * dbk / (dbk.abs() + 1e-8)) < 1e-5, k
+
+
+@pytest.mark.parametrize("TP", [16, 32])
+@pytest.mark.parametrize("n", [1, 4, 5, 7, 8, 9, 607, 608, 609, 1225])
+def test_fused_encoder_tiles(n, TP):
+    """The pair's tiles of 8 states (4 a CTA): a single state, a half, a full
+    and a ragged tile, as many tiles as CTA pairs and one more or less, two
+    tiles a pair; tasks of 1 test, of 8-test groups and between, of all."""
+    from pca_gb300.valuenet import ValueNet
+    net = ValueNet(seed=6)
+    b, (regs, flags, *_) = _batch_tp(n, TP, seed=n)
+    b["task_T"] = torch.tensor([1, 8, TP - 1, TP], dtype=torch.int32, device="cuda")
+    task = torch.arange(n, device="cuda") % (3 if TP == 16 else 4) + (1 if TP == 16 else 0)
+    b["task_io"] = torch.randint(0, 1 << 15, (4, 3, 32), dtype=torch.int16, device="cuda")
+    b["task"] = task.to(torch.int16)
+    Pf = net.encode_pool(b["regs"], b["flags"], b["live"], b["task"], b["depth"], TP,
+                         b["task_io"], b["task_T"])
+    net.check_status()
+    pad = torch.zeros(n, 8, 32, dtype=torch.int16, device="cuda")
+    pad[:, :, :TP] = b["regs"]
+    padf = torch.zeros(n, 32, dtype=torch.uint8, device="cuda")
+    padf[:, :TP] = b["flags"]
+    X = net.features(pad, padf, b["task"], 32, b["task_io"], b["task_T"])
+    net.forward(X, b["live"], b["task"], b["task_T"], b["depth"])
+    Pu = net._acts["P"]
+    # the same products summed in fp32 in both, stored as bf16: within an ulp
+    # of bf16 (2^-8) of a row's largest value
+    scale = Pu[:, :512].float().abs().amax(1, keepdim=True)
+    assert ((Pf[:, :512].float() - Pu[:, :512].float()).abs() <= 2.0 ** -7 * scale).all()
+    assert torch.equal(Pf[:, 512:], Pu[:, 512:])
