@@ -47,6 +47,8 @@ def _lib():
         "pcagb_vnet_pool": [vp, vp, vp, vp, vp, i, vp, vp, vp],
         "pcagb_vnet_pool_bwd": [vp, vp, vp, vp, vp, i, vp, vp],
         "pcagb_vnet_loss": [vp, vp, vp, i, f, vp, vp, vp, vp],
+        "pcagb_vnet_loss_value": [vp, vp, vp, i, f, vp, vp, vp, vp, vp],
+        "pcagb_vnet_adam_list": [vp, i, f, f, f, f, vp, vp],
         "pcagb_vnet_adam": [vp, vp, vp, vp, i, i, f, f, f, f, vp, vp, vp, vp],
         "pcagb_vnet_to_bf16": [vp, vp, sz, vp],
         "pcagb_vnet_encode_pool_tc": [vp, vp, vp, vp, vp, vp, vp, vp, vp, i, i, vp, vp, vp, vp,
@@ -63,6 +65,12 @@ def _lib():
 
 def _p(t):
     return ctypes.c_void_p(t.data_ptr()) if t is not None else None
+
+
+class _AdamTensor(ctypes.Structure):
+    """One tensor of pcagb_vnet_adam_list (struct AdamTensor)."""
+    _fields_ = [(k, ctypes.c_void_p) for k in ("W", "G", "m", "v", "Wb", "Wt")] + [
+        (k, ctypes.c_int) for k in ("out", "inp", "live_in", "pad")]
 
 
 class ValueNet:
@@ -135,14 +143,25 @@ class ValueNet:
             self.stream))
         return C
 
-    def _wgrad(self, dY, X, name):
+    def _gradients(self):
+        """{name: (dW, db)} of zeros, parts of one buffer (one clearing
+        launch instead of two a layer)."""
+        flat = torch.zeros(sum(out * (inp + 1) for _, out, inp in LAYERS), device=self.dev,
+                           dtype=torch.float32)
+        grads, at = {}, 0
+        for name, out, inp in LAYERS:
+            grads[name] = (flat[at:at + out * inp].view(out, inp),
+                           flat[at + out * inp:at + out * (inp + 1)])
+            at += out * (inp + 1)
+        return grads
+
+    def _wgrad(self, dY, X, name, into):
         """dW = dY^T . X as one split-K tcgen05 GEMM reading dY [M][out] and
         X [M][in] as stored (MN-major operands, no transposes), and db =
-        the column sums of dY."""
+        the column sums of dY, added to the pair `into`."""
         out, inp = self.W[name].shape
         M = dY.shape[0]
-        G = torch.zeros(out, inp, device=self.dev, dtype=torch.float32)
-        db = torch.zeros(out, device=self.dev, dtype=torch.float32)
+        G, db = into
         bn = 256 if inp > 192 else (inp + 63) // 64 * 64
         tiles = ((out + 127) // 128) * ((inp + bn - 1) // bn)
         kblocks = (M + 63) // 64
@@ -217,21 +236,21 @@ class ValueNet:
         """dL: bf16 [n,16] gradient of the loss w.r.t. the logits. Returns
         {name: (dW, db)} in fp32."""
         a = self._acts
-        grads = {}
-        grads["H"] = self._wgrad(dL, a["Z2"], "H")
+        grads = self._gradients()
+        self._wgrad(dL, a["Z2"], "H", grads["H"])
         dZ2 = self._gemm(dL, "H", False, transposed=True, mask=a["Z2"])
-        grads["T2"] = self._wgrad(dZ2, a["Z1"], "T2")
+        self._wgrad(dZ2, a["Z1"], "T2", grads["T2"])
         dZ1 = self._gemm(dZ2, "T2", False, transposed=True, mask=a["Z1"])
-        grads["T1"] = self._wgrad(dZ1, a["P"], "T1")
+        self._wgrad(dZ1, a["P"], "T1", grads["T1"])
         dP = self._gemm(dZ1, "T1", False, transposed=True)
         n = a["task"].shape[0]
         dH2 = torch.empty(n * ROWS, 256, device=self.dev, dtype=torch.bfloat16)
         self._ck(self.lib.pcagb_vnet_pool_bwd(_p(dP), _p(a["am"]), _p(a["task"]),
                                               _p(a["task_T"]), _p(a["H2"]), n, _p(dH2),
                                               self.stream))
-        grads["E2"] = self._wgrad(dH2, a["H1"], "E2")
+        self._wgrad(dH2, a["H1"], "E2", grads["E2"])
         dH1 = self._gemm(dH2, "E2", False, transposed=True, mask=a["H1"])
-        grads["E1"] = self._wgrad(dH1, a["X"], "E1")
+        self._wgrad(dH1, a["X"], "E1", grads["E1"])
         return grads
 
     def loss(self, L, label, remaining):
@@ -239,29 +258,27 @@ class ValueNet:
         gradient w.r.t. the logits."""
         n = L.shape[0]
         dL = torch.empty(n, 16, device=self.dev, dtype=torch.bfloat16)
-        stats = torch.zeros(3, device=self.dev, dtype=torch.float32)
-        npos = (label > 0.5).sum(dtype=torch.float32).reshape(1)
-        self._ck(self.lib.pcagb_vnet_loss(_p(L), _p(label), _p(remaining), n, self.pos_weight,
-                                          _p(npos), _p(dL), _p(stats), self.stream))
-        loss = stats[0] / n + 0.5 * stats[1] / npos[0].clamp(min=1.0)
+        loss = torch.empty((), device=self.dev, dtype=torch.float32)
+        self._ck(self.lib.pcagb_vnet_loss_value(_p(L), _p(label), _p(remaining), n,
+                                                self.pos_weight, None, _p(dL), None, _p(loss),
+                                                self.stream))
         return loss, dL
 
     def adam(self, grads, b1=0.9, b2=0.999, eps=1e-8):
         self.step_n += 1
         self.step_dev += 1
+        tensors = []
         for name, out, inp in LAYERS:
             G, gb = grads[name]
-            self._ck(self.lib.pcagb_vnet_adam(_p(self.W[name]), _p(G), _p(self.mW[name]),
-                                              _p(self.vW[name]), out, inp, self.lr, b1, b2, eps,
-                                              _p(self.step_dev), _p(self.Wb[name]),
-                                              _p(self.Wt[name]), self.stream))
-            self._ck(self.lib.pcagb_vnet_adam(_p(self.b[name]), _p(gb), _p(self.mb[name]),
-                                              _p(self.vb[name]), 1, out, self.lr, b1, b2, eps,
-                                              _p(self.step_dev), None, None, self.stream))
-        with torch.no_grad():
-            self.W["T1"][:, 521:] = 0.0
-            self.Wb["T1"][:, 521:] = 0.0
-            self.Wt["T1"][521:, :] = 0.0
+            live = 521 if name == "T1" else inp   # padding columns stay zero
+            tensors.append(_AdamTensor(*(t.data_ptr() for t in (
+                self.W[name], G, self.mW[name], self.vW[name], self.Wb[name], self.Wt[name])),
+                out, inp, live, 0))
+            tensors.append(_AdamTensor(*(t.data_ptr() for t in (
+                self.b[name], gb, self.mb[name], self.vb[name])), None, None, 1, out, out, 0))
+        self._ck(self.lib.pcagb_vnet_adam_list((_AdamTensor * len(tensors))(*tensors),
+                                               len(tensors), self.lr, b1, b2, eps,
+                                               _p(self.step_dev), self.stream))
 
     def train_step(self, batch):
         """One step on a batch dict (device tensors): regs, flags, live, task,

@@ -311,3 +311,83 @@ def test_fused_encoder_tiles(n, TP):
     scale = Pu[:, :512].float().abs().amax(1, keepdim=True)
     assert ((Pf[:, :512].float() - Pu[:, :512].float()).abs() <= 2.0 ** -7 * scale).all()
     assert torch.equal(Pf[:, 512:], Pu[:, 512:])
+
+
+@pytest.mark.parametrize("off", [0, 1])
+@pytest.mark.parametrize("n", [1, 7, 8, 9, 300])
+def test_pooling_and_its_gradient_by_rows(n, off):
+    """Pooling, its row of the maximum and its gradient against torch in the
+    same order of operations, from 16-byte aligned arrays and from arrays one
+    value off, at 1, 8, 9 and 32 tests."""
+    from pca_gb300.valuenet import _lib, _p
+    lib = _lib()
+    g = torch.Generator(device="cuda").manual_seed(n)
+    Ts = torch.tensor([1, 8, 9, 32], dtype=torch.int32, device="cuda")
+    task = (torch.arange(n, device="cuda") % 4).to(torch.int16)
+    T = Ts[task.long()]
+
+    def arr(count, dtype=torch.bfloat16):
+        return torch.zeros(count + off, dtype=dtype, device="cuda")[off:]
+
+    H, P, dP, dH = (arr(n * k) for k in (32 * 256, 528, 528, 32 * 256))
+    am = arr(n * 256, torch.uint8)
+    H.copy_(torch.randn(n * 32 * 256, device="cuda", generator=g).relu())
+    dP.copy_(torch.randn(n * 528, device="cuda", generator=g))
+    live = torch.full((n,), 0xA5, dtype=torch.uint8, device="cuda")
+    depth = torch.full((n,), 3, dtype=torch.uint8, device="cuda")
+    s = torch.cuda.current_stream().cuda_stream
+    assert lib.pcagb_vnet_pool(_p(H), _p(live), _p(task), _p(Ts), _p(depth), n, _p(P), _p(am), s) == 0
+    assert lib.pcagb_vnet_pool_bwd(_p(dP), _p(am), _p(task), _p(Ts), _p(H), n, _p(dH), s) == 0
+    h = H.float().view(n, 32, 256)
+    inside = torch.arange(32, device="cuda")[None, :, None] < T[:, None, None]
+    total = torch.zeros(n, 256, device="cuda")
+    best = torch.full((n, 256), -1e30, device="cuda")
+    arg = torch.zeros(n, 256, dtype=torch.long, device="cuda")
+    for t in range(32):
+        on = (t < T)[:, None]
+        total = torch.where(on, total + h[:, t], total)
+        more = on & (h[:, t] > best)
+        best = torch.where(more, h[:, t], best)
+        arg = torch.where(more, torch.full_like(arg, t), arg)
+    p = P.view(n, 528)
+    assert torch.equal(p[:, :256], (total / T[:, None]).to(torch.bfloat16))
+    assert torch.equal(p[:, 256:512], best.to(torch.bfloat16))
+    assert torch.equal(am.view(n, 256).long(), arg)
+    tail = torch.tensor([1, 0, 1, 0, 0, 1, 0, 1, 3] + [0] * 7, device="cuda", dtype=torch.bfloat16)
+    assert torch.equal(p[:, 512:], tail.expand(n, 16))
+    d = dP.float().view(n, 528)
+    hot = torch.arange(32, device="cuda")[None, :, None] == arg[:, None, :]
+    want = (d[:, None, :256] / T[:, None, None]) + torch.where(hot, d[:, None, 256:512], 0.0)
+    want = torch.where(inside & (h > 0), want, 0.0).to(torch.bfloat16)
+    assert torch.equal(dH.view(n, 32, 256), want)
+
+
+@pytest.mark.parametrize("n", [1, 31, 4096, 4097, 9001])
+def test_loss_value_is_the_sums(n):
+    """The loss, counting its own positives, against float64 and against the
+    sums with the positives given; no positives at all counts as one."""
+    from pca_gb300.valuenet import ValueNet, _p
+    net = ValueNet(seed=1)
+    g = torch.Generator(device="cuda").manual_seed(n)
+    L = torch.randn(n, 16, device="cuda", generator=g)
+    for share in (0.0, 0.2):
+        label = (torch.rand(n, device="cuda", generator=g) < share).float()
+        rem = torch.randint(0, 12, (n,), device="cuda", generator=g, dtype=torch.int32) - 1
+        loss, dL = net.loss(L, label, rem)
+        again, dL2 = net.loss(L, label, rem)
+        assert torch.equal(loss, again) and torch.equal(dL, dL2)
+        z, y = L.double(), label.double()
+        sp = torch.nn.functional.softplus
+        bce = (50 * y * sp(-z[:, 0]) + (1 - y) * sp(z[:, 0])).sum() / n
+        pos = label > 0.5
+        k = rem.clamp(0, 8).long()
+        ce = torch.nn.functional.cross_entropy(z[pos, 1:10], k[pos], reduction="sum")
+        want = bce + 0.5 * ce / max(int(pos.sum()), 1)
+        # fp32 terms and sums of n of them: 2^-24 each, tens of operations deep
+        assert abs(loss.item() - want.item()) <= 64 * 2.0 ** -24 * max(1.0, abs(want.item()))
+        stats = torch.zeros(3, device="cuda")
+        npos = pos.sum(dtype=torch.float32).reshape(1)
+        dL3 = torch.empty_like(dL)
+        assert net.lib.pcagb_vnet_loss(_p(L), _p(label), _p(rem), n, 50.0, _p(npos), _p(dL3),
+                                       _p(stats), net.stream) == 0
+        assert torch.equal(dL, dL3) and stats[2].item() == pos.sum().item()
