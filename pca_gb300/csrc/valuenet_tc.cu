@@ -672,16 +672,19 @@ k_encode_pool_tc(const __grid_constant__ CUtensorMap map_w1, const __grid_consta
  * multiple of 16), grid.z splits K. Warp 0 (one thread) streams 64-column K
  * blocks of A (128 rows) and B (bn rows) by TMA with 128-byte swizzle
  * through a two-stage mbarrier ring; warp 1 owns TMEM and one thread issues
- * four tcgen05.mma (M=128, N=bn, K=16) per block; then all four warps drain
- * the accumulators (warp w: TMEM lanes 32w..32w+31 = tile rows) with
- * tcgen05.ld. Epilogue: with one K split, + bias, x (mask > 0) (the ReLU
+ * four tcgen05.mma (M=128, N=bn, K=16) per block; then all eight warps drain
+ * the accumulators (warp w: TMEM lanes 32(w mod 4).. = tile rows, half w/4 of
+ * the columns) with tcgen05.ld. Epilogue: with one K split, + bias, x (mask > 0) (the ReLU
  * derivative through a stored activation), ReLU, stored as bf16 or fp32;
  * with several, fp32 atomic adds into C (zeroed by the caller). Out-of-range
  * rows and columns of A and B are TMA zero fill; stores are bounds checked.
  * Every wait is bounded by the global timer; a wait that runs out sets the
  * abort flag and *status, each role leaves, and TMEM is freed. Two CTAs fit
  * an SM (96 KB of shared memory at bn = 256), so one CTA's epilogue overlaps
- * the other's loads and MMAs.
+ * the other's loads and MMAs. The network's products are bound by their
+ * bytes and this epilogue: 262,144 rows of 256, 67 us beside 39 of copy rate,
+ * 90 with the mask beside 59; four warps, which found each 16-byte piece's
+ * row by a division, took 94 and 142.
  *
  * mn_major: A and B are given K-row by K-row instead ([K][M] and [K][N],
  * M and N contiguous: the weight gradient dY^T . X reads dY [batch][out]
@@ -690,8 +693,9 @@ k_encode_pool_tc(const __grid_constant__ CUtensorMap map_w1, const __grid_consta
  * bn is then a multiple of 64. */
 constexpr int kGRows = 128, kGBK = 64, kGStages = 2;
 constexpr int kGABytes = kGRows * 128;              /* 16 KB per A stage */
+constexpr int kGThreads = 256;
 
-__global__ void __launch_bounds__(128, 2)
+__global__ void __launch_bounds__(kGThreads, 2)
 k_gemm_tc(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_b,
           const float *__restrict__ bias, const __nv_bfloat16 *__restrict__ mask, int ldm,
           __nv_bfloat16 *__restrict__ Cb, float *__restrict__ Cf, int ldc, int M, int N,
@@ -796,15 +800,18 @@ k_gemm_tc(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUt
         }
     }
     __syncwarp();
-    /* epilogue: all four warps. The tile's bias goes to shared memory
+    /* epilogue: all eight warps. The tile's bias goes to shared memory
        first (every thread takes part, so the barrier below is reached by
        all of them whatever the waits return). */
     float *sbias = (float *)(ctl + 256);
-    for (int c = threadIdx.x; c < bn; c += 128) sbias[c] = (bias && n0 + c < N) ? bias[n0 + c] : 0.f;
+    for (int c = threadIdx.x; c < bn; c += kGThreads) sbias[c] = (bias && n0 + c < N) ? bias[n0 + c] : 0.f;
     bool ok = nk > 0 && mbar_wait(done_bar, 0, abort_flag, status, 13);
     ok = __all_sync(0xFFFFFFFFu, ok) && !*abort_flag;
     tc_after();
     __syncthreads();
+    /* two warps share a TMEM lane quarter (32 rows), half of the columns each */
+    const int quarter = warp & 3, half = (bn / 2 + 31) / 32 * 32;
+    const int lo = warp < 4 ? 0 : min(half, bn), hi = warp < 4 ? min(half, bn) : bn;
     if (ok && stage_mode) {
         /* Staged: each warp drains its 32 rows of accumulators (+ bias,
            ReLU, rounding) into the drained stage buffers, a row of bn values
@@ -814,28 +821,33 @@ k_gemm_tc(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUt
            on the way. stage_mode 1: bf16 C; 2: fp32 C (bn <= 112). */
         const int esz = stage_mode == 1 ? 2 : 4;
         const uint32_t S = (uint32_t)(bn * esz + 16);
-        const uint32_t lane_base = (uint32_t)(warp * 32) << 16;
-        uint8_t *myrow = smem + (uint32_t)(warp * 32 + lane) * S;
-        for (int c0 = 0; c0 < bn; c0 += 32) {
+        const uint32_t lane_base = (uint32_t)(quarter * 32) << 16;
+        uint8_t *rows = smem + (uint32_t)(quarter * 32) * S;
+        uint8_t *myrow = rows + (uint32_t)lane * S;
+        for (int c0 = lo; c0 < hi; c0 += 32) {
             uint32_t acc[32];
             tmem_ld32(tmem + lane_base + (uint32_t)c0, acc);
             if (stage_mode == 1) {
                 uint32_t w[16];
 #pragma unroll
-                for (int j = 0; j < 16; j++) {
-                    const float v0 = __uint_as_float(acc[2 * j]) + sbias[c0 + 2 * j];
-                    const float v1 = __uint_as_float(acc[2 * j + 1]) + sbias[c0 + 2 * j + 1];
+                for (int j = 0; j < 8; j++) {
+                    const float4 bv = *(const float4 *)(sbias + c0 + 4 * j);
+                    const float2 u = add_f32x2(acc[4 * j], acc[4 * j + 1], bv.x, bv.y);
+                    const float2 v = add_f32x2(acc[4 * j + 2], acc[4 * j + 3], bv.z, bv.w);
                     if (relu) {
-                        w[j] = relu_bf16x2(v0, v1);
+                        w[2 * j] = relu_bf16x2(u.x, u.y);
+                        w[2 * j + 1] = relu_bf16x2(v.x, v.y);
                     } else {
-                        __nv_bfloat162 h = __floats2bfloat162_rn(v0, v1);
-                        w[j] = *reinterpret_cast<uint32_t *>(&h);
+                        const __nv_bfloat162 hu = __floats2bfloat162_rn(u.x, u.y);
+                        const __nv_bfloat162 hv = __floats2bfloat162_rn(v.x, v.y);
+                        w[2 * j] = *reinterpret_cast<const uint32_t *>(&hu);
+                        w[2 * j + 1] = *reinterpret_cast<const uint32_t *>(&hv);
                     }
                 }
                 /* the tile may end inside this group of 32 (bn = 16) */
 #pragma unroll
                 for (int k = 0; k < 4; k++)
-                    if (c0 + 8 * k < bn)
+                    if (c0 + 8 * k < hi)
                         *(uint4 *)(myrow + c0 * 2 + 16 * k) =
                             make_uint4(w[4 * k], w[4 * k + 1], w[4 * k + 2], w[4 * k + 3]);
             } else {
@@ -847,81 +859,85 @@ k_gemm_tc(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUt
                         v[q] = __uint_as_float(acc[4 * k + q]) + sbias[c0 + 4 * k + q];
                         if (relu) v[q] = fmaxf(v[q], 0.f);
                     }
-                    if (c0 + 4 * k < bn)
+                    if (c0 + 4 * k < hi)
                         *(float4 *)(myrow + c0 * 4 + 16 * k) = make_float4(v[0], v[1], v[2], v[3]);
                 }
             }
         }
         __syncwarp();
+        /* the warp's columns of its 32 rows in 16-byte pieces, a lane a piece
+           and four at a time (their mask pieces all in flight); a lane's next
+           piece is 32 further, its row and column follow without a division */
         const int per = 16 / esz;                 /* values per 16-byte piece */
-        const int cpr = bn / per;                 /* pieces per row */
-        /* the mask's pieces of four iterations are loaded before any of
-           them is used, so each lane has four global loads in flight */
-        uint4 mkq[4];
-        for (int it = lane; it < 32 * cpr; it += 32) {
-            const int u = ((it - lane) >> 5) & 3;
-            if (stage_mode == 1 && mask && u == 0) {
+        const int cpr = (hi - lo) / per;          /* pieces per row */
+        const int dr = cpr ? 32 / cpr : 0, dc = cpr ? 32 - dr * cpr : 0;
+        int r = cpr ? lane / cpr : 32, ch = cpr ? lane - r * cpr : 0;
+        while (r < 32) {
+            int rk[4], ck[4];
+            uint4 mk[4];
 #pragma unroll
-                for (int k = 0; k < 4; k++) {
-                    const int itk = it + 32 * k;
-                    const int rk = itk / cpr, gr = m0 + warp * 32 + rk;
-                    const int gc = n0 + (itk - rk * cpr) * per;
-                    mkq[k] = itk < 32 * cpr && gr < M && gc < N
-                                 ? *(const uint4 *)(mask + (size_t)gr * ldm + gc)
-                                 : make_uint4(0u, 0u, 0u, 0u);
+            for (int k = 0; k < 4; k++) {
+                rk[k] = r;
+                ck[k] = lo + ch * per;
+                const int grow = m0 + quarter * 32 + r, gcol = n0 + ck[k];
+                if (r >= 32 || grow >= M || gcol >= N) rk[k] = -1;
+                else if (stage_mode == 1 && mask)
+                    mk[k] = *(const uint4 *)(mask + (size_t)grow * ldm + gcol);
+                ch += dc;
+                r += dr;
+                if (ch >= cpr) {
+                    ch -= cpr;
+                    r++;
                 }
             }
-            const int r = it / cpr, ch = it - r * cpr;
-            const int grow = m0 + warp * 32 + r, gcol = n0 + ch * per;
-            if (grow >= M || gcol >= N) continue;
-            const uint8_t *src = smem + (uint32_t)(warp * 32 + r) * S + ch * 16;
-            if (stage_mode == 1) {
-                uint4 v = *(const uint4 *)src;
-                if (mask) {
-                    uint4 mk = mkq[0];
 #pragma unroll
-                    for (int k = 1; k < 4; k++)
-                        if (u == k) mk = mkq[k];
-                    /* keep a value where its mask half is a positive bf16 */
-                    auto keep = [](uint32_t m) {
-                        return (__uint_as_float(m << 16) > 0.f ? 0x0000FFFFu : 0u) |
-                               (__uint_as_float(m & 0xFFFF0000u) > 0.f ? 0xFFFF0000u : 0u);
-                    };
-                    v.x &= keep(mk.x);
-                    v.y &= keep(mk.y);
-                    v.z &= keep(mk.z);
-                    v.w &= keep(mk.w);
-                }
-                if (gcol + per <= N) {
-                    *(uint4 *)(Cb + (size_t)grow * ldc + gcol) = v;
+            for (int k = 0; k < 4; k++) {
+                if (rk[k] < 0) continue;
+                const size_t grow = (size_t)(m0 + quarter * 32 + rk[k]);
+                const int gcol = n0 + ck[k];
+                const uint8_t *src = rows + (uint32_t)rk[k] * S + ck[k] * esz;
+                if (stage_mode == 1) {
+                    uint4 v = *(const uint4 *)src;
+                    if (mask) {
+                        /* keep a value where its mask half is a positive bf16 */
+                        auto keep = [](uint32_t m) {
+                            return (__uint_as_float(m << 16) > 0.f ? 0x0000FFFFu : 0u) |
+                                   (__uint_as_float(m & 0xFFFF0000u) > 0.f ? 0xFFFF0000u : 0u);
+                        };
+                        v.x &= keep(mk[k].x);
+                        v.y &= keep(mk[k].y);
+                        v.z &= keep(mk[k].z);
+                        v.w &= keep(mk[k].w);
+                    }
+                    if (gcol + per <= N) {
+                        *(uint4 *)(Cb + grow * ldc + gcol) = v;
+                    } else {
+                        const uint32_t w4[4] = {v.x, v.y, v.z, v.w};
+#pragma unroll
+                        for (int q = 0; q < 8; q++)
+                            if (gcol + q < N)
+                                reinterpret_cast<uint16_t *>(Cb)[grow * ldc + gcol + q] =
+                                    (uint16_t)(w4[q >> 1] >> (16 * (q & 1)));
+                    }
                 } else {
-                    const uint32_t w4[4] = {v.x, v.y, v.z, v.w};
+                    const float4 v = *(const float4 *)src;
+                    if (gcol + per <= N) {
+                        *(float4 *)(Cf + grow * ldc + gcol) = v;
+                    } else {
+                        const float f4[4] = {v.x, v.y, v.z, v.w};
 #pragma unroll
-                    for (int q = 0; q < 8; q++)
-                        if (gcol + q < N) {
-                            const uint32_t b = (w4[q >> 1] >> (16 * (q & 1))) & 0xFFFFu;
-                            reinterpret_cast<uint16_t *>(Cb)[(size_t)grow * ldc + gcol + q] =
-                                (uint16_t)b;
-                        }
-                }
-            } else {
-                const float4 v = *(const float4 *)src;
-                if (gcol + per <= N) {
-                    *(float4 *)(Cf + (size_t)grow * ldc + gcol) = v;
-                } else {
-                    const float f4[4] = {v.x, v.y, v.z, v.w};
-#pragma unroll
-                    for (int q = 0; q < 4; q++)
-                        if (gcol + q < N) Cf[(size_t)grow * ldc + gcol + q] = f4[q];
+                        for (int q = 0; q < 4; q++)
+                            if (gcol + q < N) Cf[grow * ldc + gcol + q] = f4[q];
+                    }
                 }
             }
         }
     } else if (ok) {
         /* direct: split-K partial sums (fp32 adds, four at a time where
            aligned) or outputs the staged forms do not cover */
-        const int row = m0 + warp * 32 + lane;
-        const uint32_t lane_base = (uint32_t)(warp * 32) << 16;
-        for (int c0 = 0; c0 < bn; c0 += 32) {
+        const int row = m0 + quarter * 32 + lane;
+        const uint32_t lane_base = (uint32_t)(quarter * 32) << 16;
+        for (int c0 = lo; c0 < hi; c0 += 32) {
             uint32_t acc[32];
             tmem_ld32(tmem + lane_base + (uint32_t)c0, acc);
             if (row >= M) continue;
@@ -1102,7 +1118,7 @@ extern "C" int pcagb_vnet_gemm_tc(const void *A, int lda, const void *B, int ldb
     const int vec_atomic = splits > 1 && ldc % 4 == 0 && !((uintptr_t)Cf & 15);
     if (attr_err != cudaSuccess) return PCAGB_ECUDA;
     dim3 grid((N + bn - 1) / bn, (M + kGRows - 1) / kGRows, splits);
-    k_gemm_tc<<<grid, 128, smem, (cudaStream_t)stream>>>(
+    k_gemm_tc<<<grid, kGThreads, smem, (cudaStream_t)stream>>>(
         ma, mb, bias, (const __nv_bfloat16 *)mask, ldm, (__nv_bfloat16 *)Cb, Cf, ldc, M, N,
         kblocks, per, bn, idesc, tcols, relu, splits > 1, stage_mode, vec_atomic, 0, status);
     return cudaGetLastError() == cudaSuccess ? PCAGB_OK : PCAGB_ECUDA;
@@ -1196,7 +1212,7 @@ extern "C" int pcagb_vnet_wgrad_tc(const void *dY, int ldy, const void *X, int l
     float *out = part ? part : C;
     const int vec_atomic = ldc % 4 == 0 && !((uintptr_t)out & 15);
     dim3 grid((N + bn - 1) / bn, (M + kGRows - 1) / kGRows, splits);
-    k_gemm_tc<<<grid, 128, smem, (cudaStream_t)stream>>>(
+    k_gemm_tc<<<grid, kGThreads, smem, (cudaStream_t)stream>>>(
         ma, mb, nullptr, nullptr, 0, nullptr, out, ldc, M, N, kblocks, per, bn, idesc, tcols, 0,
         part ? 2 : 1, 0, vec_atomic, 1, status);
     if (cudaGetLastError() != cudaSuccess) return PCAGB_ECUDA;

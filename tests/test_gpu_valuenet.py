@@ -391,3 +391,11 @@ def test_loss_value_is_the_sums(n):
         assert net.lib.pcagb_vnet_loss(_p(L), _p(label), _p(rem), n, 50.0, _p(npos), _p(dL3),
                                        _p(stats), net.stream) == 0
         assert torch.equal(dL, dL3) and stats[2].item() == pos.sum().item()
+
+
+@pytest.mark.parametrize("M,N,K", [(129, 24, 64), (64, 80, 72), (200, 112, 128), (131, 120, 40),
+                                   (33, 144, 64), (257, 272, 192)])
+def test_tc_gemm_column_halves(M, N, K):
+    """Tile widths whose two halves differ (the second empty, shorter, not a
+    multiple of 32) and tiles of one row or column over."""
+    test_tc_gemm_matches_fp32(M, N, K)
