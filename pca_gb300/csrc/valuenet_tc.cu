@@ -121,6 +121,11 @@ __device__ __forceinline__ void mbar_init(uint32_t bar, uint32_t count)
     asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(bar), "r"(count) : "memory");
 }
 
+__device__ __forceinline__ void mbar_arrive(uint32_t bar)
+{
+    asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(bar) : "memory");
+}
+
 /* arrive on the barrier at this offset of the cluster's first CTA */
 __device__ __forceinline__ void mbar_arrive_first(uint32_t bar)
 {
@@ -690,17 +695,23 @@ k_encode_pool_tc(const __grid_constant__ CUtensorMap map_w1, const __grid_consta
  * M and N contiguous: the weight gradient dY^T . X reads dY [batch][out]
  * and X [batch][in] as stored), loaded as 64 x 64 boxes (64 K-rows of 64
  * elements along M or N) and described to the MMA as MN-major operands;
- * bn is then a multiple of 64. */
+ * bn is then a multiple of 64. With kSums (mn_major only) four of the warps
+ * that otherwise wait add up A's columns over the CTA's K rows from the same
+ * stages, dY's column sums: the bias gradient without another pass over dY
+ * (which took 37 us a layer of 262,144 rows; the product with the sums takes
+ * 53 us where it took 52). A form of its own: the branches cost the others 5%. */
 constexpr int kGRows = 128, kGBK = 64, kGStages = 2;
 constexpr int kGABytes = kGRows * 128;              /* 16 KB per A stage */
 constexpr int kGThreads = 256;
+constexpr int kGSumWarps = 4;                       /* warps 2..5 */
 
+template <bool kSums>
 __global__ void __launch_bounds__(kGThreads, 2)
 k_gemm_tc(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_b,
           const float *__restrict__ bias, const __nv_bfloat16 *__restrict__ mask, int ldm,
           __nv_bfloat16 *__restrict__ Cb, float *__restrict__ Cf, int ldc, int M, int N,
           int kblocks, int kb_per_split, int bn, uint32_t idesc, uint32_t tmem_cols, int relu,
-          int atomic_out, int stage_mode, int vec_atomic, int mn_major, int *status)
+          int atomic_out, int stage_mode, int vec_atomic, int mn_major, float *part_db, int *status)
 {
     extern __shared__ uint8_t gsmem_raw[];
     uint8_t *smem = (uint8_t *)(((uintptr_t)gsmem_raw + 1023) & ~(uintptr_t)1023);
@@ -720,10 +731,12 @@ k_gemm_tc(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUt
     const int kb0 = blockIdx.z * kb_per_split;
     const int nk = min(kblocks, kb0 + kb_per_split) - kb0;
 
+    /* the columns of A are summed once per row tile and K split */
+    const bool sums = kSums && blockIdx.x == 0;
     if (threadIdx.x == 0) {
         for (int s = 0; s < kGStages; s++) {
             mbar_init(full(s), 1);
-            mbar_init(empty(s), 1);
+            mbar_init(empty(s), sums ? 1 + kGSumWarps : 1);
         }
         mbar_init(done_bar, 1);
         *abort_flag = 0;
@@ -799,6 +812,30 @@ k_gemm_tc(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUt
         while (!mbar_test(done_bar, 0) && global_ns() - t0 < kWaitNs) {
         }
     }
+    float col[8] = {};
+    const int chunk = threadIdx.x & 15, slot = ((int)threadIdx.x - 64) >> 4;
+    if (sums && warp >= 2 && warp < 2 + kGSumWarps) {
+        /* a thread adds 8 columns (a 16-byte chunk of a row; 8 chunks of a
+           64-column box's swizzled row) of every 8th K row */
+        for (int i = 0; i < nk; i++) {
+            const int st = i % kGStages;
+            const bool ok = mbar_wait(full(st), (uint32_t)(i / kGStages) & 1u, abort_flag, status, 14);
+            if (!__all_sync(0xFFFFFFFFu, ok)) break;
+            const uint8_t *box = smem + st * kGABytes + (chunk >> 3) * 8192;
+#pragma unroll
+            for (int k = 0; k < 8; k++) {
+                const uint4 v = *(const uint4 *)(box + sw128_off(slot + 8 * k, chunk & 7));
+                const uint32_t w[4] = {v.x, v.y, v.z, v.w};
+#pragma unroll
+                for (int j = 0; j < 4; j++) {
+                    col[2 * j] += __uint_as_float(w[j] << 16);
+                    col[2 * j + 1] += __uint_as_float(w[j] & 0xFFFF0000u);
+                }
+            }
+            __syncwarp();
+            if (lane == 0) mbar_arrive(empty(st));
+        }
+    }
     __syncwarp();
     /* epilogue: all eight warps. The tile's bias goes to shared memory
        first (every thread takes part, so the barrier below is reached by
@@ -809,6 +846,20 @@ k_gemm_tc(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUt
     ok = __all_sync(0xFFFFFFFFu, ok) && !*abort_flag;
     tc_after();
     __syncthreads();
+    if (sums) {
+        /* every stage is drained: the 8 row slots' sums meet there */
+        float *ssum = (float *)smem;
+        if (warp >= 2 && warp < 2 + kGSumWarps)
+#pragma unroll
+            for (int j = 0; j < 8; j++) ssum[slot * kGRows + 8 * chunk + j] = col[j];
+        __syncthreads();
+        if (ok && threadIdx.x < kGRows && m0 + (int)threadIdx.x < M) {
+            float v = 0.f;
+#pragma unroll
+            for (int y = 0; y < 8; y++) v += ssum[y * kGRows + threadIdx.x];
+            part_db[(size_t)blockIdx.z * M + m0 + threadIdx.x] = v;
+        }
+    }
     /* two warps share a TMEM lane quarter (32 rows), half of the columns each */
     const int quarter = warp & 3, half = (bn / 2 + 31) / 32 * 32;
     const int lo = warp < 4 ? 0 : min(half, bn), hi = warp < 4 ? min(half, bn) : bn;
@@ -1103,7 +1154,7 @@ extern "C" int pcagb_vnet_gemm_tc(const void *A, int lda, const void *B, int ldb
     static std::once_flag attr_once;
     static cudaError_t attr_err = cudaSuccess;
     std::call_once(attr_once, [] {
-        attr_err = cudaFuncSetAttribute(k_gemm_tc, cudaFuncAttributeMaxDynamicSharedMemorySize,
+        attr_err = cudaFuncSetAttribute(k_gemm_tc<false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                         kGStages * (kGABytes + 256 * 128) + 256 + 2048);
     });
     /* the epilogue: staged through shared memory and stored in 16-byte
@@ -1118,9 +1169,9 @@ extern "C" int pcagb_vnet_gemm_tc(const void *A, int lda, const void *B, int ldb
     const int vec_atomic = splits > 1 && ldc % 4 == 0 && !((uintptr_t)Cf & 15);
     if (attr_err != cudaSuccess) return PCAGB_ECUDA;
     dim3 grid((N + bn - 1) / bn, (M + kGRows - 1) / kGRows, splits);
-    k_gemm_tc<<<grid, kGThreads, smem, (cudaStream_t)stream>>>(
+    k_gemm_tc<false><<<grid, kGThreads, smem, (cudaStream_t)stream>>>(
         ma, mb, bias, (const __nv_bfloat16 *)mask, ldm, (__nv_bfloat16 *)Cb, Cf, ldc, M, N,
-        kblocks, per, bn, idesc, tcols, relu, splits > 1, stage_mode, vec_atomic, 0, status);
+        kblocks, per, bn, idesc, tcols, relu, splits > 1, stage_mode, vec_atomic, 0, nullptr, status);
     return cudaGetLastError() == cudaSuccess ? PCAGB_OK : PCAGB_ECUDA;
 }
 
@@ -1140,25 +1191,29 @@ bool tile_map_mn(CUtensorMap *m, const void *ptr, int krows, int cols, int ld)
               CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
 
-/* C[i] += the `splits` slabs' values at i, in slab order: a thread per
- * value, 16 slabs' loads in flight before they are added (one after the
- * other a value waits for up to 152 loads in turn: 9 to 19 us a layer,
- * so 8 to 12). */
-__global__ void k_split_sum(const float *part, int splits, size_t count, float *C)
+/* C[i] += the `splits` slabs' values at i, in slab order, and the same for
+ * db from part_db (count_db values; 0: none): a thread per value, 16 slabs'
+ * loads in flight before they are added (one after the other a value waits
+ * for up to 152 loads in turn: 9 to 19 us a layer, so 8 to 12). */
+__global__ void k_split_sum(const float *part, int splits, size_t count, float *C,
+                            const float *part_db, size_t count_db, float *db)
 {
-    for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < count;
-         i += (size_t)gridDim.x * blockDim.x) {
+    for (size_t at = (size_t)blockIdx.x * blockDim.x + threadIdx.x; at < count + count_db;
+         at += (size_t)gridDim.x * blockDim.x) {
+        const bool first = at < count;
+        const size_t i = first ? at : at - count, n = first ? count : count_db;
+        const float *src = (first ? part : part_db) + i;
         float v = 0.f;
         int z = 0;
         for (; z + 16 <= splits; z += 16) {
             float p[16];
 #pragma unroll
-            for (int k = 0; k < 16; k++) p[k] = part[(size_t)(z + k) * count + i];
+            for (int k = 0; k < 16; k++) p[k] = src[(size_t)(z + k) * n];
 #pragma unroll
             for (int k = 0; k < 16; k++) v += p[k];
         }
-        for (; z < splits; z++) v += part[(size_t)z * count + i];
-        C[i] += v;
+        for (; z < splits; z++) v += src[(size_t)z * n];
+        (first ? C : db)[i] += v;
     }
 }
 
@@ -1181,9 +1236,9 @@ extern "C" int pcagb_vnet_wgrad_splits(int K, int splits)
  * so the result is the same on every run; without it the ranges' fp32 sums
  * are added into C atomically. C is zeroed by the caller (leading dimension
  * ldc). ldy and ldx are multiples of 8 elements, dY and X 16-byte aligned. */
-extern "C" int pcagb_vnet_wgrad_tc(const void *dY, int ldy, const void *X, int ldx, float *C,
-                                   int ldc, int M, int N, int K, int splits, float *part,
-                                   int *status, void *stream)
+static int wgrad(const void *dY, int ldy, const void *X, int ldx, float *C, int ldc, int M, int N,
+                 int K, int splits, float *part, float *db, float *part_db, int *status,
+                 void *stream)
 {
     if (M <= 0 || N <= 0 || K <= 0) return PCAGB_OK;
     if (!dY || !X || !C || !status || (ldy & 7) || (ldx & 7) || ldy < M || ldx < N ||
@@ -1205,24 +1260,45 @@ extern "C" int pcagb_vnet_wgrad_tc(const void *dY, int ldy, const void *X, int l
     static std::once_flag attr_once;
     static cudaError_t attr_err = cudaSuccess;
     std::call_once(attr_once, [] {
-        attr_err = cudaFuncSetAttribute(k_gemm_tc, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                        kGStages * (kGABytes + 256 * 128) + 256 + 2048);
+        for (auto *k : {&k_gemm_tc<false>, &k_gemm_tc<true>})
+            if (attr_err == cudaSuccess)
+                attr_err = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                                kGStages * (kGABytes + 256 * 128) + 256 + 2048);
     });
     if (attr_err != cudaSuccess) return PCAGB_ECUDA;
     float *out = part ? part : C;
     const int vec_atomic = ldc % 4 == 0 && !((uintptr_t)out & 15);
     dim3 grid((N + bn - 1) / bn, (M + kGRows - 1) / kGRows, splits);
-    k_gemm_tc<<<grid, kGThreads, smem, (cudaStream_t)stream>>>(
+    (part_db ? k_gemm_tc<true> : k_gemm_tc<false>)<<<grid, kGThreads, smem, (cudaStream_t)stream>>>(
         ma, mb, nullptr, nullptr, 0, nullptr, out, ldc, M, N, kblocks, per, bn, idesc, tcols, 0,
-        part ? 2 : 1, 0, vec_atomic, 1, status);
+        part ? 2 : 1, 0, vec_atomic, 1, part_db, status);
     if (cudaGetLastError() != cudaSuccess) return PCAGB_ECUDA;
     if (part) {
         const size_t count = (size_t)M * ldc;
-        const unsigned blocks = (unsigned)std::min<size_t>((count + 63) / 64, 4096);
-        k_split_sum<<<blocks, 64, 0, (cudaStream_t)stream>>>(part, splits, count, C);
+        const size_t count_db = part_db ? (size_t)M : 0;
+        const unsigned blocks = (unsigned)std::min<size_t>((count + count_db + 63) / 64, 4096);
+        k_split_sum<<<blocks, 64, 0, (cudaStream_t)stream>>>(part, splits, count, C, part_db,
+                                                             count_db, db);
         if (cudaGetLastError() != cudaSuccess) return PCAGB_ECUDA;
     }
     return PCAGB_OK;
+}
+
+extern "C" int pcagb_vnet_wgrad_tc(const void *dY, int ldy, const void *X, int ldx, float *C,
+                                   int ldc, int M, int N, int K, int splits, float *part,
+                                   int *status, void *stream)
+{
+    return wgrad(dY, ldy, X, ldx, C, ldc, M, N, K, splits, part, nullptr, nullptr, status, stream);
+}
+
+/* The same with the bias gradient: db[M] += dY's column sums. part and
+ * part_db (pcagb_vnet_wgrad_splits(K, splits) slabs of M floats) are needed. */
+extern "C" int pcagb_vnet_wgrad_bias_tc(const void *dY, int ldy, const void *X, int ldx, float *C,
+                                        int ldc, int M, int N, int K, int splits, float *part,
+                                        float *db, float *part_db, int *status, void *stream)
+{
+    if (M > 0 && N > 0 && K > 0 && (!part || !db || !part_db)) return PCAGB_EINVAL;
+    return wgrad(dY, ldy, X, ldx, C, ldc, M, N, K, splits, part, db, part_db, status, stream);
 }
 
 

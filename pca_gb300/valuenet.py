@@ -7,9 +7,9 @@ optimizer update is one of the C kernels, called through the C ABI.
 Every matrix product runs on the fifth-generation tensor cores (TMA,
 tcgen05.mma into TMEM, FP32 accumulation): the forward layers and the input
 gradients (pcagb_vnet_gemm_tc, the ReLU derivative applied in the epilogue),
-and the weight gradients (pcagb_vnet_wgrad_tc: split-K, both operands read
-as stored, MN-major), whose bias gradients are the output gradients' column
-sums (pcagb_vnet_colsum).
+and the weight gradients (split-K, both operands read
+as stored, MN-major), which add up the output gradients' columns, the bias
+gradients, from the same tiles (pcagb_vnet_wgrad_bias_tc).
 
 Network (the reference's ValueNetwork, python/model.py:16-84, with bit
 features): per-test encoder 176 -> 256 -> 256 (ReLU), mean + max pooling
@@ -40,6 +40,7 @@ def _lib():
     sigs = {
         "pcagb_vnet_gemm_tc": [vp, i, vp, i, vp, vp, i, vp, vp, i, i, i, i, i, i, vp, vp],
         "pcagb_vnet_wgrad_tc": [vp, i, vp, i, vp, i, i, i, i, i, vp, vp, vp],
+        "pcagb_vnet_wgrad_bias_tc": [vp, i, vp, i, vp, i, i, i, i, i, vp, vp, vp, vp, vp],
         "pcagb_vnet_wgrad_splits": [i, i],
         "pcagb_vnet_colsum": [vp, ctypes.c_longlong, i, i, vp, vp, i, vp],
         "pcagb_vnet_colsum_blocks": [ctypes.c_longlong, i],
@@ -169,15 +170,10 @@ class ValueNet:
             M, max(1, min(kblocks, (2 * self.sms) // max(tiles, 1))))
         # each K split writes its own slab, added in split order: the same
         # gradients (and so the same network) on every run
-        part = torch.empty(splits * out * inp, device=self.dev, dtype=torch.float32)
-        self._ck(self.lib.pcagb_vnet_wgrad_tc(
+        part = torch.empty(splits * out * (inp + 1), device=self.dev, dtype=torch.float32)
+        self._ck(self.lib.pcagb_vnet_wgrad_bias_tc(
             _p(dY), dY.stride(0), _p(X), X.stride(0), _p(G), inp, out, inp, M, splits, _p(part),
-            _p(self._status_word()), self.stream))
-        part = torch.empty(self.lib.pcagb_vnet_colsum_blocks(M, self.sms) * out,
-                           device=self.dev, dtype=torch.float32)
-        self._ck(self.lib.pcagb_vnet_colsum(_p(dY), M, out, dY.stride(0), _p(db), _p(part),
-                                            self.sms, self.stream))
-        return G, db
+            _p(db), _p(part[splits * out * inp:]), _p(self._status_word()), self.stream))
 
     def features(self, regs, flags, task, TP, task_io, task_T):
         n = task.shape[0]

@@ -399,3 +399,40 @@ def test_tc_gemm_column_halves(M, N, K):
     """Tile widths whose two halves differ (the second empty, shorter, not a
     multiple of 32) and tiles of one row or column over."""
     test_tc_gemm_matches_fp32(M, N, K)
+
+
+@pytest.mark.parametrize("out,inp,M,splits", [(16, 128, 1, 1), (16, 128, 64, 1), (128, 256, 65, 2),
+                                              (136, 64, 1000, 3), (256, 528, 4096, 43),
+                                              (256, 176, 262144 // 16, 152)])
+def test_weight_gradient_adds_the_bias_gradient(out, inp, M, splits):
+    """dW and db from one launch: dW is the launch without db, bit for bit; db
+    against float64 (row tiles of 128 outputs and one over, K blocks of 64
+    rows and one over, more splits than blocks), the same on every run, both
+    added to what is there."""
+    from pca_gb300.valuenet import _lib, _p
+    lib = _lib()
+    g = torch.Generator(device="cuda").manual_seed(out + M)
+    dY = torch.randn(M, out, device="cuda", generator=g).to(torch.bfloat16)
+    X = torch.randn(M, inp, device="cuda", generator=g).to(torch.bfloat16)
+    status = torch.zeros(1, dtype=torch.int32, device="cuda")
+    s = torch.cuda.current_stream().cuda_stream
+    ns = lib.pcagb_vnet_wgrad_splits(M, splits)
+    part = torch.empty(ns * out * inp, device="cuda")
+    pdb = torch.empty(ns * out, device="cuda")
+    runs = []
+    for _ in range(2):
+        G = torch.full((out, inp), 2.0, device="cuda")
+        db = torch.full((out,), 3.0, device="cuda")
+        assert lib.pcagb_vnet_wgrad_bias_tc(_p(dY), out, _p(X), inp, _p(G), inp, out, inp, M, splits,
+                                            _p(part), _p(db), _p(pdb), _p(status), s) == 0
+        runs.append((G, db))
+    G0 = torch.full((out, inp), 2.0, device="cuda")
+    assert lib.pcagb_vnet_wgrad_tc(_p(dY), out, _p(X), inp, _p(G0), inp, out, inp, M, splits,
+                                   _p(part), _p(status), s) == 0
+    assert status.item() == 0
+    assert torch.equal(runs[0][0], G0) and torch.equal(runs[0][0], runs[1][0])
+    assert torch.equal(runs[0][1], runs[1][1])
+    want = dY.double().sum(0) + 3
+    # sums of at most M fp32 additions of bf16 values
+    bound = 2.0 ** -24 * (M + 8) ** 0.5 * 4 * (dY.double().abs().sum(0) + 3)
+    assert ((runs[0][1].double() - want).abs() <= bound).all()
