@@ -37,15 +37,15 @@
  * E1(i + 2) does.
  *
  * What bounds it: 27 MMAs of 128 cycles a tile, 3,456, and the hand-overs
- * between the roles: 5,600 cycles a tile, tensor pipe 60% busy. In the
+ * between the roles: 5,300 cycles a tile, tensor pipe 65% busy. In the
  * one-CTA form (weights streamed, H2 pooled through shared memory by the
  * same 16 warps) the operands, 224 KB of weight slabs a tile and H2's way
  * were 800 KB of shared-memory traffic a tile of 128 rows and each warp
  * waited for its own record loads, 10,900 cycles. Measured on the way
  * (131,072 states of 16 to 32 tests): the pair alone 1.21 -> 0.85 ms; front
  * and back apart, accumulators fetched ahead and nothing computed from a
- * record when it is loaded 0.67; the quotient below and E1 in halves 0.63.
- * 4,096 states: 47 -> 31 us.
+ * record when it is loaded 0.67; the quotient below and E1 in halves 0.63;
+ * descriptors not kept 0.60. 4,096 states: 47 -> 31 us.
  *
  * Synchronisation is by mbarriers (and one cluster barrier at each end);
  * every wait is bounded by the global timer (kWaitNs). A wait that runs out
@@ -200,15 +200,16 @@ __device__ __forceinline__ void tma_load_2d(uint32_t dst, const CUtensorMap *map
 }
 
 /* Shared-memory matrix descriptor: K-major operand in 128-byte swizzle
-   atoms (8 rows x 128 B), 8-row groups 1024 B apart. */
+   atoms (8 rows x 128 B), 8-row groups 1024 B apart; the address in the low
+   word. */
+constexpr uint64_t kSw128Desc = (uint64_t)1 << 16 |            /* leading byte offset: unused */
+                                (uint64_t)(1024 >> 4) << 32 |  /* stride byte offset */
+                                (uint64_t)1 << 46 |            /* descriptor version */
+                                (uint64_t)2 << 61;             /* 128-byte swizzle */
+
 __device__ __forceinline__ uint64_t sw128_desc(uint32_t saddr)
 {
-    uint64_t d = (uint64_t)((saddr & 0x3FFFFu) >> 4);
-    d |= (uint64_t)1 << 16;            /* leading byte offset: unused for swizzled K-major */
-    d |= (uint64_t)(1024 >> 4) << 32;  /* stride byte offset */
-    d |= (uint64_t)1 << 46;            /* descriptor version */
-    d |= (uint64_t)2 << 61;            /* 128-byte swizzle */
-    return d;
+    return kSw128Desc | (uint64_t)((saddr & 0x3FFFFu) >> 4);
 }
 
 /* Shared-memory matrix descriptor: MN-major operand in 128-byte swizzle
@@ -225,15 +226,18 @@ __device__ __forceinline__ uint64_t sw128_mn_desc(uint32_t saddr)
     return d;
 }
 
-/* one product of the pair: A and B at these offsets of both CTAs */
-__device__ __forceinline__ void mma_pair(uint32_t dtmem, uint64_t a, uint64_t b, uint32_t idesc,
+/* one product of the pair: A and B at these offsets of both CTAs, given as
+   the low words of their descriptors */
+__device__ __forceinline__ void mma_pair(uint32_t dtmem, uint32_t a, uint32_t b, uint32_t idesc,
                                          uint32_t acc)
 {
+    constexpr uint32_t high = (uint32_t)(kSw128Desc >> 32);
     asm volatile(
-        "{\n\t.reg .pred p;\n\t"
+        "{\n\t.reg .pred p;\n\t.reg .b64 da, db;\n\t"
+        "mov.b64 da, {%1, %5};\n\tmov.b64 db, {%2, %5};\n\t"
         "setp.ne.b32 p, %4, 0;\n\t"
-        "tcgen05.mma.cta_group::2.kind::f16 [%0], %1, %2, %3, p;\n\t}" ::"r"(dtmem),
-        "l"(a), "l"(b), "r"(idesc), "r"(acc)
+        "tcgen05.mma.cta_group::2.kind::f16 [%0], da, db, %3, p;\n\t}" ::"r"(dtmem),
+        "r"(a), "r"(b), "r"(idesc), "r"(acc), "r"(high)
         : "memory");
 }
 
@@ -420,20 +424,29 @@ k_encode_pool_tc(const __grid_constant__ CUtensorMap map_w1, const __grid_consta
             auto wait = [&](int which, int tile, int code) {
                 return mbar_wait(bar(which), tile & 1, abort_flag, status, code);
             };
-            /* unrolled: a product takes this thread 100 to 120 cycles to
-               issue, in a loop 190, longer than the tensor core needs */
+            /* Unrolled: a product takes this thread 100 cycles to issue, in
+               a loop 190, longer than the tensor core needs. The descriptors'
+               low words are hidden from the compiler at each use: it would
+               otherwise keep all 76 of them, and load many back from local
+               memory before their product (633 us; so 601). */
+            const uint32_t a1 = (uint32_t)sw128_desc(sA1), w1 = (uint32_t)sw128_desc(sW1);
+            const uint32_t a2 = (uint32_t)sw128_desc(sA2), w2 = (uint32_t)sw128_desc(sW2);
+            auto hidden = [](uint32_t v) {
+                asm volatile("" : "+r"(v));
+                return v;
+            };
+            /* K step k of 16: 32 bytes along the rows of a 64-column block */
+            auto step = [](int k) { return (uint32_t)((k >> 2) * (kBlock >> 4) + (k & 3) * 2); };
             auto e1 = [&](int i) {
                 if (!wait(kBarA1, i, 2)) return false;
 #pragma unroll
                 for (int u = 0; u < 2; u++) {
                     if (i && !wait(kBarFree1 + u, i - 1, 3)) return false;
                     tc_after();
+                    const uint32_t a = hidden(a1), w = hidden(w1 + u * (kBlock >> 5));
 #pragma unroll
                     for (int k = 0; k < kFeat / 16; k++)
-                        mma_pair(tmem + kHalfUnits * u,
-                                 sw128_desc(sA1 + (k >> 2) * kBlock + 32 * (k & 3)),
-                                 sw128_desc(sW1 + (k >> 2) * kBlock + u * (kBlock / 2) + 32 * (k & 3)),
-                                 kIdescE1, k != 0);
+                        mma_pair(tmem + kHalfUnits * u, a + step(k), w + step(k), kIdescE1, k != 0);
                     mma_commit_pair(bar(kBarD1 + u));
                 }
                 return true;
@@ -442,10 +455,10 @@ k_encode_pool_tc(const __grid_constant__ CUtensorMap map_w1, const __grid_consta
                 if (!wait(kBarA2, i, 4)) return false;
                 if (i && !wait(kBarFree2, i - 1, 5)) return false;
                 tc_after();
+                const uint32_t a = hidden(a2), w = hidden(w2);
 #pragma unroll
                 for (int k = 0; k < 4 * kKB2; k++) {
-                    mma_pair(tmem + kUnits, sw128_desc(sW2 + (k >> 2) * kBlock + 32 * (k & 3)),
-                             sw128_desc(sA2 + (k >> 2) * kBlock + 32 * (k & 3)), kIdescE2, k != 0);
+                    mma_pair(tmem + kUnits, w + step(k), a + step(k), kIdescE2, k != 0);
                     if ((k & 3) == 3) mma_commit_pair(bar(kBarE2 + (k >> 2)));
                 }
                 return true;
