@@ -45,28 +45,28 @@ CANDIDATES = ("candidates as the reference's enumerator counts them (tools/enume
               "counts the class evaluations its kernels execute)")
 
 # The suffix kernel's capture (profiles/k_suffix_lanes_is_power2_t32_k4.md):
-# warp instructions and DRAM bytes of the depth-4 launch (the autotuner's
-# choice there, a lane per prefix with two tests per lane), valid for the
-# kernel source it was taken from (SHA-256 of
-# pca_gb300/csrc/engine_kernels.cuh, first 16 hex).
-SUFFIX_CAPTURE = {"kernel": "k_suffix_lanes<32,2>", "choice": (2, 32), "inst": 336474909,
-                  "ms": 0.521024, "dram_bytes": 379046912 + 266496,
-                  "source_sha16": ("5e54a4b385e0443c",),
+# warp instructions and DRAM bytes of the depth-4 launch (a lane per prefix
+# with two tests per lane), valid for the kernel source it was taken from
+# (SHA-256 of pca_gb300/csrc's engine_kernels.cuh, suffix_forms.cuh and
+# value_forms.h, first 16 hex) and the autotuner's choice.
+SUFFIX_CAPTURE = {"kernel": "k_suffix_lanes<32,2>", "choice": (2, 32), "inst": 132652957,
+                  "ms": 0.238912, "dram_bytes": 376526336 + 290560,
+                  "source_sha16": ("791be789cc8eae2f",),
                   "file": "profiles/k_suffix_lanes_is_power2_t32_k4.md"}
 # The insert kernel's capture (profiles/k_expand_insert_is_power2_t32_level3.md):
 # DRAM bytes read + written by the level-3 launch (99.6% of a solve's children).
-# Valid for the captured source and for 5e54a4b3..., which differs from it
-# only inside k_suffix_lanes (its own evaluation count), a kernel the insert
-# launch neither calls nor shares code with.
-INSERT_CAPTURE = {"dram_bytes": 540317696 + 170325504,
-                  "source_sha16": ("17cc19cb3689daec", "5e54a4b385e0443c"),
+INSERT_CAPTURE = {"dram_bytes": 541437440 + 187046400,
+                  "source_sha16": ("791be789cc8eae2f",),
                   "file": "profiles/k_expand_insert_is_power2_t32_level3.md"}
 
 
 def kernel_source_sha16() -> str:
     import hashlib
-    with open(os.path.join(REPO, "pca_gb300", "csrc", "engine_kernels.cuh"), "rb") as f:
-        return hashlib.sha256(f.read()).hexdigest()[:16]
+    h = hashlib.sha256()
+    for name in ("engine_kernels.cuh", "suffix_forms.cuh", "value_forms.h"):
+        with open(os.path.join(REPO, "pca_gb300", "csrc", name), "rb") as f:
+            h.update(f.read())
+    return h.hexdigest()[:16]
 
 
 def bench_config(args, world: int) -> dict:
@@ -275,16 +275,17 @@ def run_reference_binary(exe: str, path: str, depth: int):
 def insert_roofline(sol, T: int, insert_ms: float, hbm_gbs: float, pk_kind: str) -> dict:
     """k_expand_insert against HBM. Algorithmic bytes of a level build (the
     OEP kernel's unit of work): per child an 8-byte slot probe, per child
-    that is not a new state a 17*T-byte compare of the state it equals, per
-    parent a 17*T-byte read of its state. Summed over the solve's builds
-    (levels 1..split) and divided by the insert launches' device time."""
+    that is not a new state the ids of the state it equals (its parent's
+    eight 4-byte column ids, its own and its link), per parent a 17*T-byte
+    read of its state and its ids. Summed over the solve's builds (levels
+    1..split) and divided by the insert launches' device time."""
     S = len(sol.level_survivors) - 1
     byts = 0
     for d in range(1, S + 1):
         kids, kept, parents = sol.level_children[d], sol.level_survivors[d], sol.level_survivors[d - 1]
         if kids == 0:
             continue
-        byts += kids * 8 + (kids - kept) * 17 * T + parents * 17 * T
+        byts += kids * 8 + (kids - kept) * 40 + parents * (17 * T + 32)
     achieved = byts / (insert_ms / 1000.0) / 1e9 if insert_ms > 0 else 0.0
     fresh = kernel_source_sha16() in INSERT_CAPTURE["source_sha16"]
     return {"kernel": "k_expand_insert<32> (exact OEP insert of levels 1..3)", "bound": "hbm",
@@ -295,7 +296,7 @@ def insert_roofline(sol, T: int, insert_ms: float, hbm_gbs: float, pk_kind: str)
             "traffic_note": ("DRAM bytes of the level-3 launch from one ncu capture "
                              f"({INSERT_CAPTURE['file']}); null when the kernel source changed "
                              "since that capture"),
-            "bytes_model": "per child 8 B slot + per duplicate 17*T B compare + per parent 17*T B"}
+            "bytes_model": "per child 8 B slot + per duplicate 40 B of ids + per parent 17*T + 32 B"}
 
 
 def tuned_depth1_choice(tuning: dict) -> tuple[int, int]:

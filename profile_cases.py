@@ -160,7 +160,7 @@ def _branch_case(name: str, reps: int):
     import json
     import os
     from pca_gb300.pcalib import Engine, task_from_dict
-    fx = os.path.join(os.path.dirname(os.path.dirname(os.path.abspath(__file__))), "tests",
+    fx = os.path.join(os.path.dirname(os.path.abspath(__file__)), "tests",
                       "golden", "ref_published.json")
     spec = next(t for t in json.load(open(fx)) if t["name"] == name)
     task = task_from_dict(spec["task"])
