@@ -1077,6 +1077,279 @@ k_gemm_tc(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUt
                      : "memory");
 }
 
+/* ---- the scoring trunk -------------------------------------------------------
+ *
+ * Z1 = relu(P . T1^T + b), Z2 = relu(Z1 . T2^T + b), logits = Z2 . H^T + b of
+ * 128 pooled rows a tile in one kernel, a persistent CTA per SM; Z1 and Z2
+ * stay in shared memory. Warp 0 streams P's blocks and the weights (370 KB a
+ * tile, from L2) by TMA through a two-stage ring, a thread of warp 1 issues
+ * the MMAs (M = 128; N = 256, 128, 16; the GEMM kernel's order of K blocks,
+ * so its results), eight warps (two a TMEM lane quarter) are the epilogues.
+ * The products run in the order T1(i + 1), T2(i), H(i - 1), so each
+ * epilogue's work lies beside the others' products.
+ *
+ * Bound by the operands' way from L2, 670 KB a tile. As three launches of
+ * k_gemm_tc Z1 and Z2 went through HBM: 131,072 rows 122 -> 64 us, and
+ * 4,096 rows, mostly the three calls, 57 -> 21. */
+constexpr int kTK1 = 9, kTK2 = 4, kTK3 = 2;           /* 64-column K blocks: 528, 256, 128 */
+constexpr int kTStages = 2;
+constexpr int kTStage = 3 * kBlock;                   /* A 16 KB, then B up to 32 KB */
+constexpr int kTOffZ1 = kTStages * kTStage;           /* 64 KB */
+constexpr int kTOffZ2 = kTOffZ1 + kTK2 * kBlock;      /* 32 KB */
+constexpr int kTOffBias = kTOffZ2 + kTK3 * kBlock;    /* 256 + 128 + 16 fp32 */
+constexpr int kTOffBar = kTOffBias + 400 * 4;
+constexpr int kTSmem = kTOffBar + 256 + 1024;
+constexpr int kTEpiWarps = 8, kTThreads = 64 + 32 * kTEpiWarps;
+constexpr int kTFull = 0, kTEmpty = kTStages, kTD1 = 2 * kTStages, kTD2 = kTD1 + 1,
+              kTD3 = kTD1 + 2, kTZ1 = kTD1 + 3, kTZ2 = kTD1 + 4, kTFree1 = kTD1 + 5,
+              kTFree2 = kTD1 + 6, kTFree3 = kTD1 + 7, kTDrain = kTD1 + 8, kTBars = kTD1 + 9;
+static_assert(kTSmem <= 227 * 1024 && kTOffBar % 8 == 0 && kTBars * 8 + 8 <= 256, "shared memory");
+constexpr uint32_t kTColD2 = 256, kTColD3 = 384;      /* D1: columns 0..255 */
+
+__device__ __forceinline__ void mma_one(uint32_t dtmem, uint64_t a, uint64_t b, uint32_t idesc,
+                                        uint32_t acc)
+{
+    asm volatile(
+        "{\n\t.reg .pred p;\n\t"
+        "setp.ne.b32 p, %4, 0;\n\t"
+        "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}" ::"r"(dtmem),
+        "l"(a), "l"(b), "r"(idesc), "r"(acc)
+        : "memory");
+}
+
+__global__ void __launch_bounds__(kTThreads, 1)
+k_trunk_tc(const __grid_constant__ CUtensorMap map_p, const __grid_constant__ CUtensorMap map_w1,
+           const __grid_constant__ CUtensorMap map_w2, const __grid_constant__ CUtensorMap map_w3,
+           const float *__restrict__ b1, const float *__restrict__ b2,
+           const float *__restrict__ b3, int n, float *__restrict__ logits, int *status)
+{
+    extern __shared__ uint8_t tsmem_raw[];
+    uint8_t *smem = (uint8_t *)(((uintptr_t)tsmem_raw + 1023) & ~(uintptr_t)1023);
+    const uint32_t sbase = smem_u32(smem), sBar = sbase + kTOffBar;
+    uint32_t *tmem_slot = (uint32_t *)(smem + kTOffBar + kTBars * 8);
+    volatile int *abort_flag = (volatile int *)(smem + kTOffBar + kTBars * 8 + 4);
+    float *bias = (float *)(smem + kTOffBias);
+    auto bar = [&](int i) { return sBar + 8u * (uint32_t)i; };
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int ntiles = (n + kRows - 1) / kRows;
+    const int mine = (int)blockIdx.x < ntiles ? (ntiles - 1 - (int)blockIdx.x) / (int)gridDim.x + 1 : 0;
+    auto row0 = [&](int i) { return ((int)blockIdx.x + i * (int)gridDim.x) * kRows; };
+
+    if (threadIdx.x == 0) {
+        for (int i = 0; i < kTBars; i++)
+            mbar_init(bar(i), i >= kTZ1 && i <= kTFree2 ? kTEpiWarps : i == kTFree3 ? 4 : 1);
+        *abort_flag = 0;
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+        fence_async_smem();
+    }
+    for (int i = threadIdx.x; i < 400; i += kTThreads)
+        bias[i] = i < 256 ? b1[i] : i < 384 ? b2[i - 256] : b3[i - 384];
+    if (warp == 1) {
+        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], 512;" ::"r"(
+                         smem_u32(tmem_slot))
+                     : "memory");
+        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+    }
+    tc_before();
+    __syncthreads();
+    tc_after();
+    const uint32_t tmem = *tmem_slot;
+
+    if (warp == 0) {
+        /* ---- TMA producer, in the order of the products ---- */
+        if (lane == 0) {
+            uint32_t j = 0;
+            auto stage = [&](uint32_t bytes, uint32_t &st) {
+                st = j % kTStages;
+                if (!mbar_wait(bar(kTEmpty + st), ((j / kTStages) & 1u) ^ 1u, abort_flag, status, 21))
+                    return false;
+                mbar_expect_tx(bar(kTFull + st), bytes);
+                j++;
+                return true;
+            };
+            auto t1 = [&](int i) {
+                for (int k = 0; k < kTK1; k++) {
+                    uint32_t st;
+                    if (!stage(kTStage, st)) return false;
+                    tma_load_2d(sbase + st * kTStage, &map_p, bar(kTFull + st), 64 * k, row0(i));
+                    tma_load_2d(sbase + st * kTStage + kBlock, &map_w1, bar(kTFull + st), 64 * k, 0);
+                }
+                return true;
+            };
+            auto weights = [&](const CUtensorMap *map, int blocks, uint32_t bytes) {
+                for (int k = 0; k < blocks; k++) {
+                    uint32_t st;
+                    if (!stage(bytes, st)) return false;
+                    tma_load_2d(sbase + st * kTStage + kBlock, map, bar(kTFull + st), 64 * k, 0);
+                }
+                return true;
+            };
+            bool ok = mine > 0 && t1(0);
+            for (int i = 0; i <= mine && ok; i++) {
+                if (i + 1 < mine) ok = t1(i + 1);
+                if (ok && i < mine) ok = weights(&map_w2, kTK2, kBlock);
+                if (ok && i > 0) ok = weights(&map_w3, kTK3, 16 * 128);
+            }
+            /* the copies this thread issued land before the CTA leaves */
+            for (uint32_t back = 1; back <= kTStages && back <= j; back++) {
+                const uint32_t last = j - back;
+                const unsigned long long t0 = global_ns();
+                while (!mbar_test(bar(kTFull + last % kTStages), (last / kTStages) & 1u) &&
+                       global_ns() - t0 < kWaitNs) {
+                }
+            }
+        }
+    } else if (warp == 1) {
+        /* ---- MMA issuer ---- */
+        if (lane == 0) {
+            uint32_t j = 0;
+            auto wait = [&](int which, int tile, int code) {
+                return mbar_wait(bar(which), tile & 1, abort_flag, status, code);
+            };
+            /* blocks of a product: A from the ring (z < 0) or from shared
+               memory at offset z; the last block has `last` K steps */
+            auto product = [&](int blocks, int last, int z, uint32_t col, int N, int done) {
+                const uint32_t idesc = (1u << 4) | (1u << 7) | (1u << 10) |
+                                       ((uint32_t)(N >> 3) << 17) | ((uint32_t)(kRows >> 4) << 24);
+                for (int kb = 0; kb < blocks; kb++, j++) {
+                    const uint32_t st = j % kTStages;
+                    if (!mbar_wait(bar(kTFull + st), (j / kTStages) & 1u, abort_flag, status, 22))
+                        return false;
+                    tc_after();
+                    const uint32_t ring = sbase + st * kTStage;
+                    const uint64_t da = sw128_desc(z < 0 ? ring : sbase + z + kb * kBlock);
+                    const uint64_t db = sw128_desc(ring + kBlock);
+#pragma unroll
+                    for (int k = 0; k < 4; k++)
+                        if (kb + 1 < blocks || k < last)
+                            mma_one(tmem + col, da + 2 * k, db + 2 * k, idesc, (kb | k) != 0);
+                    mma_commit(bar(kTEmpty + st));
+                }
+                mma_commit(bar(done));
+                return true;
+            };
+            auto t1 = [&](int i) {
+                if (i && !wait(kTFree1, i - 1, 23)) return false;
+                tc_after();
+                return product(kTK1, 1, -1, 0, 256, kTD1);
+            };
+            bool ok = mine > 0 && t1(0);
+            for (int i = 0; i <= mine && ok; i++) {
+                if (i + 1 < mine) ok = t1(i + 1);
+                if (ok && i < mine) {
+                    ok = wait(kTZ1, i, 24) && (!i || wait(kTFree2, i - 1, 25));
+                    tc_after();
+                    ok = ok && product(kTK2, 4, kTOffZ1, kTColD2, 128, kTD2);
+                }
+                if (ok && i > 0) {
+                    ok = wait(kTZ2, i - 1, 26) && (i < 2 || wait(kTFree3, i - 2, 27));
+                    tc_after();
+                    ok = ok && product(kTK3, 4, kTOffZ2, kTColD3, 16, kTD3);
+                }
+            }
+            /* every MMA this thread issued has finished before TMEM is freed */
+            mma_commit(bar(kTDrain));
+            const unsigned long long t0 = global_ns();
+            while (!mbar_test(bar(kTDrain), 0) && global_ns() - t0 < kWaitNs) {
+            }
+        }
+    } else {
+        /* ---- epilogues: two warps a lane quarter (32 rows), half of the
+           columns each ---- */
+        const int q = warp & 3, h = (warp - 2) >> 2;
+        const int r = q * 32 + lane;
+        const uint32_t lane_base = (uint32_t)(q * 32) << 16;
+        /* 32 columns of accumulators + bias, ReLU, bf16 */
+        auto drain = [&](uint32_t col, const float *b, uint32_t *w) {
+            uint32_t acc[32];
+            tmem_ld32(tmem + lane_base + col, acc);
+#pragma unroll
+            for (int c = 0; c < 8; c++) {
+                const float4 bv = *(const float4 *)(b + 4 * c);
+                const float2 u = add_f32x2(acc[4 * c], acc[4 * c + 1], bv.x, bv.y);
+                const float2 v = add_f32x2(acc[4 * c + 2], acc[4 * c + 3], bv.z, bv.w);
+                w[2 * c] = relu_bf16x2(u.x, u.y);
+                w[2 * c + 1] = relu_bf16x2(v.x, v.y);
+            }
+        };
+        /* a K block (64 columns) of the next product's operand */
+        auto store = [&](int off, const uint32_t *w) {
+#pragma unroll
+            for (int c = 0; c < 8; c++)
+                *(uint4 *)(smem + off + sw128_off(r, c)) =
+                    make_uint4(w[4 * c], w[4 * c + 1], w[4 * c + 2], w[4 * c + 3]);
+        };
+        auto arrive = [&](int which) {
+            __syncwarp();
+            if (lane == 0) mbar_arrive(bar(which));
+        };
+        auto wait = [&](int which, int tile, int code) {
+            const bool done = mbar_wait(bar(which), tile & 1, abort_flag, status, code);
+            return __all_sync(0xffffffffu, done) != 0;
+        };
+        for (int i = 0; i < mine + 2 && mine; i++) {
+            if (i < mine) {
+                /* T1(i) into Z1, once T2(i - 1) has read it */
+                if (!wait(kTD1, i, 28)) break;
+                tc_after();
+                uint32_t w[64];
+#pragma unroll
+                for (int g = 0; g < 4; g++)
+                    drain((uint32_t)(128 * h + 32 * g), bias + 128 * h + 32 * g, w + 16 * g);
+                tc_before();
+                arrive(kTFree1);
+                if (i && !wait(kTD2, i - 1, 29)) break;
+#pragma unroll
+                for (int k = 0; k < 2; k++) store(kTOffZ1 + (2 * h + k) * kBlock, w + 32 * k);
+                fence_async_smem();
+                arrive(kTZ1);
+            }
+            if (i >= 1 && i <= mine) {
+                /* T2(i - 1) into Z2, once H(i - 2) has read it */
+                if (!wait(kTD2, i - 1, 30)) break;
+                tc_after();
+                uint32_t w[32];
+#pragma unroll
+                for (int g = 0; g < 2; g++)
+                    drain(kTColD2 + 64 * h + 32 * g, bias + 256 + 64 * h + 32 * g, w + 16 * g);
+                tc_before();
+                arrive(kTFree2);
+                if (i >= 2 && !wait(kTD3, i - 2, 31)) break;
+                store(kTOffZ2 + h * kBlock, w);
+                fence_async_smem();
+                arrive(kTZ2);
+            }
+            if (i >= 2 && h == 0) {
+                /* H(i - 2): the logits, a row a lane */
+                if (!wait(kTD3, i - 2, 32)) break;
+                tc_after();
+                uint32_t acc[32];
+                tmem_ld32(tmem + lane_base + kTColD3, acc);
+                tc_before();
+                arrive(kTFree3);
+                const int row = row0(i - 2) + r;
+                if (row < n)
+#pragma unroll
+                    for (int c = 0; c < 4; c++) {
+                        const float4 b = *(const float4 *)(bias + 384 + 4 * c);
+                        *(float4 *)(logits + (size_t)row * 16 + 4 * c) =
+                            make_float4(__uint_as_float(acc[4 * c]) + b.x,
+                                        __uint_as_float(acc[4 * c + 1]) + b.y,
+                                        __uint_as_float(acc[4 * c + 2]) + b.z,
+                                        __uint_as_float(acc[4 * c + 3]) + b.w);
+                    }
+            }
+        }
+    }
+    __syncwarp();
+    tc_before();
+    __syncthreads();
+    tc_after();
+    if (warp == 1)
+        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, 512;" ::"r"(tmem)
+                     : "memory");
+}
+
 
 typedef CUresult (*EncodeTiledFn)(CUtensorMap *, CUtensorMapDataType, cuuint32_t, void *,
                                   const cuuint64_t *, const cuuint64_t *, const cuuint32_t *,
@@ -1344,5 +1617,39 @@ extern "C" int pcagb_vnet_encode_pool_tc(const void *W1, const float *b1, const 
     k_encode_pool_tc<<<2 * pairs, kThreads, kSmemBytes, (cudaStream_t)stream>>>(
         m1, m2, b1, b2, regs, flags, live, task, depth, TP, n, task_io, task_T,
         (__nv_bfloat16 *)P, status);
+    return cudaGetLastError() == cudaSuccess ? PCAGB_OK : PCAGB_ECUDA;
+}
+
+/* Logits [n][16] (fp32) of pooled rows P [n][528] through the trunk: T1 [256]
+ * [528], T2 [128][256], H [16][128] bf16, row-major and contiguous. P, the
+ * weights and the logits are 16-byte aligned. *status as in the other
+ * tcgen05 launches. */
+extern "C" int pcagb_vnet_trunk_tc(const void *P, int n, const void *T1, const float *b1,
+                                   const void *T2, const float *b2, const void *H, const float *b3,
+                                   float *logits, int *status, void *stream)
+{
+    if (n <= 0) return PCAGB_OK;
+    if (!P || !T1 || !T2 || !H || !b1 || !b2 || !b3 || !logits || !status ||
+        (((uintptr_t)P | (uintptr_t)T1 | (uintptr_t)T2 | (uintptr_t)H | (uintptr_t)logits) & 15))
+        return PCAGB_EINVAL;
+    CUtensorMap mp, m1, m2, m3;
+    if (!tile_map(&mp, P, n, kPoolCols, kPoolCols, kRows) ||
+        !tile_map(&m1, T1, 256, kPoolCols, kPoolCols, 256) ||
+        !tile_map(&m2, T2, 128, 256, 256, 128) || !tile_map(&m3, H, 16, 128, 128, 16))
+        return PCAGB_ECUDA;
+    int dev = 0, sms = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess ||
+        cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess)
+        return PCAGB_ECUDA;
+    static std::once_flag attr_once;
+    static cudaError_t attr_err = cudaSuccess;
+    std::call_once(attr_once, [] {
+        attr_err = cudaFuncSetAttribute(k_trunk_tc, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                        kTSmem);
+    });
+    if (attr_err != cudaSuccess) return PCAGB_ECUDA;
+    const int ntiles = (n + kRows - 1) / kRows;
+    k_trunk_tc<<<ntiles < sms ? ntiles : sms, kTThreads, kTSmem, (cudaStream_t)stream>>>(
+        mp, m1, m2, m3, b1, b2, b3, n, logits, status);
     return cudaGetLastError() == cudaSuccess ? PCAGB_OK : PCAGB_ECUDA;
 }

@@ -54,6 +54,7 @@ def _lib():
         "pcagb_vnet_to_bf16": [vp, vp, sz, vp],
         "pcagb_vnet_encode_pool_tc": [vp, vp, vp, vp, vp, vp, vp, vp, vp, i, i, vp, vp, vp, vp,
                                       vp],
+        "pcagb_vnet_trunk_tc": [vp, i, vp, vp, vp, vp, vp, vp, vp, vp, vp],
         "pcagb_vnet_gather_sample": [vp, vp, vp, vp, vp, vp, i, i, vp],
         "pcagb_vnet_compose_order": [vp, vp, i, vp, ctypes.c_ulonglong, vp],
     }
@@ -220,6 +221,15 @@ class ValueNet:
             raise RuntimeError(f"tensor-core kernel aborted (barrier wait {v} timed out)")
 
     def trunk(self, P):
+        """Logits [n][16] of pooled rows: the three layers in one launch, or
+        a product each for rows that are not contiguous."""
+        if P.is_contiguous() and P.shape[1] == 528 and P.data_ptr() % 16 == 0:
+            L = torch.empty(P.shape[0], 16, device=self.dev, dtype=torch.float32)
+            self._ck(self.lib.pcagb_vnet_trunk_tc(
+                _p(P), P.shape[0], _p(self.Wb["T1"]), _p(self.b["T1"]), _p(self.Wb["T2"]),
+                _p(self.b["T2"]), _p(self.Wb["H"]), _p(self.b["H"]), _p(L),
+                _p(self._status_word()), self.stream))
+            return L
         Z1 = self._gemm(P, "T1", True)
         Z2 = self._gemm(Z1, "T2", True)
         return self._gemm(Z2, "H", False, out_f32=True)

@@ -436,3 +436,24 @@ def test_weight_gradient_adds_the_bias_gradient(out, inp, M, splits):
     # sums of at most M fp32 additions of bf16 values
     bound = 2.0 ** -24 * (M + 8) ** 0.5 * 4 * (dY.double().abs().sum(0) + 3)
     assert ((runs[0][1].double() - want).abs() <= bound).all()
+
+
+@pytest.mark.parametrize("n", [1, 127, 128, 129, 152 * 128, 152 * 128 + 1, 2 * 152 * 128 + 77,
+                               4 * 152 * 128 - 5])
+def test_trunk_in_one_launch(n):
+    """The fused trunk against its three products, bit for bit (the same
+    order of K blocks): one row, a tile and one over, one tile a CTA, one more,
+    three and four tiles a CTA; rows that are not contiguous."""
+    from pca_gb300.valuenet import ValueNet
+    net = ValueNet(seed=9)
+    g = torch.Generator(device="cuda").manual_seed(n)
+    P = torch.randn(n, 528, device="cuda", generator=g).to(torch.bfloat16)
+    L = net.trunk(P)
+    net.check_status()
+    Z1 = net._gemm(P, "T1", True)
+    Z2 = net._gemm(Z1, "T2", True)
+    assert torch.equal(L, net._gemm(Z2, "H", False, out_f32=True))
+    wide = torch.zeros(n, 536, device="cuda", dtype=torch.bfloat16)
+    wide[:, :528] = P
+    assert torch.equal(net.trunk(wide[:, :528]), L)
+    net.check_status()
