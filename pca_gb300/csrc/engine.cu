@@ -67,6 +67,9 @@ constexpr int kMaxBatch = 8192;
 /* engine_init's budget for an engine whose arena each solve supplies */
 constexpr size_t kArenaExternal = ~size_t(0);
 /* slots of the pinned host buffer */
+/* [kPinBuild ..]: d_small[2 ..] after a build: survivors, status at 6, the
+   bitmap's set bits at 7 */
+constexpr int kPinBuild = 16;
 constexpr int kPinStatus = 0, kPinSurvivors = 1, kPinTotal = 2, kPinCount = 3,
               kPinHist = 64;
 /* A level whose children's states fit in this many bytes, or in an eighth
@@ -157,10 +160,12 @@ struct pcagb_engine {
     size_t cap = 0, bottom = 0, top = 0;
     unsigned long long *d_small = nullptr;   /* [0] sol count [1] unused [2] count
                                                 [3] value-class evaluations run
-                                                [4] the work counter of the insert and
-                                                lean materialise kernels
-                                                [5] column ids given out */
-    uint32_t *d_status = nullptr;
+                                                [4] the insert kernel's work counter
+                                                [5] column ids given out
+                                                [6] the lean materialise kernel's work
+                                                counter [8] status [9] a bitmap's set
+                                                bits */
+    uint32_t *d_status = nullptr;            /* in d_small */
     ulonglong2 *d_sol = nullptr;
     ulonglong2 *d_firsts = nullptr;          /* [cap_tasks] SolBuf::firsts */
     FirstOut *d_first_out = nullptr;         /* [cap_tasks] */
@@ -374,11 +379,13 @@ int alloc_level(pcagb_engine *e, Level &L, uint64_t n)
 
 /* Enqueue the level's (task, mask) histogram and its copy into the pinned
    buffer; take_hist reads it after the stream has been synchronised. With
-   n_dev set, L.n is an upper bound and the device holds the count. */
-int enqueue_hist(pcagb_engine *e, const Level &L, const unsigned long long *n_dev)
+   n_dev set, L.n is an upper bound and the device holds the count; with
+   cleared, d_hist is zero. */
+int enqueue_hist(pcagb_engine *e, const Level &L, const unsigned long long *n_dev,
+                 bool cleared = false)
 {
     const size_t nh = (size_t)e->ntasks * 128;
-    CK(cudaMemsetAsync(e->d_hist, 0, nh * sizeof(unsigned long long), e->stream));
+    if (!cleared) CK(cudaMemsetAsync(e->d_hist, 0, nh * sizeof(unsigned long long), e->stream));
     if (nh <= 4096)
         k_task_hist_smem<<<e->grid(2), 256, nh * sizeof(uint32_t), e->stream>>>(
             L.live, L.task, L.n, n_dev, (uint32_t)nh, e->d_hist);
@@ -410,12 +417,12 @@ uint32_t split_log2(uint64_t parents, int grid)
 
 template <int TPC>
 int launch_expand(pcagb_engine *e, const Level &P, const uint32_t *fcr_up,
-                  unsigned long long *table, uint64_t tmask, const IdDev &ids)
+                  unsigned long long *table, uint64_t tmask, const IdDev &ids, bool cleared)
 {
     const int g = e->grid(e->occ_insert);
     /* the work-item counter the kernel's warps draw from */
     uint32_t *next = reinterpret_cast<uint32_t *>(e->d_small + 4);
-    CK(cudaMemsetAsync(next, 0, 4, e->stream));
+    if (!cleared) CK(cudaMemsetAsync(next, 0, 4, e->stream));
     if (ids.tab) {
         k_state_ids<TPC><<<e->grid(4), kThreads, 0, e->stream>>>(view(P), ids, e->d_status);
         const int rc = check_launch(e);
@@ -436,7 +443,7 @@ int launch_expand(pcagb_engine *e, const Level &P, const uint32_t *fcr_up,
    insert takes 0.06-0.08 ms with ids and 0.08-0.11 without, at one parent the
    extra pass and the clearing cost more than there is to compare. */
 constexpr uint64_t kIdParents = 64;
-int alloc_ids(pcagb_engine *e, const Level &P, IdDev *out)
+int alloc_ids(pcagb_engine *e, const Level &P, IdDev *out, ClearList *clear)
 {
     IdDev D{};
     *out = D;
@@ -465,21 +472,25 @@ int alloc_ids(pcagb_engine *e, const Level &P, IdDev *out)
     D.mask = slots - 1;
     D.cap = (uint32_t)cap;
     D.next = reinterpret_cast<uint32_t *>(e->d_small + 5);
-    CK(cudaMemsetAsync(D.next, 0, 4, e->stream));
-    CK(cudaMemsetAsync(D.tab, 0, slots * 8, e->stream));
+    if (clear) {
+        clear->add(D.tab, slots * 8);   /* the caller clears next with d_small */
+    } else {
+        CK(cudaMemsetAsync(D.next, 0, 4, e->stream));
+        CK(cudaMemsetAsync(D.tab, 0, slots * 8, e->stream));
+    }
     *out = D;
     return PCAGB_OK;
 }
 
 template <int TPC>
 int launch_materialize(pcagb_engine *e, const Level &P, const uint32_t *fcr_up,
-                       const uint32_t *bitmap, const uint64_t *word_off, Level &C)
+                       const uint32_t *bitmap, const uint64_t *word_off, Level &C, bool cleared)
 {
     LevelOut out{C.regs, C.flags, C.live, C.task, C.parent, C.cidx, C.rdl, C.own, C.probe};
     const int g = e->grid(e->occ_mat);
     if (C.lean) {
-        uint32_t *next = reinterpret_cast<uint32_t *>(e->d_small + 4);
-        CK(cudaMemsetAsync(next, 0, 4, e->stream));
+        uint32_t *next = reinterpret_cast<uint32_t *>(e->d_small + 6);
+        if (!cleared) CK(cudaMemsetAsync(next, 0, 4, e->stream));
         k_materialize_probe<TPC><<<g, kThreads, 0, e->stream>>>(view(P), e->td, bitmap, word_off,
                                                                 out, split_log2(P.n, g), fcr_up,
                                                                 next);
@@ -525,22 +536,30 @@ int build_level(pcagb_engine *e, int d, bool lean = false, bool use_ids = true)
     if (!P.child_off) {
         P.child_off = (uint64_t *)e->alloc_bottom((P.n + 1) * sizeof(uint64_t));
         if (!P.child_off) return fail(PCAGB_ENOMEM);
-        CK(cudaMemsetAsync(P.child_off + P.n, 0, sizeof(uint64_t), e->stream));
-        k_child_counts<<<e->grid(2), 256, 0, e->stream>>>(P.live, P.task, e->td.active, P.n,
-                                                          P.child_off);
-        int rc = check_launch(e);
-        if (rc) return rc;
-        rc = exclusive_scan(e, P.child_off, P.n + 1, nullptr);
-        if (rc) return fail(rc);
+        if (P.n <= kSmallParents) {
+            k_child_offsets<<<1, 1024, 0, e->stream>>>(P.live, P.task, e->td.active, P.n,
+                                                       P.child_off);
+            const int rc = check_launch(e);
+            if (rc) return rc;
+        } else {
+            CK(cudaMemsetAsync(P.child_off + P.n, 0, sizeof(uint64_t), e->stream));
+            k_child_counts<<<e->grid(2), 256, 0, e->stream>>>(P.live, P.task, e->td.active, P.n,
+                                                              P.child_off);
+            int rc = check_launch(e);
+            if (rc) return rc;
+            rc = exclusive_scan(e, P.child_off, P.n + 1, nullptr);
+            if (rc) return fail(rc);
+        }
         uint64_t c = 0;
         for (size_t i = 0; i < P.hist.size(); i++)
             if (e->h_active[i >> 7]) c += P.hist[i] * (uint64_t)gt.nc((int)(i & 127));
         P.children = c;
     }
+    bool new_fcr = false;
     if (!P.fcr && !e->no_oep) {
         P.fcr = (uint32_t *)e->alloc_bottom(P.n * 8 * sizeof(uint32_t));
         if (!P.fcr) return fail(PCAGB_ENOMEM);
-        CK(cudaMemsetAsync(P.fcr, 0xFF, P.n * 8 * sizeof(uint32_t), e->stream));
+        new_fcr = true;
     }
     /* the dead-write rule of the insert kernel needs the first-child ranks
        of the level above (unset at the root) */
@@ -556,23 +575,67 @@ int build_level(pcagb_engine *e, int d, bool lean = false, bool use_ids = true)
     uint32_t *bitmap = (uint32_t *)e->alloc_top(words * 4 + 4);
     if (!bitmap) return fail(PCAGB_ENOMEM);
     uint64_t survivors = children;
+    const bool small_words = words <= kSmallWords;
+    bool cleared = false;
     if (e->no_oep) {
         k_mark_all<<<e->grid(2), 256, 0, e->stream>>>(bitmap, words, children);
         int rc = check_launch(e);
         if (rc) return rc;
     } else {
         if (P.n >= (1ull << 28)) return fail(PCAGB_ENOMEM);
-        /* mark the later flag twins of the parent level (k_twins); their
-           table lives on the scratch side only while the pass runs (stream
-           order keeps the space from being reused before it ends) */
-        CK(cudaMemsetAsync(P.twin, 0, P.n, e->stream));
-        if (P.n >= 2) {
+        uint64_t slots = 1024, tslots = 1024;
+        while (slots < 2 * children) slots <<= 1;
+        while (tslots < 2 * P.n) tslots <<= 1;
+        const bool twins = P.n >= 2;
+        unsigned long long *table = nullptr, *tt = nullptr;
+        IdDev ids{};
+        size_t top_scratch = e->top;
+        /* A small level's scratch (children up to 2^20: a table of 16 MB)
+           is laid out side by side and cleared by one launch; a larger
+           one's tables take turns and are cleared by memsets, whose rate is
+           what counts there. */
+        if (small_words) {
+            const size_t top_all = e->top;
+            table = (unsigned long long *)e->alloc_top(slots * 8);
+            top_scratch = e->top;
+            if (twins) tt = (unsigned long long *)e->alloc_top(tslots * 8);
+            if (table && (tt || !twins)) {
+                ClearList cl{};
+                cl.add(table, slots * 8);
+                if (twins) cl.add(tt, tslots * 8);
+                if (use_ids) {
+                    const int rc = alloc_ids(e, P, &ids, &cl);
+                    if (rc) return rc;
+                }
+                cl.add(bitmap, words * 4 + 4);
+                cl.add(P.twin, P.n);
+                if (new_fcr) cl.add(P.fcr, P.n * 8 * sizeof(uint32_t), ~0u);
+                cl.add(e->d_small + 2, 8);
+                cl.add(e->d_small + 4, 24);
+                cl.add(e->d_hist, (uint64_t)e->ntasks * 128 * sizeof(unsigned long long));
+                k_clear<<<e->grid(4), 256, 0, e->stream>>>(cl);
+                const int rc = check_launch(e);
+                if (rc) return rc;
+                cleared = true;
+            } else {
+                e->top = top_all;
+                table = tt = nullptr;
+            }
+        }
+        if (!cleared) {
+            if (new_fcr) CK(cudaMemsetAsync(P.fcr, 0xFF, P.n * 8 * sizeof(uint32_t), e->stream));
+            CK(cudaMemsetAsync(P.twin, 0, P.n, e->stream));
+        }
+        /* mark the later flag twins of the parent level (k_twins); a large
+           level's table lives on the scratch side only while the pass runs
+           (stream order keeps the space from being reused before it ends) */
+        if (twins) {
             const size_t top_tw = e->top;
-            uint64_t tslots = 1024;
-            while (tslots < 2 * P.n) tslots <<= 1;
-            unsigned long long *tt = (unsigned long long *)e->alloc_top(tslots * 8);
-            if (!tt) return fail(PCAGB_ENOMEM);
-            CK(cudaMemsetAsync(tt, 0, tslots * 8, e->stream));
+            if (!cleared) {
+                tt = (unsigned long long *)e->alloc_top(tslots * 8);
+                if (!tt) return fail(PCAGB_ENOMEM);
+                CK(cudaMemsetAsync(tt, 0, tslots * 8, e->stream));
+            }
             if (e->TPC == 16)
                 k_twins<16><<<e->grid(4), 256, 0, e->stream>>>(view(P), e->td, tt, tslots - 1,
                                                               P.twin, e->d_status);
@@ -581,36 +644,38 @@ int build_level(pcagb_engine *e, int d, bool lean = false, bool use_ids = true)
                                                               P.twin, e->d_status);
             const int rct = check_launch(e);
             if (rct) return rct;
-            e->top = top_tw;
+            if (!cleared) e->top = top_tw;
         }
-        uint64_t slots = 1024;
-        while (slots < 2 * children) slots <<= 1;
-        unsigned long long *table = (unsigned long long *)e->alloc_top(slots * 8);
-        if (!table) return fail(PCAGB_ENOMEM);
-        CK(cudaMemsetAsync(table, 0, slots * 8, e->stream));
-        CK(cudaMemsetAsync(bitmap, 0, words * 4 + 4, e->stream));
-        CK(cudaMemsetAsync(e->d_small + 2, 0, 8, e->stream));
+        int rc = PCAGB_OK;
+        if (!cleared) {
+            table = (unsigned long long *)e->alloc_top(slots * 8);
+            if (!table) return fail(PCAGB_ENOMEM);
+            CK(cudaMemsetAsync(table, 0, slots * 8, e->stream));
+            CK(cudaMemsetAsync(bitmap, 0, words * 4 + 4, e->stream));
+            CK(cudaMemsetAsync(e->d_small + 2, 0, 8, e->stream));
+        }
         cudaEventRecord(e->ev2, e->stream);
         /* the column ids' scratch lives on the top only while the insert
            runs, as the twins' table above */
-        const size_t top_ids = e->top;
-        IdDev ids{};
-        int rc = use_ids ? alloc_ids(e, P, &ids) : PCAGB_OK;
+        if (!cleared) {
+            top_scratch = e->top;
+            rc = use_ids ? alloc_ids(e, P, &ids, nullptr) : PCAGB_OK;
+            if (rc) return rc;
+        }
+        rc = e->TPC == 16 ? launch_expand<16>(e, P, fcr_up, table, slots - 1, ids, cleared)
+                          : launch_expand<32>(e, P, fcr_up, table, slots - 1, ids, cleared);
         if (rc) return rc;
-        rc = e->TPC == 16 ? launch_expand<16>(e, P, fcr_up, table, slots - 1, ids)
-                          : launch_expand<32>(e, P, fcr_up, table, slots - 1, ids);
-        if (rc) return rc;
-        e->top = top_ids;
+        e->top = top_scratch;
         with_ids = ids.tab != nullptr;
         cudaEventRecord(e->ev3, e->stream);
         k_mark<<<e->grid(4), 256, 0, e->stream>>>(table, slots, P.child_off, bitmap,
                                                   e->d_small + 2);
         rc = check_launch(e);
         if (rc) return rc;
-        CK(e_copy(e, &e->h_pin[kPinStatus], e->d_status, 4, cudaMemcpyDeviceToHost, e->stream));
-        CK(e_copy(e, &e->h_pin[kPinSurvivors], e->d_small + 2, 8, cudaMemcpyDeviceToHost,
-                  e->stream));
         if (!one_sync) {
+            CK(e_copy(e, &e->h_pin[kPinStatus], e->d_status, 4, cudaMemcpyDeviceToHost, e->stream));
+            CK(e_copy(e, &e->h_pin[kPinSurvivors], e->d_small + 2, 8, cudaMemcpyDeviceToHost,
+                      e->stream));
             CK(cudaStreamSynchronize(e->stream));
             if (with_ids && (uint32_t)e->h_pin[kPinStatus] == kStatusColumns) return retry();
             if ((uint32_t)e->h_pin[kPinStatus]) {
@@ -625,13 +690,22 @@ int build_level(pcagb_engine *e, int d, bool lean = false, bool use_ids = true)
     }
     uint64_t *word_off = (uint64_t *)e->alloc_top((words + 1) * sizeof(uint64_t));
     if (!word_off) return fail(PCAGB_ENOMEM);
-    CK(cudaMemsetAsync(word_off + words, 0, sizeof(uint64_t), e->stream));
-    k_popc<<<e->grid(2), 256, 0, e->stream>>>(bitmap, words, word_off);
-    int rc = check_launch(e);
-    if (rc) return rc;
-    rc = exclusive_scan(e, word_off, words + 1, nullptr);
-    if (rc) return fail(rc);
-    CK(e_copy(e, &e->h_pin[kPinTotal], word_off + words, 8, cudaMemcpyDeviceToHost, e->stream));
+    int rc;
+    if (small_words) {
+        k_word_offsets<<<1, 1024, 0, e->stream>>>(bitmap, words, word_off, e->d_small + 9);
+        rc = check_launch(e);
+        if (rc) return rc;
+    } else {
+        CK(cudaMemsetAsync(word_off + words, 0, sizeof(uint64_t), e->stream));
+        k_popc<<<e->grid(2), 256, 0, e->stream>>>(bitmap, words, word_off);
+        rc = check_launch(e);
+        if (rc) return rc;
+        rc = exclusive_scan(e, word_off, words + 1, nullptr);
+        if (rc) return fail(rc);
+        CK(e_copy(e, e->d_small + 9, word_off + words, 8, cudaMemcpyDeviceToDevice, e->stream));
+    }
+    if (!one_sync)
+        CK(e_copy(e, &e->h_pin[kPinTotal], e->d_small + 9, 8, cudaMemcpyDeviceToHost, e->stream));
     if (!one_sync) {
         /* the winners' ranks must stay inside the level about to be sized */
         CK(cudaStreamSynchronize(e->stream));
@@ -648,13 +722,20 @@ int build_level(pcagb_engine *e, int d, bool lean = false, bool use_ids = true)
     const uint64_t space = one_sync ? children : survivors;
     if (space >= (1ull << 28)) return fail(PCAGB_ENOMEM);
     if (alloc_level(e, C, space) != PCAGB_OK) return fail(PCAGB_ENOMEM);
-    rc = e->TPC == 16 ? launch_materialize<16>(e, P, fcr_up, bitmap, word_off, C)
-                      : launch_materialize<32>(e, P, fcr_up, bitmap, word_off, C);
+    rc = e->TPC == 16 ? launch_materialize<16>(e, P, fcr_up, bitmap, word_off, C, cleared)
+                      : launch_materialize<32>(e, P, fcr_up, bitmap, word_off, C, cleared);
     if (rc) return rc;
     cudaEventRecord(e->ev1, e->stream);
-    rc = enqueue_hist(e, C, one_sync && !e->no_oep ? e->d_small + 2 : nullptr);
+    rc = enqueue_hist(e, C, one_sync && !e->no_oep ? e->d_small + 2 : nullptr, cleared);
     if (rc) return rc;
+    if (one_sync)
+        CK(e_copy(e, &e->h_pin[kPinBuild], e->d_small + 2, 64, cudaMemcpyDeviceToHost, e->stream));
     CK(cudaStreamSynchronize(e->stream));
+    if (one_sync) {
+        e->h_pin[kPinSurvivors] = e->h_pin[kPinBuild];
+        e->h_pin[kPinStatus] = (uint32_t)e->h_pin[kPinBuild + 6];
+        e->h_pin[kPinTotal] = e->h_pin[kPinBuild + 7];
+    }
     if (one_sync && !e->no_oep) {
         if (with_ids && (uint32_t)e->h_pin[kPinStatus] == kStatusColumns) {
             e->insert_launches--;
@@ -2047,7 +2128,8 @@ int engine_init(pcagb_engine *e, int device, size_t budget)
         PCAGB_PRELOAD(k_leaf<16>); PCAGB_PRELOAD(k_leaf<32>);
         PCAGB_PRELOAD(k_leaf_last<16>); PCAGB_PRELOAD(k_leaf_last<32>);
         PCAGB_PRELOAD(k_count_evals); PCAGB_PRELOAD(k_mark); PCAGB_PRELOAD(k_mark_all);
-        PCAGB_PRELOAD(k_popc); PCAGB_PRELOAD(k_child_counts); PCAGB_PRELOAD(k_task_hist);
+        PCAGB_PRELOAD(k_popc); PCAGB_PRELOAD(k_child_counts); PCAGB_PRELOAD(k_clear);
+        PCAGB_PRELOAD(k_child_offsets); PCAGB_PRELOAD(k_word_offsets); PCAGB_PRELOAD(k_task_hist);
         PCAGB_PRELOAD(k_task_hist_smem); PCAGB_PRELOAD(k_scan_local); PCAGB_PRELOAD(k_scan_add);
         PCAGB_PRELOAD(k_gather_paths); PCAGB_PRELOAD(k_gather_firsts); PCAGB_PRELOAD(k_check_perm);
 #undef PCAGB_PRELOAD
@@ -2097,7 +2179,7 @@ int engine_init(pcagb_engine *e, int device, size_t budget)
     int trc = ensure_device_tables(device);
     if (trc) return trc;
     CK(cudaMalloc(&e->d_small, 256 * sizeof(unsigned long long)));
-    CK(cudaMalloc(&e->d_status, 16));
+    e->d_status = reinterpret_cast<uint32_t *>(e->d_small + 8);
     CK(cudaMalloc(&e->d_sol, e->sol_cap * sizeof(ulonglong2)));
     return ensure_tasks(e, 1);
 }
@@ -2397,7 +2479,6 @@ void pcagb_engine_destroy(pcagb_engine_t *e)
     cudaSetDevice(e->device);
     if (e->stream) cudaStreamSynchronize(e->stream);
     cudaFree(e->d_small);
-    cudaFree(e->d_status);
     cudaFree(e->d_sol);
     cudaFree(e->d_tasks);
     if (e->h_pin) cudaFreeHost(e->h_pin);

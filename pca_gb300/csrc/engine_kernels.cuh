@@ -1082,6 +1082,128 @@ __global__ void k_child_counts(const uint8_t *live, const uint16_t *task, const 
     }
 }
 
+/* ---- the bookkeeping of a small level -----------------------------------------
+   A level of a few hundred states is built in launches of a few microseconds
+   each, so their number is its time: what has to be cleared is cleared by one
+   launch (nine to ten memsets), and counts are formed and scanned by one block
+   (a counting launch, two to four of the scan and a memset). A solve that
+   builds two such levels takes 493 us where it took 574. */
+constexpr int kClearMax = 10;
+struct ClearList {
+    void *p[kClearMax];          /* 16-byte aligned */
+    uint64_t bytes[kClearMax];
+    uint32_t value[kClearMax];   /* 0 or ~0 */
+    int n;
+    void add(void *at, uint64_t count, uint32_t v = 0)
+    {
+        p[n] = at;
+        bytes[n] = count;
+        value[n++] = v;
+    }
+};
+
+__global__ void k_clear(const __grid_constant__ ClearList L)
+{
+    const uint64_t t = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    for (int r = 0; r < L.n; r++) {
+        const uint32_t v = L.value[r];
+        for (uint64_t i = t; i < L.bytes[r] / 16; i += (uint64_t)gridDim.x * blockDim.x)
+            reinterpret_cast<uint4 *>(L.p[r])[i] = make_uint4(v, v, v, v);
+        const uint64_t tail = L.bytes[r] % 16;
+        if (t < tail) reinterpret_cast<uint8_t *>(L.p[r])[L.bytes[r] - tail + t] = (uint8_t)v;
+    }
+}
+
+/* The exclusive offsets of a block's counts, four a thread (1,024 threads),
+   and their sum in every thread. */
+__device__ __forceinline__ uint32_t block_offsets(const uint32_t (&v)[4], uint32_t (&off)[4],
+                                                  uint32_t (&sums)[33])
+{
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    uint32_t s = v[0] + v[1] + v[2] + v[3], inc = s;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        const uint32_t x = __shfl_up_sync(0xFFFFFFFFu, inc, o);
+        if (lane >= o) inc += x;
+    }
+    if (lane == 31) sums[w] = inc;
+    __syncthreads();
+    if (w == 0) {
+        const uint32_t own = sums[lane];
+        uint32_t all = own;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const uint32_t x = __shfl_up_sync(0xFFFFFFFFu, all, o);
+            if (lane >= o) all += x;
+        }
+        sums[lane] = all - own;
+        if (lane == 31) sums[32] = all;
+    }
+    __syncthreads();
+    uint32_t run = sums[w] + inc - s;
+#pragma unroll
+    for (int k = 0; k < 4; k++) {
+        off[k] = run;
+        run += v[k];
+    }
+    const uint32_t total = sums[32];
+    __syncthreads();
+    return total;
+}
+
+/* child_off[0..n] of a level of at most kSmallParents states, one block. */
+constexpr uint64_t kSmallParents = 16384;
+__global__ void __launch_bounds__(1024) k_child_offsets(const uint8_t *live, const uint16_t *task,
+                                                       const uint8_t *active, uint64_t n,
+                                                       uint64_t *child_off)
+{
+    __shared__ uint32_t sums[33];
+    uint64_t carry = 0;
+    for (uint64_t base = 0; base < n; base += 4096) {
+        const uint64_t i = base + threadIdx.x * 4;
+        uint32_t v[4], off[4];
+#pragma unroll
+        for (int k = 0; k < 4; k++) {
+            v[k] = 0;
+            if (i + k < n && active[task[i + k]]) {
+                const uint32_t m = (live[i + k] >> 1) & 127u;
+                v[k] = c_cand_off[m + 1] - c_cand_off[m];
+            }
+        }
+        const uint32_t total = block_offsets(v, off, sums);
+#pragma unroll
+        for (int k = 0; k < 4; k++)
+            if (i + k < n) child_off[i + k] = carry + off[k];
+        carry += total;
+    }
+    if (threadIdx.x == 0) child_off[n] = carry;
+}
+
+/* The ranks of a bitmap of at most kSmallWords words, word_off[0..words],
+   and the number of set bits, one block. */
+constexpr uint64_t kSmallWords = 32768;
+__global__ void __launch_bounds__(1024) k_word_offsets(const uint32_t *bitmap, uint64_t words,
+                                                      uint64_t *word_off, unsigned long long *total)
+{
+    __shared__ uint32_t sums[33];
+    uint64_t carry = 0;
+    for (uint64_t base = 0; base < words; base += 4096) {
+        const uint64_t i = base + threadIdx.x * 4;
+        uint32_t v[4], off[4];
+#pragma unroll
+        for (int k = 0; k < 4; k++) v[k] = i + k < words ? __popc(bitmap[i + k]) : 0;
+        const uint32_t sum = block_offsets(v, off, sums);
+#pragma unroll
+        for (int k = 0; k < 4; k++)
+            if (i + k < words) word_off[i + k] = carry + off[k];
+        carry += sum;
+    }
+    if (threadIdx.x == 0) {
+        word_off[words] = carry;
+        *total = carry;
+    }
+}
+
 /* One warp's shared memory in the materialisation: the parent's register
    block in the level's own layout (8 columns of TPC tests) and the current
    child's new column and flags, from which each lane writes one 16-byte
