@@ -46,19 +46,17 @@ CANDIDATES = ("candidates as the reference's enumerator counts them (tools/enume
 
 # The suffix kernel's capture (profiles/k_suffix_lanes_is_power2_t32_k4.md):
 # warp instructions and DRAM bytes of the depth-4 launch (a lane per prefix
-# with two tests per lane), valid for the kernel source it was taken from
+# on the four tests of its probe), valid for the kernel source it was taken from
 # (SHA-256 of pca_gb300/csrc's engine_kernels.cuh, suffix_forms.cuh and
 # value_forms.h, first 16 hex) and the autotuner's choice.
-SUFFIX_CAPTURE = {"kernel": "k_suffix_lanes<32,2>", "choice": (2, 32), "inst": 132652957,
-                  "ms": 0.238912, "dram_bytes": 376526336 + 290560,
-                  "source_sha16": ("791be789cc8eae2f", "f5a2c7dba0fc9ed0"),
+SUFFIX_CAPTURE = {"kernel": "k_suffix_lanes<32,3>", "choice": (3, 32), "inst": 132050193,
+                  "ms": 0.222848, "dram_bytes": 366526208 + 123904,
+                  "source_sha16": ("dea4ab14bede2660",),
                   "file": "profiles/k_suffix_lanes_is_power2_t32_k4.md"}
 # The insert kernel's capture (profiles/k_expand_insert_is_power2_t32_level3.md):
 # DRAM bytes read + written by the level-3 launch (99.6% of a solve's children).
-# Both hold for the captured source, 791be789..., and for the next, which adds
-# kernels for the bookkeeping of small levels and leaves these two as they were.
-INSERT_CAPTURE = {"dram_bytes": 541437440 + 187046400,
-                  "source_sha16": ("791be789cc8eae2f", "f5a2c7dba0fc9ed0"),
+INSERT_CAPTURE = {"dram_bytes": 546621696 + 189057536,
+                  "source_sha16": ("dea4ab14bede2660",),
                   "file": "profiles/k_expand_insert_is_power2_t32_level3.md"}
 
 
@@ -326,7 +324,7 @@ def suffix_roofline(kernel_ms: float, stage_ms: float, peak_issue: float, evals_
     fresh = kernel_source_sha16() in SUFFIX_CAPTURE["source_sha16"]
     ft, shape = tuned_depth1_choice(tuning)
     same = (ft, shape) == SUFFIX_CAPTURE["choice"]
-    out = {"kernel": SUFFIX_CAPTURE["kernel"] + " (last instruction over operand pairs)",
+    out = {"kernel": SUFFIX_CAPTURE["kernel"] + " (last instruction by value forms)",
            "bound": "int_issue", "unit": "Gwarp-inst/s", "peak": peak_issue / 1e9,
            "evaluations_run_per_s": evals_run_per_s, "ncu": SUFFIX_CAPTURE["file"],
            "kernel_ms_live": kernel_ms, "suffix_stages_ms_per_step": stage_ms}

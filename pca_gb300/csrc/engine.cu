@@ -67,11 +67,8 @@ constexpr int kMaxBatch = 8192;
 /* engine_init's budget for an engine whose arena each solve supplies */
 constexpr size_t kArenaExternal = ~size_t(0);
 /* slots of the pinned host buffer */
-/* [kPinBuild ..]: d_small[2 ..] after a build: survivors, status at 6, the
-   bitmap's set bits at 7 */
-constexpr int kPinBuild = 16;
-constexpr int kPinStatus = 0, kPinSurvivors = 1, kPinTotal = 2, kPinCount = 3,
-              kPinHist = 64;
+/* (kPinStatus, kPinTotal: d_small[8], [9] after a build) */
+constexpr int kPinStatus = 0, kPinTotal = 1, kPinCount = 3, kPinHist = 64;
 /* A level whose children's states fit in this many bytes, or in an eighth
    of the arena's free space, is written into space for all of them, so its
    build needs one host round trip instead of three. */
@@ -158,7 +155,7 @@ struct pcagb_engine {
     cudaStream_t stream = nullptr;
     char *arena = nullptr;
     size_t cap = 0, bottom = 0, top = 0;
-    unsigned long long *d_small = nullptr;   /* [0] sol count [1] unused [2] count
+    unsigned long long *d_small = nullptr;   /* [0] sol count [1], [2] unused
                                                 [3] value-class evaluations run
                                                 [4] the insert kernel's work counter
                                                 [5] column ids given out
@@ -417,7 +414,8 @@ uint32_t split_log2(uint64_t parents, int grid)
 
 template <int TPC>
 int launch_expand(pcagb_engine *e, const Level &P, const uint32_t *fcr_up,
-                  unsigned long long *table, uint64_t tmask, const IdDev &ids, bool cleared)
+                  unsigned long long *table, uint64_t tmask, const IdDev &ids, uint32_t *bitmap,
+                  bool cleared)
 {
     const int g = e->grid(e->occ_insert);
     /* the work-item counter the kernel's warps draw from */
@@ -428,10 +426,12 @@ int launch_expand(pcagb_engine *e, const Level &P, const uint32_t *fcr_up,
         const int rc = check_launch(e);
         if (rc) return rc;
         k_expand_insert<TPC, true><<<g, kThreads, 0, e->stream>>>(
-            view(P), e->td, table, tmask, e->d_status, split_log2(P.n, g), fcr_up, next, ids);
+            view(P), e->td, table, tmask, e->d_status, split_log2(P.n, g), fcr_up, next, ids,
+            bitmap);
     } else {
         k_expand_insert<TPC, false><<<g, kThreads, 0, e->stream>>>(
-            view(P), e->td, table, tmask, e->d_status, split_log2(P.n, g), fcr_up, next, ids);
+            view(P), e->td, table, tmask, e->d_status, split_log2(P.n, g), fcr_up, next, ids,
+            bitmap);
     }
     return check_launch(e);
 }
@@ -507,7 +507,7 @@ int launch_materialize(pcagb_engine *e, const Level &P, const uint32_t *fcr_up,
  * same sum the device scan forms), so nothing waits before the insert. A
  * level whose children's states fit in kOneSyncBytes or an eighth of the
  * free arena is materialised into space for every child and its survivor
- * count, status, scan total and histogram come back in one round trip; a
+ * count (the bitmap's set bits), status and histogram come back in one round trip; a
  * larger level reads the survivor count first and allocates exactly. */
 int build_level(pcagb_engine *e, int d, bool lean = false, bool use_ids = true)
 {
@@ -610,7 +610,6 @@ int build_level(pcagb_engine *e, int d, bool lean = false, bool use_ids = true)
                 cl.add(bitmap, words * 4 + 4);
                 cl.add(P.twin, P.n);
                 if (new_fcr) cl.add(P.fcr, P.n * 8 * sizeof(uint32_t), ~0u);
-                cl.add(e->d_small + 2, 8);
                 cl.add(e->d_small + 4, 24);
                 cl.add(e->d_hist, (uint64_t)e->ntasks * 128 * sizeof(unsigned long long));
                 k_clear<<<e->grid(4), 256, 0, e->stream>>>(cl);
@@ -652,7 +651,6 @@ int build_level(pcagb_engine *e, int d, bool lean = false, bool use_ids = true)
             if (!table) return fail(PCAGB_ENOMEM);
             CK(cudaMemsetAsync(table, 0, slots * 8, e->stream));
             CK(cudaMemsetAsync(bitmap, 0, words * 4 + 4, e->stream));
-            CK(cudaMemsetAsync(e->d_small + 2, 0, 8, e->stream));
         }
         cudaEventRecord(e->ev2, e->stream);
         /* the column ids' scratch lives on the top only while the insert
@@ -662,29 +660,12 @@ int build_level(pcagb_engine *e, int d, bool lean = false, bool use_ids = true)
             rc = use_ids ? alloc_ids(e, P, &ids, nullptr) : PCAGB_OK;
             if (rc) return rc;
         }
-        rc = e->TPC == 16 ? launch_expand<16>(e, P, fcr_up, table, slots - 1, ids, cleared)
-                          : launch_expand<32>(e, P, fcr_up, table, slots - 1, ids, cleared);
+        rc = e->TPC == 16 ? launch_expand<16>(e, P, fcr_up, table, slots - 1, ids, bitmap, cleared)
+                          : launch_expand<32>(e, P, fcr_up, table, slots - 1, ids, bitmap, cleared);
         if (rc) return rc;
         e->top = top_scratch;
         with_ids = ids.tab != nullptr;
         cudaEventRecord(e->ev3, e->stream);
-        k_mark<<<e->grid(4), 256, 0, e->stream>>>(table, slots, P.child_off, bitmap,
-                                                  e->d_small + 2);
-        rc = check_launch(e);
-        if (rc) return rc;
-        if (!one_sync) {
-            CK(e_copy(e, &e->h_pin[kPinStatus], e->d_status, 4, cudaMemcpyDeviceToHost, e->stream));
-            CK(e_copy(e, &e->h_pin[kPinSurvivors], e->d_small + 2, 8, cudaMemcpyDeviceToHost,
-                      e->stream));
-            CK(cudaStreamSynchronize(e->stream));
-            if (with_ids && (uint32_t)e->h_pin[kPinStatus] == kStatusColumns) return retry();
-            if ((uint32_t)e->h_pin[kPinStatus]) {
-                set_err("expansion of level %d hit a device limit (status %u)", d + 1,
-                        (uint32_t)e->h_pin[kPinStatus]);
-                return PCAGB_ELIMIT;
-            }
-            survivors = e->h_pin[kPinSurvivors];
-        }
         e->insert_launches++;
         e->insert_children += children;
     }
@@ -704,16 +685,22 @@ int build_level(pcagb_engine *e, int d, bool lean = false, bool use_ids = true)
         if (rc) return fail(rc);
         CK(e_copy(e, e->d_small + 9, word_off + words, 8, cudaMemcpyDeviceToDevice, e->stream));
     }
-    if (!one_sync)
-        CK(e_copy(e, &e->h_pin[kPinTotal], e->d_small + 9, 8, cudaMemcpyDeviceToHost, e->stream));
     if (!one_sync) {
-        /* the winners' ranks must stay inside the level about to be sized */
+        CK(e_copy(e, &e->h_pin[kPinStatus], e->d_small + 8, 16, cudaMemcpyDeviceToHost, e->stream));
         CK(cudaStreamSynchronize(e->stream));
-        if (e->h_pin[kPinTotal] != survivors) {
-            set_err("internal: bitmap holds %llu winners, table %llu",
-                    (unsigned long long)e->h_pin[kPinTotal], (unsigned long long)survivors);
-            return PCAGB_ELIMIT;
+        if (!e->no_oep) {
+            if (with_ids && (uint32_t)e->h_pin[kPinStatus] == kStatusColumns) {
+                e->insert_launches--;
+                e->insert_children -= children;
+                return retry();
+            }
+            if ((uint32_t)e->h_pin[kPinStatus]) {
+                set_err("expansion of level %d hit a device limit (status %u)", d + 1,
+                        (uint32_t)e->h_pin[kPinStatus]);
+                return PCAGB_ELIMIT;
+            }
         }
+        survivors = e->h_pin[kPinTotal];
     }
     Level C;
     C.lean = lean;
@@ -726,16 +713,11 @@ int build_level(pcagb_engine *e, int d, bool lean = false, bool use_ids = true)
                       : launch_materialize<32>(e, P, fcr_up, bitmap, word_off, C, cleared);
     if (rc) return rc;
     cudaEventRecord(e->ev1, e->stream);
-    rc = enqueue_hist(e, C, one_sync && !e->no_oep ? e->d_small + 2 : nullptr, cleared);
+    rc = enqueue_hist(e, C, one_sync && !e->no_oep ? e->d_small + 9 : nullptr, cleared);
     if (rc) return rc;
     if (one_sync)
-        CK(e_copy(e, &e->h_pin[kPinBuild], e->d_small + 2, 64, cudaMemcpyDeviceToHost, e->stream));
+        CK(e_copy(e, &e->h_pin[kPinStatus], e->d_small + 8, 16, cudaMemcpyDeviceToHost, e->stream));
     CK(cudaStreamSynchronize(e->stream));
-    if (one_sync) {
-        e->h_pin[kPinSurvivors] = e->h_pin[kPinBuild];
-        e->h_pin[kPinStatus] = (uint32_t)e->h_pin[kPinBuild + 6];
-        e->h_pin[kPinTotal] = e->h_pin[kPinBuild + 7];
-    }
     if (one_sync && !e->no_oep) {
         if (with_ids && (uint32_t)e->h_pin[kPinStatus] == kStatusColumns) {
             e->insert_launches--;
@@ -747,12 +729,7 @@ int build_level(pcagb_engine *e, int d, bool lean = false, bool use_ids = true)
                     (uint32_t)e->h_pin[kPinStatus]);
             return fail(PCAGB_ELIMIT);
         }
-        survivors = e->h_pin[kPinSurvivors];
-        if (e->h_pin[kPinTotal] != survivors) {
-            set_err("internal: bitmap holds %llu winners, table %llu",
-                    (unsigned long long)e->h_pin[kPinTotal], (unsigned long long)survivors);
-            return fail(PCAGB_ELIMIT);
-        }
+        survivors = e->h_pin[kPinTotal];
         C.n = survivors;
     }
     take_hist(e, C);
@@ -2127,7 +2104,7 @@ int engine_init(pcagb_engine *e, int device, size_t budget)
         PCAGB_PRELOAD(k_twins<16>); PCAGB_PRELOAD(k_twins<32>);
         PCAGB_PRELOAD(k_leaf<16>); PCAGB_PRELOAD(k_leaf<32>);
         PCAGB_PRELOAD(k_leaf_last<16>); PCAGB_PRELOAD(k_leaf_last<32>);
-        PCAGB_PRELOAD(k_count_evals); PCAGB_PRELOAD(k_mark); PCAGB_PRELOAD(k_mark_all);
+        PCAGB_PRELOAD(k_count_evals); PCAGB_PRELOAD(k_mark_all);
         PCAGB_PRELOAD(k_popc); PCAGB_PRELOAD(k_child_counts); PCAGB_PRELOAD(k_clear);
         PCAGB_PRELOAD(k_child_offsets); PCAGB_PRELOAD(k_word_offsets); PCAGB_PRELOAD(k_task_hist);
         PCAGB_PRELOAD(k_task_hist_smem); PCAGB_PRELOAD(k_scan_local); PCAGB_PRELOAD(k_scan_add);

@@ -726,11 +726,23 @@ __device__ bool warp_child_equal(const LevelDev &P, const InsertState<TPC> &A, i
    children, 7.9M of them looked up, 5.3M kept): hashing each child's column
    and comparing columns by the warp took 943M warp instructions, 1.40 ms;
    hashing by class 695M, 1.16 ms; with ids 311M, 0.61 ms (0.75 with the
-   ids of the level's registers and the clearing of their table). */
+   ids of the level's registers and the clearing of their table).
+
+   The child bitmap is kept beside the table: a child that takes a slot
+   toggles its bit, and one that takes it from a later sibling the other's
+   too, so that in whatever order the toggles land each slot's last holder has
+   its bit set and nobody else (a scan of the 256 MB table for its holders
+   took 0.09 ms of the level and a launch, the toggles 0.06). */
+__device__ __forceinline__ void toggle_child(uint32_t *bitmap, uint64_t child)
+{
+    atomicXor(&bitmap[child >> 5], 1u << (child & 31));
+}
+
 template <int TPC, bool IDS>
 __global__ void __launch_bounds__(kThreads, 4)
 k_expand_insert(LevelDev P, TaskDev task, unsigned long long *table, uint64_t tmask,
-                uint32_t *status, uint32_t split_log2, const uint32_t *fcr_up, uint32_t *next, IdDev D)
+                uint32_t *status, uint32_t split_log2, const uint32_t *fcr_up, uint32_t *next, IdDev D,
+                uint32_t *bitmap)
 {
     __shared__ InsertState<TPC> sws[kWarpsPerBlock];
     const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
@@ -766,6 +778,7 @@ k_expand_insert(LevelDev P, TaskDev task, unsigned long long *table, uint64_t tm
         }
         if (IDS && lane < 8) ws.ids[lane] = D.ids[q * 8 + lane];
         const uint32_t live = P.live[q];
+        const uint64_t first_child = P.child_off[q];
         __syncwarp();
         if (lane >= 1 && lane < 8) ws.colh[lane] = col_final(lane, hash_column<TPC>(ws.R[lane]));
         if (lane >= 8 && lane < 12) {   /* the parent's flags, a plane a lane */
@@ -848,6 +861,7 @@ k_expand_insert(LevelDev P, TaskDev task, unsigned long long *table, uint64_t tm
                     if (s == 0) {
                         const unsigned long long old = atomicCAS(&table[idx], 0ull, mine);
                         if (old == 0) {
+                            toggle_child(bitmap, first_child + c);
                             done = true;
                         } else {
                             s = old;
@@ -914,7 +928,11 @@ k_expand_insert(LevelDev P, TaskDev task, unsigned long long *table, uint64_t tm
                         uint64_t oref = (s & kRefMask) - 1;
                         while (ref < oref) {
                             const unsigned long long old = atomicCAS(&table[idx], s, mine);
-                            if (old == s) break;
+                            if (old == s) {
+                                toggle_child(bitmap, first_child + c);
+                                toggle_child(bitmap, P.child_off[oref >> 12] + (oref & 4095));
+                                break;
+                            }
                             s = old;
                             oref = (s & kRefMask) - 1;
                         }
@@ -1019,36 +1037,6 @@ __global__ void k_twins(LevelDev P, TaskDev task, unsigned long long *table, uin
             }
         }
     }
-}
-
-/* Mark each table winner in the child bitmap; count them. A thread reads
-   four slots (two 16-byte loads, both issued before either is used) per
-   step: the table is larger than L2 and its scan is the kernel's traffic.
-   slots is a power of two >= 1024 and the table 16-byte aligned. */
-__device__ __forceinline__ uint32_t mark_slot(unsigned long long s, const uint64_t *child_off,
-                                              uint32_t *bitmap)
-{
-    if (!s) return 0;
-    const uint64_t ref = (s & kRefMask) - 1;
-    const uint64_t L = child_off[ref >> 12] + (ref & 4095);
-    atomicOr(&bitmap[L >> 5], 1u << (L & 31));
-    return 1;
-}
-
-__global__ void k_mark(const unsigned long long *table, uint64_t slots, const uint64_t *child_off,
-                       uint32_t *bitmap, unsigned long long *count)
-{
-    const ulonglong2 *t2 = reinterpret_cast<const ulonglong2 *>(table);
-    const uint64_t quads = slots / 4;
-    const uint64_t stride = (uint64_t)gridDim.x * blockDim.x;
-    uint32_t local = 0;
-    for (uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; i < quads; i += stride) {
-        const ulonglong2 a = t2[2 * i], b = t2[2 * i + 1];
-        local += mark_slot(a.x, child_off, bitmap) + mark_slot(a.y, child_off, bitmap) +
-                 mark_slot(b.x, child_off, bitmap) + mark_slot(b.y, child_off, bitmap);
-    }
-    for (int o = 16; o; o >>= 1) local += __shfl_down_sync(0xFFFFFFFFu, local, o);
-    if ((threadIdx.x & 31) == 0 && local) atomicAdd(count, (unsigned long long)local);
 }
 
 /* Keep every child (no pruning): set all bits below `total`. */
@@ -1448,12 +1436,22 @@ __global__ void k_task_hist_smem(const uint8_t *live, const uint16_t *task, uint
     __syncthreads();
     const uint64_t stride = (uint64_t)gridDim.x * blockDim.x;
     const uint64_t n_round = (n + 31) & ~31ull;
-    for (uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n_round; i += stride) {
-        const bool valid = i < n;
-        const uint32_t key = valid ? (uint32_t)task[i] * 128u + ((live[i] >> 1) & 127u) : ~0u;
-        const uint32_t peers = __match_any_sync(0xFFFFFFFFu, key);
-        if (valid && (threadIdx.x & 31) == __ffs(peers) - 1 && key < nbins)
-            atomicAdd(&sh_hist[key], (uint32_t)__popc(peers));
+    /* four states a thread in flight: one at a time, 5.3M states took 46 us,
+       waiting for their bytes; 22 so */
+    for (uint64_t i0 = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; i0 < n_round;
+         i0 += 4 * stride) {
+        uint32_t key[4];
+#pragma unroll
+        for (int k = 0; k < 4; k++) {
+            const uint64_t i = i0 + k * stride;
+            key[k] = i < n ? (uint32_t)task[i] * 128u + ((live[i] >> 1) & 127u) : ~0u;
+        }
+#pragma unroll
+        for (int k = 0; k < 4; k++) {
+            const uint32_t peers = __match_any_sync(0xFFFFFFFFu, key[k]);
+            if ((threadIdx.x & 31) == __ffs(peers) - 1 && key[k] < nbins)
+                atomicAdd(&sh_hist[key[k]], (uint32_t)__popc(peers));
+        }
     }
     __syncthreads();
     for (uint32_t b = threadIdx.x; b < nbins; b += blockDim.x)
