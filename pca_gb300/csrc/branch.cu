@@ -594,19 +594,31 @@ __device__ bool bchild_same(const BDev &P, const BWarp<TP> &A, uint32_t wa, int 
 
    Bound: integer issue. Hashing every register of every test of every child
    from global memory took 6.9 ms for relu's depth-3 last level (11 tests,
-   22.5M children, 8.2M kept); this 4.1 ms (5.9 without never_kept). */
+   22.5M children, 8.2M kept); 4.1 ms this way (5.9 without never_kept) with
+   fixed shares of the parents, 3.6 with parents drawn from a counter: their
+   costs differ widely. A child that takes a slot toggles its bit, and one that
+   takes it from a later sibling the other's too, so the holders' bits are set
+   in whatever order the toggles land (a scan of the table for them: 0.29). */
+__device__ __forceinline__ void btoggle(uint32_t *bitmap, uint64_t child)
+{
+    atomicXor(&bitmap[child >> 5], 1u << (child & 31));
+}
+
 template <int TP>
 __global__ void __launch_bounds__(kBThreads)
 k_bexpand(BDev P, BTab tab, int T, uint32_t p, unsigned long long *table, uint64_t tmask,
-          uint32_t *bitmap, uint32_t *status, uint32_t split_log2)
+          uint32_t *bitmap, uint32_t *status, uint32_t *next, uint32_t split_log2)
 {
     __shared__ BWarp<TP> sw[kWarps];
     const int lane = threadIdx.x & 31;
     BWarp<TP> &W = sw[threadIdx.x >> 5];
-    const uint64_t nw = (uint64_t)gridDim.x * kWarps;
     const uint32_t split = 1u << split_log2;
-    for (uint64_t it = ((uint64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-         it < P.n << split_log2; it += nw) {
+    const uint64_t items = P.n << split_log2;   /* far below 2^32: a state takes 200 bytes */
+    uint32_t nx = 0;
+    if (lane == 0) nx = atomicAdd(next, 1u);
+    for (uint64_t it = __shfl_sync(0xFFFFFFFFu, nx, 0); it < items;
+         it = __shfl_sync(0xFFFFFFFFu, nx, 0)) {
+        if (lane == 0) nx = atomicAdd(next, 1u);
         const uint64_t q = it >> split_log2;
         const uint32_t m = (P.live[q] >> 1) & 127u;
         const uint32_t nc = bcount(tab, m);
@@ -682,8 +694,12 @@ k_bexpand(BDev P, BTab tab, int T, uint32_t p, unsigned long long *table, uint64
                     s = *((volatile unsigned long long *)&table[idx]);
                     if (s == 0) {
                         const unsigned long long old = atomicCAS(&table[idx], 0ull, mine);
-                        if (old == 0) done = true;
-                        else s = old;
+                        if (old == 0) {
+                            btoggle(bitmap, off + c);
+                            done = true;
+                        } else {
+                            s = old;
+                        }
                     }
                     if (!done) needcmp = (s >> 40) == (mine >> 40);
                 }
@@ -709,7 +725,11 @@ k_bexpand(BDev P, BTab tab, int T, uint32_t p, unsigned long long *table, uint64
                         uint64_t oref = (s & kBRefMask) - 1;
                         while (ref < oref) {
                             const unsigned long long old = atomicCAS(&table[idx], s, mine);
-                            if (old == s) break;
+                            if (old == s) {
+                                btoggle(bitmap, off + c);
+                                btoggle(bitmap, P.child_off[oref >> 12] + (oref & 4095));
+                                break;
+                            }
                             s = old;
                             oref = (s & kBRefMask) - 1;
                         }
@@ -724,19 +744,6 @@ k_bexpand(BDev P, BTab tab, int T, uint32_t p, unsigned long long *table, uint64
                 }
             }
         }
-    }
-}
-
-__global__ void k_bmark(const unsigned long long *table, uint64_t slots, const uint64_t *child_off,
-                        uint32_t *bitmap)
-{
-    for (uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; i < slots;
-         i += (uint64_t)gridDim.x * blockDim.x) {
-        const unsigned long long s = table[i];
-        if (!s) continue;
-        const uint64_t ref = (s & kBRefMask) - 1;
-        const uint64_t L = child_off[ref >> 12] + (ref & 4095);
-        atomicOr(&bitmap[L >> 5], 1u << (L & 31));
     }
 }
 
@@ -1252,17 +1259,16 @@ int build_blevel(BranchRun &b, BLevel &P, const BLevel *up, uint32_t p, int mf, 
     if (!bitmap || !table || !rank || !P.fcr) { set_berr("device memory exhausted expanding a level"); return PCAGB_ENOMEM; }
     BCK(cudaMemsetAsync(bitmap, 0, (words + 1) * 4, b.st));
     BCK(cudaMemsetAsync(table, 0, slots * 8, b.st));
-    BCK(cudaMemsetAsync(b.d_status, 0, 4, b.st));
+    BCK(cudaMemsetAsync(b.d_status, 0, 8, b.st));
     BCK(cudaMemsetAsync(P.fcr, 0xFF, P.n * 8 * sizeof(uint32_t), b.st));
     if (b.TP == 16)
         k_bexpand<16><<<b.grid(6), kBThreads, 0, b.st>>>(bdev(P, up), tab, b.T, p, table, slots - 1,
-                                                        bitmap, b.d_status, slices(P.n, b.grid(6)));
+                                                        bitmap, b.d_status, b.d_status + 1,
+                                                        slices(P.n, b.grid(6)));
     else
         k_bexpand<32><<<b.grid(6), kBThreads, 0, b.st>>>(bdev(P, up), tab, b.T, p, table, slots - 1,
-                                                        bitmap, b.d_status, slices(P.n, b.grid(6)));
-    rc = blaunch(b);
-    if (rc) return rc;
-    k_bmark<<<b.grid(4), 256, 0, b.st>>>(table, slots, P.child_off, bitmap);
+                                                        bitmap, b.d_status, b.d_status + 1,
+                                                        slices(P.n, b.grid(6)));
     rc = blaunch(b);
     if (rc) return rc;
     BCK(cudaMemsetAsync(rank + words, 0, 8, b.st));
@@ -1600,7 +1606,7 @@ int solve_branch(pcagb_engine_t *e, const task_spec_t *task, int max_depth,
     b.T = task->num_tests;
     b.TP = b.T <= 16 ? 16 : 32;
     b.d_target = b.alloc<uint32_t>(32);
-    b.d_status = b.alloc<uint32_t>(1);
+    b.d_status = b.alloc<uint32_t>(2);   /* status, work counter */
     if (!b.d_target || !b.d_status) {
         set_berr("device memory exhausted");
         return PCAGB_ENOMEM;
