@@ -932,7 +932,12 @@ struct BSol {
    child whose registers hold the target is recorded, solving or not: a
    child with the same state as a solving one holds the same registers, so
    the records contain the depth-first first child of every solving state
-   (the one the pruner keeps) without a pass over all children. */
+   (the one the pruner keeps) without a pass over all children.
+
+   Bound: integer issue, the ops of a run of candidates diverging. A lane reads
+   the operands and the written register of a test from shared memory; reading
+   all eight registers and picking among them took is_power2's last position
+   (11 tests, 8.2M parents) 73 ms, this 59. */
 template <int TP>
 __global__ void __launch_bounds__(kBThreads)
 k_bsuffix(BDev P, BTab tab, int T, uint32_t p, const uint32_t *target, BSol *out,
@@ -973,22 +978,20 @@ k_bsuffix(BDev P, BTab tab, int T, uint32_t p, const uint32_t *target, BSol *out
             const uint32_t c = c0 + lane;
             if (c >= nc) continue;
             const uint32_t insn = bcand(tab, m, c);
-            if (never_kept(insn, buop(insn), dead)) continue;
-            const uint32_t op = insn >> 11, rdi = (insn >> 8) & 7u;
-            const uint32_t wr = (op != (uint32_t)kOpCmp && op != (uint32_t)kOpBr && rdi != 0) ? rdi : 0u;
+            const BUop u = buop(insn);
+            if (never_kept(insn, u, dead)) continue;
+            const uint32_t wr = u.wr;
             /* a register the child leaves as the parent's can hold the
                target only where the parent's column does */
             const bool kept = (pm & ~(1u << wr) & 0xFEu) != 0;
             if (!kept && !wr) continue;
             bool match = wr != 0, fault = pfault;
             for (int t = 0; t < T; t++) {
-                uint32_t R[8];
-#pragma unroll
-                for (int r = 0; r < 8; r++) R[r] = sR[r][t];
-                uint32_t v = 0, f, sk;
-                const uint32_t rd = bexec(insn, p, R, sF[t], sS[t], &v, &f, &sk);
+                uint32_t f, sk;
+                const uint32_t v = bvalue(u, p, sR[u.ra][t], sR[u.rb][t], sR[wr][t], sF[t], sS[t],
+                                          &f, &sk);
                 if (sk == kFault) fault = true;
-                if (wr) match &= (rd == wr ? v : R[wr]) == target[t];
+                if (wr) match &= v == target[t];
                 /* nothing left to record once the written register missed
                    and no other register holds the target */
                 if (!match && !kept) break;
