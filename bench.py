@@ -51,12 +51,12 @@ CANDIDATES = ("candidates as the reference's enumerator counts them (tools/enume
 # value_forms.h, first 16 hex) and the autotuner's choice.
 SUFFIX_CAPTURE = {"kernel": "k_suffix_lanes<32,3>", "choice": (3, 32), "inst": 132050193,
                   "ms": 0.222848, "dram_bytes": 366526208 + 123904,
-                  "source_sha16": ("dea4ab14bede2660",),
+                  "source_sha16": ("2a7afde722770fe4",),
                   "file": "profiles/k_suffix_lanes_is_power2_t32_k4.md"}
 # The insert kernel's capture (profiles/k_expand_insert_is_power2_t32_level3.md):
 # DRAM bytes read + written by the level-3 launch (99.6% of a solve's children).
 INSERT_CAPTURE = {"dram_bytes": 546621696 + 189057536,
-                  "source_sha16": ("dea4ab14bede2660",),
+                  "source_sha16": ("2a7afde722770fe4",),
                   "file": "profiles/k_expand_insert_is_power2_t32_level3.md"}
 
 

@@ -937,7 +937,7 @@ struct BSol {
    Bound: integer issue, the ops of a run of candidates diverging. A lane reads
    the operands and the written register of a test from shared memory; reading
    all eight registers and picking among them took is_power2's last position
-   (11 tests, 8.2M parents) 73 ms, this 59. */
+   (11 tests) 73 ms, this 59. */
 template <int TP>
 __global__ void __launch_bounds__(kBThreads)
 k_bsuffix(BDev P, BTab tab, int T, uint32_t p, const uint32_t *target, BSol *out,

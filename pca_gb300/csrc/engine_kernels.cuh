@@ -8,15 +8,17 @@
  * program. TP is 16 or 32 (test count rounded up), and test slots >= T are
  * zero in every state.
  *
- * Level expansion (the OEP kernel): one warp per parent, one lane per child
- * candidate. Each lane computes the child's new column and flags across all
- * tests, a 64-bit hash of the whole child state (incrementally from the
- * parent's per-column hashes), and inserts a 64-bit slot
+ * Level expansion (the OEP kernel): one warp per parent. It forms each value
+ * class of the parent's candidates once, a lane a class: the new column (two
+ * tests to a word), its hash, its flags as bit planes and the column's exact
+ * id; then a lane takes a child (class, destination), whose 64-bit hash comes
+ * from the parent's per-column hashes, and inserts a 64-bit slot
  *   [tag: hash bits 40..63][ref + 1: 40 bits]
  * into an open-addressed HBM table, ref = parent_rank << 12 | candidate.
- * On a tag match the two child states are rebuilt and compared in full
- * (every register of every test, flags, and live when it is part of the
- * key), so a hash collision can never merge two different states. Among
+ * On a tag match the two child states are compared exactly, by the ids of
+ * their columns or, on levels too small or too large for ids, column by
+ * column (every register of every test, flags, and live when it is part of
+ * the key), so a hash collision can never merge two different states. Among
  * equal states the smallest ref wins (atomicCAS loop), which is the first
  * child in the reference's DFS order -- the representative the reference's
  * DFS pruner keeps (tools/enumerate.c:379-384). Children that can never be
@@ -25,18 +27,20 @@
  * dead-able unread write (deadable_writes) and LDI swaps (ldi_swap); each
  * has an equal state with a smaller ref, so the winners do not change.
  *
- * The winners are then marked in a bitmap indexed by the child's linear
- * index (child_off[parent] + candidate), ranked by a scan, and written out
- * in that order, so every level stays in DFS order.
+ * The insert keeps a bitmap of the winners beside the table, indexed by the
+ * child's linear index (child_off[parent] + candidate); its bits are ranked
+ * by a scan and the winners written out in that order, so every level stays
+ * in DFS order.
  *
- * Suffix kernels: one warp per prefix state. The last instruction's value
- * does not depend on its destination (except ADDI), so only value classes
- * are evaluated, and only those that read the last write (the read rule in
- * scan_last): one lane per operand pair, every op of the pair evaluated on
- * the first two tests at once, each survivor checked on all tests by the
- * warp (lane t taking test t, __all_sync deciding). Suffix depths 2 and 3
- * enumerate the middle instructions in the warp, keeping the new columns in
- * spare shared-memory columns 8 and 9.
+ * Suffix kernels. The last instruction's value does not depend on its
+ * destination (except ADDI), so only value classes are evaluated, and only
+ * those that read the last write (the read rule in scan_last). Large levels
+ * take a lane per prefix or per state, by value forms (suffix_forms.cuh);
+ * here are the warp-per-prefix kernels of roots, small levels and forced
+ * shapes: one lane per operand pair, every op of the pair evaluated on the
+ * first two tests at once, each survivor checked on all tests by the warp
+ * (lane t taking test t, __all_sync deciding), the middle instructions of
+ * suffix depths 2 and 3 in spare shared-memory columns 8 and 9.
  */
 #pragma once
 
