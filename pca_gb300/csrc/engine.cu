@@ -1574,8 +1574,8 @@ struct OrderSpec {
     uint64_t chunk = 0;
 };
 
-int run_batch(pcagb_engine *e, std::vector<TaskRun> &runs, const pcagb_opts_t &o,
-              done_fn on_done = nullptr, void *user = nullptr, const OrderSpec *ord = nullptr)
+int search_batch(pcagb_engine *e, std::vector<TaskRun> &runs, const pcagb_opts_t &o,
+                 done_fn on_done, void *user, const OrderSpec *ord)
 {
     const GenTables &gt = gen_tables();
     auto t_start = std::chrono::steady_clock::now();
@@ -1622,38 +1622,8 @@ int run_batch(pcagb_engine *e, std::vector<TaskRun> &runs, const pcagb_opts_t &o
     e->lean_K = !o.count_levels && !ord && !warp_forced && !o.full_levels ? maxK : -1;
     e->td = TaskDev{e->d_task_T, e->d_task_target, e->d_task_active,
                     o.oep_mode == PCAGB_OEP_EXACT_LIVE, o.oep_mode != PCAGB_OEP_NONE};
-    /* level 0: one root per task. The roots go over in one copy; the test
-       order is chosen and level 0 laid out on the device (k_setup) */
     Level L0;
     if (alloc_level(e, L0, nt) != PCAGB_OK) { set_err("arena too small"); return PCAGB_ENOMEM; }
-    L0.hist.assign((size_t)nt * 128, 0);
-    for (int i = 0; i < nt; i++) {
-        const TaskRun &tr = runs[i];
-        RootIn &r = e->h_roots[i];
-        memset(&r, 0, sizeof r);
-        memcpy(r.regs, tr.root.regs, (size_t)tr.T * sizeof r.regs[0]);
-        memcpy(r.flags, tr.root.flags, tr.T);
-        memcpy(r.target, tr.target, (size_t)tr.T * 2);
-        r.live = tr.root.live;
-        r.T = (uint8_t)tr.T;
-        L0.hist[(size_t)i * 128 + ((tr.root.live >> 1) & 127)] = 1;
-    }
-    CK(e_copy(e, e->d_roots, e->h_roots, (size_t)nt * sizeof(RootIn), cudaMemcpyHostToDevice,
-              e->stream));
-    {
-        const LevelOut out{L0.regs, L0.flags, L0.live, L0.task, L0.parent, L0.cidx, L0.rdl, L0.own,
-                           L0.probe};
-        const SetupOut so{e->d_task_T, e->d_task_target, e->d_task_io, e->d_order, e->d_status,
-                          e->d_small + 3};
-        const uint32_t rounds = maxK >= 5 ? 8 : 1;
-        if (e->TPC == 16)
-            k_setup<16><<<nt, kSetupWarps * 32, 0, e->stream>>>(e->d_roots, rounds, out, L0.twin, so);
-        else
-            k_setup<32><<<nt, kSetupWarps * 32, 0, e->stream>>>(e->d_roots, rounds, out, L0.twin, so);
-        const int rc = check_launch(e);
-        if (rc) return rc;
-    }
-    e->levels.push_back(std::move(L0));
 
     /* K = 0: does a live register already hold the target? */
     for (TaskRun &tr : runs) {
@@ -1676,6 +1646,40 @@ int run_batch(pcagb_engine *e, std::vector<TaskRun> &runs, const pcagb_opts_t &o
             tr.t_done = elapsed();
         }
     }
+    /* level 0: one root per task, laid out when a task is to be searched (or
+       the caller reads the levels). The roots go over in one copy; the test
+       order is chosen and the level laid out on the device (k_setup) */
+    bool search = o.count_levels != 0;
+    for (const TaskRun &tr : runs) search |= !tr.done && tr.max_depth >= 1;
+    L0.hist.assign((size_t)nt * 128, 0);
+    if (search) {
+        for (int i = 0; i < nt; i++) {
+            const TaskRun &tr = runs[i];
+            RootIn &r = e->h_roots[i];
+            memset(&r, 0, sizeof r);
+            memcpy(r.regs, tr.root.regs, (size_t)tr.T * sizeof r.regs[0]);
+            memcpy(r.flags, tr.root.flags, tr.T);
+            memcpy(r.target, tr.target, (size_t)tr.T * 2);
+            r.live = tr.root.live;
+            r.T = (uint8_t)tr.T;
+            L0.hist[(size_t)i * 128 + ((tr.root.live >> 1) & 127)] = 1;
+        }
+        CK(e_copy(e, e->d_roots, e->h_roots, (size_t)nt * sizeof(RootIn), cudaMemcpyHostToDevice,
+                  e->stream));
+        const LevelOut out{L0.regs, L0.flags, L0.live, L0.task, L0.parent, L0.cidx, L0.rdl, L0.own,
+                           L0.probe};
+        const SetupOut so{e->d_task_T, e->d_task_target, e->d_task_io, e->d_order, e->d_status,
+                          e->d_small + 3};
+        const uint32_t rounds = maxK >= 5 ? 8 : 1;
+        if (e->TPC == 16)
+            k_setup<16><<<nt, kSetupWarps * 32, 0, e->stream>>>(e->d_roots, rounds, out, L0.twin, so);
+        else
+            k_setup<32><<<nt, kSetupWarps * 32, 0, e->stream>>>(e->d_roots, rounds, out, L0.twin, so);
+        const int rc = check_launch(e);
+        if (rc) return rc;
+    }
+    e->levels.push_back(std::move(L0));
+
     std::vector<uint8_t> notified(nt, 0);
     auto notify = [&](int i) {
         if (notified[i]) return;
@@ -1875,6 +1879,20 @@ int run_batch(pcagb_engine *e, std::vector<TaskRun> &runs, const pcagb_opts_t &o
     }
     for (int i = 0; i < nt; i++) notify(i);
     if (e->measure) store_costs(e);
+    return PCAGB_OK;
+}
+
+/* search_batch, and the end of its work on the device: however it returns, no
+   kernel or copy of it is left on the stream. The arena may belong to a server,
+   which hands it to another stream's solve next, and the pinned buffers are
+   the next solve's. (A solve that ran its stages has waited already.) */
+int run_batch(pcagb_engine *e, std::vector<TaskRun> &runs, const pcagb_opts_t &o,
+              done_fn on_done = nullptr, void *user = nullptr, const OrderSpec *ord = nullptr)
+{
+    const int rc = search_batch(e, runs, o, on_done, user, ord);
+    const cudaError_t end = cudaStreamSynchronize(e->stream);
+    if (rc) return rc;
+    CK(end);
     return PCAGB_OK;
 }
 
