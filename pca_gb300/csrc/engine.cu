@@ -1047,16 +1047,23 @@ void launch_suffix_lanes(int ft, int g, cudaStream_t st, const LevelDev &L, cons
     else k_suffix_lanes<TPC, 2><<<g, kThreads, 0, st>>>(L, td, sb, R, lean);
 }
 
-/* A long stage of a solve that shares the GPU (a server's) runs in a few
-   CTAs: a launch holds its SMs until it ends, and requests admitted meanwhile
-   would wait for them. Four CTAs leave 148 SMs to the others and take about
-   as long as the stage took before it was a lane per state (is_power2 at
-   depth 5: 0.4 s, 5 ms on the whole GPU), which is also what the serving test
-   builds on: it submits requests 0.2 s into such a solve and expects their
-   answers before its own. The stages of requests up to depth 4 (0.2 ms)
-   are below the line. */
-constexpr double kBackgroundMs = 2.0;
-constexpr int kBackgroundCtas = 4;
+/* The lane-per-state stages of a solve that shares the GPU (a server's). A
+   launch holds its SMs until it ends and other streams' kernels get in between
+   launches, so a stage or a batch's group predicted to take longer than
+   kSharedRangeMs runs as ranges of prefixes of that length on the whole GPU.
+   One task's long stage steps back at first: until kStepBackMs have passed its
+   ranges run in a few CTAs, which leave the other SMs to the requests admitted
+   meanwhile. It is a bound on the wait that is bought, not a share of the
+   stage: a two-input task's depth 5 takes 0.08 s alone and 0.47 s so (5.8 s
+   where all of it ran in four CTAs, 9.2 s before the lanes were states), and
+   no batch is slowed (40 open two-input tasks to depth 4: 5 ms either way; 194
+   in four CTAs, whose line was drawn by the sum of the tasks). The price falls
+   on stages of a few ms: is_power2 to depth 5, 7 ms alone, takes 0.39 s (0.43
+   before). It is not smaller because tests/test_gpu_serve.py submits requests
+   0.2 s after that solve and expects their answers before its own. */
+constexpr double kSharedRangeMs = 2.0;
+constexpr double kStepBackMs = 400.0, kStepBackRangeMs = 0.25;
+constexpr int kStepBackCtas = 4;
 
 /* A lane per state (k_suffix_states): per_prefix states to a prefix, and the
    shares their work is cut into so that the warps fill the GPU about twice
@@ -1064,9 +1071,9 @@ constexpr int kBackgroundCtas = 4;
    that a share only repeats the state's set-up. */
 template <int TPC, int SD>
 void launch_states(pcagb_engine *e, const LevelDev &L, const SolBuf &sb, uint32_t per_prefix,
-                   const PrefixRange &R, bool background)
+                   const PrefixRange &R, bool step_back)
 {
-    const int g = background ? kBackgroundCtas : e->grid(e->occ_states);
+    const int g = step_back ? kStepBackCtas : e->grid(e->occ_states);
     const uint64_t batches = (R.count * per_prefix + 31) / 32;
     const uint64_t warps = (uint64_t)g * kStatesWarps;
     uint32_t sl = 0;
@@ -1193,9 +1200,7 @@ int run_stage(pcagb_engine *e, int S, int K, std::vector<TaskRun> &runs, bool fi
             s == 1                ? 1u
             : chunk == kLaneShape ? (s == 2 ? 1u : std::max(1u, (uint32_t)ncmax))
                                   : std::max(1u, (uint32_t)((ncmax + chunk - 1) / chunk));
-        const bool background =
-            !e->measure && (double)evals_pred * e->t_eval_ms[s] > kBackgroundMs;
-        auto launch = [&](const PrefixRange &R) {
+        auto launch = [&](const PrefixRange &R, bool step_back = false) {
             const LevelDev V = view(L);
             if (s == 1) {
                 const bool lanes = chunk == 32;
@@ -1226,11 +1231,11 @@ int run_stage(pcagb_engine *e, int S, int K, std::vector<TaskRun> &runs, bool fi
                 }
             } else if (chunk == kLaneShape) {
                 if (t16) {
-                    if (s == 2) launch_states<16, 2>(e, V, sb, cpp, R, background);
-                    else launch_states<16, 3>(e, V, sb, cpp, R, background);
+                    if (s == 2) launch_states<16, 2>(e, V, sb, cpp, R, step_back);
+                    else launch_states<16, 3>(e, V, sb, cpp, R, step_back);
                 } else {
-                    if (s == 2) launch_states<32, 2>(e, V, sb, cpp, R, background);
-                    else launch_states<32, 3>(e, V, sb, cpp, R, background);
+                    if (s == 2) launch_states<32, 2>(e, V, sb, cpp, R, step_back);
+                    else launch_states<32, 3>(e, V, sb, cpp, R, step_back);
                 }
             } else if (s == 2) {
                 if (t16) launch_suffix<16, 2>(ft, g, e->stream, V, e->td, sb, cpp, chunk, R);
@@ -1241,11 +1246,35 @@ int run_stage(pcagb_engine *e, int S, int K, std::vector<TaskRun> &runs, bool fi
             }
             return check_launch(e);
         };
+        /* range R of the stage (or of a batch's group) that is predicted to
+           take ms on the whole GPU, R itself r_ms: in one launch or, of a
+           solve that shares the GPU, in ranges */
+        const auto stage_t0 = std::chrono::steady_clock::now();
+        auto launch_range = [&](const PrefixRange &R, double ms, double r_ms, int tasks) {
+            if (e->measure || chunk != kLaneShape || ms <= kSharedRangeMs || !R.count)
+                return launch(R);
+            for (uint64_t at = 0; at < R.count;) {
+                const bool back =
+                    tasks == 1 && std::chrono::duration<double, std::milli>(
+                                      std::chrono::steady_clock::now() - stage_t0).count() <
+                                      kStepBackMs;
+                const double share = (back ? kStepBackRangeMs : kSharedRangeMs) / r_ms;
+                const uint64_t n =
+                    std::min(R.count - at, std::max<uint64_t>(1, (uint64_t)(share * R.count)));
+                const int rc0 = launch(PrefixRange{R.order, R.begin + at, n}, back);
+                if (rc0) return rc0;
+                /* stepping back ends by the clock, so it is kept in step */
+                if (back) CK(cudaStreamSynchronize(e->stream));
+                at += n;
+            }
+            return (int)PCAGB_OK;
+        };
+        const double stage_ms = (double)evals_pred * e->t_eval_ms[s];
         tuned_ft = s == 1 ? ft : 0;   /* the deeper stages have no choices to time */
         tuned_ck = ck;
         /* task groups of the progressive mode: [first task, end task) with
-           the level range they occupy */
-        struct Group { int t0, t1; uint64_t b0, b1; };
+           the level range they occupy, their evaluations and active tasks */
+        struct Group { int t0, t1; uint64_t b0, b1; double evals; int active; };
         std::vector<Group> groups;
         if (!so && on_tasks && e->ntasks > 1) {
             const int nt = e->ntasks;
@@ -1254,7 +1283,7 @@ int run_stage(pcagb_engine *e, int S, int K, std::vector<TaskRun> &runs, bool fi
             for (int t = 0; t < nt; t++) nact += e->h_active[t] ? 1 : 0;
             if (nact > 1) {
                 uint64_t off = 0, gb0 = 0;
-                int gt0 = 0;
+                int gt0 = 0, ga = 0;
                 double acc = 0;
                 for (int t = 0; t < nt; t++) {
                     uint64_t cnt = 0, ev = 0;
@@ -1263,12 +1292,16 @@ int run_stage(pcagb_engine *e, int S, int K, std::vector<TaskRun> &runs, bool fi
                         ev += L.hist[(size_t)t * 128 + m] * gt.ev[s][m];
                     }
                     off += cnt;
-                    if (e->h_active[t]) acc += (double)ev;
+                    if (e->h_active[t]) {
+                        acc += (double)ev;
+                        ga++;
+                    }
                     if (acc >= per_group || t == nt - 1) {
-                        groups.push_back({gt0, t + 1, gb0, off});
+                        groups.push_back({gt0, t + 1, gb0, off, acc, ga});
                         gt0 = t + 1;
                         gb0 = off;
                         acc = 0;
+                        ga = 0;
                     }
                 }
                 if (off != L.n) groups.clear();   /* histogram and level disagree: one launch */
@@ -1278,7 +1311,8 @@ int run_stage(pcagb_engine *e, int S, int K, std::vector<TaskRun> &runs, bool fi
             grouped = true;
             for (const Group &G : groups) {
                 if (G.b1 > G.b0) {
-                    rc = launch(PrefixRange{nullptr, G.b0, G.b1 - G.b0});
+                    const double ms = G.evals * e->t_eval_ms[s];
+                    rc = launch_range(PrefixRange{nullptr, G.b0, G.b1 - G.b0}, ms, ms, G.active);
                     if (rc) return rc;
                 }
                 if (firsts) {
@@ -1305,7 +1339,8 @@ int run_stage(pcagb_engine *e, int S, int K, std::vector<TaskRun> &runs, bool fi
             uint64_t step = so && so->chunk ? so->chunk : std::max<uint64_t>(L.n, 1);
             for (uint64_t b0 = 0; b0 < L.n; b0 += step, step = so && so->chunk ? step * 2 : step) {
                 const PrefixRange R{so ? so->order : nullptr, b0, std::min(step, L.n - b0)};
-                rc = launch(R);
+                rc = launch_range(R, stage_ms, stage_ms * (double)R.count / (double)L.n,
+                                  nact_stage);
                 if (rc) return rc;
                 if (so && so->stop_at_first) {
                     const auto h0 = std::chrono::steady_clock::now();
