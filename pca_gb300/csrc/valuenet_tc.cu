@@ -61,6 +61,7 @@
 #include <mutex>
 
 #include "../../include/pca_gb300.h"
+#include "per_device.h"
 
 namespace {
 
@@ -1403,6 +1404,22 @@ bool tile_map(CUtensorMap *m, const void *ptr, int rows, int cols, int ld, int b
               CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
 
+/* Allow a kernel `bytes` of dynamic shared memory on the current device. */
+template <class Kernel>
+bool allow_smem(pcagb::OncePerDevice &once, Kernel *kernel, int bytes)
+{
+    int dev = 0;
+    return cudaGetDevice(&dev) == cudaSuccess && once.run(dev, [&] {
+        const bool ok = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                             bytes) == cudaSuccess;
+        if (!ok) cudaGetLastError();   /* reported here, not by the next launch */
+        return ok;
+    });
+}
+
+constexpr int kGSmemMost = kGStages * (kGABytes + 256 * 128) + 256 + 2048;
+pcagb::OncePerDevice g_gemm_smem, g_gemm_sums_smem;
+
 }  // namespace
 
 /* C[M,N] = A[M,K] . B[N,K]^T on tcgen05 (k_gemm_tc): bias[N] added, then
@@ -1437,12 +1454,6 @@ extern "C" int pcagb_vnet_gemm_tc(const void *A, int lda, const void *B, int ldb
     /* stage buffers, then 256 bytes of barriers and flags, the tile's bias
        (bn floats), 1 KB of alignment slack */
     const int smem = kGStages * (kGABytes + bn * 128) + 256 + 1024 + 1024;
-    static std::once_flag attr_once;
-    static cudaError_t attr_err = cudaSuccess;
-    std::call_once(attr_once, [] {
-        attr_err = cudaFuncSetAttribute(k_gemm_tc<false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                        kGStages * (kGABytes + 256 * 128) + 256 + 2048);
-    });
     /* the epilogue: staged through shared memory and stored in 16-byte
        pieces where the output's alignment allows */
     int stage_mode = 0;
@@ -1453,7 +1464,7 @@ extern "C" int pcagb_vnet_gemm_tc(const void *A, int lda, const void *B, int ldb
              !((uintptr_t)Cf & 15))
         stage_mode = 2;
     const int vec_atomic = splits > 1 && ldc % 4 == 0 && !((uintptr_t)Cf & 15);
-    if (attr_err != cudaSuccess) return PCAGB_ECUDA;
+    if (!allow_smem(g_gemm_smem, k_gemm_tc<false>, kGSmemMost)) return PCAGB_ECUDA;
     dim3 grid((N + bn - 1) / bn, (M + kGRows - 1) / kGRows, splits);
     k_gemm_tc<false><<<grid, kGThreads, smem, (cudaStream_t)stream>>>(
         ma, mb, bias, (const __nv_bfloat16 *)mask, ldm, (__nv_bfloat16 *)Cb, Cf, ldc, M, N,
@@ -1543,15 +1554,9 @@ static int wgrad(const void *dY, int ldy, const void *X, int ldx, float *C, int 
     const uint32_t idesc = (1u << 4) | (1u << 7) | (1u << 10) | (1u << 15) | (1u << 16) |
                            ((uint32_t)(bn >> 3) << 17) | ((uint32_t)(kGRows >> 4) << 24);
     const int smem = kGStages * (kGABytes + bn * 128) + 256 + 1024 + 1024;
-    static std::once_flag attr_once;
-    static cudaError_t attr_err = cudaSuccess;
-    std::call_once(attr_once, [] {
-        for (auto *k : {&k_gemm_tc<false>, &k_gemm_tc<true>})
-            if (attr_err == cudaSuccess)
-                attr_err = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                                kGStages * (kGABytes + 256 * 128) + 256 + 2048);
-    });
-    if (attr_err != cudaSuccess) return PCAGB_ECUDA;
+    if (!(part_db ? allow_smem(g_gemm_sums_smem, k_gemm_tc<true>, kGSmemMost)
+                  : allow_smem(g_gemm_smem, k_gemm_tc<false>, kGSmemMost)))
+        return PCAGB_ECUDA;
     float *out = part ? part : C;
     const int vec_atomic = ldc % 4 == 0 && !((uintptr_t)out & 15);
     dim3 grid((N + bn - 1) / bn, (M + kGRows - 1) / kGRows, splits);
@@ -1605,13 +1610,8 @@ extern "C" int pcagb_vnet_encode_pool_tc(const void *W1, const float *b1, const 
     if (cudaGetDevice(&dev) != cudaSuccess ||
         cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess)
         return PCAGB_ECUDA;
-    static std::once_flag attr_once;
-    static cudaError_t attr_err = cudaSuccess;
-    std::call_once(attr_once, [] {
-        attr_err = cudaFuncSetAttribute(k_encode_pool_tc, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                        kSmemBytes);
-    });
-    if (attr_err != cudaSuccess) return PCAGB_ECUDA;
+    static pcagb::OncePerDevice smem;
+    if (!allow_smem(smem, k_encode_pool_tc, kSmemBytes)) return PCAGB_ECUDA;
     const int ntiles = (n + kStatesPerTile - 1) / kStatesPerTile;
     const int pairs = ntiles < sms / 2 ? ntiles : sms / 2;
     k_encode_pool_tc<<<2 * pairs, kThreads, kSmemBytes, (cudaStream_t)stream>>>(
@@ -1641,13 +1641,8 @@ extern "C" int pcagb_vnet_trunk_tc(const void *P, int n, const void *T1, const f
     if (cudaGetDevice(&dev) != cudaSuccess ||
         cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess)
         return PCAGB_ECUDA;
-    static std::once_flag attr_once;
-    static cudaError_t attr_err = cudaSuccess;
-    std::call_once(attr_once, [] {
-        attr_err = cudaFuncSetAttribute(k_trunk_tc, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                        kTSmem);
-    });
-    if (attr_err != cudaSuccess) return PCAGB_ECUDA;
+    static pcagb::OncePerDevice smem;
+    if (!allow_smem(smem, k_trunk_tc, kTSmem)) return PCAGB_ECUDA;
     const int ntiles = (n + kRows - 1) / kRows;
     k_trunk_tc<<<ntiles < sms ? ntiles : sms, kTThreads, kTSmem, (cudaStream_t)stream>>>(
         mp, m1, m2, m3, b1, b2, b3, n, logits, status);
