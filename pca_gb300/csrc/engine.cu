@@ -215,6 +215,7 @@ struct pcagb_engine {
     int force_ft = 0, force_chunk = 0;   /* per solve: pcagb_opts_t overrides */
     bool measure = true;                 /* per solve: the GPU is its own (not
                                             shared_gpu), so its times are costs */
+    uint64_t id_limit = ~0ull;           /* most column ids of a level build (tests lower it) */
     int lean_K = -1;                     /* per solve: the last depth, whose stage
                                             reads its split level lean (-1: none) */
 
@@ -458,7 +459,8 @@ int alloc_ids(pcagb_engine *e, const Level &P, IdDev *out, ClearList *clear)
     /* distinct columns: at most the registers and classes together, measured
        a tenth of that; warps drop parts of their batches */
     const uint64_t warps = (uint64_t)e->grid(e->occ_insert) * kWarpsPerBlock;
-    const uint64_t cap = std::min<uint64_t>((classes + 7 * P.n) / 4 + warps * kIdBatch, 1u << 30);
+    const uint64_t cap = std::min<uint64_t>((classes + 7 * P.n) / 4 + warps * kIdBatch,
+                                            std::min<uint64_t>(1u << 30, e->id_limit));
     uint64_t slots = 1024;
     while (slots < 2 * cap) slots <<= 1;
     const uint64_t bytes = slots * 8 + cap * e->TPC * 2 + P.n * 32 + P.n * D.stride * 20;
@@ -515,7 +517,9 @@ int build_level(pcagb_engine *e, int d, bool lean = false, bool use_ids = true)
     Level &P = e->levels[d];
     const size_t bottom0 = e->bottom, top0 = e->top;
     bool with_ids = false;
-    /* the ids ran out: once more without them */
+    /* the ids ran out (whatever else the build met by then: it compared
+       children by ids that they do not have): once more without them */
+    auto no_ids = [&] { return with_ids && ((uint32_t)e->h_pin[kPinStatus] & kStatusColumns); };
     auto retry = [&]() -> int {
         e->bottom = bottom0;
         e->top = top0;
@@ -689,7 +693,7 @@ int build_level(pcagb_engine *e, int d, bool lean = false, bool use_ids = true)
         CK(e_copy(e, &e->h_pin[kPinStatus], e->d_small + 8, 16, cudaMemcpyDeviceToHost, e->stream));
         CK(cudaStreamSynchronize(e->stream));
         if (!e->no_oep) {
-            if (with_ids && (uint32_t)e->h_pin[kPinStatus] == kStatusColumns) {
+            if (no_ids()) {
                 e->insert_launches--;
                 e->insert_children -= children;
                 return retry();
@@ -719,7 +723,7 @@ int build_level(pcagb_engine *e, int d, bool lean = false, bool use_ids = true)
         CK(e_copy(e, &e->h_pin[kPinStatus], e->d_small + 8, 16, cudaMemcpyDeviceToHost, e->stream));
     CK(cudaStreamSynchronize(e->stream));
     if (one_sync && !e->no_oep) {
-        if (with_ids && (uint32_t)e->h_pin[kPinStatus] == kStatusColumns) {
+        if (no_ids()) {
             e->insert_launches--;
             e->insert_children -= children;
             return retry();
@@ -2463,6 +2467,8 @@ thread_local uint64_t t_last_explored = 0;
 /* For the branch-mode solver (branch.cu), which runs on the engine's stream
    and device but keeps its own levels. */
 cudaStream_t pcagb_internal_stream(pcagb_engine_t *e) { return e->stream; }
+/* For the tests of the rebuild without column ids. */
+extern "C" void pcagb_internal_limit_ids(pcagb_engine_t *e, uint64_t most) { e->id_limit = most; }
 int pcagb_internal_device(pcagb_engine_t *e) { return e->device; }
 void pcagb_internal_arena(pcagb_engine_t *e, char **base, size_t *bytes)
 {
