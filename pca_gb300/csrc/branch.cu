@@ -24,8 +24,9 @@
  * searched (BR offsets reach at most to the end of the kernel), so every
  * depth of the iterative deepening builds its levels afresh.
  *
- * Levels live in stream-ordered device allocations on the engine's stream;
- * every launch goes to that stream.
+ * Levels live in the engine's arena while no solve uses it, and in
+ * stream-ordered device allocations where it is in use or too small; every
+ * launch goes to the engine's stream.
  */
 #include <cuda_runtime.h>
 #include <stdint.h>
@@ -43,6 +44,12 @@
 #include "../../include/pca_gb300.h"
 #include "pca_isa.h"
 #include "scan.cuh"
+
+/* Internal accessors of engine.cu. */
+cudaStream_t pcagb_internal_stream(pcagb_engine_t *e);
+int pcagb_internal_device(pcagb_engine_t *e);
+bool pcagb_internal_arena_take(pcagb_engine_t *e, char **base, size_t *bytes);
+void pcagb_internal_arena_give(pcagb_engine_t *e);
 
 namespace {
 
@@ -1106,8 +1113,10 @@ struct BranchRun {
     uint32_t *d_pre_off = nullptr, *d_post_off = nullptr;
     uint16_t *d_pre = nullptr, *d_post = nullptr;
     uint32_t *d_status = nullptr;
-    /* the engine's arena, idle during a branch-mode solve, from its bottom;
-       what does not fit in it comes from the device's pool */
+    /* the engine's arena, from its bottom, where no solve is using it (a
+       solve's callback may call branch mode); what does not fit in it comes
+       from the device's pool */
+    pcagb_engine_t *arena_of = nullptr;
     char *arena = nullptr;
     size_t arena_cap = 0, arena_used = 0;
     struct Alloc {
@@ -1122,6 +1131,7 @@ struct BranchRun {
     {
         release(0);
         cudaStreamSynchronize(st);
+        if (arena_of) pcagb_internal_arena_give(arena_of);
     }
     /* free the allocations made after the first `keep` */
     void release(size_t keep)
@@ -1216,8 +1226,6 @@ uint32_t slices(uint64_t parents, int grid)
     return l;
 }
 
-/* Expand level P (position p of a depth-K pass) into C. Fills the number of
-   generated children. */
 /* Children of every state of P at a position with mf forward offsets:
    P.child_off (exclusive scan) and P.children. */
 int count_bchildren(BranchRun &b, BLevel &P, int mf)
@@ -1245,7 +1253,8 @@ int count_bchildren(BranchRun &b, BLevel &P, int mf)
     return PCAGB_OK;
 }
 
-/* `up`: the level above P (null at the root). */
+/* Expand level P (position p of a depth-K pass) into C; up: the level above P
+   (null at the root). */
 int build_blevel(BranchRun &b, BLevel &P, const BLevel *up, uint32_t p, int mf, BLevel &C)
 {
     const BTab tab = b.tab(mf);
@@ -1546,11 +1555,6 @@ int64_t branch_suffix(BranchRun &b, const BranchTables &bt, std::vector<BLevel> 
 
 }  // namespace
 
-/* Internal accessors of engine.cu. */
-cudaStream_t pcagb_internal_stream(pcagb_engine_t *e);
-int pcagb_internal_device(pcagb_engine_t *e);
-void pcagb_internal_arena(pcagb_engine_t *e, char **base, size_t *bytes);
-
 extern "C" {
 
 const char *pcagb_branch_last_error(void) { return g_berr.c_str(); }
@@ -1595,7 +1599,7 @@ int solve_branch(pcagb_engine_t *e, const task_spec_t *task, int max_depth,
     b.st = pcagb_internal_stream(e);
     BCK(cudaSetDevice(pcagb_internal_device(e)));
     BCK(cudaDeviceGetAttribute(&b.sms, cudaDevAttrMultiProcessorCount, pcagb_internal_device(e)));
-    pcagb_internal_arena(e, &b.arena, &b.arena_cap);
+    if (pcagb_internal_arena_take(e, &b.arena, &b.arena_cap)) b.arena_of = e;
     {
         const DevTables *dt = nullptr;
         const int rc = device_tables(pcagb_internal_device(e), &dt);

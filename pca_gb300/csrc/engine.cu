@@ -26,6 +26,7 @@
 
 #include <algorithm>
 #include <chrono>
+#include <condition_variable>
 #include <cstdarg>
 #include <cstdio>
 #include <cstring>
@@ -244,9 +245,34 @@ struct pcagb_engine {
         return arena + top;
     }
     int grid(int per_sm = 4) const { return sms * per_sm; }
+
+    /* who uses the arena: solves (one, or a solve inside its own callbacks),
+       or a branch-mode search, which takes it when nobody does */
+    std::mutex arena_mu;
+    std::condition_variable arena_cv;
+    int arena_solves = 0;
+    bool arena_branch = false;
 };
 
 namespace {
+
+/* A solve's use of its engine's arena; waits for a branch-mode search of
+   another thread that holds it. */
+struct ArenaUse {
+    pcagb_engine *e;
+    explicit ArenaUse(pcagb_engine *eng) : e(eng)
+    {
+        std::unique_lock<std::mutex> lk(e->arena_mu);
+        e->arena_cv.wait(lk, [&] { return !e->arena_branch; });
+        e->arena_solves++;
+    }
+    ~ArenaUse()
+    {
+        std::lock_guard<std::mutex> lk(e->arena_mu);
+        e->arena_solves--;
+    }
+    ArenaUse(const ArenaUse &) = delete;
+};
 
 /* Unit costs the engines of one device have measured (the autotuner's
    model), shared so that a new engine, e.g. a server's slot, starts from
@@ -1928,6 +1954,7 @@ int search_batch(pcagb_engine *e, std::vector<TaskRun> &runs, const pcagb_opts_t
 int run_batch(pcagb_engine *e, std::vector<TaskRun> &runs, const pcagb_opts_t &o,
               done_fn on_done = nullptr, void *user = nullptr, const OrderSpec *ord = nullptr)
 {
+    const ArenaUse use(e);
     const int rc = search_batch(e, runs, o, on_done, user, ord);
     const cudaError_t end = cudaStreamSynchronize(e->stream);
     if (rc) return rc;
@@ -2470,10 +2497,25 @@ cudaStream_t pcagb_internal_stream(pcagb_engine_t *e) { return e->stream; }
 /* For the tests of the rebuild without column ids. */
 extern "C" void pcagb_internal_limit_ids(pcagb_engine_t *e, uint64_t most) { e->id_limit = most; }
 int pcagb_internal_device(pcagb_engine_t *e) { return e->device; }
-void pcagb_internal_arena(pcagb_engine_t *e, char **base, size_t *bytes)
+/* The arena for a branch-mode search, if no solve (whose callback may have
+   called it) and no other search uses it; to be given back once its work on
+   the stream has ended. */
+bool pcagb_internal_arena_take(pcagb_engine_t *e, char **base, size_t *bytes)
 {
+    std::lock_guard<std::mutex> lk(e->arena_mu);
+    if (!e->arena || e->arena_solves || e->arena_branch) return false;
+    e->arena_branch = true;
     *base = e->arena;
-    *bytes = e->arena ? e->cap : 0;
+    *bytes = e->cap;
+    return true;
+}
+void pcagb_internal_arena_give(pcagb_engine_t *e)
+{
+    {
+        std::lock_guard<std::mutex> lk(e->arena_mu);
+        e->arena_branch = false;
+    }
+    e->arena_cv.notify_all();
 }
 
 extern "C" {
@@ -2724,6 +2766,7 @@ int pcagb_record(pcagb_engine_t *e, const task_spec_t *task, int max_depth, uint
     o.count_levels = 1;
     std::vector<TaskRun> runs(1);
     if (!make_run(task, o, &runs[0])) return PCAGB_EINVAL;
+    const ArenaUse use(e);   /* to the end: the records are read from the levels */
     int rc = run_batch(e, runs, o);
     if (rc) return rc;
     const int cap = 100;  /* the reference's MAX_SOLUTIONS */
