@@ -165,24 +165,24 @@ struct pcagb_engine {
                                                 bits */
     uint32_t *d_status = nullptr;            /* in d_small */
     ulonglong2 *d_sol = nullptr;
-    ulonglong2 *d_firsts = nullptr;          /* [cap_tasks] SolBuf::firsts */
-    FirstOut *d_first_out = nullptr;         /* [cap_tasks] */
+    ulonglong2 *d_firsts = nullptr;          /* [kMaxBatch] SolBuf::firsts */
+    FirstOut *d_first_out = nullptr;         /* [kMaxBatch] */
     uint64_t sol_cap = 1u << 20;
     /* batch task table */
     int32_t *d_task_T = nullptr;
     uint32_t *d_task_target = nullptr;
     uint8_t *d_task_active = nullptr;
-    uint16_t *d_task_io = nullptr;           /* [cap_tasks][3][32] in0, in1, target */
-    uint8_t *d_order = nullptr;              /* [cap_tasks][32] the caller's test at each place */
-    RootIn *d_roots = nullptr;               /* [cap_tasks] */
-    int cap_tasks = 0;                       /* tasks the per-task arrays hold (ensure_tasks) */
-    char *d_tasks = nullptr;                 /* the allocation behind the device ones */
-    unsigned long long *d_hist = nullptr;    /* [cap_tasks][128] */
+    uint16_t *d_task_io = nullptr;           /* [kMaxBatch][3][32] in0, in1, target */
+    uint8_t *d_order = nullptr;              /* [kMaxBatch][32] the caller's test at each place */
+    RootIn *d_roots = nullptr;               /* [kMaxBatch] */
+    char *d_tasks = nullptr;                 /* the allocation behind the per-task arrays */
+    unsigned long long *d_hist = nullptr;    /* [kMaxBatch][128] */
     /* pinned host mirror of the small results (kPin* slots) and of d_hist:
        device-to-host reads of these never wait on their own */
     unsigned long long *h_pin = nullptr;
-    /* pinned too: first-only results, roots and active flags on their way to
-       the device */
+    /* pinned too: first-only results, roots (in the histogram's place: they
+       are on the device before the first one comes back) and active flags on
+       their way to the device */
     FirstOut *h_first_out = nullptr;
     RootIn *h_roots = nullptr;
     uint8_t *h_up_active = nullptr;
@@ -1630,8 +1630,6 @@ int validate_order(pcagb_engine *e, const uint32_t *order, uint64_t n)
     return PCAGB_OK;
 }
 
-int ensure_tasks(pcagb_engine *e, int nt);
-
 /* Core batched IDDFS shared by every solve entry point. */
 struct OrderSpec {
     pcagb_order_cb cb = nullptr;
@@ -1676,7 +1674,6 @@ int search_batch(pcagb_engine *e, std::vector<TaskRun> &runs, const pcagb_opts_t
         tr.res.optimal_depth = -1;
     }
     CK(cudaSetDevice(e->device));
-    if (int prc = ensure_tasks(e, nt)) return prc;
     e->TPC = maxT <= 16 ? 16 : 32;
     e->no_oep = o.oep_mode == PCAGB_OEP_NONE;
     /* the last depth's split level may be built lean when nothing but its
@@ -2102,22 +2099,13 @@ int ensure_device_tables(int device)
     return PCAGB_OK;
 }
 
-/* The per-task arrays, on the device and pinned on the host, for a batch of
-   nt tasks: 256 at first, grown by the first larger batch (8,192, the most,
-   take 25 MB of both, whose allocation would take longer than the rest of an
-   engine's creation). */
-int ensure_tasks(pcagb_engine *e, int nt)
+/* The per-task arrays, on the device and pinned on the host, for the largest
+   batch: no solve allocates. (Growing them with the first large batch made an
+   engine 0.35 ms sooner; that batch then freed and allocated, which waits for
+   every engine of the device.) */
+int alloc_tasks(pcagb_engine *e)
 {
-    if (nt <= e->cap_tasks) return PCAGB_OK;
-    int cap = std::max(e->cap_tasks, 256);
-    while (cap < nt) cap *= 2;
-    const size_t n = (size_t)cap;
-    CK(cudaStreamSynchronize(e->stream));
-    e->cap_tasks = 0;
-    CK(cudaFree(e->d_tasks));
-    if (e->h_pin) CK(cudaFreeHost(e->h_pin));
-    e->d_tasks = nullptr;
-    e->h_pin = nullptr;
+    const size_t n = kMaxBatch;
     struct { void **p; size_t bytes; } dev[] = {
         {(void **)&e->d_firsts, n * sizeof(ulonglong2)},
         {(void **)&e->d_first_out, n * sizeof(FirstOut)},
@@ -2136,14 +2124,14 @@ int ensure_tasks(pcagb_engine *e, int nt)
         *x.p = at;
         at += (x.bytes + 255) & ~size_t(255);
     }
+    static_assert(sizeof(RootIn) <= 128 * sizeof(unsigned long long), "a root in a histogram's place");
     const size_t pins = (kPinHist + n * 128) * sizeof(unsigned long long);
     char *p = nullptr;
-    CK(cudaMallocHost(&p, pins + n * (sizeof(RootIn) + sizeof(FirstOut) + 1)));
+    CK(cudaMallocHost(&p, pins + n * (sizeof(FirstOut) + 1)));
     e->h_pin = (unsigned long long *)p;
-    e->h_roots = (RootIn *)(p + pins);
-    e->h_first_out = (FirstOut *)(e->h_roots + n);
+    e->h_roots = (RootIn *)(e->h_pin + kPinHist);
+    e->h_first_out = (FirstOut *)(p + pins);
     e->h_up_active = (uint8_t *)(e->h_first_out + n);
-    e->cap_tasks = cap;
     return PCAGB_OK;
 }
 
@@ -2242,7 +2230,7 @@ int engine_init(pcagb_engine *e, int device, size_t budget)
     CK(cudaMalloc(&e->d_small, 256 * sizeof(unsigned long long)));
     e->d_status = reinterpret_cast<uint32_t *>(e->d_small + 8);
     CK(cudaMalloc(&e->d_sol, e->sol_cap * sizeof(ulonglong2)));
-    return ensure_tasks(e, 1);
+    return alloc_tasks(e);
 }
 
 bool make_run(const task_spec_t *task, const pcagb_opts_t &o, TaskRun *tr)
