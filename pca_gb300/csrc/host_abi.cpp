@@ -11,6 +11,7 @@
 #include "pca_isa.h"
 
 #include <algorithm>
+#include <array>
 #include <cctype>
 #include <cstdio>
 #include <cstdlib>
@@ -214,22 +215,39 @@ static GenTables build_tables()
                     for (uint32_t x = 1; x < 8; x++)
                         if (a == x || b == x) last[(m * 8 + r) * 8 + x] += n;
                 }
+        /* A middle's evaluations depend on the pair only by which of its
+           registers the middle reads: with none left unread the whole last
+           position, with one left (not the one it overwrites) the classes
+           reading that too. So each candidate adds to the sums of its operand
+           set, eight of them, and the sets (at most 29 of a mask) to the
+           pairs; every pair of every candidate took 12 ms of a process's
+           start. */
         t.ev_mid.assign(2 * 128 * 64, 0);
-        for (int m = 0; m < 128; m++)
+        std::vector<std::array<uint32_t, 8>> sums(2 * 256);   /* [no same-state ones][set] */
+        for (int m = 0; m < 128; m++) {
+            std::vector<uint32_t> sets;
             for (uint32_t i = t.cand_off[m]; i < t.cand_off[m + 1]; i++) {
                 const uint32_t u = t.cand_uop[i], rd = UOP_RD(u);
-                const uint32_t reads = 1u << UOP_A(u) | 1u << UOP_B(u);
+                const uint32_t reads = (1u << UOP_A(u) | 1u << UOP_B(u)) & 0xFEu;
                 const uint32_t *l = &last[(((m | 1u << (rd - 1)) & 127u) * 8 + rd) * 8];
-                for (uint32_t A = 0; A < 8; A++)
-                    for (uint32_t B = 0; B < 8; B++) {
-                        const uint32_t a = A && !(reads >> A & 1u) ? A : 0u;
-                        const uint32_t b = B && !(reads >> B & 1u) ? B : 0u;
-                        if ((a && b) || (a && a == rd) || (b && b == rd)) continue;
-                        const uint32_t n = l[a ? a : b];
-                        t.ev_mid[(m * 8 + A) * 8 + B] += n;
-                        if (!t.cand_dupe[i]) t.ev_mid[((128 + m) * 8 + A) * 8 + B] += n;
-                    }
+                if (std::find(sets.begin(), sets.end(), reads) == sets.end()) {
+                    sets.push_back(reads);
+                    sums[reads].fill(0);
+                    sums[256 + reads].fill(0);
+                }
+                for (uint32_t d = 0; d < 2 - t.cand_dupe[i]; d++)
+                    for (uint32_t r = 0; r < 8; r++)
+                        if (r != rd) sums[d * 256 + reads][r] += l[r];
             }
+            for (uint32_t d = 0; d < 2; d++)
+                for (uint32_t set : sets)
+                    for (uint32_t A = 0; A < 8; A++)
+                        for (uint32_t B = 0; B < 8; B++) {
+                            const uint32_t a = set >> A & 1u ? 0u : A, b = set >> B & 1u ? 0u : B;
+                            if (!a || !b)
+                                t.ev_mid[((d * 128 + m) * 8 + A) * 8 + B] += sums[d * 256 + set][a + b];
+                        }
+        }
     }
     for (int s = 0; s < 5; s++) t.ev[s].assign(128, 0);
     for (int m = 0; m < 128; m++) t.ev[1][m] = t.vc_off[m + 1] - t.vc_off[m];
