@@ -110,9 +110,15 @@ class ValueNet:
             raise RuntimeError(f"value-net kernel failed ({rc})")
 
     def _refresh_bf16(self):
+        """The bf16 copies of the weights, in place once they exist: captured
+        graphs (training steps, rankings) read and write them where they
+        are."""
         for name, out, inp in LAYERS:
-            self.Wb[name] = self.W[name].to(torch.bfloat16).contiguous()
-            self.Wt[name] = self.W[name].t().contiguous().to(torch.bfloat16)
+            if name not in self.Wb:
+                self.Wb[name] = torch.empty(out, inp, device=self.dev, dtype=torch.bfloat16)
+                self.Wt[name] = torch.empty(inp, out, device=self.dev, dtype=torch.bfloat16)
+            self.Wb[name].copy_(self.W[name])
+            self.Wt[name].copy_(self.W[name].t())
 
     def n_params(self):
         return sum(w.numel() + self.b[k].numel() for k, w in self.W.items())
