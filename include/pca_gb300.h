@@ -416,7 +416,9 @@ void *pcagb_engine_stream(pcagb_engine_t *e);
  * chunk_choices[s][c] first instructions per work item, 1024 meaning a lane
  * per state, for s = 1 the prefixes a warp scans at once, 1 or
  * 32) with the number of stages it was measured on; the host round trip of
- * a chunked launch. */
+ * a chunked launch. Choices are tried at s = 1 only: at s = 2 and 3 a lane
+ * per state is taken, on a fixed number of tests, unless the caller forces a
+ * shape, so of their entries only chunk_ms[s][3] is measured. */
 typedef struct {
     double   t_eval_ms[4];
     double   t_child_ms;

@@ -1204,7 +1204,9 @@ int run_stage(pcagb_engine *e, int S, int K, std::vector<TaskRun> &runs, bool fi
                     8, std::max<uint64_t>(1, L.n * (uint64_t)ncmax / ((uint64_t)g * kWarpsPerBlock)));
             } else if (s >= 2 && e->force_chunk < 1) {
                 /* a lane per state: measured 30-100x faster than the fastest
-                   warp-per-item chunk on every stage, so nothing is explored */
+                   warp-per-item chunk on every stage, so nothing is explored
+                   (its cost is kept all the same: pcagb_tuning) */
+                ck = 3;
                 chunk = kLaneShape;
             } else if (e->force_chunk >= 1) {
                 chunk = s == 1 ? (e->force_chunk >= 32 ? 32u : 1u)
