@@ -530,6 +530,7 @@ int task_load(const char *path, task_spec_t *spec)
 int task_evaluate(const task_spec_t *spec, const uint16_t *prog, int prog_len)
 {
     int passed = 0;
+    if (spec->num_tests < 1) return 0;   /* no test: the program is not looked at */
     pca_vm_t vm;
     pca_init(&vm);
     pca_load(&vm, prog, (size_t)prog_len);
