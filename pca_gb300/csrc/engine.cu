@@ -1986,7 +1986,7 @@ int ensure_device_tables(int device)
         }
     }
     uint32_t *cand_uop = nullptr, *vc_uop = nullptr, *chunks = nullptr, *vcr_uop_d = nullptr;
-    uint16_t *vc_first = nullptr, *vcr = nullptr;
+    uint16_t *vc_first = nullptr;
     uint8_t *vc_n = nullptr;
     {
         std::vector<uint32_t> vcr_uop(gt.vcr.size());
@@ -1994,14 +1994,10 @@ int ensure_device_tables(int device)
             for (uint32_t k = gt.vcr_off[m * 8]; k < gt.vcr_off[m * 8 + 8]; k++)
                 vcr_uop[k] = gt.vc_uop[gt.vc_off[m] + gt.vcr[k]];
         CK(cudaMalloc(&vcr_uop_d, std::max<size_t>(vcr_uop.size(), 1) * 4));
-        CK(cudaMalloc(&vcr, std::max<size_t>(gt.vcr.size(), 1) * 2));
         CK(cudaMemcpy(vcr_uop_d, vcr_uop.data(), vcr_uop.size() * 4, cudaMemcpyHostToDevice));
-        CK(cudaMemcpy(vcr, gt.vcr.data(), gt.vcr.size() * 2, cudaMemcpyHostToDevice));
         const uint32_t *vu = vcr_uop_d;
-        const uint16_t *vr = vcr;
         CK(cudaMemcpyToSymbol(c_vcr_off, gt.vcr_off.data(), gt.vcr_off.size() * 4));
         CK(cudaMemcpyToSymbol(c_vcr_uop, &vu, sizeof vu));
-        CK(cudaMemcpyToSymbol(c_vcr, &vr, sizeof vr));
     }
     {
         uint32_t *pr = nullptr;

@@ -77,7 +77,6 @@ __constant__ const uint16_t *c_kid;        /* [class][8] candidate of the class 
                                               0xFFFF: none, or a same-state duplicate */
 __constant__ uint32_t c_vcr_off[128 * 8 + 1]; /* [mask*8 + r]: classes reading r */
 __constant__ const uint32_t *c_vcr_uop;    /* their micro-ops */
-__constant__ const uint16_t *c_vcr;        /* their indices in the mask's class list */
 __constant__ uint32_t c_pr_off[128 * 8 + 1];  /* [mask*8 + r]: the same, by operand pair */
 __constant__ const uint32_t *c_pr;         /* a | b << 3 | opmask << 6 | imm << 16 */
 __constant__ const uint16_t *c_pr_cls;     /* [entry][10] class index per opmask bit */
@@ -1660,7 +1659,6 @@ __device__ __forceinline__ void scan_last(const WarpState<TPC> &ws, int T,
     }
     const uint32_t vbase = c_vc_off[m];
     const uint32_t *uops = c_vc_uop + vbase;
-    const uint16_t *list = nullptr;
     const uint32_t nvc = c_vc_off[m + 1] - vbase;
     for (uint32_t b0 = 0; b0 < nvc; b0 += 32) {
         const uint32_t i = b0 + lane;
@@ -1689,10 +1687,7 @@ __device__ __forceinline__ void scan_last(const WarpState<TPC> &ws, int T,
             rb = rb == rd2 ? 9u : rb == rd1 ? 8u : rb;
             bool ok = true;
             if (lane < T) ok = pca_alu(UOP_OP(uj), ws.R[ra][lane], ws.R[rb][lane], UOP_IMM(uj)) == tgt;
-            if (__all_sync(0xFFFFFFFFu, ok) && lane == 0) {
-                const uint32_t cj = list ? (uint32_t)list[b0 + j] : b0 + j;
-                record_solution(S, q, m1, m2, cj, m);
-            }
+            if (__all_sync(0xFFFFFFFFu, ok) && lane == 0) record_solution(S, q, m1, m2, b0 + j, m);
         }
     }
 }

@@ -261,13 +261,6 @@ PCA_HD uint32_t self_value2(uint32_t f, uint32_t x)
     }
 }
 
-PCA_HD uint32_t form_value2(uint32_t kind, uint32_t f, uint32_t x, uint32_t y)
-{
-    return kind == kKindPair   ? pair_value2(f, x, y)
-           : kind == kKindSelf ? self_value2(f, x)
-                               : ldi_imm(f) * 0x10001u;
-}
-
 /* which forms give t on both tests */
 PCA_HD uint32_t pair_mask2(uint32_t v, uint32_t x, uint32_t t)
 {

@@ -619,14 +619,6 @@ int pcagb_vnet_adam_list(const void *tensors, int count, float lr, float b1, flo
     return PCAGB_OK;
 }
 
-int pcagb_vnet_adam(float *W, const float *G, float *m, float *v, int out, int in, float lr,
-                    float b1, float b2, float eps, const int *step, void *Wb, void *Wt,
-                    void *stream)
-{
-    const AdamTensor t{W, G, m, v, (__nv_bfloat16 *)Wb, (__nv_bfloat16 *)Wt, out, in, in, 0};
-    return pcagb_vnet_adam_list(&t, 1, lr, b1, b2, eps, step, stream);
-}
-
 int pcagb_vnet_to_bf16(const float *src, void *dst, size_t count, void *stream)
 {
     k_to_bf16<<<1024, 256, 0, (cudaStream_t)stream>>>(src, (__nv_bfloat16 *)dst, count);

@@ -50,7 +50,6 @@ def _lib():
         "pcagb_vnet_loss": [vp, vp, vp, i, f, vp, vp, vp, vp],
         "pcagb_vnet_loss_value": [vp, vp, vp, i, f, vp, vp, vp, vp, vp],
         "pcagb_vnet_adam_list": [vp, i, f, f, f, f, vp, vp],
-        "pcagb_vnet_adam": [vp, vp, vp, vp, i, i, f, f, f, f, vp, vp, vp, vp],
         "pcagb_vnet_to_bf16": [vp, vp, sz, vp],
         "pcagb_vnet_encode_pool_tc": [vp, vp, vp, vp, vp, vp, vp, vp, vp, i, i, vp, vp, vp, vp,
                                       vp],
