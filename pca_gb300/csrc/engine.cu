@@ -2542,17 +2542,18 @@ void pcagb_engine_destroy(pcagb_engine_t *e)
     if (!e) return;
     cudaSetDevice(e->device);
     if (e->stream) cudaStreamSynchronize(e->stream);
-    /* Freeing the arena leaves the driver a millisecond of work, which it does
-       at the free of the last of several blocks, or else at the next engine's
-       allocation of its arena. So the arena goes first and the histogram, a
-       block of its own, last: an engine made after another was closed takes
-       0.87 ms and the closing 6.3 (1.39 and 4.85 with the arena last). */
+    /* Freeing the arena leaves the driver milliseconds of work, which it does
+       at one of the frees that follow, or else at the next engine's allocation
+       of its arena. So the arena goes first, and the histogram is a block of
+       its own: an engine of 4, 8, 16, 24 or 48 GB made after another was closed
+       takes 0.8, 0.9, 3.3, 1.7 or 2.1 ms, as it did with a block for every
+       array (one block, the arena last: 1.7, 1.3, 2.5 to 3.6, 3.7 to 4.8, 7.2). */
     cudaFree(e->arena);
     cudaFree(e->d_small);
     cudaFree(e->d_sol);
     cudaFree(e->d_tasks);
-    if (e->h_pin) cudaFreeHost(e->h_pin);
     cudaFree(e->d_hist);
+    if (e->h_pin) cudaFreeHost(e->h_pin);
     for (cudaEvent_t ev : {e->ev0, e->ev1, e->ev2, e->ev3, e->evk0, e->evk1})
         if (ev) cudaEventDestroy(ev);
     if (e->stream) cudaStreamDestroy(e->stream);
