@@ -217,6 +217,7 @@ struct pcagb_engine {
     bool measure = true;                 /* per solve: the GPU is its own (not
                                             shared_gpu), so its times are costs */
     uint64_t id_limit = ~0ull;           /* most column ids of a level build (tests lower it) */
+    bool quiet = true;                   /* per solve: nothing of it is on the stream */
     int lean_K = -1;                     /* per solve: the last depth, whose stage
                                             reads its split level lean (-1: none) */
 
@@ -1653,6 +1654,7 @@ int search_batch(pcagb_engine *e, std::vector<TaskRun> &runs, const pcagb_opts_t
         return PCAGB_EINVAL;
     }
     e->ntasks = nt;
+    e->quiet = true;
     e->levels.clear();
     e->bottom = 0;
     e->top = e->cap;
@@ -1728,6 +1730,7 @@ int search_batch(pcagb_engine *e, std::vector<TaskRun> &runs, const pcagb_opts_t
             r.T = (uint8_t)tr.T;
             L0.hist[(size_t)i * 128 + ((tr.root.live >> 1) & 127)] = 1;
         }
+        e->quiet = false;
         CK(e_copy(e, e->d_roots, e->h_roots, (size_t)nt * sizeof(RootIn), cudaMemcpyHostToDevice,
                   e->stream));
         const LevelOut out{L0.regs, L0.flags, L0.live, L0.task, L0.parent, L0.cidx, L0.rdl, L0.own,
@@ -1773,6 +1776,7 @@ int search_batch(pcagb_engine *e, std::vector<TaskRun> &runs, const pcagb_opts_t
         }
         if (!nact) break;
         memcpy(e->h_up_active, active.data(), nt);
+        e->quiet = false;
         CK(e_copy(e, e->d_task_active, e->h_up_active, nt, cudaMemcpyHostToDevice, e->stream));
         e->h_active = active;
         int S_target = o.count_levels ? K : K - 1;
@@ -1921,6 +1925,7 @@ int search_batch(pcagb_engine *e, std::vector<TaskRun> &runs, const pcagb_opts_t
         const bool stage_first_only = o.first_only != 0 || (ord && !ordered_stage);
         int rc = run_stage(e, S, K, runs, stage_first_only, sop, sop ? nullptr : &on_tasks);
         if (rc) return rc;
+        e->quiet = true;   /* a stage ends by reading its results */
         for (int i = 0; i < nt; i++) finish(i);
     }
     const double total = elapsed();
@@ -1947,15 +1952,17 @@ int search_batch(pcagb_engine *e, std::vector<TaskRun> &runs, const pcagb_opts_t
 }
 
 /* search_batch, and the end of its work on the device: however it returns, no
-   kernel or copy of it is left on the stream. The arena may belong to a server,
-   which hands it to another stream's solve next, and the pinned buffers are
-   the next solve's. (A solve that ran its stages has waited already.) */
+   kernel or copy of it is left on the stream (a solve whose last stage ran has
+   waited already). The arena may belong to a server, which hands it to another
+   stream's solve next, and the pinned buffers are the next solve's. */
 int run_batch(pcagb_engine *e, std::vector<TaskRun> &runs, const pcagb_opts_t &o,
               done_fn on_done = nullptr, void *user = nullptr, const OrderSpec *ord = nullptr)
 {
     const ArenaUse use(e);
     const int rc = search_batch(e, runs, o, on_done, user, ord);
+    if (e->quiet) return rc;
     const cudaError_t end = cudaStreamSynchronize(e->stream);
+    e->quiet = true;
     if (rc) return rc;
     CK(end);
     return PCAGB_OK;
