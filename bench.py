@@ -50,13 +50,13 @@ CANDIDATES = ("candidates as the reference's enumerator counts them (tools/enume
 # (SHA-256 of pca_gb300/csrc's engine_kernels.cuh, suffix_forms.cuh and
 # value_forms.h, first 16 hex) and the autotuner's choice.
 SUFFIX_CAPTURE = {"kernel": "k_suffix_lanes<32,3>", "choice": (3, 32), "inst": 132050193,
-                  "ms": 0.222848, "dram_bytes": 366526208 + 123904,
-                  "source_sha16": ("2a7afde722770fe4",),
+                  "ms": 0.224864, "dram_bytes": 366522112 + 70400,
+                  "source_sha16": ("8036a31d3fcd457a",),
                   "file": "profiles/k_suffix_lanes_is_power2_t32_k4.md"}
 # The insert kernel's capture (profiles/k_expand_insert_is_power2_t32_level3.md):
 # DRAM bytes read + written by the level-3 launch (99.6% of a solve's children).
-INSERT_CAPTURE = {"dram_bytes": 546621696 + 189057536,
-                  "source_sha16": ("2a7afde722770fe4",),
+INSERT_CAPTURE = {"dram_bytes": 546178816 + 188960256,
+                  "source_sha16": ("8036a31d3fcd457a",),
                   "file": "profiles/k_expand_insert_is_power2_t32_level3.md"}
 
 

@@ -208,7 +208,9 @@ typedef struct {
     int shared_gpu;     /* 1: the solve shares the GPU with other solves (a
                            server's): its stage times measure the mix, so
                            they update none of the autotuner's costs and no
-                           launch choice is explored on it                   */
+                           launch choice is explored on it; its long stages
+                           run in ranges of about 2 ms, a single task's at
+                           first in a few CTAs, for 0.4 s at most            */
     int full_levels;    /* 1: every level with its register block; 0: the
                            last depth's split level, which only its
                            last-position stage reads, holds links and the
@@ -379,7 +381,9 @@ int  pcagb_record(pcagb_engine_t *e, const task_spec_t *task, int max_depth, uin
  * of each depth is built on the engine's stream, so the per-depth counters
  * (tried, pruned_cum) are the reference's, up to the 100th solution at the
  * optimal depth as its walk stops there; the first sol_cap programs in
- * depth-first order are returned. Errors: see pcagb_branch_last_error. */
+ * depth-first order are returned. Errors: see pcagb_branch_last_error. The
+ * levels take the engine's arena where no solve is using it (a solve's
+ * callbacks may call this), stream-ordered allocations otherwise. */
 int  pcagb_solve_branch(pcagb_engine_t *e, const task_spec_t *task, int max_depth,
                         pcagb_result_t *res, uint16_t *sol_progs, int *sol_lens, int sol_cap);
 /* The same with the size rule of the last position explicit: when a depth's

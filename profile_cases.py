@@ -1,6 +1,6 @@
 """Fixed small workloads, one per kernel family, for profiling under ncu.
 
-    python profile_cases.py engine_depths   # k_suffix<32, 2/3>, k_leaf
+    python profile_cases.py engine_depths   # k_suffix<32, 2/3>, k_suffix_states, leaf check
     python profile_cases.py suffix_depth2   # one k_suffix<32, 2> depth-4 stage
     python profile_cases.py noalloc         # k_suffix_noalloc
     python profile_cases.py valuenet        # training and scoring kernels
@@ -31,7 +31,7 @@ def _events():
 def case_engine_depths(reps: int):
     """is_power2 (32 tests) to kernel depth 4 with the suffix stage started
     from level 1 and level 2 (suffix depths 3 and 2), each with a warp per
-    (prefix, chunk of 16 middles) and with a lane per innermost middle, and
+    (prefix, chunk of 16 middles) and with a lane per state, and
     depth 3 from level 3 (the leaf check)."""
     from pca_gb300.pcalib import Engine
     from pca_gb300.taskgen import is_power2_task
