@@ -1085,7 +1085,7 @@ void launch_suffix_lanes(int ft, int g, cudaStream_t st, const LevelDev &L, cons
    One task's long stage steps back at first: until kStepBackMs have passed its
    ranges run in a few CTAs, which leave the other SMs to the requests admitted
    meanwhile. It is a bound on the wait that is bought, not a share of the
-   stage: a two-input task's depth 5 takes 0.08 s alone and 0.47 s so (5.8 s
+   stage: a two-input task's depth 5 takes 0.08 s alone and 0.49 s so (5.8 s
    where all of it ran in four CTAs, 9.2 s before the lanes were states), and
    no batch is slowed (40 open two-input tasks to depth 4: 5 ms either way; 194
    in four CTAs, whose line was drawn by the sum of the tasks). The price falls
