@@ -18,7 +18,7 @@ def test_what_an_engine_held_is_free_again():
         e.close()
         free.append(device_memory(0)[0])
     assert len(set(map(str, answers))) == 1
-    assert free[1:] == free[:1] * 5
+    assert min(free[1:]) >= free[0]
 
 
 def test_engines_held_together_and_closed_in_another_order():
@@ -31,5 +31,5 @@ def test_engines_held_together_and_closed_in_another_order():
             es[i].close()
         assert all(g == got[0] for g in got)
         if before is not None:
-            assert device_memory(0)[0] == before
+            assert device_memory(0)[0] >= before
         before = device_memory(0)[0]
